@@ -76,7 +76,7 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // the same in all lanes, and known to be
   const int lane = threadIdx.x & 31;
   constexpr int CTAS = PAIR ? 2 : 1;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
@@ -129,7 +129,7 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
   __syncthreads();
   if (PAIR) cluster_sync_all();  // the other CTA's barriers exist before anything is sent to them
   tc_fence_after_sync();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   // barriers, tensor memory and descriptors are ready: from here on the kernel touches tensors that the
   // kernel before it in the stream may still be writing
   grid_dependency_wait();
@@ -153,85 +153,78 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    // one lane per TMA copy (issuing is what costs): lanes 0/1 the weight planes of a tap,
-    // lanes 2/3 the patch planes of a channel block; lane 0 owns the barrier traffic
-    const bool b_issuer = lane < PLANES;
-    const bool a_issuer = lane >= 2 && lane < 2 + PLANES;
-    const int plane = lane & 1;
-    // (PAIR: the bytes of both CTAs are counted on CTA 0's barriers, armed by CTA 0)
-    const uint32_t a_tx = CTAS * PLANES * static_cast<uint32_t>(p.patch_h * p.patch_w) * 128u;
-    const uint32_t b_tx = CTAS * PLANES * static_cast<uint32_t>(b_rows) * 128u;
-    int s = 0, ab = 0;
-    uint32_t ph = 0, a_ph = 0;
-    long long a_issued = 0, b_issued = 0;
-    bool ok = true;
-    for (int tile = worker; tile < total_tiles && ok; tile += workers) {
-      int img, oy0, ox0, n0;
-      bool valid;
-      decode(tile, &img, &oy0, &ox0, &n0, &valid);
-      n0 += static_cast<int>(rank) * b_rows;
-      for (int cb = 0; cb < p.c_blocks && ok; ++cb) {
-        const uint32_t ab_bar = PAIR ? map_to_cta(smem_u32(&a_full[ab]), 0u) : smem_u32(&a_full[ab]);
-        int w = 1;
-        if (lane == 0) {
-          w = mbar_wait_bounded(smem_u32(&a_empty[ab]), a_ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-          if (w && rank == 0) mbar_arrive_expect_tx(smem_u32(&a_full[ab]), a_tx);
-        }
-        w = __shfl_sync(0xffffffffu, w, 0);
-        if (!w) {
-          ok = false;
-          break;
-        }
-        if (a_issuer) {
-          const uint32_t dst = smem_base + static_cast<uint32_t>(ab) * a_buf_bytes + plane * patch_bytes;
-          if (PAIR) tma_load_4d_pair(dst, plane ? &map_a1 : &map_a0, ab_bar, cb * p.k_elems, ox0 - p.pad_l, oy0 - p.pad_t, img);
-          else tma_load_4d(dst, plane ? &map_a1 : &map_a0, ab_bar, cb * p.k_elems, ox0 - p.pad_l, oy0 - p.pad_t, img);
-        }
-        ++a_issued;
-        ab ^= 1;
-        if (ab == 0) a_ph ^= 1u;
-        for (int tap = 0; tap < p.taps; ++tap) {
-          const uint32_t fb = PAIR ? map_to_cta(smem_u32(&b_full[s]), 0u) : smem_u32(&b_full[s]);
-          if (lane == 0) {
-            w = mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-            if (w && rank == 0) mbar_arrive_expect_tx(smem_u32(&b_full[s]), b_tx);
-          }
-          w = __shfl_sync(0xffffffffu, w, 0);
-          if (!w) {
+    // (one elected thread: tc_gemm.cuh says why)
+    if (elect_one()) {
+      // (PAIR: the bytes of both CTAs are counted on CTA 0's barriers, armed by CTA 0)
+      const uint32_t a_tx = CTAS * PLANES * static_cast<uint32_t>(p.patch_h * p.patch_w) * 128u;
+      const uint32_t b_tx = CTAS * PLANES * static_cast<uint32_t>(b_rows) * 128u;
+      int s = 0, ab = 0;
+      uint32_t ph = 0, a_ph = 0;
+      long long a_issued = 0, b_issued = 0;
+      bool ok = true;
+      for (int tile = worker; tile < total_tiles && ok; tile += workers) {
+        int img, oy0, ox0, n0;
+        bool valid;
+        decode(tile, &img, &oy0, &ox0, &n0, &valid);
+        n0 += static_cast<int>(rank) * b_rows;
+        for (int cb = 0; cb < p.c_blocks && ok; ++cb) {
+          const uint32_t ab_bar = PAIR ? map_to_cta(smem_u32(&a_full[ab]), 0u) : smem_u32(&a_full[ab]);
+          if (!mbar_wait_bounded(smem_u32(&a_empty[ab]), a_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
             ok = false;
             break;
           }
-          const bool ptr_ = p.trace != nullptr && worker == workers / 2 && rank == 0 && tile == worker && cb == 0 && lane == 0 && tap < 16;
-          if (ptr_) p.trace[16 + 4 * tap + 2] = clock64();
-          if (b_issuer) {
-            const uint32_t dst = b_ring + static_cast<uint32_t>(s) * b_stage_bytes + plane * b_bytes;
-            if (PAIR) tma_load_2d_pair(dst, plane ? &map_b1 : &map_b0, fb, (tap * p.c_blocks + cb) * p.k_elems, n0);
-            else tma_load_2d(dst, plane ? &map_b1 : &map_b0, fb, (tap * p.c_blocks + cb) * p.k_elems, n0);
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&a_full[ab]), a_tx);
+#pragma unroll
+          for (int plane = 0; plane < PLANES; ++plane) {
+            const uint32_t dst = smem_base + static_cast<uint32_t>(ab) * a_buf_bytes + static_cast<uint32_t>(plane) * patch_bytes;
+            const CUtensorMap* map = plane ? &map_a1 : &map_a0;
+            if (PAIR) tma_load_4d_pair(dst, map, ab_bar, cb * p.k_elems, ox0 - p.pad_l, oy0 - p.pad_t, img);
+            else tma_load_4d(dst, map, ab_bar, cb * p.k_elems, ox0 - p.pad_l, oy0 - p.pad_t, img);
           }
-          ++b_issued;
-          if (++s == S) {
-            s = 0;
-            ph ^= 1u;
+          ++a_issued;
+          ab ^= 1;
+          if (ab == 0) a_ph ^= 1u;
+          for (int tap = 0; tap < p.taps; ++tap) {
+            const uint32_t fb = PAIR ? map_to_cta(smem_u32(&b_full[s]), 0u) : smem_u32(&b_full[s]);
+            if (!mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+              ok = false;
+              break;
+            }
+            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&b_full[s]), b_tx);
+            const bool ptr_ = p.trace != nullptr && worker == workers / 2 && rank == 0 && tile == worker && cb == 0 && tap < 16;
+            if (ptr_) p.trace[16 + 4 * tap + 2] = clock64();
+#pragma unroll
+            for (int plane = 0; plane < PLANES; ++plane) {
+              const uint32_t dst = b_ring + static_cast<uint32_t>(s) * b_stage_bytes + static_cast<uint32_t>(plane) * b_bytes;
+              const CUtensorMap* map = plane ? &map_b1 : &map_b0;
+              if (PAIR) tma_load_2d_pair(dst, map, fb, (tap * p.c_blocks + cb) * p.k_elems, n0);
+              else tma_load_2d(dst, map, fb, (tap * p.c_blocks + cb) * p.k_elems, n0);
+            }
+            ++b_issued;
+            if (++s == S) {
+              s = 0;
+              ph ^= 1u;
+            }
           }
         }
       }
-    }
-    if (lane == 0) {
-      if (!ok) {
-        if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
-      }
-      if (*abort_ptr != 0 && rank == 0) {
-        // copies may still be landing (CTA 0's barriers count both CTAs' bytes): wait (bounded) for the last ones
-        int zero = 0;
-        for (long long i = b_issued > S ? b_issued - S : 0; i < b_issued; ++i)
-          mbar_wait_bounded(smem_u32(&b_full[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
-        for (long long i = a_issued > 2 ? a_issued - 2 : 0; i < a_issued; ++i)
-          mbar_wait_bounded(smem_u32(&a_full[i % 2]), static_cast<uint32_t>((i / 2) & 1), &zero, 200000000ull);
+      {
+        if (!ok) {
+          if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
+        }
+        if (*abort_ptr != 0 && rank == 0) {
+          // copies may still be landing (CTA 0's barriers count both CTAs' bytes): wait (bounded) for the last ones
+          int zero = 0;
+          for (long long i = b_issued > S ? b_issued - S : 0; i < b_issued; ++i)
+            mbar_wait_bounded(smem_u32(&b_full[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
+          for (long long i = a_issued > 2 ? a_issued - 2 : 0; i < a_issued; ++i)
+            mbar_wait_bounded(smem_u32(&a_full[i % 2]), static_cast<uint32_t>((i / 2) & 1), &zero, 200000000ull);
+        }
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc =
           instr_desc(1u, KIND == GEMM_BF16X3 ? 1u : 2u, kTcBlockM * CTAS, static_cast<uint32_t>(p.block_n));
       // A: 128-byte rows, 128B swizzle, 8-row groups one patch row apart

@@ -111,7 +111,7 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // the same in all lanes, and known to be
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(dwp_smem_raw) + 1023u) & ~1023u;
   const int P = EXPAND ? 2 : p.patch_bufs;  // EXPAND: one patch per depthwise group, filled by the group itself
@@ -187,7 +187,7 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   grid_dependency_wait();
 
   // channel blocks of one pixel tile are neighbours, so CTAs working side by side share the patch in L2
@@ -205,109 +205,98 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    // lane 0: the fp32 patch of a channel block (EXPAND: both planes of the tile's input patch); lanes 1, 2: the
-    // two planes of that block's projection weights; lanes 3, 4 (EXPAND): the two planes of its expand weights
-    const uint32_t patch_tx = static_cast<uint32_t>(NPX * kDwpChannels * 4);
-    const uint32_t x_tx = 2u * static_cast<uint32_t>(NPX) * static_cast<uint32_t>(p.x_row_bytes);
-    const uint32_t b_tx = 2u * static_cast<uint32_t>(p.block_n) * 64u + (EXPAND ? 2u * 32u * static_cast<uint32_t>(p.x_row_bytes) : 0u);
-    int s = 0, pb = 0;
-    uint32_t ph = 0, p_ph = 0;
-    long long patches = 0, weights = 0, tiles_done = 0, x_issued = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++tiles_done) {
-      int img, oy0, ox0, n0;
-      decode(tile, &img, &oy0, &ox0, &n0);
-      if (EXPAND) {
-        // With two buffers the patch of the NEXT tile is requested here (the first tile's before the loop): its
-        // buffer was released by the tile before this one, so the wait cannot hold up this tile's weight copies.
-        // With one buffer the patch of THIS tile is requested, once the previous tile's expand MMAs have read theirs.
-        const long long first = XB == 2 ? (tiles_done == 0 ? 0 : tiles_done + 1) : tiles_done;
-        const long long last = XB == 2 ? tiles_done + 1 : tiles_done;
-        for (long long tl = first; tl <= last && ok; ++tl) {
-          const int t2 = static_cast<int>(blockIdx.x) + static_cast<int>(tl) * static_cast<int>(gridDim.x);
-          if (t2 >= total_tiles) break;
-          int img2, oy2, ox2, n2;
-          decode(t2, &img2, &oy2, &ox2, &n2);
-          const int xb = static_cast<int>(tl % XB);
-          const uint32_t x_ph = static_cast<uint32_t>((tl / XB) & 1);
-          int w = 1;
-          if (lane == 0) {
-            w = mbar_wait_bounded(smem_u32(&x_empty[xb]), x_ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-            if (w) {
-              const uint32_t dst = x_base + static_cast<uint32_t>(xb) * 2u * x_plane;
-              mbar_arrive_expect_tx(smem_u32(&x_full[xb]), x_tx);
-              tma_load_4d(dst, &map_x, smem_u32(&x_full[xb]), 0, ox2 * STRIDE - p.pad_l, oy2 * STRIDE - p.pad_t, img2);
-              tma_load_4d(dst + x_plane, &map_x1, smem_u32(&x_full[xb]), 0, ox2 * STRIDE - p.pad_l, oy2 * STRIDE - p.pad_t, img2);
+    // per channel block the fp32 patch (EXPAND: per tile both planes of the input patch), the two planes of the block's
+    // projection weights and (EXPAND) of its expand weights; one elected thread (tc_gemm.cuh says why)
+    if (elect_one()) {
+      const uint32_t patch_tx = static_cast<uint32_t>(NPX * kDwpChannels * 4);
+      const uint32_t x_tx = 2u * static_cast<uint32_t>(NPX) * static_cast<uint32_t>(p.x_row_bytes);
+      const uint32_t b_tx = 2u * static_cast<uint32_t>(p.block_n) * 64u + (EXPAND ? 2u * 32u * static_cast<uint32_t>(p.x_row_bytes) : 0u);
+      int s = 0, pb = 0;
+      uint32_t ph = 0, p_ph = 0;
+      long long patches = 0, weights = 0, tiles_done = 0, x_issued = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++tiles_done) {
+        int img, oy0, ox0, n0;
+        decode(tile, &img, &oy0, &ox0, &n0);
+        if (EXPAND) {
+          // With two buffers the patch of the NEXT tile is requested here (the first tile's before the loop): its
+          // buffer was released by the tile before this one, so the wait cannot hold up this tile's weight copies.
+          // With one buffer the patch of THIS tile is requested, once the previous tile's expand MMAs have read theirs.
+          const long long first = XB == 2 ? (tiles_done == 0 ? 0 : tiles_done + 1) : tiles_done;
+          const long long last = XB == 2 ? tiles_done + 1 : tiles_done;
+          for (long long tl = first; tl <= last && ok; ++tl) {
+            const int t2 = static_cast<int>(blockIdx.x) + static_cast<int>(tl) * static_cast<int>(gridDim.x);
+            if (t2 >= total_tiles) break;
+            int img2, oy2, ox2, n2;
+            decode(t2, &img2, &oy2, &ox2, &n2);
+            const int xb = static_cast<int>(tl % XB);
+            const uint32_t x_ph = static_cast<uint32_t>((tl / XB) & 1);
+            if (!mbar_wait_bounded(smem_u32(&x_empty[xb]), x_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+              ok = false;
+              break;
             }
+            const uint32_t dst = x_base + static_cast<uint32_t>(xb) * 2u * x_plane;
+            mbar_arrive_expect_tx(smem_u32(&x_full[xb]), x_tx);
+            tma_load_4d(dst, &map_x, smem_u32(&x_full[xb]), 0, ox2 * STRIDE - p.pad_l, oy2 * STRIDE - p.pad_t, img2);
+            tma_load_4d(dst + x_plane, &map_x1, smem_u32(&x_full[xb]), 0, ox2 * STRIDE - p.pad_l, oy2 * STRIDE - p.pad_t, img2);
+            ++x_issued;
           }
-          w = __shfl_sync(0xffffffffu, w, 0);
-          if (!w) ok = false;
-          else ++x_issued;
+          if (!ok) break;
         }
-        if (!ok) break;
-      }
-      for (int cb = 0; cb < p.c_blocks && ok; ++cb) {
-        int w = 1;
-        if (!EXPAND) {
-          if (lane == 0) {
-            w = mbar_wait_bounded(smem_u32(&patch_empty[pb]), p_ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-            if (w) {
-              mbar_arrive_expect_tx(smem_u32(&patch_full[pb]), patch_tx);
-              tma_load_4d(patch_base + static_cast<uint32_t>(pb) * kPatchBytes, &map_x, smem_u32(&patch_full[pb]),
-                          cb * kDwpChannels, ox0 * STRIDE - p.pad_l, oy0 * STRIDE - p.pad_t, img);
+        for (int cb = 0; cb < p.c_blocks && ok; ++cb) {
+          if (!EXPAND) {
+            if (!mbar_wait_bounded(smem_u32(&patch_empty[pb]), p_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(smem_u32(&patch_full[pb]), patch_tx);
+            tma_load_4d(patch_base + static_cast<uint32_t>(pb) * kPatchBytes, &map_x, smem_u32(&patch_full[pb]), cb * kDwpChannels,
+                        ox0 * STRIDE - p.pad_l, oy0 * STRIDE - p.pad_t, img);
+            ++patches;
+            if (++pb == P) {
+              pb = 0;
+              p_ph ^= 1u;
             }
           }
-          w = __shfl_sync(0xffffffffu, w, 0);
-          if (!w) {
+          if (!mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
             ok = false;
             break;
           }
-          ++patches;
-          if (++pb == P) {
-            pb = 0;
-            p_ph ^= 1u;
+          const uint32_t fb = smem_u32(&b_full[s]);
+          mbar_arrive_expect_tx(fb, b_tx);
+          const uint32_t stage = b_base + static_cast<uint32_t>(s) * b_stage_bytes;
+          tma_load_2d(stage, &map_b0, fb, cb * kDwpChannels, n0);
+          tma_load_2d(stage + b_bytes, &map_b1, fb, cb * kDwpChannels, n0);
+          if (EXPAND) {
+            tma_load_2d(stage + 2u * b_bytes, &map_e0, fb, 0, cb * kDwpChannels);
+            tma_load_2d(stage + 2u * b_bytes + kExWeightBytes, &map_e1, fb, 0, cb * kDwpChannels);
+          }
+          ++weights;
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
           }
         }
-        if (lane == 0) {
-          w = mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-          if (w) mbar_arrive_expect_tx(smem_u32(&b_full[s]), b_tx);
-        }
-        w = __shfl_sync(0xffffffffu, w, 0);
-        if (!w) {
-          ok = false;
-          break;
-        }
-        const uint32_t stage = b_base + static_cast<uint32_t>(s) * b_stage_bytes;
-        if (lane == 1 || lane == 2)
-          tma_load_2d(stage + (lane - 1) * b_bytes, lane == 1 ? &map_b0 : &map_b1, smem_u32(&b_full[s]), cb * kDwpChannels, n0);
-        if (EXPAND && (lane == 3 || lane == 4))
-          tma_load_2d(stage + 2u * b_bytes + (lane - 3) * kExWeightBytes, lane == 3 ? &map_e0 : &map_e1, smem_u32(&b_full[s]), 0,
-                      cb * kDwpChannels);
-        ++weights;
-        if (++s == S) {
-          s = 0;
-          ph ^= 1u;
-        }
       }
-    }
-    if (lane == 0) {
-      if (!ok) {
-        if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
-      }
-      if (*abort_ptr != 0) {
-        // copies issued by this warp may still be landing: wait (bounded) for the last ones
-        int zero = 0;
-        for (long long i = weights > S ? weights - S : 0; i < weights; ++i)
-          mbar_wait_bounded(smem_u32(&b_full[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
-        for (long long i = patches > P ? patches - P : 0; i < patches; ++i)
-          mbar_wait_bounded(smem_u32(&patch_full[i % P]), static_cast<uint32_t>((i / P) & 1), &zero, 200000000ull);
-        for (long long i = x_issued > XB ? x_issued - XB : 0; i < x_issued; ++i)
-          mbar_wait_bounded(smem_u32(&x_full[i % XB]), static_cast<uint32_t>((i / XB) & 1), &zero, 200000000ull);
+      {
+        if (!ok) {
+          if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
+        }
+        if (*abort_ptr != 0) {
+          // copies issued by this warp may still be landing: wait (bounded) for the last ones
+          int zero = 0;
+          for (long long i = weights > S ? weights - S : 0; i < weights; ++i)
+            mbar_wait_bounded(smem_u32(&b_full[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
+          for (long long i = patches > P ? patches - P : 0; i < patches; ++i)
+            mbar_wait_bounded(smem_u32(&patch_full[i % P]), static_cast<uint32_t>((i / P) & 1), &zero, 200000000ull);
+          for (long long i = x_issued > XB ? x_issued - XB : 0; i < x_issued; ++i)
+            mbar_wait_bounded(smem_u32(&x_full[i % XB]), static_cast<uint32_t>((i / XB) & 1), &zero, 200000000ull);
+        }
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc(1u, 1u, kTcBlockM, static_cast<uint32_t>(p.block_n));
       const uint32_t idesc_ex = instr_desc(1u, 1u, kTcBlockM, 32u);
       const uint64_t fixed = smem_desc_kmajor(0u, 64u);  // 64-byte rows, 64-byte swizzle

@@ -770,7 +770,8 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  // (the shuffle tells the compiler that the warp number is the same in all lanes: see the issuing roles below)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
   const uint32_t slot = static_cast<uint32_t>(kTcBlockM) * p.row_bytes;
@@ -813,7 +814,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   // barriers, tensor memory and descriptors are ready: from here on the kernel touches tensors that the
   // kernel before it in the stream may still be writing
   grid_dependency_wait();
@@ -825,107 +826,101 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
 
   if (warp == 0 || warp == 6) {
     // ------------------------------------------------------------ producers
-    // Arming a stage and issuing its copies costs the issuing thread several hundred cycles per
-    // K block (about 450 for the barrier hand-shake plus about 120 per TMA instruction, whatever
-    // the box size), more than the MMAs of a narrow K block take.  So the work is split: warp 0
-    // feeds the A tiles, warp 6 the B tiles, each arming the stage for its own bytes (the full
-    // barrier counts two arrivals).  Within a warp lane p issues plane p.
+    // warp 0 feeds the A tiles, warp 6 the B tiles, each arming the stage for its own bytes (the full barrier
+    // counts two arrivals).  The issuing roles (these two and the MMA warp) run in one thread picked by
+    // elect.sync under a warp number that is the same in all lanes: TMA and tcgen05 instructions take their
+    // operands from uniform registers, and only then can the compiler keep descriptors and coordinates there.
+    // Chosen by `lane == 0` instead, every instruction first moves its operands over, one by one: 54 (unrolled)
+    // to 148 clocks between narrow MMAs against 40-64, which is the tensor pipe's own pace.
     const bool is_b = warp == 6;
-    // (paired tiles: lanes PLANES..2*PLANES-1 of the A warp issue the second half's planes)
-    // (int8 with several K blocks per stage, never paired: lane b issues the copy of the stage's K block b, so
-    // the copies of a stage cost the warp one instruction's time, not one each)
-    const bool by_block = KIND == GEMM_I8 && SUB > 1;
-    const bool issuer = by_block ? lane < SUB : lane < (is_b ? PLANES : PLANES * AS);
-    const int my_sb = by_block ? lane : 0;
-    const int my_plane = by_block ? 0 : lane % PLANES;
-    const int my_half = is_b || by_block ? 0 : lane / PLANES;
-    const CUtensorMap* my_map = is_b ? (my_plane ? &map_b1 : &map_b0) : (my_plane ? &map_a1 : &map_a0);
-    const uint32_t my_lane_slot = by_block ? 0u : static_cast<uint32_t>(lane);
-    const uint32_t my_off = is_b ? static_cast<uint32_t>(PLANES * AS) * slot + my_lane_slot * b_slot : my_lane_slot * slot;
-    const uint32_t b_tx = PLANES * static_cast<uint32_t>(p.block_n) * p.row_bytes;
-    int s = 0;
-    uint32_t ph = 0;
-    long long issued = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-      const int m_blk = tile / p.tiles_n;
-      const int n_blk = tile - m_blk * p.tiles_n;
-      const bool pair_tile = m_blk < p.pair_rows;
-      // a second half that starts past the last row repeats the first (its results are never stored)
-      long long m0 = pair_tile ? static_cast<long long>(m_blk) * (2 * kTcBlockM)
-                               : static_cast<long long>(p.pair_rows) * (2 * kTcBlockM) +
-                                     static_cast<long long>(m_blk - p.pair_rows) * kTcBlockM;
-      if (pair_tile && m0 + static_cast<long long>(my_half) * kTcBlockM < p.M) m0 += static_cast<long long>(my_half) * kTcBlockM;
-      const bool issues = issuer && (is_b || pair_tile || my_half == 0);
-      const uint32_t my_tx = is_b ? b_tx : static_cast<uint32_t>(PLANES * (pair_tile ? 2 : 1)) * slot;
-      const int n0 = n_blk * p.block_n;
-      int img = 0, h_base = 0, w_base = 0;
-      if (p.a_im2col) {
-        const long long per_img = static_cast<long long>(p.OH) * p.OW;
-        img = static_cast<int>(m0 / per_img);
-        const int r = static_cast<int>(m0 - img * per_img);
-        const int oh = r / p.OW;
-        const int ow = r - oh * p.OW;
-        h_base = oh * p.stride_h - p.pad_t;
-        w_base = ow * p.stride_w - p.pad_l;
-      }
-      if (p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[(tile / gridDim.x) * 16 + 0] = clock64();
-      // this lane's K block: channel block, filter row and column (lanes that issue by block start at theirs)
-      int cb = 0, kh = 0, kw = 0;
-      auto next_k_block = [&]() {
-        if (++cb == p.c_blocks) {
-          cb = 0;
-          if (++kw == p.KW) {
-            kw = 0;
-            ++kh;
+    if (elect_one()) {
+      const uint32_t b_tx = PLANES * static_cast<uint32_t>(p.block_n) * p.row_bytes;
+      const uint32_t b_off = static_cast<uint32_t>(PLANES * AS) * slot;
+      int s = 0;
+      uint32_t ph = 0;
+      long long issued = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+        const int m_blk = tile / p.tiles_n;
+        const int n_blk = tile - m_blk * p.tiles_n;
+        const bool pair_tile = m_blk < p.pair_rows;
+        const long long m0 = pair_tile ? static_cast<long long>(m_blk) * (2 * kTcBlockM)
+                                       : static_cast<long long>(p.pair_rows) * (2 * kTcBlockM) +
+                                             static_cast<long long>(m_blk - p.pair_rows) * kTcBlockM;
+        const int halves = pair_tile ? 2 : 1;
+        // a second half that starts past the last row repeats the first (its results are never stored)
+        const long long m1 = pair_tile && m0 + kTcBlockM < p.M ? m0 + kTcBlockM : m0;
+        const uint32_t my_tx = is_b ? b_tx : static_cast<uint32_t>(PLANES * halves) * slot;
+        const int n0 = n_blk * p.block_n;
+        int img[2] = {0, 0}, h_base[2] = {0, 0}, w_base[2] = {0, 0};
+        if (p.a_im2col && !is_b) {
+          const long long per_img = static_cast<long long>(p.OH) * p.OW;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            if (half == 1 && !pair_tile) break;
+            const long long m = half ? m1 : m0;
+            img[half] = static_cast<int>(m / per_img);
+            const int r = static_cast<int>(m - img[half] * per_img);
+            const int oh = r / p.OW;
+            const int ow = r - oh * p.OW;
+            h_base[half] = oh * p.stride_h - p.pad_t;
+            w_base[half] = ow * p.stride_w - p.pad_l;
           }
         }
-      };
-      for (int kg = 0; kg < k_groups; ++kg) {
-        const uint32_t fb = smem_u32(&full_bar[s]);
-        int w = 1;
-        if (lane == 0) {
-          w = mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, wait_limit) ? 1 : 0;
-          if (w && !(test_stall && kg == 0 && tile == static_cast<int>(blockIdx.x))) mbar_arrive_expect_tx(fb, my_tx * static_cast<uint32_t>(SUB));
-        }
-        w = __shfl_sync(0xffffffffu, w, 0);
-        if (!w) {
-          ok = false;
-          break;
-        }
-        const bool tr = p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0 && tile == static_cast<int>(gridDim.x) && kg < 32;
-        if (tr) p.trace[1024 + kg * 4 + 0] = clock64();
-        {
-          const int kb = kg * SUB + my_sb;
-          if (by_block) {
-            // (computed, not stepped: lanes that step by different amounts would diverge and issue one by one)
-            const int tap = kb / p.c_blocks;
-            cb = kb - tap * p.c_blocks;
-            kh = tap / p.KW;
-            kw = tap - kh * p.KW;
+        if (p.trace != nullptr && blockIdx.x == 0 && !is_b) p.trace[(tile / gridDim.x) * 16 + 0] = clock64();
+        // the current K block: channel block, filter row and column
+        int cb = 0, kh = 0, kw = 0;
+        for (int kg = 0; kg < k_groups; ++kg) {
+          const uint32_t fb = smem_u32(&full_bar[s]);
+          const bool stall = test_stall && kg == 0 && tile == static_cast<int>(blockIdx.x);
+          if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, wait_limit)) {
+            ok = false;
+            break;
           }
-          if (issues && !(test_stall && kg == 0 && tile == static_cast<int>(blockIdx.x))) {
-            const uint32_t dst = smem_base + static_cast<uint32_t>(s * SUB + my_sb) * stage_bytes + my_off;
-            if (is_b) {
-              tma_load_2d(dst, my_map, fb, kb * p.k_elems, n0);
-            } else if (p.a_im2col) {
-              tma_load_im2col_4d(dst, my_map, fb, cb * p.k_elems, w_base, h_base, img,
-                                 static_cast<uint16_t>(kw * p.dil_w), static_cast<uint16_t>(kh * p.dil_h));
-            } else {
-              tma_load_2d(dst, my_map, fb, kb * p.k_elems, static_cast<int>(m0));
+          const bool tr = p.trace != nullptr && blockIdx.x == 0 && !is_b && tile == static_cast<int>(gridDim.x) && kg < 32;
+          if (tr) p.trace[1024 + kg * 4 + 0] = clock64();
+          if (!stall) {
+            mbar_arrive_expect_tx(fb, my_tx * static_cast<uint32_t>(SUB));
+            for (int sb = 0; sb < SUB; ++sb) {
+              const uint32_t dst = smem_base + static_cast<uint32_t>(s * SUB + sb) * stage_bytes;
+              if (is_b) {
+                const int k = (kg * SUB + sb) * p.k_elems;
+                tma_load_2d(dst + b_off, &map_b0, fb, k, n0);
+                if (PLANES == 2) tma_load_2d(dst + b_off + b_slot, &map_b1, fb, k, n0);
+              } else {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                  if (half == 1 && !pair_tile) break;
+                  const uint32_t at = dst + static_cast<uint32_t>(half * PLANES) * slot;
+                  if (p.a_im2col) {
+                    const uint16_t dw = static_cast<uint16_t>(kw * p.dil_w), dh = static_cast<uint16_t>(kh * p.dil_h);
+                    tma_load_im2col_4d(at, &map_a0, fb, cb * p.k_elems, w_base[half], h_base[half], img[half], dw, dh);
+                    if (PLANES == 2)
+                      tma_load_im2col_4d(at + slot, &map_a1, fb, cb * p.k_elems, w_base[half], h_base[half], img[half], dw, dh);
+                  } else {
+                    const int k = (kg * SUB + sb) * p.k_elems;
+                    tma_load_2d(at, &map_a0, fb, k, static_cast<int>(half ? m1 : m0));
+                    if (PLANES == 2) tma_load_2d(at + slot, &map_a1, fb, k, static_cast<int>(half ? m1 : m0));
+                  }
+                }
+                if (++cb == p.c_blocks) {
+                  cb = 0;
+                  if (++kw == p.KW) {
+                    kw = 0;
+                    ++kh;
+                  }
+                }
+              }
             }
           }
-          if (!by_block) next_k_block();
-        }
-        if (tr) p.trace[1024 + kg * 4 + 1] = clock64();
-        ++issued;
-        if (++s == S) {
-          s = 0;
-          ph ^= 1u;
+          if (tr) p.trace[1024 + kg * 4 + 1] = clock64();
+          ++issued;
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
-    }
-    if (lane == 0) {
       if (!ok) {
         if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
       }
@@ -943,7 +938,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // formats: kind::i8 s32 <- s8 (2, 1); kind::tf32 f32 <- tf32 (1, 2); kind::f16 f32 <- bf16 (1, 1)
       const uint32_t idesc = KIND == GEMM_I8
                                  ? instr_desc(2u, 1u, kTcBlockM, static_cast<uint32_t>(p.block_n))

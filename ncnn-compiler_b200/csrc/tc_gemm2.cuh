@@ -127,7 +127,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // the same in all lanes, and known to be
   const int lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
   constexpr int CTAS = PAIR ? 2 : 1;               // CTAs per worker
@@ -177,117 +177,111 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
   __syncthreads();
   if (PAIR) cluster_sync_all();  // the other CTA's barriers exist before anything is sent to them
   tc_fence_after_sync();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   // barriers, tensor memory and descriptors are ready: from here on the kernel touches tensors that the
   // kernel before it in the stream may still be writing
   grid_dependency_wait();
 
   if (warp == 0 || warp == 6) {
     // ------------------------------------------------------------ producers
-    // Warp 0 feeds this CTA's 128 rows of A, warp 6 its half of the B rows; lane p issues plane p.
+    // Warp 0 feeds this CTA's 128 rows of A, warp 6 its half of the B rows, in one elected thread (why: tc_gemm.cuh).
     // The bytes are counted on CTA 0's full barrier, armed by CTA 0's two producer warps for both CTAs.
     const bool is_b = warp == 6;
-    const bool issuer = lane < PLANES;
-    const CUtensorMap* my_map = is_b ? (lane ? &map_b1 : &map_b0) : (lane ? &map_a1 : &map_a0);
-    const uint32_t my_off = is_b ? static_cast<uint32_t>(PLANES) * slot + lane * b_slot : lane * slot;
-    const uint32_t tx_both = static_cast<uint32_t>(CTAS) * PLANES * (is_b ? static_cast<uint32_t>(b_rows) * p.row_bytes : slot);
-    int s = 0;
-    uint32_t ph = 0;
-    long long issued = 0;
-    bool ok = true;
-    for (int i = 0; i < work.nseg && ok; ++i) {
-      int tile, kb0, kb1, owned;
-      work.seg(i, &tile, &kb0, &kb1, &owned);
-      const int m_blk = tile / p.tiles_n;
-      const int n_blk = tile - m_blk * p.tiles_n;
-      // a second half that starts past the last row repeats the first (its results are never stored)
-      long long m0 = static_cast<long long>(m_blk) * TILE_M;
-      if (m0 + static_cast<long long>(rank) * kTcBlockM < p.M) m0 += static_cast<long long>(rank) * kTcBlockM;
-      const int n0 = n_blk * p.block_n + static_cast<int>(rank) * b_rows;
-      int img = 0, h_base = 0, w_base = 0;
-      if (p.a_im2col) {
-        const long long per_img = static_cast<long long>(p.OH) * p.OW;
-        img = static_cast<int>(m0 / per_img);
-        const int r = static_cast<int>(m0 - img * per_img);
-        const int oh = r / p.OW;
-        const int ow = r - oh * p.OW;
-        h_base = oh * p.stride_h - p.pad_t;
-        w_base = ow * p.stride_w - p.pad_l;
-      }
-      const int tap0 = kb0 / p.c_blocks;
-      int cb = kb0 - tap0 * p.c_blocks;
-      int kh = tap0 / p.KW;
-      int kw = tap0 - kh * p.KW;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const uint32_t fb = PAIR ? map_to_cta(smem_u32(&full_bar[s]), 0u) : smem_u32(&full_bar[s]);
-        int w = 1;
-        if (lane == 0) {
-          w = mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-          if (w && rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), tx_both);
+    if (elect_one()) {
+      const uint32_t my_off = is_b ? static_cast<uint32_t>(PLANES) * slot : 0u;
+      const uint32_t my_plane = is_b ? b_slot : slot;
+      const uint32_t tx_both = static_cast<uint32_t>(CTAS) * PLANES * (is_b ? static_cast<uint32_t>(b_rows) * p.row_bytes : slot);
+      int s = 0;
+      uint32_t ph = 0;
+      long long issued = 0;
+      bool ok = true;
+      for (int i = 0; i < work.nseg && ok; ++i) {
+        int tile, kb0, kb1, owned;
+        work.seg(i, &tile, &kb0, &kb1, &owned);
+        const int m_blk = tile / p.tiles_n;
+        const int n_blk = tile - m_blk * p.tiles_n;
+        // a second half that starts past the last row repeats the first (its results are never stored)
+        long long m0 = static_cast<long long>(m_blk) * TILE_M;
+        if (m0 + static_cast<long long>(rank) * kTcBlockM < p.M) m0 += static_cast<long long>(rank) * kTcBlockM;
+        const int n0 = n_blk * p.block_n + static_cast<int>(rank) * b_rows;
+        int img = 0, h_base = 0, w_base = 0;
+        if (p.a_im2col) {
+          const long long per_img = static_cast<long long>(p.OH) * p.OW;
+          img = static_cast<int>(m0 / per_img);
+          const int r = static_cast<int>(m0 - img * per_img);
+          const int oh = r / p.OW;
+          const int ow = r - oh * p.OW;
+          h_base = oh * p.stride_h - p.pad_t;
+          w_base = ow * p.stride_w - p.pad_l;
         }
-        w = __shfl_sync(0xffffffffu, w, 0);
-        if (!w) {
-          ok = false;
-          break;
-        }
-        const bool tr = p.trace != nullptr && blockIdx.x == trace_cta && threadIdx.x == 0 && i == 0 && kb - kb0 < 40;
-        if (tr) p.trace[16 + 4 * (kb - kb0) + 2] = clock64();
-        if (issuer) {
-          const uint32_t dst = smem_base + s * stage_bytes + my_off;
-          if (PAIR) {
+        const int tap0 = kb0 / p.c_blocks;
+        int cb = kb0 - tap0 * p.c_blocks;
+        int kh = tap0 / p.KW;
+        int kw = tap0 - kh * p.KW;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const uint32_t fb = PAIR ? map_to_cta(smem_u32(&full_bar[s]), 0u) : smem_u32(&full_bar[s]);
+          if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+            ok = false;
+            break;
+          }
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), tx_both);
+          const bool tr = p.trace != nullptr && blockIdx.x == trace_cta && !is_b && i == 0 && kb - kb0 < 40;
+          if (tr) p.trace[16 + 4 * (kb - kb0) + 2] = clock64();
+          const uint32_t dst0 = smem_base + s * stage_bytes + my_off;
+#pragma unroll
+          for (int plane = 0; plane < PLANES; ++plane) {
+            const uint32_t dst = dst0 + static_cast<uint32_t>(plane) * my_plane;
             if (is_b) {
-              tma_load_2d_pair(dst, my_map, fb, kb * p.k_elems, n0);
-            } else if (p.a_im2col) {
-              tma_load_im2col_4d_pair(dst, my_map, fb, cb * p.k_elems, w_base, h_base, img,
-                                      static_cast<uint16_t>(kw * p.dil_w), static_cast<uint16_t>(kh * p.dil_h));
+              const CUtensorMap* map = plane ? &map_b1 : &map_b0;
+              if (PAIR) tma_load_2d_pair(dst, map, fb, kb * p.k_elems, n0);
+              else tma_load_2d(dst, map, fb, kb * p.k_elems, n0);
             } else {
-              tma_load_2d_pair(dst, my_map, fb, kb * p.k_elems, static_cast<int>(m0));
-            }
-          } else {
-            if (is_b) {
-              tma_load_2d(dst, my_map, fb, kb * p.k_elems, n0);
-            } else if (p.a_im2col) {
-              tma_load_im2col_4d(dst, my_map, fb, cb * p.k_elems, w_base, h_base, img,
-                                 static_cast<uint16_t>(kw * p.dil_w), static_cast<uint16_t>(kh * p.dil_h));
-            } else {
-              tma_load_2d(dst, my_map, fb, kb * p.k_elems, static_cast<int>(m0));
+              const CUtensorMap* map = plane ? &map_a1 : &map_a0;
+              const uint16_t dw = static_cast<uint16_t>(kw * p.dil_w), dh = static_cast<uint16_t>(kh * p.dil_h);
+              if (p.a_im2col) {
+                if (PAIR) tma_load_im2col_4d_pair(dst, map, fb, cb * p.k_elems, w_base, h_base, img, dw, dh);
+                else tma_load_im2col_4d(dst, map, fb, cb * p.k_elems, w_base, h_base, img, dw, dh);
+              } else {
+                if (PAIR) tma_load_2d_pair(dst, map, fb, kb * p.k_elems, static_cast<int>(m0));
+                else tma_load_2d(dst, map, fb, kb * p.k_elems, static_cast<int>(m0));
+              }
             }
           }
-        }
-        if (tr) p.trace[16 + 4 * (kb - kb0) + 3] = clock64();
-        ++issued;
-        if (++cb == p.c_blocks) {
-          cb = 0;
-          if (++kw == p.KW) {
-            kw = 0;
-            ++kh;
+          if (tr) p.trace[16 + 4 * (kb - kb0) + 3] = clock64();
+          ++issued;
+          if (++cb == p.c_blocks) {
+            cb = 0;
+            if (++kw == p.KW) {
+              kw = 0;
+              ++kh;
+            }
+          }
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
           }
         }
-        if (++s == S) {
-          s = 0;
-          ph ^= 1u;
+      }
+      {
+        if (!ok) {
+          if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
         }
-      }
-    }
-    if (lane == 0) {
-      if (!ok) {
-        if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
-      }
-      if (*abort_ptr != 0 && rank == 0) {
-        // Some role gave up.  Copies may still be landing in shared memory: wait (bounded) for the
-        // last S fills that were armed (CTA 0's barriers count both CTAs' bytes).
-        int zero = 0;
-        const long long first = issued > S ? issued - S : 0;
-        for (long long i = first; i < issued; ++i) {
-          const int st = static_cast<int>(i % S);
-          const uint32_t par = static_cast<uint32_t>((i / S) & 1);
-          mbar_wait_bounded(smem_u32(&full_bar[st]), par, &zero, 200000000ull);
+        if (*abort_ptr != 0 && rank == 0) {
+          // Some role gave up.  Copies may still be landing in shared memory: wait (bounded) for the
+          // last S fills that were armed (CTA 0's barriers count both CTAs' bytes).
+          int zero = 0;
+          const long long first = issued > S ? issued - S : 0;
+          for (long long i = first; i < issued; ++i) {
+            const int st = static_cast<int>(i % S);
+            const uint32_t par = static_cast<uint32_t>((i / S) & 1);
+            mbar_wait_bounded(smem_u32(&full_bar[st]), par, &zero, 200000000ull);
+          }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer (CTA 0 only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = KIND == GEMM_I8
                                  ? instr_desc(2u, 1u, TILE_M, static_cast<uint32_t>(p.block_n))
                                  : instr_desc(1u, KIND == GEMM_BF16X3 ? 1u : 2u, TILE_M,

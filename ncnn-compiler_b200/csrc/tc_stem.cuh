@@ -76,7 +76,7 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // the same in all lanes, and known to be
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(stem_smem_raw) + 1023u) & ~1023u;
   const int S = p.stages;
@@ -117,69 +117,63 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   // barriers, tensor memory and descriptors are ready: from here on the kernel touches tensors that the
   // kernel before it in the stream may still be writing
   grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer: weights once, then rows
-    const CUtensorMap* map_a = lane ? &map_a1 : &map_a0;
-    const CUtensorMap* map_b = lane ? &map_b1 : &map_b0;
-    const uint32_t wb = smem_u32(&weights_bar);
-    if (lane == 0) mbar_arrive_expect_tx(wb, static_cast<uint32_t>(p.KH * PLANES) * static_cast<uint32_t>(p.N) * 64u);
-    __syncwarp();
-    if (lane < PLANES) {
+    if (elect_one()) {  // (one elected thread: tc_gemm.cuh says why)
+      const uint32_t wb = smem_u32(&weights_bar);
+      mbar_arrive_expect_tx(wb, static_cast<uint32_t>(p.KH * PLANES) * static_cast<uint32_t>(p.N) * 64u);
       // (the K coordinate counts elements: 32 bf16 or 64 int8 per filter row)
-      for (int kh = 0; kh < p.KH; ++kh)
-        tma_load_2d(b_region + static_cast<uint32_t>(kh * PLANES + lane) * p.b_slot, map_b, wb,
-                    kh * (KIND == GEMM_I8 ? 64 : 32), 0);
-    }
-    int s = 0;
-    uint32_t ph = 0;
-    long long issued = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
-      const int img = tile / p.OH;
-      const int oh = tile - img * p.OH;
-      const uint32_t fb = smem_u32(&full_bar[s]);
-      int w = 1;
-      if (lane == 0) {
-        w = mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0;
-        if (w) mbar_arrive_expect_tx(fb, static_cast<uint32_t>(PLANES * p.KH) * static_cast<uint32_t>(p.row_bytes));
+      for (int kh = 0; kh < p.KH; ++kh) {
+        const uint32_t dst = b_region + static_cast<uint32_t>(kh * PLANES) * p.b_slot;
+        tma_load_2d(dst, &map_b0, wb, kh * (KIND == GEMM_I8 ? 64 : 32), 0);
+        if (PLANES == 2) tma_load_2d(dst + static_cast<uint32_t>(p.b_slot), &map_b1, wb, kh * 32, 0);
       }
-      w = __shfl_sync(0xffffffffu, w, 0);
-      if (!w) {
-        ok = false;
-        break;
+      int s = 0;
+      uint32_t ph = 0;
+      long long issued = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+        const int img = tile / p.OH;
+        const int oh = tile - img * p.OH;
+        const uint32_t fb = smem_u32(&full_bar[s]);
+        if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+          ok = false;
+          break;
+        }
+        mbar_arrive_expect_tx(fb, static_cast<uint32_t>(PLANES * p.KH) * static_cast<uint32_t>(p.row_bytes));
+        // rows above or below the image are filled with zeros by the copy
+        const uint32_t dst = a_region + static_cast<uint32_t>(s) * stage_bytes;
+        tma_load_4d(dst, &map_a0, fb, 0, 0, oh * p.stride_h - p.pad_t, img);
+        if (PLANES == 2) tma_load_4d(dst + static_cast<uint32_t>(p.a_plane_bytes), &map_a1, fb, 0, 0, oh * p.stride_h - p.pad_t, img);
+        ++issued;
+        if (++s == S) {
+          s = 0;
+          ph ^= 1u;
+        }
       }
-      // rows above or below the image are filled with zeros by the copy
-      if (lane < PLANES)
-        tma_load_4d(a_region + static_cast<uint32_t>(s) * stage_bytes + static_cast<uint32_t>(lane) * p.a_plane_bytes,
-                    map_a, fb, 0, 0, oh * p.stride_h - p.pad_t, img);
-      ++issued;
-      if (++s == S) {
-        s = 0;
-        ph ^= 1u;
-      }
-    }
-    if (lane == 0) {
-      if (!ok && atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
-      if (*abort_ptr != 0) {
-        // copies this warp issued may still be landing: wait (bounded) for them before the CTA ends
-        int zero = 0;
-        mbar_wait_bounded(wb, 0, &zero, 200000000ull);
-        const long long first = issued > S ? issued - S : 0;
-        for (long long i = first; i < issued; ++i)
-          mbar_wait_bounded(smem_u32(&full_bar[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
+      {
+        if (!ok && atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
+        if (*abort_ptr != 0) {
+          // copies this warp issued may still be landing: wait (bounded) for them before the CTA ends
+          int zero = 0;
+          mbar_wait_bounded(wb, 0, &zero, 200000000ull);
+          const long long first = issued > S ? issued - S : 0;
+          for (long long i = first; i < issued; ++i)
+            mbar_wait_bounded(smem_u32(&full_bar[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
+        }
       }
     }
   } else if (warp == 1 || (warp == 6 && issuers == 2)) {
     // ---------------------------------------------------------- MMA issuers
-    // One thread issues a narrow MMA every 75-150 cycles, the tensor pipe takes one every ~48: with four
-    // accumulators warps 1 and 6 issue alternate tiles (MMAs into one accumulator must come from one thread).
+    // With four accumulators warps 1 and 6 issue alternate tiles, so that one waits for its rows while the other's
+    // MMAs run (MMAs into one accumulator must come from one thread).
     const int me = warp == 1 ? 0 : 1;
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = KIND == GEMM_I8 ? instr_desc(2u, 1u, kTcBlockM, static_cast<uint32_t>(p.N))
                                              : instr_desc(1u, 1u, kTcBlockM, static_cast<uint32_t>(p.N));
       bool ok = mbar_wait_bounded(smem_u32(&weights_bar), 0, abort_ptr, kTcWaitLimitNs);
