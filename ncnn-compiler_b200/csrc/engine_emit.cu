@@ -6,6 +6,52 @@ namespace nb {
 
 static cudaError_t launch_ok() { return cudaGetLastError(); }
 
+// fp32 contraction on the CUDA cores as a tiled kernel (conv_f32.cuh).  Needs plain fp32 input and 32-bit pixel numbers.
+static bool conv_f32_applies(const ActRef& in, const ConvGeom& g) {
+  const long long rows = g.images * g.OH * g.OW, pixels = g.images * g.H * g.W;
+  return in.fmt == FMT_F32 && rows < (1ll << 30) && pixels < (1ll << 30) && static_cast<long long>(g.KH) * g.KW * g.C < (1ll << 30);
+}
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& out, const void* w, const ConvGeom& g, const ConvEpilogue& e) {
+  F32ConvParams p{};
+  p.g = g;
+  p.weights = static_cast<const float*>(w);
+  p.e = e;
+  p.K = g.KH * g.KW * g.C;
+  f32_chunks(p.K, &p.chunks, &p.chunk_k);
+  const long long rows = g.images * g.OH * g.OW;
+  p.tiles_n = (g.O + kF32Bn - 1) / kF32Bn;
+  // 128-row tiles move 25 % fewer operand bytes; 64-row tiles fill the last wave better.  Two 128-thread blocks or four
+  // 64-thread blocks live on an SM, so the large tiles pay from about two full waves on.
+  const bool large = (rows + 127) / 128 * p.tiles_n >= 4ll * sm_count_;
+  const int bm = large ? 128 : 64;
+  const long long tiles = (rows + bm - 1) / bm * p.tiles_n;
+  // fewer tiles than the four blocks an SM holds: the chunks of a tile go to different blocks (as far as the workspace reaches)
+  const size_t ws = static_cast<size_t>(tiles) * p.chunks * bm * kF32Bn * 4;
+  p.split = !large && p.chunks > 1 && tiles < 4ll * sm_count_ && tiles <= kTcSplitFlagCount && ws <= kTcSplitWorkspaceBytes ? 1 : 0;
+  p.partials = reinterpret_cast<float*>(d_split_ws_);
+  p.counters = d_split_flags_;
+  p.vec_a = g.C % 4 == 0 && aligned16(in.p0) ? 1 : 0;
+  p.vec_b = g.O % 2 == 0 ? 1 : 0;
+  p.vec_o = g.O % 4 == 0 ? 1 : 0;
+  p.plain = p.vec_o && out.fmt == FMT_F32 && (!e.has_res || e.res.fmt == FMT_F32) && (e.act == ACT_NONE || e.act == ACT_RELU || e.act == ACT_CLIP) ? 1 : 0;
+  p.clamp_lo = e.act == ACT_RELU ? 0.0f : (e.act == ACT_CLIP ? e.act_a : -std::numeric_limits<float>::infinity());
+  p.clamp_hi = e.act == ACT_CLIP ? e.act_b : std::numeric_limits<float>::infinity();
+  const float* x = in.p0;
+  const dim3 grid(static_cast<unsigned>(tiles), p.split ? p.chunks : 1);
+  const cudaError_t ae = large ? cudaFuncSetAttribute(k_conv_f32<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem_bytes(128))
+                               : cudaFuncSetAttribute(k_conv_f32<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem_bytes(64));
+  if (ae != cudaSuccess) return cudaGetErrorString(ae);
+  s->kernel = p.split ? "k_conv_f32:split" : "k_conv_f32";
+  s->run = [=](cudaStream_t st) {
+    if (large) k_conv_f32<128><<<grid, 128, f32_smem_bytes(128), st>>>(x, out, p);
+    else k_conv_f32<64><<<grid, 64, f32_smem_bytes(64), st>>>(x, out, p);
+    return launch_ok();
+  };
+  return {};
+}
+
 
 bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string* err) {
   const Tensor& to = tensors_[resolve(node.out)];
@@ -332,6 +378,9 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
           }
           return launch_ok();
         };
+      } else if (!i8 && conv_f32_applies(in, g)) {
+        const std::string ferr = emit_conv_f32(&s, in, out, w, g, e);
+        if (!ferr.empty()) return fail(err, "layer " + node.name + ": " + ferr);
       } else {
         const int grid = grid_for(n * node.OH * node.OW * node.O);
         s.kernel = i8 ? "k_conv_direct<i8>" : "k_conv_direct<f32>";
@@ -346,6 +395,15 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       const long long M = (to.rank == 2 ? static_cast<long long>(ti.h) : 1) * n;
       const int K = node.K, N = node.O;
       const void* w = node.d_w0;
+      ConvGeom g{};
+      g.images = M;
+      g.C = K;
+      g.O = N;
+      g.H = g.W = g.OH = g.OW = g.KH = g.KW = g.sh = g.sw = g.dh = g.dw = 1;
+      if (!i8 && conv_f32_applies(in, g)) {
+        const std::string ferr = emit_conv_f32(&s, in, out, w, g, e);
+        if (!ferr.empty()) return fail(err, "layer " + node.name + ": " + ferr);
+      } else {
       const int grid = grid_for(M * N);
       s.kernel = i8 ? "k_matmul_direct<i8>" : "k_matmul_direct<f32>";
       s.run = [=](cudaStream_t st) {
@@ -353,6 +411,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         else k_matmul_direct<false><<<grid, 256, 0, st>>>(in, out, w, M, K, N, e, 0.0f);
         return launch_ok();
       };
+      }
       plan.steps.push_back(std::move(s));
     }
     if (node.kind == N_GEMM && node.alpha != 1.0f && !(node.impl == IMPL_TC && node.act == ACT_NONE)) {
@@ -609,7 +668,7 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
           k_chw_to_nhwc_small_x4<<<grid, 256, 0, st>>>(src_ptr, dst, ep);
           return launch_ok();
         };
-      } else if (t.c <= 4 && (t.Cp == 4 || t.Cp == 16 || (t.Cp == 8 && t.fmt == FMT_I8))) {
+      } else if (t.c <= 4 && (t.Cp == 4 || t.Cp == 16 || (t.Cp == 8 && t.fmt == FMT_I8) || (t.Cp == t.c && t.input_quant_scale <= 0.0f))) {
         const int grid = grid_for(n * t.h * t.w);
         s.kernel = "k_chw_to_nhwc_small";
         s.run = [=](cudaStream_t st) {

@@ -13,6 +13,7 @@
 #include <map>
 #include <sstream>
 
+#include "conv_f32.cuh"
 #include "ip_rows.cuh"
 #include "kernels.cuh"
 #include "loader.h"
@@ -334,6 +335,7 @@ class EngineImpl {
   bool prepare_weights(std::string* err);
   void plan_memory();
   ActRef ref(int tensor, int64_t n) const;
+  std::string emit_conv_f32(Step* s, const ActRef& in, const ActRef& out, const void* w, const ConvGeom& g, const ConvEpilogue& e);
   bool emit_node(Plan& plan, const Node& node, int64_t n, std::string* err);
   void restore_padding(int64_t n, cudaStream_t st);
   int64_t last_run_n_ = 0;  // batch size of the previous run (0: none yet)

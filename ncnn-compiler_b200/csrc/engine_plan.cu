@@ -581,7 +581,7 @@ bool EngineImpl::prepare_weights(std::string* err) {
           }
         }
       } else {
-        // direct kernel: [KH*KW][C][O]
+        // CUDA cores: [KH*KW][C][O] (int8), pairs of k (fp32)
         const size_t total = static_cast<size_t>(n.KH) * n.KW * C * n.O;
         if (i8) {
           std::vector<int8_t> v(total);
@@ -591,11 +591,11 @@ bool EngineImpl::prepare_weights(std::string* err) {
                 v[(static_cast<size_t>(t) * C + c) * n.O + o] = n.w_i8[(static_cast<size_t>(o) * C + c) * n.KH * n.KW + t];
           n.d_w0 = upload(v);
         } else {
-          std::vector<float> v(total);
+          std::vector<float> v((static_cast<size_t>(n.KH) * n.KW * C + 1) / 2 * 2 * n.O, 0.0f);
           for (int o = 0; o < n.O; ++o)
             for (int c = 0; c < C; ++c)
               for (int t = 0; t < n.KH * n.KW; ++t)
-                v[(static_cast<size_t>(t) * C + c) * n.O + o] = n.w_f32[(static_cast<size_t>(o) * C + c) * n.KH * n.KW + t];
+                v[f32_weight_at(static_cast<long long>(t) * C + c, o, n.O)] = n.w_f32[(static_cast<size_t>(o) * C + c) * n.KH * n.KW + t];
           n.d_w0 = upload(v);
         }
       }
@@ -652,16 +652,16 @@ bool EngineImpl::prepare_weights(std::string* err) {
           if (kind == GEMM_TF32X3) n.d_w1 = upload(lo);
         }
       } else {
-        // direct kernel: [K][N]
+        // CUDA cores: [K][N] (int8), pairs of k (fp32)
         if (i8) {
           std::vector<int8_t> v(n.w_i8.size());
           for (int o = 0; o < n.O; ++o)
             for (int k = 0; k < n.K; ++k) v[static_cast<size_t>(k) * n.O + o] = n.w_i8[static_cast<size_t>(o) * n.K + perm[k]];
           n.d_w0 = upload(v);
         } else {
-          std::vector<float> v(n.w_f32.size());
+          std::vector<float> v((static_cast<size_t>(n.K) + 1) / 2 * 2 * n.O, 0.0f);
           for (int o = 0; o < n.O; ++o)
-            for (int k = 0; k < n.K; ++k) v[static_cast<size_t>(k) * n.O + o] = n.w_f32[static_cast<size_t>(o) * n.K + perm[k]];
+            for (int k = 0; k < n.K; ++k) v[f32_weight_at(k, o, n.O)] = n.w_f32[static_cast<size_t>(o) * n.K + perm[k]];
           n.d_w0 = upload(v);
         }
       }

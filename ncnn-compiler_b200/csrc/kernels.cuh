@@ -137,7 +137,8 @@ static __global__ void k_chw_to_nhwc_tiled(const float* __restrict__ src, ActRef
   }
 }
 
-// Few channels (C <= 4): one thread per pixel, one 16-byte store per plane.
+// Few channels (C <= 4): one thread per pixel, one 16-byte store per plane (dense pixels of fewer than 4 channels: one
+// store per channel; the 32-channel tiles of the general kernel would be nine tenths empty: 56 -> 8 us for 8 x 3 x 224 x 224).
 static __global__ void k_chw_to_nhwc_small(const float* __restrict__ src, ActRef dst, EdgeParams p) {
   const long long hw = static_cast<long long>(p.H) * p.W;
   const long long total = p.images * hw;
@@ -156,6 +157,8 @@ static __global__ void k_chw_to_nhwc_small(const float* __restrict__ src, ActRef
         w0 |= (static_cast<uint32_t>(quantize_rha(v[c], p.quant_scale)) & 0xffu) << (8 * c);
       if (p.Cp == 8) *reinterpret_cast<uint2*>(dst.q + o) = make_uint2(w0, 0u);
       else *reinterpret_cast<uint4*>(dst.q + o) = make_uint4(w0, 0u, 0u, 0u);
+    } else if (p.Cp < 4) {
+      for (int c = 0; c < p.C; ++c) act_store(dst, o + c, v[c]);  // dense pixels of one to three channels
     } else {
       act_store4(dst, o, make_float4(v[0], v[1], v[2], v[3]));
     }
@@ -735,8 +738,11 @@ static __global__ void __launch_bounds__(256) k_maxpool3x3s2_tile(ActRef in, Act
 }
 
 // ----------------------------------------------------------------- direct conv / matmul
-// CUDA-core convolution: exact fp32 accumulation (fused multiply-add), any geometry.
-// Weights are stored [KH*KW][C][O].  One thread per (pixel, output channel); threads
+// Where the CUDA-core fp32 contractions keep weight (k, o): rows of two k, [K/2][O][2] (conv_f32.cuh reads pairs).
+__host__ __device__ __forceinline__ long long f32_weight_at(long long k, int o, int O) { return ((k >> 1) * O + o) * 2 + (k & 1); }
+
+// CUDA-core convolution: exact fp32 accumulation (fused multiply-add), any geometry (int8, and fp32 inputs that are not
+// one plain plane).  Weights are stored [KH*KW][C][O] (int8), f32_weight_at (fp32).  One thread per (pixel, output channel); threads
 // of a warp share the pixel, so activation reads are broadcasts and weight reads coalesce.
 template <bool INT8>
 static __global__ void k_conv_direct(ActRef in, ActRef out, const void* __restrict__ weights, ConvGeom g,
@@ -761,12 +767,12 @@ static __global__ void k_conv_direct(ActRef in, ActRef out, const void* __restri
         const int iw = ow * g.sw - g.pl + kw * g.dw;
         if (iw < 0 || iw >= g.W) continue;
         const long long xb = ((img * g.H + ih) * g.W + iw) * g.C;
-        const long long wb = static_cast<long long>(kh * g.KW + kw) * g.C * g.O + o;
+        const long long k0 = static_cast<long long>(kh * g.KW + kw) * g.C;
         for (int c = 0; c < g.C; ++c) {
           if (INT8) {
-            iacc += static_cast<int>(in.q[xb + c]) * static_cast<int>(wq[wb + static_cast<long long>(c) * g.O]);
+            iacc += static_cast<int>(in.q[xb + c]) * static_cast<int>(wq[(k0 + c) * g.O + o]);
           } else {
-            acc = fmaf(act_load(in, xb + c), wf[wb + static_cast<long long>(c) * g.O], acc);
+            acc = fmaf(act_load(in, xb + c), wf[f32_weight_at(k0 + c, o, g.O)], acc);
           }
         }
       }
@@ -779,7 +785,7 @@ static __global__ void k_conv_direct(ActRef in, ActRef out, const void* __restri
 }
 
 // InnerProduct / Gemm on CUDA cores: y[m][n] = sum_k a[m][k] * w[k][n] (weights
-// stored [K][N]); bias is added after the sum, as the reference's matmul + add does.
+// stored [K][N] (int8), f32_weight_at (fp32)); bias is added after the sum, as the reference's matmul + add does.
 template <bool INT8>
 static __global__ void k_matmul_direct(ActRef a, ActRef out, const void* __restrict__ weights,
                                 long long M, int K, int N, ConvEpilogue e, float gemm_beta_unused) {
@@ -796,7 +802,7 @@ static __global__ void k_matmul_direct(ActRef a, ActRef out, const void* __restr
       if (INT8) {
         iacc += static_cast<int>(a.q[m * K + k]) * static_cast<int>(wq[static_cast<long long>(k) * N + n]);
       } else {
-        acc = fmaf(act_load(a, m * K + k), wf[static_cast<long long>(k) * N + n], acc);
+        acc = fmaf(act_load(a, m * K + k), wf[f32_weight_at(k, n, N)], acc);
       }
     }
     float y;
