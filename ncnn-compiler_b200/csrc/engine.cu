@@ -104,9 +104,10 @@ Plan* EngineImpl::plan_for(int64_t n) {
   cudaStreamSynchronize(stream_);
   Plan plan;
   plan.n = n;
-  for (const Node& node : nodes_) {
+  plan.node_steps.resize(nodes_.size());
+  for (size_t k = 0; k < nodes_.size(); ++k) {
     std::string err;
-    if (!emit_node(plan, node, n, &err)) {
+    if (!emit_node(plan.node_steps[k], nodes_[k], n, &err)) {
       error_ = err;
       return nullptr;
     }
@@ -186,30 +187,72 @@ cudaGraphExec_t EngineImpl::capture_steps(const std::vector<Step>& steps) {
   return exec;
 }
 
-// Enqueues one pass of `plan` on `st`: input edges, layers, output edges; as a replay of the
-// captured graph when graphs are enabled (re-captured when the edge pointers changed).
-int EngineImpl::launch(Plan* plan, const std::vector<const float*>& d_in, const std::vector<float*>& d_out,
-                       cudaStream_t st) {
-  const int64_t n = plan->n;
-  restore_padding(n, st);
-  std::vector<Step> all, post;
-  make_edge_steps(n, d_in, d_out, &all, &post);
-  all.insert(all.end(), plan->steps.begin(), plan->steps.end());
-  all.insert(all.end(), post.begin(), post.end());
-  if (!opt_.use_cuda_graph) return issue_steps(all, st) ? 0 : 6;
-  std::vector<const void*> ptrs;
-  for (auto p : d_in) ptrs.push_back(p);
-  for (auto p : d_out) ptrs.push_back(p);
-  if (plan->graph == nullptr || plan->graph_ptrs != ptrs) {
-    if (plan->graph != nullptr) {
-      cudaGraphExecDestroy(plan->graph);
-      plan->graph = nullptr;
+// Every launch of one pass of `plan` over the given caller arrays: input edges, layers, output edges.  Arrays whose
+// layout is the tensor's own are used in place, so their edge steps fall away and the layers that touch them are
+// emitted with the caller's pointers.
+bool EngineImpl::assemble(const Plan& plan, const std::vector<const float*>& d_in, const std::vector<float*>& d_out, std::vector<Step>* all) {
+  const int64_t n = plan.n;
+  caller_array_.assign(tensors_.size(), nullptr);
+  for (size_t i = 0; i < inputs_.size(); ++i)
+    if (reads_caller_array(static_cast<int>(i), n, d_in[i])) caller_array_[resolve(inputs_[i])] = const_cast<float*>(d_in[i]);
+  for (size_t i = 0; i < outputs_.size(); ++i)
+    if (caller_array_[resolve(outputs_[i])] == nullptr && writes_caller_array(static_cast<int>(i), d_out[i]))
+      caller_array_[resolve(outputs_[i])] = d_out[i];
+  std::vector<Step> post;
+  make_edge_steps(n, d_in, d_out, all, &post);
+  bool ok = true;
+  for (size_t k = 0; k < nodes_.size() && ok; ++k) {
+    const Node& node = nodes_[k];
+    bool touched = caller_array_[resolve(node.out)] != nullptr || (node.res >= 0 && caller_array_[resolve(node.res)] != nullptr);
+    for (int t : node.in) touched = touched || caller_array_[resolve(t)] != nullptr;
+    // (an InnerProduct that quantises its own rows reads the Quantize step's input)
+    const int q = absorbed_quantize(node, n);
+    touched = touched || (q >= 0 && caller_array_[resolve(nodes_[q].in[0])] != nullptr);
+    if (!touched) {
+      all->insert(all->end(), plan.node_steps[k].begin(), plan.node_steps[k].end());
+      continue;
     }
-    plan->graph = capture_steps(all);
-    if (plan->graph == nullptr) return 6;
-    plan->graph_ptrs = ptrs;
+    std::string err;
+    ok = emit_node(*all, node, n, &err);
+    if (!ok) error_ = err;
   }
-  const cudaError_t e = cudaGraphLaunch(plan->graph, st);
+  caller_array_.clear();
+  all->insert(all->end(), post.begin(), post.end());
+  return ok;
+}
+
+// Enqueues one pass of `plan` on `st`, as a replay of the graph captured for these caller arrays when graphs are
+// enabled.  A plan remembers the launches for the last few sets of arrays: a call with known arrays builds nothing.
+int EngineImpl::launch(Plan* plan, const float* const* d_in, float* const* d_out, cudaStream_t st) {
+  restore_padding(plan->n, st);
+  const size_t ni = inputs_.size(), no = outputs_.size();
+  Pass* pass = nullptr;
+  for (Pass& p : plan->passes) {
+    if (!std::equal(p.ptrs.begin(), p.ptrs.begin() + ni, d_in) || !std::equal(p.ptrs.begin() + ni, p.ptrs.end(), d_out)) continue;
+    pass = &p;
+    break;
+  }
+  if (pass == nullptr) {
+    Pass fresh;
+    fresh.ptrs.assign(d_in, d_in + ni);
+    fresh.ptrs.insert(fresh.ptrs.end(), d_out, d_out + no);
+    if (!assemble(*plan, std::vector<const float*>(d_in, d_in + ni), std::vector<float*>(d_out, d_out + no), &fresh.steps)) return 6;
+    if (opt_.use_cuda_graph) {
+      fresh.graph = capture_steps(fresh.steps);
+      if (fresh.graph == nullptr) return 6;
+      fresh.steps.clear();
+    }
+    if (plan->passes.size() >= kMaxPasses) {
+      auto oldest = std::min_element(plan->passes.begin(), plan->passes.end(), [](const Pass& a, const Pass& b) { return a.last_used < b.last_used; });
+      if (oldest->graph != nullptr) cudaGraphExecDestroy(oldest->graph);
+      plan->passes.erase(oldest);
+    }
+    plan->passes.push_back(std::move(fresh));
+    pass = &plan->passes.back();
+  }
+  pass->last_used = ++use_counter_;
+  if (!opt_.use_cuda_graph) return issue_steps(pass->steps, st) ? 0 : 6;
+  const cudaError_t e = cudaGraphLaunch(pass->graph, st);
   if (e != cudaSuccess) {
     error_ = std::string("launch failed: ") + cudaGetErrorString(e);
     return 6;
@@ -252,6 +295,12 @@ bool EngineImpl::build_pipeline(Plan* plan) {
         cnt * node.OH * node.OW < 2ll * kTcBlockM * sm_count_)
       break;
     if (node.kind == N_IP || node.kind == N_GEMM) break;
+    // (whether an InnerProduct quantises its own rows depends on the batch it runs with: its Quantize step stays beside it)
+    if (node.kind == N_UNARY && node.un.op == UN_QUANT) {
+      bool feeds_ip = false;
+      for (const Node& ip : nodes_) feeds_ip = feeds_ip || (ip.kind == N_IP && resolve(ip.in[0]) == resolve(node.out));
+      if (feeds_ip) break;
+    }
   }
   for (int c = 0; c < chunks; ++c) {
     layout_n_ = n;
@@ -262,25 +311,21 @@ bool EngineImpl::build_pipeline(Plan* plan) {
     std::vector<Step> post;
     plan->head[c].clear();
     make_edge_steps(cnt, d_in, plan->d_out, &plan->head[c], &post);
-    Plan piece;
-    piece.n = cnt;
     bool ok = true;
     for (int k = 0; k < head_end && ok; ++k) {
       std::string err;
-      ok = emit_node(piece, nodes_[k], cnt, &err);
+      ok = emit_node(plan->head[c], nodes_[k], cnt, &err);
       if (!ok) error_ = err;
     }
     layout_n_ = 0;
     img0_ = 0;
     if (!ok) return false;
-    plan->head[c].insert(plan->head[c].end(), piece.steps.begin(), piece.steps.end());
   }
   {
-    Plan piece;
-    piece.n = n;
+    plan->tail.clear();
     for (size_t k = head_end; k < nodes_.size(); ++k) {
       std::string err;
-      if (!emit_node(piece, nodes_[k], n, &err)) {
+      if (!emit_node(plan->tail, nodes_[k], n, &err)) {
         error_ = err;
         return false;
       }
@@ -288,7 +333,6 @@ bool EngineImpl::build_pipeline(Plan* plan) {
     std::vector<const float*> d_in(plan->d_in.begin(), plan->d_in.end());
     std::vector<Step> pre, post;
     make_edge_steps(n, d_in, plan->d_out, &pre, &post);
-    plan->tail = piece.steps;
     plan->tail.insert(plan->tail.end(), post.begin(), post.end());
   }
   if (opt_.use_cuda_graph) {
@@ -376,27 +420,15 @@ int EngineImpl::run(int64_t n, const float* const* in, float* const* out, bool h
     if (upload >= kPipelineUploadBytes) return run_host_pipelined(plan, in, out);
   }
   cudaStream_t st = host ? stream_ : user_stream;
-  std::vector<const float*> d_in(inputs_.size());
-  std::vector<float*> d_out(outputs_.size());
-  if (host) {
-    if (!ensure_staging(plan)) return 6;
-    for (size_t i = 0; i < inputs_.size(); ++i) {
-      d_in[i] = plan->d_in[i];
-      cudaMemcpyAsync(plan->d_in[i], in[i], tensors_[resolve(inputs_[i])].logical() * 4 * n, cudaMemcpyHostToDevice, st);
-    }
-    for (size_t i = 0; i < outputs_.size(); ++i) d_out[i] = plan->d_out[i];
-  } else {
-    for (size_t i = 0; i < inputs_.size(); ++i) d_in[i] = in[i];
-    for (size_t i = 0; i < outputs_.size(); ++i) d_out[i] = out[i];
-  }
-  const int rc = launch(plan, d_in, d_out, st);
+  if (!host) return launch(plan, in, out, st);
+  if (!ensure_staging(plan)) return 6;
+  for (size_t i = 0; i < inputs_.size(); ++i)
+    cudaMemcpyAsync(plan->d_in[i], in[i], tensors_[resolve(inputs_[i])].logical() * 4 * n, cudaMemcpyHostToDevice, st);
+  const int rc = launch(plan, plan->d_in.data(), plan->d_out.data(), st);
   if (rc != 0) return rc;
-  if (host) {
-    for (size_t i = 0; i < outputs_.size(); ++i)
-      cudaMemcpyAsync(out[i], plan->d_out[i], tensors_[resolve(outputs_[i])].logical() * 4 * n, cudaMemcpyDeviceToHost, st);
-    return finish_host_run(st);
-  }
-  return 0;
+  for (size_t i = 0; i < outputs_.size(); ++i)
+    cudaMemcpyAsync(out[i], plan->d_out[i], tensors_[resolve(outputs_[i])].logical() * 4 * n, cudaMemcpyDeviceToHost, st);
+  return finish_host_run(st);
 }
 
 int EngineImpl::profile(int64_t n, int repeat, std::vector<LayerTiming>* out) {
@@ -404,18 +436,11 @@ int EngineImpl::profile(int64_t n, int repeat, std::vector<LayerTiming>* out) {
   if (plan == nullptr) return 6;
   restore_padding(n, stream_);
   out->clear();
-  // every launch of one run: input edges, layers, output edges
+  // every launch of one run over the staging arrays: input edges, layers, output edges
   std::vector<Step> all;
-  if (ensure_staging(plan) && !plan->d_in.empty()) {
-    std::vector<Step> pre, post;
-    std::vector<const float*> d_in(plan->d_in.begin(), plan->d_in.end());
-    make_edge_steps(n, d_in, plan->d_out, &pre, &post);
-    all = pre;
-    all.insert(all.end(), plan->steps.begin(), plan->steps.end());
-    all.insert(all.end(), post.begin(), post.end());
-  } else {
-    all = plan->steps;
-  }
+  if (!ensure_staging(plan) ||
+      !assemble(*plan, std::vector<const float*>(plan->d_in.begin(), plan->d_in.end()), plan->d_out, &all))
+    return 6;
   struct Events {
     std::vector<cudaEvent_t> ev;
     explicit Events(size_t n) : ev(n, nullptr) {
@@ -540,7 +565,11 @@ int Engine::launches_per_run(int64_t n) {
   DeviceGuard guard(impl_->device_);
   Plan* p = impl_->plan_for(n);
   if (p == nullptr) return -1;
-  return static_cast<int>(p->steps.size() + impl_->inputs_.size() + impl_->outputs_.size());
+  // (the arena stands in for the caller's arrays: aligned, as a caller's allocation is)
+  std::vector<Step> all;
+  float* any = reinterpret_cast<float*>(impl_->arena_);
+  if (!impl_->assemble(*p, std::vector<const float*>(impl_->inputs_.size(), any), std::vector<float*>(impl_->outputs_.size(), any), &all)) return -1;
+  return static_cast<int>(all.size());
 }
 const std::string& Engine::last_error() const { return impl_->error_; }
 
@@ -549,9 +578,12 @@ std::string Engine::plan_summary(int64_t n) {
   Plan* p = impl_->plan_for(n);
   std::ostringstream o;
   if (p == nullptr) return "error: " + impl_->error_;
-  o << "batch " << n << ": " << p->steps.size() << " launches, arena "
+  size_t launches = 0;
+  for (const auto& steps : p->node_steps) launches += steps.size();
+  o << "batch " << n << ": " << launches << " launches, arena "
     << (impl_->arena_per_image_ * n >> 10) << " KiB\n";
-  for (const Step& s : p->steps) o << "  " << s.kernel << "  " << s.name << "\n";
+  for (const auto& steps : p->node_steps)
+    for (const Step& s : steps) o << "  " << s.kernel << "  " << s.name << "\n";
   return o.str();
 }
 

@@ -53,7 +53,62 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
 }
 
 
-bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string* err) {
+// True when an InnerProduct / Gemm of this batch size runs on the kernel for a handful of rows (ip_rows.cuh): one pass
+// over the weights on the CUDA cores instead of mostly empty 128-row tiles.
+bool EngineImpl::takes_rows(const Node& node, int64_t n) const {
+  if ((node.kind != N_IP && node.kind != N_GEMM) || node.impl != IMPL_TC || env_flag_off("NCNN_B200_IP_ROWS")) return false;
+  const Tensor& ti = tensors_[resolve(node.in[0])];
+  const Tensor& to = tensors_[resolve(node.out)];
+  const bool i8 = node.term != 0;
+  if (!i8 && ti.fmt != FMT_BF16X2) return false;
+  const long long M = (to.rank == 2 ? static_cast<long long>(ti.h) : 1) * n;
+  const int out_mode = to.fmt == FMT_I8 ? OUT_I8 : (to.fmt == FMT_BF16X2 ? OUT_BF16X2 : (to.fmt == FMT_F32 ? OUT_F32 : OUT_F32_SPLIT));
+  return ip_rows_applies(M, ti.row_pitch > 0 ? ti.row_pitch : node.K, node.O, i8, out_mode, node.res >= 0, !node.side_q.empty());
+}
+
+// The Quantize step that the rows kernel of an int8 InnerProduct does itself while it loads its rows, or -1: a step of
+// its own for this layer, reading one plain fp32 plane.
+int EngineImpl::absorbed_quantize(const Node& node, int64_t n) const {
+  if (node.kind != N_IP || node.term == 0 || !takes_rows(node, n)) return -1;
+  for (size_t k = 0; k < nodes_.size(); ++k) {
+    const Node& q = nodes_[k];
+    if (q.kind != N_UNARY || q.un.op != UN_QUANT || resolve(q.out) != resolve(node.in[0])) continue;
+    return q.side_q.empty() && q.un.nscale == 1 && tensors_[resolve(q.in[0])].fmt == FMT_F32 ? static_cast<int>(k) : -1;
+  }
+  return -1;
+}
+
+// A graph input whose storage is the caller's own layout is read where it is: plain fp32 in channel-last order that
+// equals the caller's order (one channel, or one pixel), or rows for the kernel that converts them itself.
+bool EngineImpl::reads_caller_array(int input, int64_t n, const void* ptr) const {
+  const int id = resolve(inputs_[input]);
+  const Tensor& t = tensors_[id];
+  const bool flat = t.rank != 3 || ((t.c == 1 || t.h * t.w == 1) && t.Cp == t.c && t.Wp == t.w && t.w_off == 0);
+  if (!flat || t.dedicated || t.input_quant_scale > 0.0f || !aligned16(ptr)) return false;
+  if (t.fmt == FMT_F32) return true;
+  if (t.fmt != FMT_BF16X2) return false;
+  for (int o : outputs_)
+    if (resolve(o) == id) return false;
+  for (const Node& node : nodes_) {
+    if (node.res >= 0 && resolve(node.res) == id) return false;
+    for (int in : node.in)
+      if (resolve(in) == id && !(takes_rows(node, n) && node.term == 0)) return false;
+  }
+  return true;
+}
+
+// A graph output that a node writes as plain fp32 in the caller's order goes straight into the caller's array.
+bool EngineImpl::writes_caller_array(int output, const void* ptr) const {
+  const int id = resolve(outputs_[output]);
+  const Tensor& t = tensors_[id];
+  const bool flat = t.rank != 3 || ((t.c == 1 || t.h * t.w == 1) && t.Cp == t.c && t.Wp == t.w && t.w_off == 0);
+  if (!flat || t.is_input || t.fmt != FMT_F32 || t.row_pitch > 0 || !aligned16(ptr)) return false;
+  for (const Node& node : nodes_)
+    if (resolve(node.out) == id) return true;
+  return false;
+}
+
+bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n, std::string* err) {
   const Tensor& to = tensors_[resolve(node.out)];
   const ActRef out = ref(node.out, n);
   Step s;
@@ -93,7 +148,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         k_gemm_i8_rowscale<<<static_cast<unsigned>(M), 128, K, st>>>(in, out, wq, K, N, s_b, c_bias, alpha, beta, has_c, scale_alpha);
         return launch_ok();
       };
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
       return true;
     }
     if (node.impl == IMPL_TC) {
@@ -179,7 +234,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         s.kernel = node.ex_fused ? (node.dw_stride == 2 ? "tc_dw_project_kernel:expand+stride2<bf16x3>" : "tc_dw_project_kernel:expand<bf16x3>")
                                  : "tc_dw_project_kernel<bf16x3>";
         s.run = [dl](cudaStream_t st) { return tc_launch_dw_project(*dl, st); };
-        plan.steps.push_back(std::move(s));
+        steps.push_back(std::move(s));
         return true;
       }
       // stride-1 filters with spatial extent: the patch-resident kernel loads each input pixel
@@ -207,7 +262,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         if (tc_plan_conv_halo(hl.get(), kind, hc, te, sm_count_, halo_level() >= 2).empty()) {
           s.kernel = std::string(hl->pair ? "tc_conv_halo_kernel:pairs<" : "tc_conv_halo_kernel<") + kind_name + ">";
           s.run = [hl](cudaStream_t st) { return tc_launch_halo(*hl, st); };
-          plan.steps.push_back(std::move(s));
+          steps.push_back(std::move(s));
           return true;
         }
       }
@@ -234,14 +289,14 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
           s.name = node.name + "+" + node.pool_name;
           s.kernel = std::string("tc_stem_pool_kernel<") + kind_name + ">";
           s.run = [pl](cudaStream_t st) { return tc_launch_stem_pool(*pl, st); };
-          plan.steps.push_back(std::move(s));
+          steps.push_back(std::move(s));
           return true;
         }
         auto sl = std::make_shared<TcStemLaunch>();
         if (tc_plan_stem(sl.get(), sc, te, sm_count_).empty()) {
           s.kernel = std::string("tc_stem_kernel<") + kind_name + ">";
           s.run = [sl](cudaStream_t st) { return tc_launch_stem(*sl, st); };
-          plan.steps.push_back(std::move(s));
+          steps.push_back(std::move(s));
           return true;
         }
       }
@@ -290,13 +345,21 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         const long long M = (to.rank == 2 ? static_cast<long long>(ti.h) : 1) * n;
         const void* a0 = i8 ? static_cast<const void*>(in.q) : static_cast<const void*>(in.p0);
         // a handful of rows: one pass over the weights on the CUDA cores instead of mostly empty 128-row tiles
-        if ((kind == GEMM_BF16X3 || kind == GEMM_I8) && !env_flag_off("NCNN_B200_IP_ROWS") &&
-            ip_rows_applies(M, node.K, node.O, i8, te.out_mode, te.res0 != nullptr, te.side_count > 0)) {
+        const int row = ti.row_pitch > 0 ? ti.row_pitch : node.K;  // elements between rows of the operand
+        if (takes_rows(node, n)) {
           IpRowsParams ip{};
           ip.M = static_cast<int>(M);
-          ip.K = node.K;
+          ip.K = i8 ? row : node.K;  // (padded rows end in zeros on both sides)
           ip.N = node.O;
-          ip.lda = node.K;
+          ip.lda = row;
+          const int q = absorbed_quantize(node, n);
+          if (q >= 0 || in.fmt == FMT_F32) {
+            // rows straight from the fp32 tensor (the caller's own array, or what a Quantize step would have read)
+            const ActRef src = q >= 0 ? ref(nodes_[q].in[0], n) : in;
+            ip.x = src.p0;
+            ip.x_len = node.K;
+            ip.x_scale = node.s_in;
+          }
           ip.ldw = (node.K + node.k_elems - 1) / node.k_elems * node.k_elems;
           ip.a0 = a0;
           ip.a1 = in.p1;
@@ -313,6 +376,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
           ip.out1 = te.out1;
           ip.outq = te.outq;
           ip.ldo = te.ldo;
+          ip.x_vec = ip.x != nullptr && node.K % 4 == 0 && aligned16(ip.x) ? 1 : 0;
           const int smem = static_cast<int>(ip_rows_smem_bytes(ip.M, ip.K, i8));
           const cudaError_t ae = i8 ? cudaFuncSetAttribute(k_ip_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)
                                     : cudaFuncSetAttribute(k_ip_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
@@ -325,15 +389,15 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
             else k_ip_rows<false><<<grid, kIpRowsThreads, smem, st>>>(ip);
             return launch_ok();
           };
-          plan.steps.push_back(std::move(s));
+          steps.push_back(std::move(s));
           return true;
         }
-        perr = tc_plan_gemm(launch.get(), kind, a0, in.p1, M, node.K, node.K, node.d_w0, node.d_w1, node.O, te, sm_count_);
+        perr = tc_plan_gemm(launch.get(), kind, a0, in.p1, M, node.K, row, node.d_w0, node.d_w1, node.O, te, sm_count_);
       }
       if (!perr.empty()) return fail(err, "layer " + node.name + ": " + perr);
       s.kernel = std::string(launch->cta2 == 2 ? (launch->p.streamk ? "tc_gemm2_kernel:pairs+split<" : "tc_gemm2_kernel:pairs<") : (launch->cta2 == 1 ? "tc_gemm2_kernel:split<" : "tc_gemm_kernel<")) + kind_name + ">";
       s.run = [launch](cudaStream_t st) { return tc_launch(*launch, st); };
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
     } else if (node.kind == N_CONV || node.kind == N_DW) {
       ConvGeom g{};
       g.images = n;
@@ -390,7 +454,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
           return launch_ok();
         };
       }
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
     } else {
       const long long M = (to.rank == 2 ? static_cast<long long>(ti.h) : 1) * n;
       const int K = node.K, N = node.O;
@@ -412,7 +476,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         return launch_ok();
       };
       }
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
     }
     if (node.kind == N_GEMM && node.alpha != 1.0f && !(node.impl == IMPL_TC && node.act == ACT_NONE)) {
       Step m;
@@ -428,7 +492,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         k_binary<1><<<grid, 256, 0, st>>>(out, out, out, count, bp);
         return launch_ok();
       };
-      plan.steps.push_back(std::move(m));
+      steps.push_back(std::move(m));
     }
     return true;
   }
@@ -447,7 +511,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         k_maxpool3x3s2_tile<<<grid, 256, 0, st>>>(in, out, p);
         return launch_ok();
       };
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
       return true;
     }
     // one window over the whole image (global pooling, or a window at least as large as an unpadded image)
@@ -459,7 +523,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         k_global_pool4<<<grid, 128, 0, st>>>(in, out, p);
         return launch_ok();
       };
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
       return true;
     }
     const int grid = grid_for(n * p.OH * p.OW * (vec ? p.C / 4 : p.C));
@@ -469,7 +533,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       else k_pool<1><<<grid, 256, 0, st>>>(in, out, p);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_DECONV) {
@@ -484,7 +548,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       k_deconv2x2<<<grid, 256, 0, st>>>(in, out, w, bias, dp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_REDUCE) {
@@ -497,7 +561,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       k_reduce_mean<<<grid, 256, 0, st>>>(in, out, rp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_REMAP) {
@@ -510,7 +574,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       k_remap<<<grid, 256, 0, st>>>(in, out, rp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_BINARY && node.broadcast) {
@@ -525,7 +589,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       k_binary_broadcast<<<grid, 256, 0, st>>>(a, b, out, bp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_BINARY) {
@@ -541,11 +605,29 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       else k_binary<1><<<grid, 256, 0, st>>>(a, b, out, count, bp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_UNARY) {
+    if (node.un.op == UN_QUANT)
+      for (const Node& ip : nodes_)
+        if (ip.kind == N_IP && resolve(ip.in[0]) == resolve(node.out) && absorbed_quantize(ip, n) >= 0) return true;  // the rows kernel quantises
     const ActRef in = ref(node.in[0], n);
+    if (to.row_pitch > 0) {
+      const Tensor& ts = tensors_[resolve(node.in[0])];
+      const int K = static_cast<int>(ts.rank == 2 ? ts.w : ts.logical());
+      const long long rows = n * (ts.rank == 2 ? ts.h : 1);
+      const int pitch = to.row_pitch;
+      const float scale = node.un_scale[0];
+      const int grid = grid_for(rows * (pitch / 4));
+      s.kernel = "k_quantize_rows";
+      s.run = [=](cudaStream_t st) {
+        k_quantize_rows<<<grid, 256, 0, st>>>(in, out.q, rows, K, pitch, scale);
+        return launch_ok();
+      };
+      steps.push_back(std::move(s));
+      return true;
+    }
     const UnaryParams up = node.un;
     const long long count = to.logical() * n;
     const bool vec = count % 4 == 0;
@@ -562,7 +644,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         k_quantize16<<<grid16, 256, 0, st>>>(xp, yp, count / 16, scale, y2, scale2);
         return launch_ok();
       };
-      plan.steps.push_back(std::move(s));
+      steps.push_back(std::move(s));
       return true;
     }
     const int grid = grid_for(vec ? count / 4 : count);
@@ -572,7 +654,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       else k_unary<1><<<grid, 256, 0, st>>>(in, out, count, up);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_SOFTMAX) {
@@ -585,7 +667,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       k_softmax<<<grid, 256, 0, st>>>(in, out, sp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   if (node.kind == N_CONCAT) {
@@ -603,7 +685,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
         k_concat_copy<<<grid, 256, 0, st>>>(in, out, cp);
         return launch_ok();
       };
-      plan.steps.push_back(std::move(c));
+      steps.push_back(std::move(c));
     }
     return true;
   }
@@ -617,7 +699,7 @@ bool EngineImpl::emit_node(Plan& plan, const Node& node, int64_t n, std::string*
       k_relayout<<<grid, 256, 0, st>>>(in, out, rp);
       return launch_ok();
     };
-    plan.steps.push_back(std::move(s));
+    steps.push_back(std::move(s));
     return true;
   }
   return fail(err, "internal: unknown node kind");
@@ -628,6 +710,7 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
                                  std::vector<Step>* post) {
   for (size_t i = 0; i < inputs_.size(); ++i) {
     const Tensor& t = tensors_[resolve(inputs_[i])];
+    if (!caller_array_.empty() && caller_array_[resolve(inputs_[i])] != nullptr) continue;
     const ActRef dst = ref(inputs_[i], n);
     const float* src_ptr = d_in[i];
     Step s;
@@ -705,6 +788,7 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
     const Tensor& t = tensors_[resolve(outputs_[i])];
     const ActRef src = ref(outputs_[i], n);
     float* dst_ptr = d_out[i];
+    if (!caller_array_.empty() && caller_array_[resolve(outputs_[i])] == dst_ptr) continue;
     Step s;
     s.name = "output:" + t.name;
     s.bytes = static_cast<double>(t.logical()) * n * (4 + t.elem_bytes() * t.planes());

@@ -36,6 +36,7 @@ struct Tensor {
   // storage
   int fmt = FMT_F32;
   int Cp = 1, Wp = 1, w_off = 0;  // padded layout of a stem input
+  int row_pitch = 0;  // > 0: rows of an InnerProduct operand whose length is no multiple of 16 bytes, padded with zeros
   float input_quant_scale = 0.0f;  // > 0: the input edge quantises to int8
   size_t plane_elems = 0;          // storage elements per image and plane
   size_t plane_bytes = 0;          // per image, rounded to 256
@@ -44,6 +45,11 @@ struct Tensor {
   bool dedicated = false;          // never shares arena space (padding must stay zero)
 
   long long logical() const { return static_cast<long long>(c) * d * h * w; }
+  // storage elements of one image and plane
+  size_t image_elems() const {
+    if (row_pitch > 0) return static_cast<size_t>(rank == 2 ? h : 1) * row_pitch;
+    return rank == 3 ? static_cast<size_t>(h) * Wp * Cp : static_cast<size_t>(logical());
+  }
   int planes() const { return fmt == FMT_SPLIT || fmt == FMT_BF16X2 ? 2 : 1; }
   int elem_bytes() const { return fmt == FMT_I8 ? 1 : (fmt == FMT_BF16X2 ? 2 : 4); }
 };
@@ -132,13 +138,22 @@ struct Step {
 
 constexpr int kMaxChunks = 4;
 
+// One pass of a plan over one set of caller arrays: every launch, and the captured graph.
+struct Pass {
+  std::vector<const void*> ptrs;  // inputs, then outputs
+  std::vector<Step> steps;
+  cudaGraphExec_t graph = nullptr;
+  uint64_t last_used = 0;
+};
+
+constexpr size_t kMaxPasses = 4;  // sets of caller arrays a plan remembers (a caller that alternates between buffers)
+
 struct Plan {
   int64_t n = 0;
   uint64_t last_used = 0;  // for the bounded plan cache
-  std::vector<Step> steps;
+  std::vector<std::vector<Step>> node_steps;  // launches of every node
   std::vector<float*> d_in, d_out;  // staging used by host-pointer runs
-  cudaGraphExec_t graph = nullptr;
-  std::vector<const void*> graph_ptrs;  // the edge pointers the graph was captured with
+  std::vector<Pass> passes;
   // Pipelined host-pointer runs: the batch is uploaded in `chunks` pieces; as soon as a piece
   // has landed, its input edge and the first `head_end` layers run on its images alone
   // (head[c]); the remaining layers and the output edges run once on the whole batch (tail).
@@ -148,8 +163,9 @@ struct Plan {
   cudaGraphExec_t head_graph[kMaxChunks] = {};
   cudaGraphExec_t tail_graph = nullptr;
   void release() {
-    if (graph != nullptr) cudaGraphExecDestroy(graph);
-    graph = nullptr;
+    for (Pass& p : passes)
+      if (p.graph != nullptr) cudaGraphExecDestroy(p.graph);
+    passes.clear();
     for (cudaGraphExec_t& g : head_graph) {
       if (g != nullptr) cudaGraphExecDestroy(g);
       g = nullptr;
@@ -244,7 +260,12 @@ class EngineImpl {
   bool ensure_staging(Plan* plan);
   bool issue_steps(const std::vector<Step>& steps, cudaStream_t st);
   cudaGraphExec_t capture_steps(const std::vector<Step>& steps);
-  int launch(Plan* plan, const std::vector<const float*>& d_in, const std::vector<float*>& d_out, cudaStream_t st);
+  bool assemble(const Plan& plan, const std::vector<const float*>& d_in, const std::vector<float*>& d_out, std::vector<Step>* all);
+  bool reads_caller_array(int input, int64_t n, const void* ptr) const;
+  bool writes_caller_array(int output, const void* ptr) const;
+  bool takes_rows(const Node& node, int64_t n) const;
+  int absorbed_quantize(const Node& node, int64_t n) const;
+  int launch(Plan* plan, const float* const* d_in, float* const* d_out, cudaStream_t st);
   int finish_host_run(cudaStream_t st);
   void choose_head_limit();
   void fold_channel_concats();
@@ -279,6 +300,9 @@ class EngineImpl {
   // image window applied by ref(): tensors are laid out for layout_n_ images (0: the n
   // passed in) and pointers start at image img0_
   int64_t layout_n_ = 0, img0_ = 0;
+  // while a pass is put together: the caller array that a tensor lives in instead of the arena (by tensor id, null
+  // elsewhere; empty outside assemble())
+  std::vector<float*> caller_array_;
   int head_limit_ = 0;  // layers [0, head_limit_) may run per chunk (their tensors never share arena space)
   bool any_fp32_tc_ = false;
 
@@ -336,7 +360,7 @@ class EngineImpl {
   void plan_memory();
   ActRef ref(int tensor, int64_t n) const;
   std::string emit_conv_f32(Step* s, const ActRef& in, const ActRef& out, const void* w, const ConvGeom& g, const ConvEpilogue& e);
-  bool emit_node(Plan& plan, const Node& node, int64_t n, std::string* err);
+  bool emit_node(std::vector<Step>& steps, const Node& node, int64_t n, std::string* err);
   void restore_padding(int64_t n, cudaStream_t st);
   int64_t last_run_n_ = 0;  // batch size of the previous run (0: none yet)
   void make_edge_steps(int64_t n, const std::vector<const float*>& d_in, const std::vector<float*>& d_out,

@@ -173,7 +173,8 @@ bool EngineImpl::choose_impl(std::string* err) {
       n.impl = IMPL_DIRECT;
       if (n.kind == N_GEMM && i8) continue;  // per-row dynamic scales: dedicated kernel
       const int es = i8 ? 1 : 4;
-      if ((!exact || i8) && (static_cast<long long>(n.K) * es) % 16 == 0) n.impl = IMPL_TC;
+      // (the rows of an int8 InnerProduct are written by its Quantize step, which pads them: any K will do)
+      if ((!exact || i8) && ((static_cast<long long>(n.K) * es) % 16 == 0 || (i8 && n.kind == N_IP))) n.impl = IMPL_TC;
       if (n.impl == IMPL_TC && !i8) any_fp32_tc_ = true;
     } else if (n.kind == N_DW) {
       n.impl = IMPL_DIRECT;
@@ -252,7 +253,7 @@ void EngineImpl::fuse_quantize_steps() {
     if (q.kind != N_UNARY || q.un.op != UN_QUANT || q.un.nscale != 1 || q.un_scale.empty()) continue;
     const int src = resolve(q.in[0]);
     const Tensor& ts = tensors_[src];
-    if (ts.fmt != FMT_F32 || ts.is_input) continue;
+    if (ts.fmt != FMT_F32 || ts.is_input || tensors_[resolve(q.out)].row_pitch > 0) continue;
     int pj = -1;
     for (size_t j = 0; j < k; ++j)
       if (resolve(nodes_[j].out) == src) pj = static_cast<int>(j);
@@ -273,14 +274,16 @@ void EngineImpl::fuse_quantize_steps() {
   // and the downsample convolution, each with its own scale) become one pass with two int8 results.
   for (size_t a = 0; a < nodes_.size(); ++a) {
     Node& q1 = nodes_[a];
-    if (q1.kind != N_UNARY || q1.un.op != UN_QUANT || q1.un.nscale != 1 || q1.un_scale.size() != 1 || !q1.side_q.empty()) continue;
+    if (q1.kind != N_UNARY || q1.un.op != UN_QUANT || q1.un.nscale != 1 || q1.un_scale.size() != 1 || !q1.side_q.empty() ||
+        tensors_[resolve(q1.out)].row_pitch > 0)
+      continue;
     const int src = resolve(q1.in[0]);
     // (only where the 16-wide kernel runs at every batch size: it is the one with the second result)
     if (tensors_[src].fmt != FMT_F32 || tensors_[src].logical() % 16 != 0) continue;
     for (size_t b = a + 1; b < nodes_.size(); ++b) {
       const Node& q2 = nodes_[b];
       if (q2.kind != N_UNARY || q2.un.op != UN_QUANT || q2.un.nscale != 1 || q2.un_scale.size() != 1 || !q2.side_q.empty() ||
-          resolve(q2.in[0]) != src)
+          resolve(q2.in[0]) != src || tensors_[resolve(q2.out)].row_pitch > 0)
         continue;
       q1.side_q.emplace_back(q2.out, q2.un_scale[0]);
       nodes_.erase(nodes_.begin() + b);
@@ -468,6 +471,7 @@ bool EngineImpl::prepare_weights(std::string* err) {
     tq.alias = -1;
     tq.is_input = false;
     tq.i8 = true;
+    if (n.kind == N_IP && n.K % 16 != 0) tq.row_pitch = static_cast<int>(round_up(n.K, 16));
     n.in[0] = q.out;
     nodes_.insert(nodes_.begin() + k, std::move(q));
     ++k;
@@ -702,7 +706,7 @@ void EngineImpl::plan_memory() {
   // sizes
   for (Tensor& t : tensors_) {
     if (t.alias >= 0) continue;
-    t.plane_elems = t.rank == 3 ? static_cast<size_t>(t.h) * t.Wp * t.Cp : static_cast<size_t>(t.logical());
+    t.plane_elems = t.image_elems();
     if (t.dedicated) t.plane_elems += 256;  // the last window may read past the last row
     t.plane_bytes = round_up(t.plane_elems * t.elem_bytes(), 256);
   }
@@ -724,6 +728,14 @@ void EngineImpl::plan_memory() {
       if (sq.first_def < 0) sq.first_def = k;
       sq.last_use = std::max(sq.last_use, k);
     }
+  }
+  // (the rows kernel of an int8 InnerProduct may read what the Quantize step in front of it would have read)
+  for (int k = 0; k < end; ++k) {
+    const Node& ip = nodes_[k];
+    if (ip.kind != N_IP || ip.term == 0) continue;
+    for (int j = 0; j < k; ++j)
+      if (nodes_[j].kind == N_UNARY && nodes_[j].un.op == UN_QUANT && resolve(nodes_[j].out) == resolve(ip.in[0]))
+        tensors_[resolve(nodes_[j].in[0])].last_use = std::max(tensors_[resolve(nodes_[j].in[0])].last_use, k);
   }
   for (int t : inputs_) {
     tensors_[resolve(t)].first_def = -1;
@@ -783,8 +795,12 @@ ActRef EngineImpl::ref(int tensor, int64_t n) const {
   r.fmt = t.fmt;
   // layout for `ln` images; pointers start at image img0_ (images are dense inside a plane)
   const size_t ln = static_cast<size_t>(layout_n_ > 0 ? layout_n_ : n);
-  const size_t image_elems = t.rank == 3 ? static_cast<size_t>(t.h) * t.Wp * t.Cp : static_cast<size_t>(t.logical());
-  uint8_t* base = arena_ + t.offset * ln + static_cast<size_t>(img0_) * image_elems * t.elem_bytes();
+  if (!caller_array_.empty() && caller_array_[resolve(tensor)] != nullptr) {
+    r.fmt = FMT_F32;
+    r.p0 = caller_array_[resolve(tensor)];
+    return r;
+  }
+  uint8_t* base = arena_ + t.offset * ln + static_cast<size_t>(img0_) * t.image_elems() * t.elem_bytes();
   if (t.fmt == FMT_I8) {
     r.q = reinterpret_cast<int8_t*>(base);
   } else {

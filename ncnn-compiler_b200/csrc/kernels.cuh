@@ -316,6 +316,23 @@ static __global__ void k_quantize16(const float* __restrict__ x, int8_t* __restr
   }
 }
 
+// Quantize of rows whose length K is no multiple of 16: rows of `pitch` bytes, zeros behind the K-th, so that the
+// tensor-core path can address them (TMA wants 16-byte row strides): 200 rows of 1001 through a layer of 1537 take
+// 14 us, 155 us on the CUDA cores.  Four results and one 4-byte store per thread.
+static __global__ void k_quantize_rows(ActRef in, int8_t* __restrict__ y, long long rows, int K, int pitch, float scale) {
+  const int quads = pitch / 4;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < rows * quads;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long row = i / quads;
+    const int k = static_cast<int>(i - row * quads) * 4;
+    uint32_t word = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (k + e < K) word |= (static_cast<uint32_t>(quantize_rha(act_load(in, row * K + k + e), scale)) & 0xffu) << (8 * e);
+    reinterpret_cast<uint32_t*>(y)[i] = word;
+  }
+}
+
 // out = act(op(a * ca?, b * cb?)): Eltwise SUM with coefficients (a coefficient of
 // exactly 1 is skipped, as the reference does) and BinaryOp add/sub/mul/max.
 enum : int { BIN_ADD = 0, BIN_SUB = 1, BIN_MUL = 2, BIN_MAX = 4 };

@@ -36,3 +36,41 @@ def test_fp32_inner_product_of_odd_extents(pkg, oracle, tmp_path, m, k, n):
     want = oracle_rows(oracle, param, bin_, x)
     assert rel_l2(pkg.Model(param, bin_).run(x)[0], want) <= 1e-5
     assert rel_l2(pkg.Model(param, bin_, accuracy_mode=pkg.FP32_CUDA).run(x)[0], want) <= 2e-6
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 17, 3), (127, 31, 130), (200, 1001, 1537), (2, 4099, 2053), (8, 4097, 2051), (9, 4097, 2051)])
+def test_int8_inner_product_of_odd_extents(pkg, oracle, tmp_path, m, k, n):
+    """Rows that are no multiple of 16 bytes: padded by the Quantize step, or quantised by the rows kernel (M <= 8)."""
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n, int8=True)
+    x = np.random.default_rng(5).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    rows = sorted({0, m // 2, m - 1})
+    got = pkg.Model(param, bin_).run(x)[0]
+    assert np.array_equal(got[rows], oracle_rows(oracle, param, bin_, x[rows]))
+
+
+@pytest.mark.parametrize("m", [1, 8, 40])
+@pytest.mark.parametrize("int8", [False, True])
+def test_device_arrays_in_place_at_any_alignment(pkg, tmp_path, m, int8):
+    """Aligned caller arrays are read and written in place, others through the edge launches; a handle that meets more
+    sets of arrays than it remembers still answers the same."""
+    import torch
+    k, n = 2048, 4096
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n, int8=int8)
+    x = np.random.default_rng(6).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    model = pkg.Model(param, bin_)
+    want = model.run(x)[0]
+    src = torch.from_numpy(x.reshape(-1)).cuda()
+    for round_ in range(2):
+        for shift_in, shift_out in [(0, 0), (4, 0), (0, 4), (8, 8), (1, 0), (0, 3), (2, 1)]:
+            xin = torch.zeros(m * k + 8, device="cuda")
+            xin[shift_in:shift_in + m * k] = src
+            y = torch.full((m * n + 8,), 7.0, device="cuda")
+            model.run_device(m, [xin.data_ptr() + 4 * shift_in], [y.data_ptr() + 4 * shift_out], torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            got = y.cpu().numpy()
+            ref = got[shift_out:shift_out + m * n].reshape(m, n)
+            if int8 or m > 8:
+                assert np.array_equal(ref, want.reshape(m, n))
+            else:  # the rows kernel reads fp32 rows in place, bf16 pairs behind an edge launch
+                assert rel_l2(ref, want.reshape(m, n)) <= 1e-5
+            assert (got[:shift_out] == 7.0).all() and (got[shift_out + m * n:] == 7.0).all()
