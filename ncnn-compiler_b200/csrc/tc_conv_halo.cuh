@@ -12,7 +12,7 @@
 // on absolute shared-memory address bits, so a descriptor may start at any 128-byte row;
 // checked on hardware.)  Only the weights stream per tap.
 //
-// Roles, accumulator double-buffering, bounded waits and the staged TMA-store epilogue are
+// Roles, accumulator double-buffering, bounded waits and the epilogue are
 // those of tc_gemm_kernel; floating-point kinds only (tf32, tf32x3, bf16x3), outputs in rows
 // of 16 bytes.
 //
@@ -29,7 +29,7 @@ namespace nb {
 
 constexpr int kHaloTileH = 16;
 constexpr int kHaloTileW = 8;
-constexpr int kHaloThreads = 192;  // warps: 0 producer, 1 MMA issuer, 2-5 epilogue
+constexpr int kHaloThreads = 320;  // warps: 0 producer, 1 MMA issuer, 2-5 and 6-9 epilogue
 
 struct TcHaloParams {
   int images, OH, OW, N;
@@ -40,8 +40,12 @@ struct TcHaloParams {
   int patch_bytes;   // one plane of one patch buffer, rounded to 1 KB
   int b_bytes;       // one plane of one B stage, rounded to 1 KB
   int stages;        // B ring depth
-  int out_bufs;      // output staging tiles (>= 2)
+  int wide;          // rows of result and residual are multiples of 32 bytes, 32-byte aligned
   const float* bias;
+  float* out0;
+  float* out1;
+  const float* res0;
+  const float* res1;
   int res_mode;      // RES_*
   int out_mode;
   int act;
@@ -55,11 +59,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1)
 tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constant__ CUtensorMap map_a0,
                     const __grid_constant__ CUtensorMap map_a1,
                     const __grid_constant__ CUtensorMap map_b0,
-                    const __grid_constant__ CUtensorMap map_b1,
-                    const __grid_constant__ CUtensorMap map_o0,
-                    const __grid_constant__ CUtensorMap map_o1,
-                    const __grid_constant__ CUtensorMap map_r0,
-                    const __grid_constant__ CUtensorMap map_r1) {
+                    const __grid_constant__ CUtensorMap map_b1) {
   using namespace ptx;
   grid_dependency_trigger();  // the next kernel of the stream may begin its preamble
   constexpr int PLANES = tc_planes(KIND);
@@ -71,8 +71,6 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
   __shared__ __align__(8) uint64_t b_empty[kTcMaxStages];
   __shared__ __align__(8) uint64_t tfull_bar[2];
   __shared__ __align__(8) uint64_t tempty_bar[2];
-  __shared__ __align__(8) uint64_t res_bar;
-  __shared__ __align__(16) float tile_bias[256];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -90,8 +88,6 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
   const uint32_t b_stage_bytes = PLANES * b_bytes;
   const uint32_t b_ring = smem_base + 2u * a_buf_bytes;
   const int S = p.stages;
-  const uint32_t res_stage = b_ring + static_cast<uint32_t>(S) * b_stage_bytes;
-  const uint32_t out_stage = res_stage + (p.res_mode != RES_NONE ? 16384u : 0u);
   const int tiles_per_image = p.tiles_y * p.tiles_x;
   const int pixel_tiles = p.images * tiles_per_image;
   // work items: a pixel tile (PAIR: two consecutive pixel tiles) times a channel block
@@ -104,17 +100,15 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
       mbar_init(smem_u32(&a_full[i]), 1);
       mbar_init(smem_u32(&a_empty[i]), 1);
       mbar_init(smem_u32(&tfull_bar[i]), 1);
-      mbar_init(smem_u32(&tempty_bar[i]), 4u * CTAS);
+      mbar_init(smem_u32(&tempty_bar[i]), 8u * CTAS);
     }
     for (int i = 0; i < S; ++i) {
       mbar_init(smem_u32(&b_full[i]), 1);
       mbar_init(smem_u32(&b_empty[i]), 1);
     }
-    mbar_init(smem_u32(&res_bar), 1);
     fence_mbar_init();
     prefetch_tensormap(&map_a0);
     prefetch_tensormap(&map_b0);
-    prefetch_tensormap(&map_o0);
   }
   if (warp == 1) {
     if (PAIR) {
@@ -326,24 +320,21 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
   } else {
     // ------------------------------------------------------------ epilogue
     const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;  // accumulator row = pixel (row / 8, row % 8) of the tile
-    TcStageCfg cfg{};
-    cfg.bar_base = 1;
-    cfg.res_stage = res_stage;
-    cfg.out_stage = out_stage;
-    cfg.res_bar = smem_u32(&res_bar);
-    cfg.out_bufs = p.out_bufs;
-    cfg.out_mode = p.out_mode;
-    cfg.res_mode = p.res_mode;
-    cfg.act = p.act;
-    cfg.act_a = p.act_a;
-    cfg.act_b = p.act_b;
-    cfg.N = p.N;
-    cfg.block_n = p.block_n;
-    cfg.wide = (p.out_mode == OUT_BF16X2 || p.res_mode == RES_BF16X2) ? 1 : 0;
-    const int e_N = p.N;
-    int acc = 0, out_slot = 0;
-    uint32_t acc_ph = 0, res_ph = 0;
+    const int group = warp >= 6 ? 1 : 0;      // half of the columns
+    const int row = quarter * 32 + lane;      // accumulator row = pixel (row / 8, row % 8) of the tile
+    const int half_cols = ((p.block_n / 2) + 15) & ~15;
+    const int c_first = group ? half_cols : 0, cols = group ? p.block_n - half_cols : half_cols;
+    const TcHaloParams lp = p;
+    TcDirect d{};
+    d.out_mode = p.out_mode;
+    d.res_mode = p.res_mode;
+    d.act = p.act;
+    d.act_a = p.act_a;
+    d.act_b = p.act_b;
+    d.wide = p.wide;
+    d.stage = b_ring + static_cast<uint32_t>(S) * b_stage_bytes + static_cast<uint32_t>(group * 4 + quarter) * kDrainWarpBytes;
+    int acc = 0;
+    uint32_t acc_ph = 0;
     bool ok = true;
     const uint32_t acc_stride = p.block_n > 128 ? 256u : 128u;
     const uint32_t tempty0 = PAIR ? map_to_cta(smem_u32(&tempty_bar[0]), 0u) : smem_u32(&tempty_bar[0]);
@@ -358,28 +349,25 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
       tc_fence_after_sync();
       const uint32_t t_row =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * acc_stride;
-      for (int t = static_cast<int>(threadIdx.x) - 64; t < p.block_n; t += 128) {
-        const int n = n0 + t;
-        tile_bias[t] = (p.bias != nullptr && n < e_N) ? __ldg(p.bias + n) : 0.0f;
-      }
-      struct {
-        const CUtensorMap *o0, *o1, *r0, *r1;
-        int x, y, img;
-        __device__ __forceinline__ void load_res(int plane, uint32_t dst, uint32_t bar, int col) const {
-          ptx::tma_load_4d(dst, plane ? r1 : r0, bar, col, x, y, img);
-        }
-        __device__ __forceinline__ void store_out(int plane, uint32_t src, int col) const {
-          ptx::tma_store_4d(plane ? o1 : o0, src, col, x, y, img);
-        }
-        __device__ __forceinline__ void store_side(int, uint32_t, int) const {}
-      } io{&map_o0, &map_o1, &map_r0, &map_r1, ox0, oy0, img};
       const bool etr = p.trace != nullptr && worker == workers / 2 && rank == 0 && tile == worker && threadIdx.x == 64;
       if (etr) p.trace[4] = clock64();
-      if (valid) {
-        ok = tc_staged_epilogue<KIND>(cfg, io, t_row, n0, row, threadIdx.x == 64, tile_bias, tile_bias, res_ph,
-                                      out_slot, abort_ptr);
-        if (!ok) break;
-      }
+      const int oy = oy0 + (row >> 3), ox = ox0 + (row & 7);
+      const bool inside = valid && oy < lp.OH && ox < lp.OW;
+      const long long at = (((static_cast<long long>(img) * lp.OH + oy) * lp.OW + ox)) * lp.N + n0 + c_first;
+      const int es = lp.out_mode == OUT_BF16X2 ? 2 : 4, rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
+      // (a warp's rows are four rows of eight pixels)
+      const long long warp_at = at - (static_cast<long long>(lane >> 3) * lp.OW + (lane & 7)) * lp.N;
+      d.o0 = reinterpret_cast<uint8_t*>(lp.out0) + warp_at * es;
+      d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + warp_at * es;
+      d.pitch = static_cast<long long>(lp.N) * es;
+      d.pitch8 = d.pitch * lp.OW;
+      d.rows = valid ? 32 : 0;
+      d.xs = lp.OW - ox0;
+      d.ys = lp.OH - (oy0 + 4 * quarter);
+      d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + at * rs;
+      d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + at * rs;
+      d.bias = lp.bias != nullptr ? lp.bias + n0 + c_first : nullptr;
+      tc_drain<KIND, false, false, false>(d, t_row + static_cast<uint32_t>(c_first), cols, lp.N - n0 - c_first, inside);
       if (etr) p.trace[5] = clock64();
       tc_fence_before_sync();
       __syncwarp();
@@ -393,7 +381,6 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
     if (!ok && lane == 0) {
       if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_EPILOGUE);
     }
-    if (threadIdx.x == 64) tma_store_wait_all();
   }
 
   // (a pair: neither CTA leaves while the other may still signal its barriers or read its shared memory)

@@ -60,7 +60,7 @@ struct TcDwProjParams {
   int stages;           // weight ring depth
   int patch_bufs;       // input patch ring depth, 2 or 4 (even: a slot then always serves the same depthwise group)
   int b_bytes;          // one plane of a weight stage, rounded to 1 KB
-  int out_bufs;
+  int wide;             // rows of result and residual are multiples of 32 bytes, 32-byte aligned
   const float* dw_weights;  // [9][C], tap-major
   const float* dw_bias;     // [C] or null
   int dw_act;
@@ -78,6 +78,10 @@ struct TcDwProjParams {
   const float* bias;        // projection bias [N] or null
   int res_mode, out_mode, act;
   float act_a, act_b;
+  float* out0;
+  float* out1;
+  const float* res0;
+  const float* res1;
   int* status;
 };
 
@@ -87,9 +91,7 @@ __global__ void __launch_bounds__(kDwpThreads, 1)
 tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_x1, const __grid_constant__ CUtensorMap map_e0,
                      const __grid_constant__ CUtensorMap map_e1,
-                     const __grid_constant__ CUtensorMap map_b0, const __grid_constant__ CUtensorMap map_b1,
-                     const __grid_constant__ CUtensorMap map_o0, const __grid_constant__ CUtensorMap map_o1,
-                     const __grid_constant__ CUtensorMap map_r0, const __grid_constant__ CUtensorMap map_r1) {
+                     const __grid_constant__ CUtensorMap map_b0, const __grid_constant__ CUtensorMap map_b1) {
   using namespace ptx;
   constexpr int TH = dwp_tile_h(STRIDE), TW = kDwpTileW;
   constexpr int PH = dwp_patch_h(STRIDE), PW = dwp_patch_w(STRIDE), NPX = PH * PW;
@@ -106,8 +108,6 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
   __shared__ __align__(8) uint64_t a_full[2], a_empty[2];
   __shared__ __align__(8) uint64_t b_full[kDwpMaxStages], b_empty[kDwpMaxStages];
   __shared__ __align__(8) uint64_t tfull_bar[2], tempty_bar[2];
-  __shared__ __align__(8) uint64_t res_bar;
-  __shared__ __align__(16) float tile_bias[256];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -125,11 +125,9 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
   const uint32_t b_bytes = static_cast<uint32_t>(p.b_bytes);
   const uint32_t b_stage_bytes = 2u * b_bytes + (EXPAND ? 2u * kExWeightBytes : 0u);  // (+ the block's expand weights)
   const int S = p.stages;
-  const uint32_t res_stage = b_base + static_cast<uint32_t>(S) * b_stage_bytes;
-  const uint32_t out_stage = res_stage + (p.res_mode != RES_NONE ? 16384u : 0u);
-  const bool wide_out = p.out_mode == OUT_BF16X2 || p.res_mode == RES_BF16X2;
   // the depthwise filter and bias of every channel, [10][c_blocks * 32] fp32 (taps 0..8, then the bias; zero past C)
-  const uint32_t table = out_stage + static_cast<uint32_t>(p.out_bufs) * (wide_out ? 16384u : 8192u);
+  const uint32_t drain = b_base + static_cast<uint32_t>(S) * b_stage_bytes;  // one block per epilogue warp
+  const uint32_t table = drain + 4u * kDrainWarpBytes;
   const int c_pad = p.c_blocks * kDwpChannels;
   // EXPAND: the expand layer's bias [c_pad] (zero past C)
   const uint32_t ex_table = table + static_cast<uint32_t>(10 * c_pad) * 4u;
@@ -160,12 +158,10 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
       mbar_init(smem_u32(&b_full[i]), 1);
       mbar_init(smem_u32(&b_empty[i]), 1);
     }
-    mbar_init(smem_u32(&res_bar), 1);
     fence_mbar_init();
     prefetch_tensormap(&map_x);
     prefetch_tensormap(&map_b0);
     prefetch_tensormap(&map_b1);
-    prefetch_tensormap(&map_o0);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&tmem_slot), kTcTmemCols);
@@ -401,22 +397,17 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
     // ------------------------------------------------------------ epilogue (warps 2-5)
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;  // accumulator row = pixel (row / 8, row % 8) of the tile
-    TcStageCfg cfg{};
-    cfg.bar_base = 1;
-    cfg.res_stage = res_stage;
-    cfg.out_stage = out_stage;
-    cfg.res_bar = smem_u32(&res_bar);
-    cfg.out_bufs = p.out_bufs;
-    cfg.out_mode = p.out_mode;
-    cfg.res_mode = p.res_mode;
-    cfg.act = p.act;
-    cfg.act_a = p.act_a;
-    cfg.act_b = p.act_b;
-    cfg.N = p.N;
-    cfg.block_n = p.block_n;
-    cfg.wide = wide_out ? 1 : 0;
-    int acc = 0, out_slot = 0;
-    uint32_t acc_ph = 0, res_ph = 0;
+    const TcDwProjParams lp = p;
+    TcDirect d{};
+    d.out_mode = p.out_mode;
+    d.res_mode = p.res_mode;
+    d.act = p.act;
+    d.act_a = p.act_a;
+    d.act_b = p.act_b;
+    d.wide = p.wide;
+    d.stage = drain + static_cast<uint32_t>(quarter) * kDrainWarpBytes;
+    int acc = 0;
+    uint32_t acc_ph = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       int img, oy0, ox0, n0;
@@ -426,26 +417,24 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
       if (!ok) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * acc_stride;
-      for (int t = static_cast<int>(threadIdx.x) - 64; t < p.block_n; t += 128) {
-        const int n = n0 + t;
-        tile_bias[t] = (p.bias != nullptr && n < p.N) ? __ldg(p.bias + n) : 0.0f;
-      }
-      // (the boxes of the output and residual maps are TH x TW pixels: of a stride-2 tile only the first 64
-      // staging rows leave)
-      struct {
-        const CUtensorMap *o0, *o1, *r0, *r1;
-        int x, y, img;
-        __device__ __forceinline__ void load_res(int plane, uint32_t dst, uint32_t bar, int col) const {
-          ptx::tma_load_4d(dst, plane ? r1 : r0, bar, col, x, y, img);
-        }
-        __device__ __forceinline__ void store_out(int plane, uint32_t src, int col) const {
-          ptx::tma_store_4d(plane ? o1 : o0, src, col, x, y, img);
-        }
-        __device__ __forceinline__ void store_side(int, uint32_t, int) const {}
-      } io{&map_o0, &map_o1, &map_r0, &map_r1, ox0, oy0, img};
-      ok = tc_staged_epilogue<KIND>(cfg, io, t_row, n0, row, threadIdx.x == 64, tile_bias, tile_bias, res_ph,
-                                           out_slot, abort_ptr);
-      if (!ok) break;
+      // (of a stride-2 tile only the first 64 rows are pixels)
+      const int oy = oy0 + (row >> 3), ox = ox0 + (row & 7);
+      const bool inside = row < TH * TW && oy < lp.H && ox < lp.W;
+      const long long at = ((static_cast<long long>(img) * lp.H + oy) * lp.W + ox) * lp.N + n0;
+      const int es = lp.out_mode == OUT_BF16X2 ? 2 : 4, rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
+      // (a warp's rows are four rows of eight pixels)
+      const long long warp_at = at - (static_cast<long long>(lane >> 3) * lp.W + (lane & 7)) * lp.N;
+      d.o0 = reinterpret_cast<uint8_t*>(lp.out0) + warp_at * es;
+      d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + warp_at * es;
+      d.pitch = static_cast<long long>(lp.N) * es;
+      d.pitch8 = d.pitch * lp.W;
+      d.rows = TH * TW - 32 * quarter;
+      d.xs = lp.W - ox0;
+      d.ys = lp.H - (oy0 + 4 * quarter);
+      d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + at * rs;
+      d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + at * rs;
+      d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
+      tc_drain<KIND, false, false, false>(d, t_row, lp.block_n, lp.N - n0, inside);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
@@ -455,7 +444,6 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
     if (!ok && lane == 0) {
       if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_EPILOGUE);
     }
-    if (threadIdx.x == 64) tma_store_wait_all();
   } else {
     // ------------------------------------------------------------ depthwise (warps 6-13, 256 threads)
     // Two groups of four warps take alternate channel blocks (group g: blocks g, g+2, ... of the CTA's sequence,

@@ -110,9 +110,38 @@ std::string encode_im2col(CUtensorMap* map, int kind, const void* base, const Tc
 // memory (barriers and per-tile constants: 1.2 KB, 2.2 KB for the int8 kernel with its
 // dequantisation factors), minus 1 KB of alignment slack.
 constexpr int tc_smem_budget(int kind) { return (kind == GEMM_I8 ? 223 : 224) * 1024; }
-// From this many K blocks per tile on, the main loop of the next tile hides even the slower
-// direct epilogue, and a third ring stage is worth more than the staging tiles.
-constexpr int kDirectEpilogueDepth = 32;
+constexpr int kDrainBytes = 8 * kDrainWarpBytes;  // shared memory of the eight epilogue warps
+
+int res_mode_of(const TcEpilogue& e) {
+  return e.res0 == nullptr ? RES_NONE : (e.res_bf16 ? RES_BF16X2 : (e.res1 != nullptr ? RES_SPLIT : RES_F32));
+}
+
+int out_elem_bytes(int out_mode) { return out_mode == OUT_I8 ? 1 : (out_mode == OUT_BF16X2 ? 2 : 4); }
+
+// True when tc_drain can write these results: rows (of `N` columns, `ldo` apart) made of 16-byte pieces in every format
+// that takes part.  *wide: of 32-byte pieces, so that stores and loads are whole sectors.
+bool direct_rows(int kind, const TcEpilogue& e, int N, int* wide) {
+  // (a residual of fp32 hi / lo planes takes part beside operands of that format only)
+  bool ok = kind == GEMM_TF32X3 || res_mode_of(e) != RES_SPLIT, all32 = true;
+  auto plane = [&](const void* p, int es) {
+    if (p == nullptr) return;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    ok = ok && at % 16 == 0 && e.ldo * es % 16 == 0 && static_cast<long long>(N) * es % 16 == 0;
+    all32 = all32 && at % 32 == 0 && e.ldo * es % 32 == 0;
+  };
+  if (e.out_mode == OUT_I8) {
+    plane(e.outq, 1);
+  } else if (e.out_mode != OUT_CHW) {
+    plane(e.out0, out_elem_bytes(e.out_mode));
+    plane(e.out1, out_elem_bytes(e.out_mode));
+  }
+  const int rs = e.res_bf16 ? 2 : 4;
+  plane(e.res0, rs);
+  plane(e.res1, rs);
+  for (int i = 0; i < e.side_count; ++i) plane(e.side_q[i], 1);
+  *wide = all32 ? 1 : 0;
+  return ok;
+}
 
 // Tile width: every multiple of 16 up to 128 is a legal UMMA N.  Cost model:
 // waves over the SMs times (columns computed + a fixed per-tile term for the
@@ -145,93 +174,16 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   p.M = static_cast<int>(M);
   p.N = N;
   p.tiles_m = static_cast<int>((M + kTcBlockM - 1) / kTcBlockM);
-  // a bf16-pair output or residual is staged 32 columns at a time
-  const int res_mode = e.res0 == nullptr ? RES_NONE : (e.res_bf16 ? RES_BF16X2 : (e.res1 != nullptr ? RES_SPLIT : RES_F32));
-  // Shallow contractions are bound by the epilogue: plain fp32 results then also go out 32 columns
-  // at a time (half as many barriers and store rounds per tile).
-  const bool shallow_f32 = e.out_mode == OUT_F32 && res_mode != RES_SPLIT && N % 16 == 0 && N >= 32 && p.k_blocks <= 4;
-  const bool wide = e.out_mode == OUT_BF16X2 || res_mode == RES_BF16X2 || shallow_f32;
-  // int8 results can leave through TMA stores in chunks of 64 columns when every tile is a
-  // multiple of 64 wide, rows are 16-byte multiples and nothing is added after requantisation
-  const bool i8_staged = e.out_mode == OUT_I8 && N % 64 == 0 && e.ldo % 16 == 0 && e.res0 == nullptr &&
-                         (reinterpret_cast<uintptr_t>(e.outq) & 15) == 0;
-  // int8 copies of an fp32 result (TcEpilogue::side_q) leave 64 columns at a time through staging tiles of
-  // their own (two [128][64] tiles per copy) when rows and tiles come in 64-channel units
-  const bool side_staged = e.side_count > 0 && e.out_mode != OUT_I8 && N % 64 == 0 && e.ldo % 16 == 0 &&
-                           (reinterpret_cast<uintptr_t>(e.side_q[0]) & 15) == 0 &&
-                           (reinterpret_cast<uintptr_t>(e.side_q[1]) & 15) == 0;
-  const int side_bytes = side_staged ? e.side_count * 16384 : 0;
-  p.block_n = choose_block_n(p.tiles_m, N, sm_count, (i8_staged || side_staged) ? 64 : (wide ? 32 : 16));
+  const int res_mode = res_mode_of(e);
+  p.direct = direct_rows(kind, e, N, &p.wide) ? 1 : 0;
+  p.block_n = choose_block_n(p.tiles_m, N, sm_count, 16);
   p.tiles_n = (N + p.block_n - 1) / p.block_n;
   const int kTcSmemBudget = tc_smem_budget(kind);
   const int planes = tc_planes(kind);
   // a stage holds the A tile(s) and block_n rows of B, every sub-buffer 1 KB aligned
   const int b_bytes = (p.block_n * p.row_bytes + 1023) / 1024 * 1024;
   p.stage_bytes = planes * (kTcBlockM * p.row_bytes + b_bytes);
-  // fp32 results leave through TMA stores when rows are 16-byte multiples; the staging
-  // tiles (out hi/lo, residual hi/lo, 8 KB each) sit behind the ring
-  const bool f32_out = e.out_mode != OUT_I8;
-  const bool aligned = e.ldo % (wide ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(e.out0) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(e.out1) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(e.res0) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(e.res1) & 15) == 0;
-  // (a wide chunk cannot carry fp32 hi/lo planes: that pairing does not occur, the direct path covers it)
-  p.tma_store = f32_out && aligned && !(wide && (e.out_mode == OUT_F32_SPLIT || e.out_mode == OUT_F32_TF32 ||
-                                                  res_mode == RES_SPLIT))
-                    ? 1
-                    : 0;
-  if (i8_staged) p.tma_store = 1;
-  // residual tiles (16 KB) + two to four output tiles of 8 KB per plane; fewer when the
-  // operand ring would drop below three stages
-  const int out_tile = (e.out_mode != OUT_I8 && (e.out_mode == OUT_F32_SPLIT || wide) ? 2 : 1) * 8192;
-  int staging = 0;
-  p.out_bufs = 2;
-  if (p.tma_store) {
-    for (int bufs : {4, 3, 2}) {
-      p.out_bufs = bufs;
-      staging = ((res_mode != RES_NONE ? 16384 : 0) + side_bytes) + bufs * out_tile;
-      if ((kTcSmemBudget - staging) / p.stage_bytes >= 3 || bufs == 2) break;
-    }
-    // Deep contractions hide even a slow epilogue behind the next tile's main loop; there a third
-    // ring stage is worth more than the staging tiles.  With one tile per CTA nothing hides the
-    // epilogue, and the direct one takes several times as long as the staged one.
-    const int with = (kTcSmemBudget - staging) / p.stage_bytes;
-    const int without = (kTcSmemBudget) / p.stage_bytes;
-    const long long tiles_all = static_cast<long long>(p.tiles_m) * p.tiles_n;
-    if (with < 3 && without >= 3 && p.k_blocks >= kDirectEpilogueDepth && tiles_all > sm_count) {
-      p.tma_store = 0;
-      staging = 0;
-    }
-  }
-  // Shallow contractions (a few K blocks per tile) are bound by the epilogue, which runs one warp
-  // per scheduler and so pays every instruction's latency in full: a second epilogue group drains
-  // every other tile, with a staging area of its own.  Two groups with two staging tiles each beat
-  // one group with four, so the tile count per group is reduced before the second group is given up.
   const long long tiles_total = static_cast<long long>(p.tiles_m) * p.tiles_n;
-  // The same holds for deeper contractions whose K blocks are cheap (int8: a K block is 128 channels
-  // and one or two MMAs): estimate both sides per tile, in cycles, from measured figures -- about 1800
-  // cycles per fp32 chunk and 3000 per 64-column int8 chunk in the epilogue; per K block the larger of
-  // the MMA issue time and the operand fetch at 45 bytes per cycle.
-  const int chunk_cols = e.out_mode == OUT_I8 ? 64 : (wide ? 32 : 16);
-  const double epi_cycles = static_cast<double>((p.block_n + chunk_cols - 1) / chunk_cols) * (e.out_mode == OUT_I8 ? 3000.0 : 1800.0);
-  const double mma_cycles = (planes == 2 ? 3.0 : 1.0) * (p.row_bytes / 32) * (p.block_n <= 64 ? 48.0 : 64.0 * p.block_n / 128.0);
-  const double main_cycles = p.k_blocks * std::max(mma_cycles, p.stage_bytes / 45.0);
-  const bool epilogue_bound = env_int("NCNN_B200_EPI2", 1) != 0 && epi_cycles > 1.2 * main_cycles;
-  p.epi_groups = 1;
-  if (p.tma_store && (p.k_blocks <= 4 || epilogue_bound) && tiles_total >= 2ll * sm_count) {
-    const int res_bytes = (res_mode != RES_NONE ? 16384 : 0) + side_bytes;
-    for (int bufs : {4, 3, 2}) {
-      const int both = 2 * (res_bytes + bufs * out_tile);
-      if (bufs > p.out_bufs) continue;
-      // (a tile of one or two K blocks needs no more than the next tile's operands in flight)
-      if ((kTcSmemBudget - both) / p.stage_bytes >= (bufs == 2 ? (p.k_blocks <= 2 ? 2 : 3) : 4)) {
-        p.epi_groups = 2;
-        p.out_bufs = bufs;
-        staging = both;
-        break;
-      }
-    }
-  }
   // Paired tiles: two 128-row halves share every B tile, so a K block moves 256 + block_n operand
   // rows for twice the output instead of 2 x (128 + block_n).  Worth it where the operand fetch sets
   // the pace (deep contractions over full 128-byte rows; the stem's 64-byte window rows ran 9%
@@ -239,17 +191,8 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   // (larger) stages.
   p.pair = 0;
   p.pair_rows = 0;
-  if (pair_enabled() && p.tma_store && p.epi_groups == 1 && p.k_blocks >= 6 && p.block_n <= 128 &&
-      p.row_bytes >= 128) {
+  if (pair_enabled() && p.k_blocks >= 6 && p.block_n <= 128 && p.row_bytes >= 128) {
     const int pair_stage = planes * (2 * kTcBlockM * p.row_bytes + b_bytes);
-    // as many output tiles as still leave two stages (the leader waits less for stores to drain)
-    int pair_bufs = 2;
-    for (int bufs : {4, 3})
-      if ((kTcSmemBudget - ((res_mode != RES_NONE ? 16384 : 0) + side_bytes) - bufs * out_tile) / pair_stage >= 2) {
-        pair_bufs = bufs;
-        break;
-      }
-    const int pair_staging = ((res_mode != RES_NONE ? 16384 : 0) + side_bytes) + pair_bufs * out_tile;
     const long long waves_single = (tiles_total + sm_count - 1) / sm_count;
     const double cost_single = static_cast<double>(waves_single) * (kTcBlockM + p.block_n);
     // whole waves of pairs first, single tiles for what is left; k waves of pairs cover
@@ -272,17 +215,14 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
     }
     const long long tiles_mixed = static_cast<long long>(p.tiles_m - best_rows) * p.tiles_n;
     if (best_rows > 0 && best < 0.97 * cost_single && tiles_mixed * 10 >= 9ll * sm_count &&
-        (kTcSmemBudget - pair_staging) / pair_stage >= 2) {
+        (kTcSmemBudget - kDrainBytes) / pair_stage >= 2) {
       p.pair = 1;
       p.pair_rows = best_rows;
       p.tiles_m = p.tiles_m - best_rows;  // tile rows: best_rows pairs, then singles
       p.stage_bytes = pair_stage;
-      p.out_bufs = pair_bufs;
-      staging = pair_staging;
     }
   }
-  p.staging_bytes = staging / p.epi_groups;
-  const int budget = kTcSmemBudget - staging;
+  const int budget = kTcSmemBudget - kDrainBytes;
   // int8 K blocks are two to four MMAs over 12-32 KB: arming and releasing a ring stage (~450 cycles of barrier
   // hand-shake per block, more than the block's copies and MMAs take) sets the pace.  A stage then holds several
   // K blocks (a divisor of their count, at least three stages deep): one hand-shake for all of them.
@@ -294,7 +234,7 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
         break;
       }
   p.stages = std::max(2, std::min(kTcMaxStages, budget / (p.sub_blocks * p.stage_bytes)));
-  L->smem_bytes = p.stages * p.sub_blocks * p.stage_bytes + staging + 1024;
+  L->smem_bytes = p.stages * p.sub_blocks * p.stage_bytes + kDrainBytes + 1024;
   // never fewer bytes than half an SM's shared memory: two CTAs must not share an
   // SM, each allocates tensor memory for itself
   L->smem_bytes = std::max(L->smem_bytes, 120 * 1024);
@@ -309,7 +249,6 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   p.res0 = e.res0;
   p.res1 = e.res1;
   p.res_mode = res_mode;
-  p.wide = wide ? 1 : 0;
   p.ldo = e.ldo;
   p.out_mode = e.out_mode;
   p.act = e.act;
@@ -318,14 +257,12 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   p.out_scale = e.out_scale;
   p.status = e.status;
   p.trace = e.trace;
-  p.side_staged = side_staged && p.tma_store ? 1 : 0;
   p.side_count = e.side_count;
   p.side_ld = e.ldo;
   p.side_q0 = e.side_q[0];
   p.side_q1 = e.side_q[1];
   p.side_scale0 = e.side_scale[0];
   p.side_scale1 = e.side_scale[1];
-  L->map_o0 = L->map_o1 = L->map_r0 = L->map_r1 = L->map_s0 = L->map_s1 = CUtensorMap{};
 }
 
 // ---- CTA pairs (tc_gemm2.cuh)
@@ -402,21 +339,11 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   TcGemmParams& p = L->p;
   if (env_int("NCNN_B200_CTA2", 1) == 0 || sm_count < 2) return false;
   if (p.k_blocks < env_int("NCNN_B200_CTA2_MIN_KB", 6)) return false;
-  const int res_mode = e.res0 == nullptr ? RES_NONE : (e.res_bf16 ? RES_BF16X2 : (e.res1 != nullptr ? RES_SPLIT : RES_F32));
-  const bool wide = e.out_mode == OUT_BF16X2 || res_mode == RES_BF16X2;
-  const bool i8_staged = e.out_mode == OUT_I8 && N % 64 == 0 && e.ldo % 16 == 0 && e.res0 == nullptr &&
-                         (reinterpret_cast<uintptr_t>(e.outq) & 15) == 0;
-  const bool f32_out = e.out_mode != OUT_I8;
-  const bool aligned = e.ldo % (wide ? 8 : 4) == 0 && (reinterpret_cast<uintptr_t>(e.out0) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(e.out1) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(e.res0) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(e.res1) & 15) == 0;
-  const bool staged = i8_staged || (f32_out && aligned &&
-                                    !(wide && (e.out_mode == OUT_F32_SPLIT || e.out_mode == OUT_F32_TF32 ||
-                                               res_mode == RES_SPLIT)));
-  if (!staged) return false;  // this kernel has the staged epilogue only
+  const int res_mode = res_mode_of(e);
+  p.direct = direct_rows(kind, e, N, &p.wide) ? 1 : 0;
+  if (!p.direct || e.out_mode == OUT_CHW) return false;  // this kernel drains dense rows only
   if (e.side_count > 0) return false;  // int8 copies of the result: the one-CTA kernel writes those
-  const int step = i8_staged ? 64 : (wide ? 32 : 16);
+  const int step = 16;
   auto even_width = [&](int widest) {
     const int n_tiles = (N + widest - 1) / widest;
     return ((N + n_tiles - 1) / n_tiles + step - 1) / step * step;
@@ -464,60 +391,28 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   p.tiles_n = (N + p.block_n - 1) / p.block_n;
   const int budget_all = tc_smem_budget(kind);
   const int planes = tc_planes(kind);
-  p.tma_store = 1;
-  const int out_tile = (e.out_mode != OUT_I8 && (e.out_mode == OUT_F32_SPLIT || wide) ? 2 : 1) * 8192;
-  const int res_bytes = res_mode != RES_NONE ? 16384 : 0;
-  // Choose epilogue groups, K-block size and staging tiles.  Two groups (each half of the columns) come
-  // first: the epilogue of a wide tile is what a worker with one or two tiles cannot hide.  Then full-size
-  // K blocks, then as many staging tiles as leave the ring deep enough to cover the copy latency.
-  const bool two_groups_ok = env_int("NCNN_B200_CTA2_GROUPS", 2) >= 2 && p.block_n >= 128 && (p.block_n / 2) % step == 0;
+  // Full-size K blocks with a ring deep enough to cover the copy latency, else half-size ones.
   const int full_rb = p.row_bytes, full_cb = p.c_blocks, full_ke = p.k_elems;
-  bool chosen = false;
-  int staging = 0;
-  auto try_config = [&](int groups, bool half_blocks, int bufs, int min_stages) {
+  auto try_config = [&](bool half_blocks, int min_stages) {
     const int rb = half_blocks ? full_rb / 2 : full_rb;
     const int b_bytes = ((p.block_n / ctas) * rb + 1023) / 1024 * 1024;
     const int stage = planes * (kTcBlockM * rb + b_bytes);
-    const int stg = groups * (res_bytes + bufs * out_tile);
-    const int stages = std::min(kTcMaxStages, (budget_all - stg) / stage);
+    const int stages = std::min(kTcMaxStages, (budget_all - kDrainBytes) / stage);
     if (stages < min_stages) return false;
-    p.epi_groups = groups;
-    p.out_bufs = bufs;
     p.row_bytes = rb;
     p.k_elems = half_blocks ? full_ke / 2 : full_ke;
     p.c_blocks = half_blocks ? full_cb * 2 : full_cb;
     p.k_blocks = half_blocks ? full_kb * 2 : full_kb;
     p.stage_bytes = stage;
     p.stages = stages;
-    staging = stg;
     return true;
   };
   const bool halves = half_blocks_ok && full_rb == 128 && kind == GEMM_BF16X3;
-  for (int groups : {2, 1}) {
-    if (groups == 2 && !two_groups_ok) continue;
-    for (int hb = 0; hb < 2 && !chosen; ++hb) {
-      if (hb == 1 && !halves) continue;
-      for (int bufs : {4, 3, 2})
-        if (!chosen && try_config(groups, hb == 1, bufs, hb ? 4 : 3)) chosen = true;
-    }
-    if (chosen) break;
-  }
-  // last resort: one group, one or two staging tiles, two stages
-  if (!chosen)
-    for (int bufs : {2, 1})
-      if (!chosen && (bufs >= 2 || e.out_mode != OUT_I8) && try_config(1, false, bufs, 2)) chosen = true;
-  if (!chosen) {
-    p.row_bytes = full_rb;
-    p.k_elems = full_ke;
-    p.c_blocks = full_cb;
-    p.k_blocks = full_kb;
-    return false;
-  }
+  if (!try_config(false, 3) && !(halves && try_config(true, 4)) && !try_config(false, 2)) return false;
   p.pair = 0;
   p.pair_rows = 0;
   p.sub_blocks = 1;
-  p.staging_bytes = staging / p.epi_groups;
-  L->smem_bytes = std::max(p.stages * p.stage_bytes + staging + 1024, 120 * 1024);
+  L->smem_bytes = std::max(p.stages * p.stage_bytes + kDrainBytes + 1024, 120 * 1024);
   L->kind = kind;
   L->cta2 = ctas;
   // workers: one per TPC (pairs) or per SM, all resident at once
@@ -525,6 +420,7 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   if (workers < 1) return false;
   const long long tiles = static_cast<long long>(p.tiles_m) * p.tiles_n;
   const long long units = tiles * p.k_blocks;
+  if (forced_split == 1) workers = static_cast<int>(std::max<long long>(1, std::min<long long>(workers, units / 4)));
   // Splitting tiles pays when whole tiles leave SMs idle in the last wave; the worker that finishes a
   // split tile spends about three K blocks' time on the partial sums.
   const double cost_whole = static_cast<double>((tiles + workers - 1) / workers) * p.k_blocks;
@@ -561,7 +457,6 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   p.res0 = e.res0;
   p.res1 = e.res1;
   p.res_mode = res_mode;
-  p.wide = wide ? 1 : 0;
   p.ldo = e.ldo;
   p.out_mode = e.out_mode;
   p.act = e.act;
@@ -570,67 +465,13 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   p.out_scale = e.out_scale;
   p.status = e.status;
   p.trace = e.trace;
-  p.side_staged = 0;  // (this kernel stores the int8 copies thread by thread)
   p.side_count = e.side_count;
   p.side_ld = e.ldo;
   p.side_q0 = e.side_q[0];
   p.side_q1 = e.side_q[1];
   p.side_scale0 = e.side_scale[0];
   p.side_scale1 = e.side_scale[1];
-  L->map_o0 = L->map_o1 = L->map_r0 = L->map_r1 = CUtensorMap{};
   return true;
-}
-
-// [M][N] plane seen as a 2-D tensor (N innermost) with boxes of 64 bytes (16 fp32 or 32 bf16)
-// x 128 rows, 64-byte swizzle
-std::string encode_plane(CUtensorMap* map, const void* base, long long M, int N, long long ld, bool bf16) {
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * (bf16 ? 2 : 4)};
-  const cuuint32_t box[2] = {bf16 ? 32u : 16u, static_cast<cuuint32_t>(kTcBlockM)};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  const CUresult r = g_encode_tiled(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-                                    const_cast<void*>(base),
-                                    dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                    CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    return "cuTensorMapEncodeTiled failed for an output plane with code " + std::to_string(static_cast<int>(r));
-  return {};
-}
-
-std::string encode_epilogue_maps(TcLaunch* L, const TcEpilogue& e) {
-  if (!L->p.tma_store) return {};
-  if (e.out_mode == OUT_I8) {
-    // [M][N] int8 plane, boxes of 64 columns x 128 rows, 64-byte swizzle
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(L->p.N), static_cast<cuuint64_t>(L->p.M)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(e.ldo)};
-    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(kTcBlockM)};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    const CUresult r = g_encode_tiled(&L->map_o0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, e.outq, dims, strides, box,
-                                      elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-      return "cuTensorMapEncodeTiled failed for an int8 output plane with code " + std::to_string(static_cast<int>(r));
-    return {};
-  }
-  const bool ob = e.out_mode == OUT_BF16X2;
-  std::string err = encode_plane(&L->map_o0, e.out0, L->p.M, L->p.N, e.ldo, ob);
-  if (err.empty() && (e.out_mode == OUT_F32_SPLIT || ob))
-    err = encode_plane(&L->map_o1, e.out1, L->p.M, L->p.N, e.ldo, ob);
-  if (err.empty() && e.res0 != nullptr) err = encode_plane(&L->map_r0, e.res0, L->p.M, L->p.N, e.ldo, e.res_bf16);
-  if (err.empty() && e.res1 != nullptr) err = encode_plane(&L->map_r1, e.res1, L->p.M, L->p.N, e.ldo, e.res_bf16);
-  for (int i = 0; i < e.side_count && err.empty() && L->p.side_staged; ++i) {
-    // [M][N] int8 plane, boxes of 64 columns x 128 rows, 64-byte swizzle
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(L->p.N), static_cast<cuuint64_t>(L->p.M)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(e.ldo)};
-    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(kTcBlockM)};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    const CUresult r = g_encode_tiled(i ? &L->map_s1 : &L->map_s0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, e.side_q[i], dims,
-                                      strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) err = "cuTensorMapEncodeTiled failed for an int8 copy of the result with code " + std::to_string(static_cast<int>(r));
-  }
-  return err;
 }
 
 }  // namespace
@@ -702,7 +543,7 @@ std::string tc_plan_conv(TcLaunch* L, int kind, const TcIm2colView& v, const voi
   } else {
     L->map_b1 = L->map_b0;
   }
-  return encode_epilogue_maps(L, e);
+  return {};
 }
 
 std::string tc_plan_gemm(TcLaunch* L, int kind, const void* a0, const void* a1, long long M, int K,
@@ -743,7 +584,7 @@ std::string tc_plan_gemm(TcLaunch* L, int kind, const void* a0, const void* a1, 
   } else {
     L->map_b1 = L->map_b0;
   }
-  return encode_epilogue_maps(L, e);
+  return {};
 }
 
 namespace {
@@ -771,7 +612,7 @@ cudaError_t prepare_worker_kernels() {
 
 template <int KIND>
 int pairs_resident(int smem_bytes, int sm_count) {
-  KernelLaunchConfig wc(sm_count / 2 * 2, kTc2ThreadsTwoEpi, smem_bytes, true, nullptr);
+  KernelLaunchConfig wc(sm_count / 2 * 2, kTc2Threads, smem_bytes, true, nullptr);
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, tc_gemm2_kernel<KIND, true>, &wc.cfg) != cudaSuccess) {
     cudaGetLastError();
@@ -799,12 +640,10 @@ int max_pairs_resident(int kind, int smem_bytes, int sm_count) {
 template <int KIND>
 cudaError_t launch_workers(const TcLaunch& L, cudaStream_t stream) {
   const bool pair = L.cta2 == 2;
-  KernelLaunchConfig wc(L.grid, L.p.epi_groups == 2 ? kTc2ThreadsTwoEpi : kTc2Threads, L.smem_bytes, pair, stream);
+  KernelLaunchConfig wc(L.grid, kTc2Threads, L.smem_bytes, pair, stream);
   if (pair)
-    return cudaLaunchKernelEx(&wc.cfg, tc_gemm2_kernel<KIND, true>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1,
-                              L.map_o0, L.map_o1, L.map_r0, L.map_r1);
-  return cudaLaunchKernelEx(&wc.cfg, tc_gemm2_kernel<KIND, false>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1,
-                            L.map_o0, L.map_o1, L.map_r0, L.map_r1);
+    return cudaLaunchKernelEx(&wc.cfg, tc_gemm2_kernel<KIND, true>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  return cudaLaunchKernelEx(&wc.cfg, tc_gemm2_kernel<KIND, false>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
 }
 
 cudaError_t tc_launch_workers(const TcLaunch& L, cudaStream_t stream) {
@@ -844,29 +683,24 @@ cudaError_t tc_launch(const TcLaunch& L, cudaStream_t stream) {
     return e;
   });
   if (attr_err != cudaSuccess) return attr_err;
-  KernelLaunchConfig lc(L.grid, L.p.epi_groups == 2 ? kTcThreadsTwoEpi : kTcThreads, L.smem_bytes, false, stream);
+  KernelLaunchConfig lc(L.grid, kTcThreads, L.smem_bytes, false, stream);
   cudaError_t e;
   switch (L.kind) {
     case GEMM_TF32:
-      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_TF32>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                             L.map_o1, L.map_r0, L.map_r1, L.map_s0, L.map_s1);
+      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_TF32>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
       break;
     case GEMM_TF32X3:
-      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_TF32X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                             L.map_o1, L.map_r0, L.map_r1, L.map_s0, L.map_s1);
+      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_TF32X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
       break;
     case GEMM_BF16X3:
-      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_BF16X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                             L.map_o1, L.map_r0, L.map_r1, L.map_s0, L.map_s1);
+      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_BF16X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
       break;
     default:
       // (int8 copies of an fp32 result are written by an instantiation of its own)
       if (L.p.side_count > 0)
-        e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_I8, true>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                               L.map_o1, L.map_r0, L.map_r1, L.map_s0, L.map_s1);
+        e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_I8, true>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
       else
-        e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_I8>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                               L.map_o1, L.map_r0, L.map_r1, L.map_s0, L.map_s1);
+        e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_I8>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
       break;
   }
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -915,11 +749,9 @@ std::string tc_plan_conv_halo(TcHaloLaunch* L, int kind, const TcHaloConv& c, co
   std::memset(&p, 0, sizeof(p));
   const int planes = tc_planes(kind);
   const bool a_bf16 = kind == GEMM_BF16X3;
-  const int res_mode = e.res0 == nullptr ? RES_NONE : (e.res_bf16 ? RES_BF16X2 : (e.res1 != nullptr ? RES_SPLIT : RES_F32));
-  const bool out_bf16 = e.out_mode == OUT_BF16X2;
-  const bool wide = out_bf16 || res_mode == RES_BF16X2;
-  if (wide && (e.out_mode == OUT_F32_SPLIT || e.out_mode == OUT_F32_TF32 || res_mode == RES_SPLIT))
-    return "fp32 hi/lo planes cannot be staged together with a bf16-pair tensor";
+  const int res_mode = res_mode_of(e);
+  if (e.out_mode == OUT_CHW || e.out_mode == OUT_I8 || e.side_count > 0 || !direct_rows(kind, e, c.out_channels, &p.wide))
+    return "the patch-resident kernel writes channel-last rows of 16-byte pieces";
   if (e.ldo != c.out_channels) return "the patch-resident kernel writes dense channel-last rows";
   p.images = c.images;
   p.OH = c.OH;
@@ -928,7 +760,7 @@ std::string tc_plan_conv_halo(TcHaloLaunch* L, int kind, const TcHaloConv& c, co
   p.tiles_y = (c.OH + kHaloTileH - 1) / kHaloTileH;
   p.tiles_x = (c.OW + kHaloTileW - 1) / kHaloTileW;
   // an MMA of any N <= 128 costs the same issue time: take the widest tile
-  const int step = wide ? 32 : 16;
+  const int step = pair ? 32 : 16;
   const int widest = pair ? 256 : 128;  // a pair's CTA holds half of the weight rows of a tap
   {
     const int n_tiles = (c.out_channels + widest - 1) / widest;
@@ -950,24 +782,22 @@ std::string tc_plan_conv_halo(TcHaloLaunch* L, int kind, const TcHaloConv& c, co
   p.b_bytes = ((p.block_n / ctas) * 128 + 1023) / 1024 * 1024;
   p.bias = e.bias;
   p.res_mode = res_mode;
+  p.out0 = e.out0;
+  p.out1 = e.out1;
+  p.res0 = e.res0;
+  p.res1 = e.res1;
   p.out_mode = e.out_mode;
   p.act = e.act;
   p.act_a = e.act_a;
   p.act_b = e.act_b;
   p.status = e.status;
   p.trace = e.trace;
-  const int out_tile = (e.out_mode == OUT_F32_SPLIT || wide ? 2 : 1) * 8192;
-  const int fixed = 2 * planes * p.patch_bytes + (res_mode != RES_NONE ? 16384 : 0);
-  p.out_bufs = 4;
-  const int kTcSmemBudget = 222 * 1024;  // the halo kernel's own static shared memory is ~2 KB
-  p.stages = (kTcSmemBudget - fixed - p.out_bufs * out_tile) / (planes * p.b_bytes);
-  if (p.stages < 4) {
-    p.out_bufs = 2;
-    p.stages = (kTcSmemBudget - fixed - p.out_bufs * out_tile) / (planes * p.b_bytes);
-  }
+  const int fixed = 2 * planes * p.patch_bytes + kDrainBytes;
+  const int kTcSmemBudget = 224 * 1024;
+  p.stages = (kTcSmemBudget - fixed) / (planes * p.b_bytes);
   p.stages = std::min(p.stages, kTcMaxStages);
   if (p.stages < 2) return "shared memory cannot hold the patch buffers and two weight stages";
-  L->smem_bytes = fixed + p.out_bufs * out_tile + p.stages * planes * p.b_bytes + 1024;
+  L->smem_bytes = fixed + p.stages * planes * p.b_bytes + 1024;
   L->smem_bytes = std::max(L->smem_bytes, 120 * 1024);
   const long long pixel_tiles = static_cast<long long>(c.images) * p.tiles_y * p.tiles_x;
   const long long tiles = ((pixel_tiles + ctas - 1) / ctas) * p.tiles_n;
@@ -988,15 +818,6 @@ std::string tc_plan_conv_halo(TcHaloLaunch* L, int kind, const TcHaloConv& c, co
     err = encode_tiled_2d(&L->map_b1, kind, c.w1, k_total, c.out_channels, k_total * tc_elem_bytes(kind), p.k_elems,
                           p.block_n / ctas, 128);
   if (!err.empty()) return err;
-  // outputs and residuals: [image][OH][OW][N], tiles of 64 bytes of channels x 8 x 16 pixels, 64-byte swizzle
-  auto plane = [&](CUtensorMap* map, const void* base, bool bf16) {
-    return encode_tiled_4d(map, bf16, base, c.out_channels, c.OW, c.OH, c.images, bf16 ? 32 : 16, kHaloTileW,
-                           kHaloTileH, CU_TENSOR_MAP_SWIZZLE_64B);
-  };
-  err = plane(&L->map_o0, e.out0, out_bf16);
-  if (err.empty() && (e.out_mode == OUT_F32_SPLIT || out_bf16)) err = plane(&L->map_o1, e.out1, out_bf16);
-  if (err.empty() && e.res0 != nullptr) err = plane(&L->map_r0, e.res0, e.res_bf16);
-  if (err.empty() && e.res1 != nullptr) err = plane(&L->map_r1, e.res1, e.res_bf16);
   return err;
 }
 
@@ -1027,8 +848,7 @@ cudaError_t tc_launch_halo(const TcHaloLaunch& L, cudaStream_t stream) {
   KernelLaunchConfig lc(L.grid, kHaloThreads, L.smem_bytes, L.pair != 0, stream);
   cudaError_t e;
 #define NB_LAUNCH_HALO(KIND, PAIRED)                                                                             \
-  e = cudaLaunchKernelEx(&lc.cfg, tc_conv_halo_kernel<KIND, PAIRED>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, \
-                         L.map_o0, L.map_o1, L.map_r0, L.map_r1)
+  e = cudaLaunchKernelEx(&lc.cfg, tc_conv_halo_kernel<KIND, PAIRED>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1)
   if (L.kind == GEMM_BF16X3) {
     if (L.pair) NB_LAUNCH_HALO(GEMM_BF16X3, true);
     else NB_LAUNCH_HALO(GEMM_BF16X3, false);
@@ -1047,7 +867,7 @@ cudaError_t tc_launch_halo(const TcHaloLaunch& L, cudaStream_t stream) {
 namespace {
 
 struct DwProjShape {
-  int block_n = 0, tiles_n = 0, stages = 0, out_bufs = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, smem = 0;
+  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, smem = 0;
   bool ok = false;
 };
 
@@ -1056,27 +876,25 @@ struct DwProjShape {
 // every ring stage, the expand bias beside the depthwise table).
 DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int stride, bool expand, int cin = 32) {
   DwProjShape r;
-  const bool wide = out_mode == OUT_BF16X2 || res_mode == RES_BF16X2;
   if (out_mode != OUT_BF16X2 && out_mode != OUT_F32) return r;
-  if (wide && res_mode == RES_SPLIT) return r;
+  if (res_mode == RES_SPLIT) return r;
   if (stride != 1 && stride != 2) return r;
   if (stride == 2 && !expand) return r;  // (patches loaded by TMA are built for stride 1 only)
-  const int step = wide ? 32 : 16;
+  const int step = 16;
   const int n_tiles = (N + 255) / 256;
   r.block_n = ((N + n_tiles - 1) / n_tiles + step - 1) / step * step;
   if (r.block_n > 256 || r.block_n % 16 != 0) return r;
   if (expand && r.block_n > 128) return r;  // (the expand accumulators take the TMEM columns past two 128-column ones)
   r.tiles_n = (N + r.block_n - 1) / r.block_n;
   r.b_bytes = (r.block_n * 64 + 1023) / 1024 * 1024;
-  const int out_tile = wide ? 16384 : 8192;
-  const int budget = 222 * 1024;  // the kernel's own static shared memory is ~2 KB
+  const int budget = 224 * 1024;  // the kernel's own static shared memory is ~2 KB
   const int c_pad = (C + kDwpChannels - 1) / kDwpChannels * kDwpChannels;
   const int table = (c_pad * (expand ? 11 : 10) * 4 + 1023) / 1024 * 1024;  // depthwise filter and bias (+ expand bias)
   const int stage = 2 * r.b_bytes + (expand ? 4096 : 0);
   r.x_row_bytes = cin <= 16 ? 32 : 64;
   r.x_plane_bytes = expand ? (dwp_patch_pixels(stride) * r.x_row_bytes + 1023) / 1024 * 1024 : 0;
-  // Deep patch ring first (a patch load outlasts one block's arithmetic), then three weight stages, then
-  // output staging tiles; the last resort is two of each.  With the expand layer: two input patch buffers if they
+  // Deep patch ring first (a patch load outlasts one block's arithmetic), then three weight stages; the last
+  // resort is two of each.  With the expand layer: two input patch buffers if they
   // fit, and never fewer than three stages (the expand MMAs run two blocks ahead of the projection's).
   for (int min_stages : {4, 3, 2}) {
     if (expand ? min_stages < 3 : min_stages > 3) continue;  // (without the expand layer three stages are plenty)
@@ -1089,20 +907,16 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int strid
       // patch, about once in 10^5 loads with the L2 flushed)
       for (int patches : {4, 2}) {
         if (expand && patches != 2) continue;
-        for (int bufs : {4, 3, 2}) {
-          if (expand && bufs == 4) continue;
-          const int fixed = (expand ? x_bufs * 2 * r.x_plane_bytes : 0) + patches * dwp_patch_bytes(stride) +
-                            2 * 2 * dwp_a_plane_bytes(stride) + (res_mode != RES_NONE ? 16384 : 0) + table;
-          const int stages = std::min(kDwpMaxStages, (budget - fixed - bufs * out_tile) / stage);
-          if (stages >= min_stages) {
-            r.stages = stages;
-            r.out_bufs = bufs;
-            r.patches = patches;
-            r.x_bufs = expand ? x_bufs : 0;
-            r.smem = fixed + bufs * out_tile + stages * stage + 1024;
-            r.ok = true;
-            return r;
-          }
+        const int fixed = (expand ? x_bufs * 2 * r.x_plane_bytes : 0) + patches * dwp_patch_bytes(stride) +
+                          2 * 2 * dwp_a_plane_bytes(stride) + 4 * kDrainWarpBytes + table;
+        const int stages = std::min(kDwpMaxStages, (budget - fixed) / stage);
+        if (stages >= min_stages) {
+          r.stages = stages;
+          r.patches = patches;
+          r.x_bufs = expand ? x_bufs : 0;
+          r.smem = fixed + stages * stage + 1024;
+          r.ok = true;
+          return r;
         }
       }
     }
@@ -1146,7 +960,8 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   if (!g_driver_error.empty()) return g_driver_error;
   TcDwProjParams& p = L->p;
   std::memset(&p, 0, sizeof(p));
-  const int res_mode = e.res0 == nullptr ? RES_NONE : (e.res_bf16 ? RES_BF16X2 : (e.res1 != nullptr ? RES_SPLIT : RES_F32));
+  const int res_mode = res_mode_of(e);
+  if (!direct_rows(GEMM_BF16X3, e, c.out_channels, &p.wide)) return "the fused depthwise + projection kernel writes rows of 16-byte pieces";
   const bool expand = c.ex_w0 != nullptr;
   const int stride = c.stride;
   const DwProjShape shape = dw_project_shape(c.out_channels, e.out_mode, res_mode, c.C, stride, expand, expand ? c.Cin : 32);
@@ -1156,7 +971,6 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   if ((reinterpret_cast<uintptr_t>(c.x) & 15) != 0 || (static_cast<size_t>(x_channels) * (expand ? 2 : 4)) % 16 != 0 ||
       (expand && (c.x1 == nullptr || (reinterpret_cast<uintptr_t>(c.x1) & 15) != 0)))
     return "input rows of the fused kernel must be 16-byte aligned";
-  const bool out_bf16 = e.out_mode == OUT_BF16X2;
   const int th = dwp_tile_h(stride);
   p.images = c.images;
   p.H = c.H;
@@ -1175,7 +989,6 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   p.stages = shape.stages;
   p.patch_bufs = shape.patches;
   p.b_bytes = shape.b_bytes;
-  p.out_bufs = shape.out_bufs;
   p.dw_weights = c.dw_weights;
   p.dw_bias = c.dw_bias;
   p.dw_act = c.dw_act;
@@ -1192,6 +1005,10 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   p.ex_act_b = c.ex_act_b;
   p.bias = e.bias;
   p.res_mode = res_mode;
+  p.out0 = e.out0;
+  p.out1 = e.out1;
+  p.res0 = e.res0;
+  p.res1 = e.res1;
   p.out_mode = e.out_mode;
   p.act = e.act;
   p.act_a = e.act_a;
@@ -1223,14 +1040,6 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   if (err.empty())
     err = encode_tiled_2d(&L->map_b1, GEMM_BF16X3, c.w1, k_total, c.out_channels, k_total * 2, kDwpChannels, p.block_n, 64);
   if (!err.empty()) return err;
-  auto plane = [&](CUtensorMap* map, const void* base, bool bf16) {
-    return encode_tiled_4d(map, bf16, base, c.out_channels, c.W, c.H, c.images, bf16 ? 32 : 16, kDwpTileW, th,
-                           CU_TENSOR_MAP_SWIZZLE_64B);
-  };
-  err = plane(&L->map_o0, e.out0, out_bf16);
-  if (err.empty() && out_bf16) err = plane(&L->map_o1, e.out1, true);
-  if (err.empty() && e.res0 != nullptr) err = plane(&L->map_r0, e.res0, e.res_bf16);
-  if (err.empty() && e.res1 != nullptr) err = plane(&L->map_r1, e.res1, e.res_bf16);
   return err;
 }
 
@@ -1246,11 +1055,11 @@ cudaError_t tc_launch_dw_project(const TcDwProjLaunch& L, cudaStream_t stream) {
   KernelLaunchConfig lc(L.grid, kDwpThreads, L.smem_bytes, false, stream);
   cudaError_t e;
   if (!L.expand)
-    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 1, false>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1, L.map_o0, L.map_o1, L.map_r0, L.map_r1);
+    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 1, false>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
   else if (L.stride == 1)
-    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 1, true>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1, L.map_o0, L.map_o1, L.map_r0, L.map_r1);
+    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 1, true>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
   else
-    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 2, true>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1, L.map_o0, L.map_o1, L.map_r0, L.map_r1);
+    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 2, true>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1351,8 +1160,6 @@ std::string tc_plan_stem(TcStemLaunch* L, const TcStemConv& c, const TcEpilogue&
   if (e.out_mode != OUT_F32 && !(e.out_mode == OUT_BF16X2 && !i8) && !(i8_out && i8))
     return "output format not handled by the stem kernel";
   const bool bf16_out = e.out_mode == OUT_BF16X2;
-  if (bf16_out && N % 32 != 0) return "bf16-pair results need channels in multiples of 32";
-  if (i8_out && N % 64 != 0) return "int8 results need channels in multiples of 64";
   if (e.ldo != N || (reinterpret_cast<uintptr_t>(e.out0) & 15) != 0 || (reinterpret_cast<uintptr_t>(e.out1) & 15) != 0 ||
       (reinterpret_cast<uintptr_t>(e.outq) & 15) != 0)
     return "the stem kernel writes dense, 16-byte aligned rows";
@@ -1380,32 +1187,22 @@ std::string tc_plan_stem(TcStemLaunch* L, const TcStemConv& c, const TcEpilogue&
   p.act_a = e.act_a;
   p.act_b = e.act_b;
   p.status = e.status;
-  p.wide = !i8_out && (bf16_out || N % 32 == 0) ? 1 : 0;
-  const int out_tile = p.wide ? 16384 : 8192;
+  p.out0 = e.out0;
+  p.out1 = e.out1;
+  p.outq = e.outq;
+  if (!direct_rows(c.kind, e, N, &p.wide)) return "the stem kernel writes rows of 16-byte pieces";
   const int budget = tc_smem_budget(c.kind);
   const int weights = c.KH * planes * p.b_slot;
   const int stage = planes * p.a_plane_bytes;
-  // the epilogue of a 64-channel row takes longer than its 42 MMAs: two epilogue groups when they fit, and
-  // staging tiles before a third row stage (a stage holds a whole tile's input: two are a double buffer)
-  p.epi_groups = 0;
-  for (int groups : {2, 1}) {
-    for (int bufs : {4, 3, 2}) {
-      if ((budget - weights - groups * bufs * out_tile) / stage >= 2) {
-        p.epi_groups = groups;
-        p.out_bufs = bufs;
-        break;
-      }
-    }
-    if (p.epi_groups != 0) break;
-  }
-  if (p.epi_groups == 0) return "shared memory cannot hold the weights, two row stages and the staging tiles";
-  if (p.tiles < 2 * sm_count) p.epi_groups = 1;
-  p.staging_bytes = p.out_bufs * out_tile;
-  p.stages = std::min(kStemMaxStages, (budget - weights - p.epi_groups * p.staging_bytes) / stage);
+  // (a stage holds a whole tile's input: two are a double buffer)
+  p.stages = std::min(kStemMaxStages, (budget - weights - kDrainBytes) / stage);
+  if (p.stages < 2) return "shared memory cannot hold the weights and two row stages";
+  // the epilogue of a 64-channel row takes longer than its 42 MMAs: two epilogue groups on alternate tiles
+  p.epi_groups = p.tiles < 2 * sm_count ? 1 : 2;
   // four accumulators of 64 columns where they fit, and then a second MMA-issuing warp for alternate tiles
   p.accs = N <= 64 ? 4 : 2;
   p.issuers = p.accs == 4 && env_int("NCNN_B200_STEM_ISSUERS", 2) >= 2 ? 2 : 1;
-  L->smem_bytes = weights + p.stages * stage + p.epi_groups * p.staging_bytes + 1024;
+  L->smem_bytes = weights + p.stages * stage + kDrainBytes + 1024;
   L->smem_bytes = std::max(L->smem_bytes, 120 * 1024);  // one CTA per SM: each allocates tensor memory
   L->grid = std::min(p.tiles, sm_count);
   // input planes: [images][H][row_bytes / 128][64 bf16], KH whole rows per copy, dense in shared memory
@@ -1434,21 +1231,6 @@ std::string tc_plan_stem(TcStemLaunch* L, const TcStemConv& c, const TcEpilogue&
   if (err.empty() && !i8)
     err = encode_tiled_2d(&L->map_b1, c.kind, c.w1, k_total, N, k_total * 2, static_cast<uint32_t>(window), N, 64);
   if (!err.empty()) return err;
-  // outputs: [pixels][N], boxes of 64 bytes x OW rows (one output row of the image), 64-byte swizzle
-  auto plane = [&](CUtensorMap* map, const void* base) -> std::string {
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(p.M)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(N) * (i8_out ? 1 : (bf16_out ? 2 : 4))};
-    const cuuint32_t box[2] = {i8_out ? 64u : (bf16_out ? 32u : 16u), static_cast<cuuint32_t>(c.OW)};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    const CUresult r = g_encode_tiled(map, i8_out ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : (bf16_out ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32),
-                                      2, const_cast<void*>(base), dims, strides, box, elem_strides,
-                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled failed for a stem output plane with code " + std::to_string(static_cast<int>(r));
-    return {};
-  };
-  err = plane(&L->map_o0, i8_out ? static_cast<const void*>(e.outq) : static_cast<const void*>(e.out0));
-  if (err.empty() && bf16_out) err = plane(&L->map_o1, e.out1);
   return err;
 }
 
@@ -1466,10 +1248,9 @@ cudaError_t tc_launch_stem(const TcStemLaunch& L, cudaStream_t stream) {
   KernelLaunchConfig lc(L.grid, kStemThreads, L.smem_bytes, false, stream);
   cudaError_t e;
   if (L.kind == GEMM_I8)
-    e = cudaLaunchKernelEx(&lc.cfg, tc_stem_kernel<GEMM_I8>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0, L.map_o1);
+    e = cudaLaunchKernelEx(&lc.cfg, tc_stem_kernel<GEMM_I8>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
   else
-    e = cudaLaunchKernelEx(&lc.cfg, tc_stem_kernel<GEMM_BF16X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                           L.map_o1);
+    e = cudaLaunchKernelEx(&lc.cfg, tc_stem_kernel<GEMM_BF16X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1545,8 +1326,8 @@ cudaError_t tc_launch_stem_pool(const TcStemPoolLaunch& L, cudaStream_t stream) 
   KernelLaunchConfig lc(L.grid, kStemPoolThreads, L.smem_bytes, false, stream);
   const cudaError_t e =
       L.kind == GEMM_I8 ? cudaLaunchKernelEx(&lc.cfg, tc_stem_pool_kernel<GEMM_I8>, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0, L.map_o1)
-                        : cudaLaunchKernelEx(&lc.cfg, tc_stem_pool_kernel<GEMM_BF16X3>, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1,
-                                             L.map_o0, L.map_o1);
+                        : cudaLaunchKernelEx(&lc.cfg, tc_stem_pool_kernel<GEMM_BF16X3>, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
+                                             L.map_o1);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

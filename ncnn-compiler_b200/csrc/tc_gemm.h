@@ -24,12 +24,6 @@ struct TcLaunch {
   alignas(64) CUtensorMap map_a1{};
   alignas(64) CUtensorMap map_b0{};
   alignas(64) CUtensorMap map_b1{};
-  alignas(64) CUtensorMap map_o0{};  // output planes, boxes of 16 columns x 128 rows
-  alignas(64) CUtensorMap map_o1{};
-  alignas(64) CUtensorMap map_r0{};  // residual planes
-  alignas(64) CUtensorMap map_r1{};
-  alignas(64) CUtensorMap map_s0{};  // int8 copies of the result (TcEpilogue::side_q)
-  alignas(64) CUtensorMap map_s1{};
   int kind = GEMM_TF32;
   int grid = 0;
   int smem_bytes = 0;
@@ -126,10 +120,6 @@ struct TcHaloLaunch {
   alignas(64) CUtensorMap map_a1{};
   alignas(64) CUtensorMap map_b0{};
   alignas(64) CUtensorMap map_b1{};
-  alignas(64) CUtensorMap map_o0{};
-  alignas(64) CUtensorMap map_o1{};
-  alignas(64) CUtensorMap map_r0{};
-  alignas(64) CUtensorMap map_r1{};
   int kind = GEMM_TF32;
   int grid = 0;
   int smem_bytes = 0;
@@ -164,10 +154,6 @@ struct TcDwProjLaunch {
   alignas(64) CUtensorMap map_e1{};
   alignas(64) CUtensorMap map_b0{};  // projection weights, bf16 hi / mid planes
   alignas(64) CUtensorMap map_b1{};
-  alignas(64) CUtensorMap map_o0{};
-  alignas(64) CUtensorMap map_o1{};
-  alignas(64) CUtensorMap map_r0{};
-  alignas(64) CUtensorMap map_r1{};
   int grid = 0;
   int smem_bytes = 0;
   int stride = 1;
@@ -214,8 +200,6 @@ struct TcStemLaunch {
   alignas(64) CUtensorMap map_a1{};
   alignas(64) CUtensorMap map_b0{};
   alignas(64) CUtensorMap map_b1{};
-  alignas(64) CUtensorMap map_o0{};
-  alignas(64) CUtensorMap map_o1{};
   int kind = GEMM_BF16X3;
   int grid = 0;
   int smem_bytes = 0;

@@ -1,7 +1,7 @@
 // Tensor-core contraction on CTA pairs, with an even split of the K blocks over the pairs.
 //
 // Same contract as tc_gemm_kernel (out[M,N] = epilogue(A[M,K] * B[N,K]^T), A by im2col or tiled
-// TMA, B the packed weights, the staged TMA-store epilogue), different shape of the work:
+// TMA, B the packed weights, the same epilogue), different shape of the work:
 //
 // * A tile is 256 rows x block_n columns (block_n up to 256) and belongs to a cluster of two CTAs
 //   on the two SMs of one TPC.  Each CTA loads its own 128 rows of A and HALF of the B rows into
@@ -35,8 +35,7 @@
 
 namespace nb {
 
-constexpr int kTc2Threads = 224;        // warps: 0 A producer, 1 MMA issuer, 2-5 epilogue, 6 B producer
-constexpr int kTc2ThreadsTwoEpi = 352;  // + warps 7-10: a second epilogue group for the other half of the columns
+constexpr int kTc2Threads = 352;  // warps: 0 A producer, 1 MMA issuer, 2-5 and 7-10 two epilogue groups, 6 B producer
 constexpr int kTc2TileM = 256;  // rows of a pair's tile
 constexpr int kTc2MaxBlockN = 256;
 constexpr int kTc2AccStride = 256;  // tensor-memory columns between the two accumulators
@@ -103,15 +102,11 @@ struct Tc2Work {
 };
 
 template <int KIND, bool PAIR>
-__global__ void __launch_bounds__(kTc2ThreadsTwoEpi, 1)
+__global__ void __launch_bounds__(kTc2Threads, 1)
 tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ CUtensorMap map_a0,
                 const __grid_constant__ CUtensorMap map_a1,
                 const __grid_constant__ CUtensorMap map_b0,
-                const __grid_constant__ CUtensorMap map_b1,
-                const __grid_constant__ CUtensorMap map_o0,
-                const __grid_constant__ CUtensorMap map_o1,
-                const __grid_constant__ CUtensorMap map_r0,
-                const __grid_constant__ CUtensorMap map_r1) {
+                const __grid_constant__ CUtensorMap map_b1) {
   using namespace ptx;
   grid_dependency_trigger();  // the next kernel of the stream may begin its preamble
   constexpr int PLANES = tc_planes(KIND);
@@ -121,9 +116,6 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
   __shared__ __align__(8) uint64_t empty_bar[kTcMaxStages];  // per CTA: the MMAs that read the stage are done
   __shared__ __align__(8) uint64_t tfull_bar[2];             // per CTA: accumulator complete
   __shared__ __align__(8) uint64_t tempty_bar[2];            // used in CTA 0: both CTAs' epilogues have drained it
-  __shared__ __align__(8) uint64_t res_bar[2];
-  __shared__ __align__(16) float tile_bias[kTc2MaxBlockN];
-  __shared__ __align__(16) float tile_scale[KIND == GEMM_I8 ? kTc2MaxBlockN : 4];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -152,10 +144,8 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&tfull_bar[i]), 1);
-      mbar_init(smem_u32(&tempty_bar[i]), 4u * CTAS * static_cast<uint32_t>(p.epi_groups));  // every epilogue warp of the worker
+      mbar_init(smem_u32(&tempty_bar[i]), 8u * CTAS);  // every epilogue warp of the worker
     }
-    mbar_init(smem_u32(&res_bar[0]), 1);
-    mbar_init(smem_u32(&res_bar[1]), 1);
     fence_mbar_init();
     prefetch_tensormap(&map_a0);
     prefetch_tensormap(&map_b0);
@@ -387,44 +377,34 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
     }
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs)
-    // One group (warps 2-5) drains all block_n columns; with two groups (352 threads) warps 2-5 take
-    // the first half of the columns and warps 7-10 the second, each with its own staging tiles,
-    // barriers, residual barrier and workspace flags.  An epilogue warp runs alone on its scheduler
-    // and pays every instruction's latency, so two groups nearly halve the time of a wide tile.
-    const int groups = p.epi_groups;
+    // Warps 2-5 take the first half of the columns and warps 7-10 the second, each with its own workspace flags.
     const int group = warp >= 7 ? 1 : 0;
-    const int first_thread = group ? 224 : 64;
-    const bool leader = static_cast<int>(threadIdx.x) == first_thread;
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+31] belong to this warp
+    const bool leader = threadIdx.x == (group ? 224u : 64u);
     const int row = quarter * 32 + lane;
-    const int half = p.block_n / groups;  // columns of this group
-    const int col0 = group * half;        // first column of the group inside the tile
+    const int half_cols = ((p.block_n / 2) + 15) & ~15;
+    const int half = group ? p.block_n - half_cols : half_cols;  // columns of this group
+    const int col0 = group ? half_cols : 0;                      // first column of the group inside the tile
     const size_t slot_words = static_cast<size_t>(kTcBlockM) * p.block_n;
-    const int bar_base = 1 + 3 * group;   // named barriers bar_base .. bar_base + 2
+    const int bar_base = 1 + group;  // this group's named barrier
     const int my_flag = static_cast<int>(blockIdx.x) * 2 + group;
     const int flag_step = 2 * CTAS;  // flag words between this CTA and the same CTA of the worker before
-    float* my_bias = tile_bias + col0;
-    float* my_scale = tile_scale + (KIND == GEMM_I8 ? col0 : 0);
     int acc = 0;
     uint32_t acc_ph = 0;
-    uint32_t res_ph = 0;
-    int out_slot = 0;
     bool ok = true;
-    TcStageCfg cfg{};
-    cfg.res_stage = smem_base + static_cast<uint32_t>(S) * stage_bytes + static_cast<uint32_t>(group) * p.staging_bytes;
-    cfg.out_stage = cfg.res_stage + (p.res_mode != RES_NONE ? 16384u : 0u);
-    cfg.res_bar = smem_u32(&res_bar[group]);
-    cfg.out_bufs = p.out_bufs;
-    cfg.out_mode = p.out_mode;
-    cfg.res_mode = p.res_mode;
-    cfg.act = p.act;
-    cfg.act_a = p.act_a;
-    cfg.act_b = p.act_b;
-    cfg.N = p.N;
-    cfg.block_n = half;
-    cfg.wide = p.wide;
-    cfg.bar_base = bar_base;
-    cfg.fix_stride = -static_cast<long long>(CTAS) * static_cast<long long>(slot_words);  // the same CTA of the worker before
+    const TcGemmParams lp = p;
+    TcDirect d{};
+    d.out_mode = p.out_mode;
+    d.res_mode = p.res_mode;
+    d.act = p.act;
+    d.act_a = p.act_a;
+    d.act_b = p.act_b;
+    d.out_scale = p.out_scale;
+    d.wide = p.wide;
+    d.xs = 8;
+    d.ys = 4;
+    d.stage = smem_base + static_cast<uint32_t>(S) * stage_bytes + static_cast<uint32_t>(group * 4 + quarter) * kDrainWarpBytes;
+    d.fix_stride = -static_cast<long long>(CTAS) * static_cast<long long>(slot_words);  // the same CTA of the worker before
     const uint32_t tempty0 = PAIR ? map_to_cta(smem_u32(&tempty_bar[0]), 0u) : smem_u32(&tempty_bar[0]);
     const uint32_t tempty1 = PAIR ? map_to_cta(smem_u32(&tempty_bar[1]), 0u) : smem_u32(&tempty_bar[1]);
     for (int i = 0; i < work.nseg && ok; ++i) {
@@ -471,7 +451,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           }
         }
         __threadfence();
-        named_barrier_sync(bar_base + 2, 128);
+        named_barrier_sync(bar_base, 128);
         if (leader) st_release_gpu(p.sk_flags + my_flag, 1);
       } else {
         const int fix = work.contributors(tile, kb0);
@@ -506,56 +486,26 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
             p.trace[512 + 8 * i + 7] = fix;
           }
         }
-        if (m_first < p.M) {
-          cfg.side_count = p.side_count;
-          cfg.side_ld = p.side_ld;
-          cfg.side_rows = static_cast<int>(p.M - m_first < kTcBlockM ? p.M - m_first : kTcBlockM);
-          cfg.side_q0 = p.side_q0 != nullptr ? p.side_q0 + m_first * p.side_ld + n0 : nullptr;
-          cfg.side_q1 = p.side_q1 != nullptr ? p.side_q1 + m_first * p.side_ld + n0 : nullptr;
-          cfg.side_scale0 = p.side_scale0;
-          cfg.side_scale1 = p.side_scale1;
-          cfg.fix_count = row_valid ? fix : 0;  // (a row past the end skips the loads; its results are clipped)
-          cfg.fix_ws = fix > 0 ? p.sk_ws + static_cast<size_t>(static_cast<int>(blockIdx.x) - CTAS) * slot_words + ws_group
-                               : nullptr;
-          // per-column constants of this tile (every warp of the group has left the previous tile's last
-          // chunk: it ends with a barrier)
-          for (int t = static_cast<int>(threadIdx.x) - first_thread; t < half; t += 128) {
-            const int n = n0 + t;
-            my_bias[t] = (p.bias != nullptr && n < p.N) ? __ldg(p.bias + n) : 0.0f;
-            if (KIND == GEMM_I8) my_scale[t] = n < p.N ? __ldg(p.scale + n) : 0.0f;
-          }
-          const int m_row = static_cast<int>(m_first);
-          struct {
-            const CUtensorMap *o0, *o1, *r0, *r1;
-            int m_first;
-            __device__ __forceinline__ void load_res(int plane, uint32_t dst, uint32_t bar, int col) const {
-              ptx::tma_load_2d(dst, plane ? r1 : r0, bar, col, m_first);
-            }
-            __device__ __forceinline__ void store_out(int plane, uint32_t src, int col) const {
-              ptx::tma_store_2d(plane ? o1 : o0, src, col, m_first);
-            }
-            __device__ __forceinline__ void store_side(int, uint32_t, int) const {}
-          } io{&map_o0, &map_o1, &map_r0, &map_r1, m_row};
-          const bool extras = fix > 0 || p.side_count > 0;
-          if (p.out_mode == OUT_I8) {
-            if (extras)
-              tc_staged_epilogue_i8<KIND, decltype(io), true>(cfg, p.out_scale, io, t_row, n0, row, leader, my_bias, my_scale,
-                                                              out_slot);
-            else
-              tc_staged_epilogue_i8<KIND>(cfg, p.out_scale, io, t_row, n0, row, leader, my_bias, my_scale, out_slot);
-          } else {
-            if (extras)
-              ok = tc_staged_epilogue<KIND, decltype(io), true>(cfg, io, t_row, n0, row, leader, my_bias, my_scale, res_ph,
-                                                                out_slot, abort_ptr);
-            else
-              ok = tc_staged_epilogue<KIND>(cfg, io, t_row, n0, row, leader, my_bias, my_scale, res_ph, out_slot,
-                                            abort_ptr);
-            if (!ok) break;
-          }
-        }
+        const long long m = m_first + row;
+        const int es = lp.out_mode == OUT_I8 ? 1 : (lp.out_mode == OUT_BF16X2 ? 2 : 4);
+        const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
+        d.o0 = (lp.out_mode == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + ((m - lane) * lp.ldo + n0) * es;
+        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + ((m - lane) * lp.ldo + n0) * es;
+        d.pitch = lp.ldo * es;
+        d.pitch8 = 8 * d.pitch;
+        const long long rows_left = lp.M - (m - lane);
+        d.rows = rows_left > 32 ? 32 : static_cast<int>(rows_left);
+        d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n0) * rs;
+        d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n0) * rs;
+        d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
+        d.scale = lp.scale + n0;
+        d.fix_count = fix;
+        d.fix_ws = lp.sk_ws + static_cast<long long>(static_cast<int>(blockIdx.x) - CTAS) * static_cast<long long>(slot_words) +
+                   ws_group + static_cast<size_t>(row) * 16;
+        tc_drain<KIND, false, true, false>(d, t_row, half, lp.N - n0, row_valid);
         if (fix > 0) {
-          // every warp of the group has read the slots (it passed the chunk barriers, or this one): free them
-          named_barrier_sync(bar_base + 2, 128);
+          // every warp of the group has read the slots: free them
+          named_barrier_sync(bar_base, 128);
           if (leader)
             for (int c = 1; c <= fix; ++c) p.sk_flags[my_flag - flag_step * c] = 0;
         }
@@ -574,7 +524,6 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
     if (!ok && lane == 0) {
       if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_EPILOGUE);
     }
-    if (leader) tma_store_wait_all();  // stores still read shared memory
   }
 
   // Neither CTA leaves while the other may still signal its barriers or read its shared memory.

@@ -40,7 +40,10 @@ struct TcStemParams {
   float out_scale;     // int8 results: requantisation scale
   int out_mode, act;
   float act_a, act_b;
-  int wide, out_bufs, staging_bytes, epi_groups;
+  int wide, epi_groups;
+  float* out0;
+  float* out1;
+  int8_t* outq;
   int* status;
 };
 
@@ -59,8 +62,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kStemThreads, 1)
 tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ CUtensorMap map_a0,
                const __grid_constant__ CUtensorMap map_a1, const __grid_constant__ CUtensorMap map_b0,
-               const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_o0,
-               const __grid_constant__ CUtensorMap map_o1) {
+               const __grid_constant__ CUtensorMap map_b1) {
   using namespace ptx;
   grid_dependency_trigger();  // the next kernel of the stream may begin its preamble
   constexpr int PLANES = tc_planes(KIND);
@@ -70,9 +72,6 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
   __shared__ __align__(8) uint64_t tfull_bar[4];
   __shared__ __align__(8) uint64_t tempty_bar[4];
   __shared__ __align__(8) uint64_t weights_bar;
-  __shared__ __align__(8) uint64_t unused_res_bar[2];
-  __shared__ __align__(16) float tile_bias_all[2][128];
-  __shared__ __align__(16) float tile_scale_all[2][KIND == GEMM_I8 ? 128 : 4];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -83,7 +82,6 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
   const uint32_t b_region = smem_base;  // [KH][plane][b_slot]
   const uint32_t a_region = b_region + static_cast<uint32_t>(p.KH * PLANES) * static_cast<uint32_t>(p.b_slot);
   const uint32_t stage_bytes = static_cast<uint32_t>(PLANES) * static_cast<uint32_t>(p.a_plane_bytes);
-  const uint32_t staging = a_region + static_cast<uint32_t>(S) * stage_bytes;
   volatile int* abort_ptr = &abort_flag;
   // tile i of this CTA's sequence: stage i % S, accumulator i % accs, issuer i % issuers
   const int accs = p.accs == 4 ? 4 : 2;
@@ -100,7 +98,6 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
       mbar_init(smem_u32(&tfull_bar[i]), 1);
       mbar_init(smem_u32(&tempty_bar[i]), 4);
     }
-    for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&unused_res_bar[i]), 1);
     mbar_init(smem_u32(&weights_bar), 1);
     fence_mbar_init();
     prefetch_tensormap(&map_a0);
@@ -225,35 +222,24 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
     const int group = warp >= 7 ? 1 : 0;
     const int groups = p.epi_groups;
     if (group < groups) {
-      const int first_thread = group ? 224 : 64;
-      const bool leader = static_cast<int>(threadIdx.x) == first_thread;
       const int quarter = warp & 3;
-      float* tile_bias = tile_bias_all[group];
-      float* tile_scale = tile_scale_all[group];
-      {
-        const int t = static_cast<int>(threadIdx.x) - first_thread;
-        tile_bias[t] = (p.bias != nullptr && t < p.N) ? __ldg(p.bias + t) : 0.0f;
-        if (KIND == GEMM_I8) tile_scale[t] = t < p.N ? __ldg(p.scale + t) : 0.0f;
-        else if (t < 4) tile_scale[t] = 0.0f;
-      }
-      int i = groups == 2 ? group : 0;  // position in this CTA's tile sequence
-      uint32_t res_ph = 0;
-      int out_slot = 0;
+      const int row = quarter * 32 + lane;  // pixel of the output row; rows past OW hold whatever followed the input row
+      int i = groups == 2 ? group : 0;      // position in this CTA's tile sequence
       bool ok = true;
-      TcStageCfg cfg{};
-      cfg.res_stage = staging + static_cast<uint32_t>(group) * p.staging_bytes;
-      cfg.out_stage = cfg.res_stage;
-      cfg.res_bar = smem_u32(&unused_res_bar[group]);
-      cfg.out_bufs = p.out_bufs;
-      cfg.out_mode = p.out_mode;
-      cfg.res_mode = RES_NONE;
-      cfg.act = p.act;
-      cfg.act_a = p.act_a;
-      cfg.act_b = p.act_b;
-      cfg.N = p.N;
-      cfg.block_n = p.N;
-      cfg.wide = p.wide;
-      cfg.bar_base = 1 + 3 * group;
+      const TcStemParams lp = p;
+      TcDirect d{};
+      d.out_mode = p.out_mode;
+      d.act = p.act;
+      d.act_a = p.act_a;
+      d.act_b = p.act_b;
+      d.out_scale = p.out_scale;
+      d.wide = p.wide;
+      d.rows = p.OW - quarter * 32;
+      d.xs = 8;
+      d.ys = 4;
+      d.stage = a_region + static_cast<uint32_t>(S) * stage_bytes + static_cast<uint32_t>(group * 4 + quarter) * kDrainWarpBytes;
+      d.bias = p.bias;
+      d.scale = p.scale;
       const int tile_step = static_cast<int>(gridDim.x) * groups;
       for (int tile = blockIdx.x + (groups == 2 ? group * static_cast<int>(gridDim.x) : 0); tile < p.tiles && ok;
            tile += tile_step, i += groups) {
@@ -265,32 +251,19 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
         tc_fence_after_sync();
         const uint32_t t_row =
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * acc_cols;
-        // the stores take OW rows of the staging tile (their box is OW rows high); rows beyond hold
-        // whatever followed the input row in shared memory and go nowhere
-        struct {
-          const CUtensorMap *o0, *o1;
-          int m_first;
-          __device__ __forceinline__ void load_res(int, uint32_t, uint32_t, int) const {}
-          __device__ __forceinline__ void store_out(int plane, uint32_t src, int col) const {
-            ptx::tma_store_2d(plane ? o1 : o0, src, col, m_first);
-          }
-          __device__ __forceinline__ void store_side(int, uint32_t, int) const {}
-        } io{&map_o0, &map_o1, tile * p.OW};
-        if (KIND == GEMM_I8 && p.out_mode == OUT_I8) {
-          tc_staged_epilogue_i8<KIND>(cfg, p.out_scale, io, t_row, 0, quarter * 32 + lane, leader, tile_bias, tile_scale,
-                                      out_slot);
-        } else {
-          ok = tc_staged_epilogue<KIND>(cfg, io, t_row, 0, quarter * 32 + lane, leader, tile_bias, tile_scale, res_ph,
-                                        out_slot, abort_ptr);
-          if (!ok) break;
-        }
+        const long long at = (static_cast<long long>(tile) * lp.OW + quarter * 32) * lp.N;
+        const int es = lp.out_mode == OUT_I8 ? 1 : (lp.out_mode == OUT_BF16X2 ? 2 : 4);
+        d.o0 = (lp.out_mode == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + at * es;
+        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at * es;
+        d.pitch = static_cast<long long>(lp.N) * es;
+        d.pitch8 = 8 * d.pitch;
+        tc_drain<KIND, false, false, false>(d, t_row, lp.N, lp.N, row < lp.OW);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
       }
       if (!ok && lane == 0 && atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0)
         atomicCAS(p.status, 0, TC_TIMEOUT_EPILOGUE);
-      if (leader) tma_store_wait_all();
     }
   }
 
