@@ -54,7 +54,7 @@ struct TcHaloParams {
   long long* trace;  // optional (bring-up): clock stamps of the first work item of a worker in the middle of the grid
 };
 
-template <int KIND, bool PAIR = false>
+template <int KIND, bool PAIR, int EPI>
 __global__ void __launch_bounds__(kHaloThreads, 1)
 tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constant__ CUtensorMap map_a0,
                     const __grid_constant__ CUtensorMap map_a1,
@@ -367,7 +367,7 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
       d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + at * rs;
       d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + at * rs;
       d.bias = lp.bias != nullptr ? lp.bias + n0 + c_first : nullptr;
-      tc_drain<KIND, false, false, false>(d, t_row + static_cast<uint32_t>(c_first), cols, lp.N - n0 - c_first, inside);
+      tc_drain<KIND, EPI, false, false>(d, t_row + static_cast<uint32_t>(c_first), cols, lp.N - n0 - c_first, inside);
       if (etr) p.trace[5] = clock64();
       tc_fence_before_sync();
       __syncwarp();

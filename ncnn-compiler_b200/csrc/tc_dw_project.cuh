@@ -86,7 +86,7 @@ struct TcDwProjParams {
 };
 
 // (KIND: the projection's arithmetic; bf16 pairs are the only form built)
-template <int KIND, int STRIDE, bool EXPAND>
+template <int KIND, int STRIDE, bool EXPAND, int EPI>
 __global__ void __launch_bounds__(kDwpThreads, 1)
 tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_x1, const __grid_constant__ CUtensorMap map_e0,
@@ -434,7 +434,7 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
       d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + at * rs;
       d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + at * rs;
       d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
-      tc_drain<KIND, false, false, false>(d, t_row, lp.block_n, lp.N - n0, inside);
+      tc_drain<KIND, EPI, false, false>(d, t_row, lp.block_n, lp.N - n0, inside);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

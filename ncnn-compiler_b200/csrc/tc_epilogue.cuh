@@ -97,11 +97,12 @@ struct TcFlushLane {
   __device__ __forceinline__ void init(const TcDirect& d) {
     const int r0 = static_cast<int>(threadIdx.x & 31) / CHUNKS;
     first = (r0 >> 3) * d.pitch8 + (r0 & 7) * d.pitch;
-    rows = 0;
+    rows = (1u << CHUNKS) - 1u;
+    if (d.rows >= 32 && d.xs >= 8 && d.ys >= 4) return;
 #pragma unroll
     for (int i = 0; i < CHUNKS; ++i) {
       const int r = r0 + i * (32 / CHUNKS);
-      if (r < d.rows && (r & 7) < d.xs && (r >> 3) < d.ys) rows |= 1u << i;
+      if (!(r < d.rows && (r & 7) < d.xs && (r >> 3) < d.ys)) rows &= ~(1u << i);
     }
   }
 };
@@ -309,10 +310,10 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
         put(4 + q, lo + 4 * q);
       }
       tc_flush<8>(d, fl, d.o0 + 4 * c, d.o1 + 4 * c, 64, 4 * min(have, 16));
-    } else if constexpr (OUT == OUT_F32) {
+    } else if constexpr (OUT == OUT_F32 || OUT == OUT_F32_TF32) {
       uint32_t w[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(d.out_mode == OUT_F32_TF32 ? round_tf32(y[j]) : y[j]);
+      for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(OUT == OUT_F32_TF32 ? round_tf32(y[j]) : y[j]);
 #pragma unroll
       for (int q = 0; q < 4; ++q) put(4 * h + q, w + 4 * q);
       if (full) tc_flush<8>(d, fl, d.o0 + 4 * c32, nullptr, 128, 4 * step_cols);
@@ -320,30 +321,20 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
   }
 }
 
+// The epilogue a kernel is compiled with: an output format, with or without a residual.  One kernel per form: a kernel
+// with all of them behind run-time branches spends its tiles on instruction fetch (24 -> 144 channels, 64 images of 112 x 112:
+// 233 us with ten forms in one kernel, 198 with eight, 176 with one).
+constexpr int epi_form(int out_mode, bool res) { return out_mode * 2 + (res ? 1 : 0); }
+constexpr int kEpiAny = -1;  // element by element, any format and alignment
+
 // Drains `cols` accumulator columns (a multiple of 16) of this warp's 32 rows, of which `left` exist in the result (a
 // multiple of the 16-byte piece of every format involved).  `valid`: this thread's row exists.  Every lane of the warp
-// must call it.  SIDE: int8 copies may take part; FIX: partial accumulators may; CHW: the caller's layout may.
-// One loop per output format, with and without a residual: the branches of a combined loop stall on instruction fetch.
-template <int KIND, bool SIDE, bool FIX, bool CHW>
-__device__ __forceinline__ void tc_drain(const TcDirect d, uint32_t t_row, int cols, int left, bool valid) {
+// must call it.  SIDE: int8 copies may take part; FIX: partial accumulators may.
+template <int KIND, int EPI, bool SIDE, bool FIX>
+__device__ __forceinline__ void tc_drain(const TcDirect& d, uint32_t t_row, int cols, int left, bool valid) {
   if (cols > left) cols = (left + 15) & ~15;
   if (cols <= 0) return;
-  const bool res = d.res_mode != RES_NONE;
-  if (KIND == GEMM_I8 && d.out_mode == OUT_I8) {
-    tc_drain_as<KIND, OUT_I8, false, false, FIX>(d, t_row, cols, left, valid);
-  } else if (CHW && d.out_mode == OUT_CHW) {
-    if (res) tc_drain_as<KIND, OUT_CHW, true, false, FIX>(d, t_row, cols, left, valid);
-    else tc_drain_as<KIND, OUT_CHW, false, false, FIX>(d, t_row, cols, left, valid);
-  } else if (d.out_mode == OUT_BF16X2) {
-    if (res) tc_drain_as<KIND, OUT_BF16X2, true, false, FIX>(d, t_row, cols, left, valid);
-    else tc_drain_as<KIND, OUT_BF16X2, false, false, FIX>(d, t_row, cols, left, valid);
-  } else if (d.out_mode == OUT_F32_SPLIT) {
-    if (res) tc_drain_as<KIND, OUT_F32_SPLIT, true, false, FIX>(d, t_row, cols, left, valid);
-    else tc_drain_as<KIND, OUT_F32_SPLIT, false, false, FIX>(d, t_row, cols, left, valid);
-  } else {
-    if (res) tc_drain_as<KIND, OUT_F32, true, SIDE, FIX>(d, t_row, cols, left, valid);
-    else tc_drain_as<KIND, OUT_F32, false, SIDE, FIX>(d, t_row, cols, left, valid);
-  }
+  tc_drain_as<KIND, EPI / 2, EPI % 2 == 1, SIDE, FIX>(d, t_row, cols, left, valid);
 }
 
 }  // namespace nb

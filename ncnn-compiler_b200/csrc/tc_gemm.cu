@@ -4,7 +4,9 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace nb {
 namespace {
@@ -118,11 +120,24 @@ int res_mode_of(const TcEpilogue& e) {
 
 int out_elem_bytes(int out_mode) { return out_mode == OUT_I8 ? 1 : (out_mode == OUT_BF16X2 ? 2 : 4); }
 
+// The formats that kernels of a kind are compiled for; the rest (networks that mix kinds in unusual ways) goes out
+// element by element.
+bool drains(int kind, int out_mode, int res_mode) {
+  if (res_mode == RES_SPLIT && kind != GEMM_TF32X3) return false;
+  switch (out_mode) {
+    case OUT_F32:
+    case OUT_CHW: return true;
+    case OUT_I8: return kind == GEMM_I8 && res_mode == RES_NONE;
+    case OUT_BF16X2: return kind == GEMM_BF16X3 || kind == GEMM_TF32X3;
+    case OUT_F32_SPLIT: return kind == GEMM_TF32X3;
+    default: return kind == GEMM_TF32;
+  }
+}
+
 // True when tc_drain can write these results: rows (of `N` columns, `ldo` apart) made of 16-byte pieces in every format
 // that takes part.  *wide: of 32-byte pieces, so that stores and loads are whole sectors.
 bool direct_rows(int kind, const TcEpilogue& e, int N, int* wide) {
-  // (a residual of fp32 hi / lo planes takes part beside operands of that format only)
-  bool ok = kind == GEMM_TF32X3 || res_mode_of(e) != RES_SPLIT, all32 = true;
+  bool ok = drains(kind, e.out_mode, res_mode_of(e)), all32 = true;
   auto plane = [&](const void* p, int es) {
     if (p == nullptr) return;
     const uintptr_t at = reinterpret_cast<uintptr_t>(p);
@@ -589,32 +604,64 @@ std::string tc_plan_gemm(TcLaunch* L, int kind, const void* a0, const void* a1, 
 
 namespace {
 
-template <int KIND>
-cudaError_t prepare_worker_kernel() {
-  cudaError_t e = cudaFuncSetAttribute(tc_gemm2_kernel<KIND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       tc_smem_budget(KIND) + 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tc_gemm2_kernel<KIND, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             tc_smem_budget(KIND) + 1024);
-  return e;
+// Calls f(std::integral_constant<int, EPI>) for the epilogue form of a launch (see `drains`).
+template <int KIND, bool CHW, class F>
+cudaError_t with_form(int out_mode, bool res, F&& f) {
+#define NB_FORM(OUT, RES) \
+  if (out_mode == OUT && res == RES) return f(std::integral_constant<int, epi_form(OUT, RES)>{})
+  NB_FORM(OUT_F32, false);
+  NB_FORM(OUT_F32, true);
+  if constexpr (CHW) {
+    NB_FORM(OUT_CHW, false);
+    NB_FORM(OUT_CHW, true);
+  }
+  if constexpr (KIND == GEMM_I8) {
+    NB_FORM(OUT_I8, false);
+  }
+  if constexpr (KIND == GEMM_BF16X3 || KIND == GEMM_TF32X3) {
+    NB_FORM(OUT_BF16X2, false);
+    NB_FORM(OUT_BF16X2, true);
+  }
+  if constexpr (KIND == GEMM_TF32X3) {
+    NB_FORM(OUT_F32_SPLIT, false);
+    NB_FORM(OUT_F32_SPLIT, true);
+  }
+  if constexpr (KIND == GEMM_TF32) {
+    NB_FORM(OUT_F32_TF32, false);
+    NB_FORM(OUT_F32_TF32, true);
+  }
+#undef NB_FORM
+  return cudaErrorInvalidValue;
 }
 
-cudaError_t prepare_worker_kernels() {
-  static PerDeviceOnce once;
-  return once.run([] {
-    cudaError_t e = prepare_worker_kernel<GEMM_TF32>();
-    if (e == cudaSuccess) e = prepare_worker_kernel<GEMM_TF32X3>();
-    if (e == cudaSuccess) e = prepare_worker_kernel<GEMM_I8>();
-    if (e == cudaSuccess) e = prepare_worker_kernel<GEMM_BF16X3>();
-    return e;
-  });
+// Opts a kernel in to `smem` bytes of dynamic shared memory, once per device.
+template <class K>
+cudaError_t opt_in(K kernel, int smem) {
+  static std::mutex mutex;
+  static std::map<std::pair<const void*, int>, cudaError_t> done;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mutex);
+  const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), device);
+  const auto it = done.find(key);
+  if (it != done.end()) return it->second;
+  return done[key] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}
+
+template <class K, class... Args>
+cudaError_t launch_opted(K kernel, int max_smem, KernelLaunchConfig& lc, const Args&... args) {
+  const cudaError_t e = opt_in(kernel, max_smem);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchKernelEx(&lc.cfg, kernel, args...);
 }
 
 template <int KIND>
 int pairs_resident(int smem_bytes, int sm_count) {
   KernelLaunchConfig wc(sm_count / 2 * 2, kTc2Threads, smem_bytes, true, nullptr);
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, tc_gemm2_kernel<KIND, true>, &wc.cfg) != cudaSuccess) {
+  const auto kernel = tc_gemm2_kernel<KIND, true, epi_form(OUT_F32, false)>;
+  if (opt_in(kernel, tc_smem_budget(KIND) + 1024) != cudaSuccess || cudaOccupancyMaxActiveClusters(&clusters, kernel, &wc.cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -628,7 +675,6 @@ int max_pairs_resident(int kind, int smem_bytes, int sm_count) {
     cudaGetLastError();
     return sm_count / 2;
   }
-  if (prepare_worker_kernels() != cudaSuccess) return 0;
   switch (kind) {
     case GEMM_TF32: return pairs_resident<GEMM_TF32>(smem_bytes, sm_count);
     case GEMM_TF32X3: return pairs_resident<GEMM_TF32X3>(smem_bytes, sm_count);
@@ -641,14 +687,14 @@ template <int KIND>
 cudaError_t launch_workers(const TcLaunch& L, cudaStream_t stream) {
   const bool pair = L.cta2 == 2;
   KernelLaunchConfig wc(L.grid, kTc2Threads, L.smem_bytes, pair, stream);
-  if (pair)
-    return cudaLaunchKernelEx(&wc.cfg, tc_gemm2_kernel<KIND, true>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-  return cudaLaunchKernelEx(&wc.cfg, tc_gemm2_kernel<KIND, false>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  return with_form<KIND, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
+    constexpr int EPI = decltype(form)::value;
+    if (pair) return launch_opted(tc_gemm2_kernel<KIND, true, EPI>, tc_smem_budget(KIND) + 1024, wc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+    return launch_opted(tc_gemm2_kernel<KIND, false, EPI>, tc_smem_budget(KIND) + 1024, wc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  });
 }
 
 cudaError_t tc_launch_workers(const TcLaunch& L, cudaStream_t stream) {
-  const cudaError_t prep = prepare_worker_kernels();
-  if (prep != cudaSuccess) return prep;
   cudaError_t e;
   switch (L.kind) {
     case GEMM_TF32: e = launch_workers<GEMM_TF32>(L, stream); break;
@@ -659,49 +705,36 @@ cudaError_t tc_launch_workers(const TcLaunch& L, cudaStream_t stream) {
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+template <int KIND>
+cudaError_t launch_gemm(const TcLaunch& L, cudaStream_t stream) {
+  KernelLaunchConfig lc(L.grid, kTcThreads, L.smem_bytes, false, stream);
+  const int max_smem = tc_smem_budget(KIND) + 1024;  // contents + alignment slack
+  // (int8 copies of an fp32 result are written by instantiations of their own)
+  if constexpr (KIND == GEMM_I8) {
+    if (L.p.side_count > 0) {
+      if (!L.p.direct || L.p.out_mode != OUT_F32)
+        return launch_opted(tc_gemm_kernel<KIND, kEpiAny, true>, max_smem, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+      if (L.p.res_mode != RES_NONE)
+        return launch_opted(tc_gemm_kernel<KIND, epi_form(OUT_F32, true), true>, max_smem, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+      return launch_opted(tc_gemm_kernel<KIND, epi_form(OUT_F32, false), true>, max_smem, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+    }
+  }
+  if (!L.p.direct) return launch_opted(tc_gemm_kernel<KIND, kEpiAny>, max_smem, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  return with_form<KIND, true>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
+    return launch_opted(tc_gemm_kernel<KIND, decltype(form)::value>, max_smem, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  });
+}
+
 }  // namespace
 
 cudaError_t tc_launch(const TcLaunch& L, cudaStream_t stream) {
   if (L.cta2) return tc_launch_workers(L, stream);
-  static PerDeviceOnce attr_once;
-  const cudaError_t attr_err = attr_once.run([] {
-    const int max_smem = tc_smem_budget(GEMM_TF32) + 1024;  // contents + alignment slack
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<GEMM_TF32>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_gemm_kernel<GEMM_TF32X3>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_gemm_kernel<GEMM_I8>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem_budget(GEMM_I8) + 1024);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_gemm_kernel<GEMM_BF16X3>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_gemm_kernel<GEMM_I8, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem_budget(GEMM_I8) + 1024);
-    return e;
-  });
-  if (attr_err != cudaSuccess) return attr_err;
-  KernelLaunchConfig lc(L.grid, kTcThreads, L.smem_bytes, false, stream);
   cudaError_t e;
   switch (L.kind) {
-    case GEMM_TF32:
-      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_TF32>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-      break;
-    case GEMM_TF32X3:
-      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_TF32X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-      break;
-    case GEMM_BF16X3:
-      e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_BF16X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-      break;
-    default:
-      // (int8 copies of an fp32 result are written by an instantiation of its own)
-      if (L.p.side_count > 0)
-        e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_I8, true>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-      else
-        e = cudaLaunchKernelEx(&lc.cfg, tc_gemm_kernel<GEMM_I8>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-      break;
+    case GEMM_TF32: e = launch_gemm<GEMM_TF32>(L, stream); break;
+    case GEMM_TF32X3: e = launch_gemm<GEMM_TF32X3>(L, stream); break;
+    case GEMM_BF16X3: e = launch_gemm<GEMM_BF16X3>(L, stream); break;
+    default: e = launch_gemm<GEMM_I8>(L, stream); break;
   }
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -822,44 +855,19 @@ std::string tc_plan_conv_halo(TcHaloLaunch* L, int kind, const TcHaloConv& c, co
 }
 
 cudaError_t tc_launch_halo(const TcHaloLaunch& L, cudaStream_t stream) {
-  static PerDeviceOnce attr_once;
-  const cudaError_t attr_err = attr_once.run([] {
-    const int max_smem = 223 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(tc_conv_halo_kernel<GEMM_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_conv_halo_kernel<GEMM_TF32X3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_conv_halo_kernel<GEMM_BF16X3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_conv_halo_kernel<GEMM_TF32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_conv_halo_kernel<GEMM_TF32X3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               max_smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_conv_halo_kernel<GEMM_BF16X3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               max_smem);
-    return e;
-  });
-  if (attr_err != cudaSuccess) return attr_err;
   KernelLaunchConfig lc(L.grid, kHaloThreads, L.smem_bytes, L.pair != 0, stream);
+  auto launch = [&](auto kind) {
+    constexpr int KIND = decltype(kind)::value;
+    return with_form<KIND, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
+      constexpr int EPI = decltype(form)::value;
+      if (L.pair) return launch_opted(tc_conv_halo_kernel<KIND, true, EPI>, 225 * 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+      return launch_opted(tc_conv_halo_kernel<KIND, false, EPI>, 225 * 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+    });
+  };
   cudaError_t e;
-#define NB_LAUNCH_HALO(KIND, PAIRED)                                                                             \
-  e = cudaLaunchKernelEx(&lc.cfg, tc_conv_halo_kernel<KIND, PAIRED>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1)
-  if (L.kind == GEMM_BF16X3) {
-    if (L.pair) NB_LAUNCH_HALO(GEMM_BF16X3, true);
-    else NB_LAUNCH_HALO(GEMM_BF16X3, false);
-  } else if (L.kind == GEMM_TF32X3) {
-    if (L.pair) NB_LAUNCH_HALO(GEMM_TF32X3, true);
-    else NB_LAUNCH_HALO(GEMM_TF32X3, false);
-  } else {
-    if (L.pair) NB_LAUNCH_HALO(GEMM_TF32, true);
-    else NB_LAUNCH_HALO(GEMM_TF32, false);
-  }
-#undef NB_LAUNCH_HALO
+  if (L.kind == GEMM_BF16X3) e = launch(std::integral_constant<int, GEMM_BF16X3>{});
+  else if (L.kind == GEMM_TF32X3) e = launch(std::integral_constant<int, GEMM_TF32X3>{});
+  else e = launch(std::integral_constant<int, GEMM_TF32>{});
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1044,22 +1052,14 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
 }
 
 cudaError_t tc_launch_dw_project(const TcDwProjLaunch& L, cudaStream_t stream) {
-  static PerDeviceOnce attr_once;
-  const cudaError_t attr_err = attr_once.run([] {
-    cudaError_t e = cudaFuncSetAttribute(tc_dw_project_kernel<GEMM_BF16X3, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(tc_dw_project_kernel<GEMM_BF16X3, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(tc_dw_project_kernel<GEMM_BF16X3, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-    return e;
-  });
-  if (attr_err != cudaSuccess) return attr_err;
   KernelLaunchConfig lc(L.grid, kDwpThreads, L.smem_bytes, false, stream);
-  cudaError_t e;
-  if (!L.expand)
-    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 1, false>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
-  else if (L.stride == 1)
-    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 1, true>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
-  else
-    e = cudaLaunchKernelEx(&lc.cfg, tc_dw_project_kernel<GEMM_BF16X3, 2, true>, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
+  constexpr int max_smem = 225 * 1024;
+  const cudaError_t e = with_form<GEMM_BF16X3, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
+    constexpr int EPI = decltype(form)::value;
+    if (!L.expand) return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 1, false, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
+    if (L.stride == 1) return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 1, true, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
+    return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 2, true, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
+  });
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1235,22 +1235,15 @@ std::string tc_plan_stem(TcStemLaunch* L, const TcStemConv& c, const TcEpilogue&
 }
 
 cudaError_t tc_launch_stem(const TcStemLaunch& L, cudaStream_t stream) {
-  static PerDeviceOnce attr_once;
-  const cudaError_t attr_err = attr_once.run([] {
-    cudaError_t e = cudaFuncSetAttribute(tc_stem_kernel<GEMM_BF16X3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tc_smem_budget(GEMM_BF16X3) + 1024);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_stem_kernel<GEMM_I8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               tc_smem_budget(GEMM_I8) + 1024);
-    return e;
-  });
-  if (attr_err != cudaSuccess) return attr_err;
   KernelLaunchConfig lc(L.grid, kStemThreads, L.smem_bytes, false, stream);
-  cudaError_t e;
-  if (L.kind == GEMM_I8)
-    e = cudaLaunchKernelEx(&lc.cfg, tc_stem_kernel<GEMM_I8>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-  else
-    e = cudaLaunchKernelEx(&lc.cfg, tc_stem_kernel<GEMM_BF16X3>, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  auto launch = [&](auto kind) {
+    constexpr int KIND = decltype(kind)::value;
+    return with_form<KIND, false>(L.p.out_mode, false, [&](auto form) {
+      if constexpr (decltype(form)::value % 2 == 1) return cudaErrorInvalidValue;  // (a stem has no residual)
+      else return launch_opted(tc_stem_kernel<KIND, decltype(form)::value>, tc_smem_budget(KIND) + 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+    });
+  };
+  const cudaError_t e = L.kind == GEMM_I8 ? launch(std::integral_constant<int, GEMM_I8>{}) : launch(std::integral_constant<int, GEMM_BF16X3>{});
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

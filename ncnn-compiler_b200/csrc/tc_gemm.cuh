@@ -189,7 +189,7 @@ __device__ __forceinline__ void tc_epilogue_chunk(const TcGemmParams& p, const u
 
 // SIDE: the instantiation that also writes int8 copies of its fp32 result (TcGemmParams::side_q); kept out
 // of the plain kernel so that layers without such copies run exactly the code they ran before.
-template <int KIND, bool SIDE = false>
+template <int KIND, int EPI, bool SIDE = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
 tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ CUtensorMap map_a0,
                const __grid_constant__ CUtensorMap map_a1,
@@ -517,6 +517,11 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
     d.out_scale = p.out_scale;
     d.wide = p.wide;
     d.chw = static_cast<long long>(p.OH) * p.OW;
+    constexpr int es = EPI / 2 == OUT_I8 ? 1 : (EPI / 2 == OUT_BF16X2 ? 2 : 4);
+    uint8_t* const out0 = EPI / 2 == OUT_I8 ? reinterpret_cast<uint8_t*>(p.outq) : reinterpret_cast<uint8_t*>(p.out0);
+    uint8_t* const out1 = reinterpret_cast<uint8_t*>(p.out1);
+    d.pitch = p.ldo * es;
+    d.pitch8 = 8 * d.pitch;
     d.xs = 8;
     d.ys = 4;
     d.stage = smem_base + static_cast<uint32_t>(S * SUB) * stage_bytes + static_cast<uint32_t>(group * 4 + quarter) * kDrainWarpBytes;
@@ -547,30 +552,29 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       if (tracing) p.trace[(tile / gridDim.x) * 16 + 4] = clock64();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                              static_cast<uint32_t>(acc) * (p.pair ? 256u : 128u) + (pair_tile && group ? 128u : 0u) + static_cast<uint32_t>(c_first);
-      if (lp.direct) {
-        const int es = lp.out_mode == OUT_I8 ? 1 : (lp.out_mode == OUT_BF16X2 ? 2 : 4);
-        long long at = m * lp.ldo + n_first;
-        if (lp.out_mode == OUT_CHW) {
+      if constexpr (EPI != kEpiAny) {
+        if (EPI / 2 == OUT_CHW) {
           const int img = static_cast<int>(m / d.chw);
-          at = (static_cast<long long>(img) * lp.N + n_first) * d.chw + (m - img * d.chw);
+          d.o0 = out0 + ((static_cast<long long>(img) * lp.N + n_first) * d.chw + (m - img * d.chw)) * 4;
+        } else {
+          const long long at = (m - lane) * d.pitch + static_cast<long long>(n_first) * es;  // (the warp's first row)
+          d.o0 = out0 + at;
+          d.o1 = out1 + at;
+          const long long rows_left = lp.M - (m - lane);
+          d.rows = rows_left > 32 ? 32 : static_cast<int>(rows_left);
         }
-        if (lp.out_mode != OUT_CHW) at -= lane * lp.ldo;  // (the warp's first row)
-        d.o0 = (lp.out_mode == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + at * es;
-        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at * es;
-        d.pitch = lp.ldo * es;
-        d.pitch8 = 8 * d.pitch;
-        const long long rows_left = lp.M - (m - lane);
-        d.rows = rows_left > 32 ? 32 : static_cast<int>(rows_left);
-        const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
-        d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n_first) * rs;
-        d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n_first) * rs;
+        if (EPI % 2 == 1) {
+          const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
+          d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n_first) * rs;
+          d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n_first) * rs;
+        }
         d.bias = lp.bias != nullptr ? lp.bias + n_first : nullptr;
         d.scale = lp.scale + n_first;
         if (SIDE) {
           d.side_q0 = lp.side_q0 + m * lp.side_ld + n_first;
           d.side_q1 = lp.side_q1 + m * lp.side_ld + n_first;
         }
-        tc_drain<KIND, SIDE, false, true>(d, t_row, cols, lp.N - n_first, valid);
+        tc_drain<KIND, EPI, SIDE, false>(d, t_row, cols, lp.N - n_first, valid);
       } else {
         const bool bf16_io = lp.out_mode == OUT_BF16X2 || lp.res_mode == RES_BF16X2;
         for (int c0 = 0; c0 < cols; c0 += 16) {

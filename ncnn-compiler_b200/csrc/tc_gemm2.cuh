@@ -101,7 +101,7 @@ struct Tc2Work {
   }
 };
 
-template <int KIND, bool PAIR>
+template <int KIND, bool PAIR, int EPI>
 __global__ void __launch_bounds__(kTc2Threads, 1)
 tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ CUtensorMap map_a0,
                 const __grid_constant__ CUtensorMap map_a1,
@@ -487,22 +487,25 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           }
         }
         const long long m = m_first + row;
-        const int es = lp.out_mode == OUT_I8 ? 1 : (lp.out_mode == OUT_BF16X2 ? 2 : 4);
-        const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
-        d.o0 = (lp.out_mode == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + ((m - lane) * lp.ldo + n0) * es;
-        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + ((m - lane) * lp.ldo + n0) * es;
+        constexpr int es = EPI / 2 == OUT_I8 ? 1 : (EPI / 2 == OUT_BF16X2 ? 2 : 4);
+        const long long at = ((m - lane) * lp.ldo + n0) * es;
+        d.o0 = (EPI / 2 == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + at;
+        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at;
         d.pitch = lp.ldo * es;
         d.pitch8 = 8 * d.pitch;
         const long long rows_left = lp.M - (m - lane);
         d.rows = rows_left > 32 ? 32 : static_cast<int>(rows_left);
-        d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n0) * rs;
-        d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n0) * rs;
+        if (EPI % 2 == 1) {
+          const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
+          d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n0) * rs;
+          d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n0) * rs;
+        }
         d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
         d.scale = lp.scale + n0;
         d.fix_count = fix;
         d.fix_ws = lp.sk_ws + static_cast<long long>(static_cast<int>(blockIdx.x) - CTAS) * static_cast<long long>(slot_words) +
                    ws_group + static_cast<size_t>(row) * 16;
-        tc_drain<KIND, false, true, false>(d, t_row, half, lp.N - n0, row_valid);
+        tc_drain<KIND, EPI, false, true>(d, t_row, half, lp.N - n0, row_valid);
         if (fix > 0) {
           // every warp of the group has read the slots: free them
           named_barrier_sync(bar_base, 128);

@@ -58,7 +58,7 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t smem_addr, uint32_t
 }
 
 // KIND is GEMM_BF16X3 (two planes: hi, mid) or GEMM_I8 (one plane)
-template <int KIND>
+template <int KIND, int EPI>
 __global__ void __launch_bounds__(kStemThreads, 1)
 tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ CUtensorMap map_a0,
                const __grid_constant__ CUtensorMap map_a1, const __grid_constant__ CUtensorMap map_b0,
@@ -257,7 +257,7 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
         d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at * es;
         d.pitch = static_cast<long long>(lp.N) * es;
         d.pitch8 = 8 * d.pitch;
-        tc_drain<KIND, false, false, false>(d, t_row, lp.N, lp.N, row < lp.OW);
+        tc_drain<KIND, EPI, false, false>(d, t_row, lp.N, lp.N, row < lp.OW);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
