@@ -65,6 +65,7 @@ __device__ __forceinline__ void cp_async_4(uint32_t smem_dst, const void* src, i
 
 template <int BM>
 static __global__ void __launch_bounds__(BM, 256 / BM) k_conv_f32(const float* __restrict__ x, ActRef out, const F32ConvParams p) {
+  ptx::grid_begin();
   constexpr int NT = BM;  // 8 x 8 results per thread
   constexpr int TX = kF32Bn / 8;
   constexpr int TY = NT / TX;  // thread (ty, tx): rows ty + TY * i, columns 16 * j + 2 * tx + {0, 1}

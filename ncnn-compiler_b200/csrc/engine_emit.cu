@@ -6,6 +6,24 @@ namespace nb {
 
 static cudaError_t launch_ok() { return cudaGetLastError(); }
 
+// Launches one of the plain kernels with programmatic stream serialisation, like the tensor-core kernels: its blocks are
+// set up while the kernel before it drains, and wait (grid_begin) before they touch any tensor.  A single image's pass
+// is a chain of launches of a few microseconds each, of which one or two were the gap to the next.
+template <class... Params, class... Args>
+static void launch_plain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = tc_pdl_enabled() ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 // fp32 contraction on the CUDA cores as a tiled kernel (conv_f32.cuh).  Needs plain fp32 input and 32-bit pixel numbers.
 static bool conv_f32_applies(const ActRef& in, const ConvGeom& g) {
   const long long rows = g.images * g.OH * g.OW, pixels = g.images * g.H * g.W;
@@ -45,8 +63,8 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
   if (ae != cudaSuccess) return cudaGetErrorString(ae);
   s->kernel = p.split ? "k_conv_f32:split" : "k_conv_f32";
   s->run = [=](cudaStream_t st) {
-    if (large) k_conv_f32<128><<<grid, 128, f32_smem_bytes(128), st>>>(x, out, p);
-    else k_conv_f32<64><<<grid, 64, f32_smem_bytes(64), st>>>(x, out, p);
+    if (large) launch_plain(k_conv_f32<128>, grid, 128, f32_smem_bytes(128), st, x, out, p);
+    else launch_plain(k_conv_f32<64>, grid, 64, f32_smem_bytes(64), st, x, out, p);
     return launch_ok();
   };
   return {};
@@ -97,10 +115,38 @@ bool EngineImpl::reads_caller_array(int input, int64_t n, const void* ptr) const
   return true;
 }
 
+// True when the tensor is a graph output in [channel][pixel] order whose only toucher is a convolution on
+// tc_gemm_kernel: its epilogue can write that order (one lane per pixel), which saves a pass over the result.
+bool EngineImpl::chw_result(int id) const {
+  const Tensor& t = tensors_[id];
+  if (t.rank != 3 || t.c == 1 || t.h * t.w == 1 || t.fmt != FMT_F32 || t.is_input || t.Cp != t.c || t.Wp != t.w) return false;
+  int entries = 0;
+  for (int o : outputs_) entries += resolve(o) == id ? 1 : 0;
+  if (entries != 1) return false;
+  const Node* producer = nullptr;
+  for (const Node& node : nodes_) {
+    for (int in : node.in)
+      if (resolve(in) == id) return false;
+    if (node.res >= 0 && resolve(node.res) == id) return false;
+    if (resolve(node.out) != id) continue;
+    if (producer != nullptr) return false;
+    producer = &node;
+  }
+  if (producer == nullptr) return false;
+  const Node& p = *producer;
+  if (p.kind != N_CONV || p.impl != IMPL_TC || p.stem || p.dw_fused || p.out_ld > 0 || !p.side_q.empty()) return false;
+  // (residual rows are read in 16-byte pieces)
+  if (p.res < 0) return true;
+  const int res_fmt = tensors_[resolve(p.res)].fmt;
+  return (res_fmt == FMT_F32 && p.O % 4 == 0) || (res_fmt == FMT_BF16X2 && p.O % 8 == 0);
+}
+
 // A graph output that a node writes as plain fp32 in the caller's order goes straight into the caller's array.
+// (A tensor-core convolution whose result nobody else reads writes [channel][pixel] order itself: OUT_CHW.)
 bool EngineImpl::writes_caller_array(int output, const void* ptr) const {
   const int id = resolve(outputs_[output]);
   const Tensor& t = tensors_[id];
+  if (chw_result(id)) return true;
   const bool flat = t.rank != 3 || ((t.c == 1 || t.h * t.w == 1) && t.Cp == t.c && t.Wp == t.w && t.w_off == 0);
   if (!flat || t.is_input || t.fmt != FMT_F32 || t.row_pitch > 0 || !aligned16(ptr)) return false;
   for (const Node& node : nodes_)
@@ -145,7 +191,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const int has_c = node.has_bias, scale_alpha = node.alpha != 1.0f;
       s.kernel = "k_gemm_i8_rowscale";
       s.run = [=](cudaStream_t st) {
-        k_gemm_i8_rowscale<<<static_cast<unsigned>(M), 128, K, st>>>(in, out, wq, K, N, s_b, c_bias, alpha, beta, has_c, scale_alpha);
+        launch_plain(k_gemm_i8_rowscale, static_cast<unsigned>(M), 128, K, st, in, out, wq, K, N, s_b, c_bias, alpha, beta, has_c, scale_alpha);
         return launch_ok();
       };
       steps.push_back(std::move(s));
@@ -186,7 +232,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       te.sk_ws_bytes = kTcSplitWorkspaceBytes;
       te.sk_flags = d_split_flags_;
       te.sk_flag_count = kTcSplitFlagCount;
-      te.out_mode = to.fmt == FMT_I8 ? OUT_I8 : (to.fmt == FMT_SPLIT ? OUT_F32_SPLIT : (to.fmt == FMT_TF32 ? OUT_F32_TF32 : (to.fmt == FMT_BF16X2 ? OUT_BF16X2 : OUT_F32)));
+      const bool caller_chw = !caller_array_.empty() && caller_array_[resolve(node.out)] != nullptr && chw_result(resolve(node.out));
+      te.out_mode = caller_chw ? OUT_CHW : to.fmt == FMT_I8 ? OUT_I8 : (to.fmt == FMT_SPLIT ? OUT_F32_SPLIT : (to.fmt == FMT_TF32 ? OUT_F32_TF32 : (to.fmt == FMT_BF16X2 ? OUT_BF16X2 : OUT_F32)));
       if (node.res >= 0) {
         const ActRef r = ref(node.res, n);
         te.res0 = r.p0;
@@ -385,8 +432,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
           const int grid = std::max(1, std::min(sm_count_, tasks));
           s.kernel = i8 ? "k_ip_rows<i8>" : "k_ip_rows<bf16x2>";
           s.run = [=](cudaStream_t st) {
-            if (i8) k_ip_rows<true><<<grid, kIpRowsThreads, smem, st>>>(ip);
-            else k_ip_rows<false><<<grid, kIpRowsThreads, smem, st>>>(ip);
+            if (i8) launch_plain(k_ip_rows<true>, grid, kIpRowsThreads, smem, st, ip);
+            else launch_plain(k_ip_rows<false>, grid, kIpRowsThreads, smem, st, ip);
             return launch_ok();
           };
           steps.push_back(std::move(s));
@@ -423,8 +470,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         const float* wf = static_cast<const float*>(w);
         s.kernel = "k_depthwise3x3_tile";
         s.run = [=](cudaStream_t st) {
-          if (stride == 1) k_depthwise3x3_tile<1><<<grid, 256, 0, st>>>(in, out, wf, g, e);
-          else k_depthwise3x3_tile<2><<<grid, 256, 0, st>>>(in, out, wf, g, e);
+          if (stride == 1) launch_plain(k_depthwise3x3_tile<1>, grid, 256, 0, st, in, out, wf, g, e);
+          else launch_plain(k_depthwise3x3_tile<2>, grid, 256, 0, st, in, out, wf, g, e);
           return launch_ok();
         };
       } else if (node.kind == N_DW) {
@@ -434,11 +481,11 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         s.kernel = i8 ? "k_depthwise<i8>" : "k_depthwise<f32>";
         s.run = [=](cudaStream_t st) {
           if (i8) {
-            if (vec) k_depthwise<4, true><<<grid, 256, 0, st>>>(in, out, w, g, e);
-            else k_depthwise<1, true><<<grid, 256, 0, st>>>(in, out, w, g, e);
+            if (vec) launch_plain(k_depthwise<4, true>, grid, 256, 0, st, in, out, w, g, e);
+            else launch_plain(k_depthwise<1, true>, grid, 256, 0, st, in, out, w, g, e);
           } else {
-            if (vec) k_depthwise<4, false><<<grid, 256, 0, st>>>(in, out, w, g, e);
-            else k_depthwise<1, false><<<grid, 256, 0, st>>>(in, out, w, g, e);
+            if (vec) launch_plain(k_depthwise<4, false>, grid, 256, 0, st, in, out, w, g, e);
+            else launch_plain(k_depthwise<1, false>, grid, 256, 0, st, in, out, w, g, e);
           }
           return launch_ok();
         };
@@ -449,8 +496,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         const int grid = grid_for(n * node.OH * node.OW * node.O);
         s.kernel = i8 ? "k_conv_direct<i8>" : "k_conv_direct<f32>";
         s.run = [=](cudaStream_t st) {
-          if (i8) k_conv_direct<true><<<grid, 256, 0, st>>>(in, out, w, g, e);
-          else k_conv_direct<false><<<grid, 256, 0, st>>>(in, out, w, g, e);
+          if (i8) launch_plain(k_conv_direct<true>, grid, 256, 0, st, in, out, w, g, e);
+          else launch_plain(k_conv_direct<false>, grid, 256, 0, st, in, out, w, g, e);
           return launch_ok();
         };
       }
@@ -471,8 +518,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const int grid = grid_for(M * N);
       s.kernel = i8 ? "k_matmul_direct<i8>" : "k_matmul_direct<f32>";
       s.run = [=](cudaStream_t st) {
-        if (i8) k_matmul_direct<true><<<grid, 256, 0, st>>>(in, out, w, M, K, N, e, 0.0f);
-        else k_matmul_direct<false><<<grid, 256, 0, st>>>(in, out, w, M, K, N, e, 0.0f);
+        if (i8) launch_plain(k_matmul_direct<true>, grid, 256, 0, st, in, out, w, M, K, N, e, 0.0f);
+        else launch_plain(k_matmul_direct<false>, grid, 256, 0, st, in, out, w, M, K, N, e, 0.0f);
         return launch_ok();
       };
       }
@@ -489,7 +536,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const long long count = to.logical() * n;
       const int grid = grid_for(count);
       m.run = [=](cudaStream_t st) {
-        k_binary<1><<<grid, 256, 0, st>>>(out, out, out, count, bp);
+        launch_plain(k_binary<1>, grid, 256, 0, st, out, out, out, count, bp);
         return launch_ok();
       };
       steps.push_back(std::move(m));
@@ -508,7 +555,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const dim3 grid(((p.OH + 7) / 8) * ((p.OW + 7) / 8), (p.C / 4 + 7) / 8, static_cast<unsigned>(n));
       s.kernel = "k_maxpool3x3s2_tile";
       s.run = [=](cudaStream_t st) {
-        k_maxpool3x3s2_tile<<<grid, 256, 0, st>>>(in, out, p);
+        launch_plain(k_maxpool3x3s2_tile, grid, 256, 0, st, in, out, p);
         return launch_ok();
       };
       steps.push_back(std::move(s));
@@ -520,7 +567,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const dim3 grid((p.C / 4 + 127) / 128, static_cast<unsigned>(n));
       s.kernel = "k_global_pool4";
       s.run = [=](cudaStream_t st) {
-        k_global_pool4<<<grid, 128, 0, st>>>(in, out, p);
+        launch_plain(k_global_pool4, grid, 128, 0, st, in, out, p);
         return launch_ok();
       };
       steps.push_back(std::move(s));
@@ -529,8 +576,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(n * p.OH * p.OW * (vec ? p.C / 4 : p.C));
     s.kernel = "k_pool";
     s.run = [=](cudaStream_t st) {
-      if (vec) k_pool<4><<<grid, 256, 0, st>>>(in, out, p);
-      else k_pool<1><<<grid, 256, 0, st>>>(in, out, p);
+      if (vec) launch_plain(k_pool<4>, grid, 256, 0, st, in, out, p);
+      else launch_plain(k_pool<1>, grid, 256, 0, st, in, out, p);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -545,7 +592,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(to.logical() * n);
     s.kernel = "k_deconv2x2";
     s.run = [=](cudaStream_t st) {
-      k_deconv2x2<<<grid, 256, 0, st>>>(in, out, w, bias, dp);
+      launch_plain(k_deconv2x2, grid, 256, 0, st, in, out, w, bias, dp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -558,7 +605,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(to.logical() * n);
     s.kernel = "k_reduce_mean";
     s.run = [=](cudaStream_t st) {
-      k_reduce_mean<<<grid, 256, 0, st>>>(in, out, rp);
+      launch_plain(k_reduce_mean, grid, 256, 0, st, in, out, rp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -571,7 +618,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(to.logical() * n);
     s.kernel = "k_remap";
     s.run = [=](cudaStream_t st) {
-      k_remap<<<grid, 256, 0, st>>>(in, out, rp);
+      launch_plain(k_remap, grid, 256, 0, st, in, out, rp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -586,7 +633,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(bp.o_image * n);
     s.kernel = "k_binary_broadcast";
     s.run = [=](cudaStream_t st) {
-      k_binary_broadcast<<<grid, 256, 0, st>>>(a, b, out, bp);
+      launch_plain(k_binary_broadcast, grid, 256, 0, st, a, b, out, bp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -601,8 +648,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(vec ? count / 4 : count);
     s.kernel = "k_binary";
     s.run = [=](cudaStream_t st) {
-      if (vec) k_binary<4><<<grid, 256, 0, st>>>(a, b, out, count, bp);
-      else k_binary<1><<<grid, 256, 0, st>>>(a, b, out, count, bp);
+      if (vec) launch_plain(k_binary<4>, grid, 256, 0, st, a, b, out, count, bp);
+      else launch_plain(k_binary<1>, grid, 256, 0, st, a, b, out, count, bp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -622,7 +669,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const int grid = grid_for(rows * (pitch / 4));
       s.kernel = "k_quantize_rows";
       s.run = [=](cudaStream_t st) {
-        k_quantize_rows<<<grid, 256, 0, st>>>(in, out.q, rows, K, pitch, scale);
+        launch_plain(k_quantize_rows, grid, 256, 0, st, in, out.q, rows, K, pitch, scale);
         return launch_ok();
       };
       steps.push_back(std::move(s));
@@ -641,7 +688,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const float scale2 = node.side_q.empty() ? 0.0f : node.side_q[0].second;
       s.kernel = node.side_q.empty() ? "k_quantize16" : "k_quantize16:two results";
       s.run = [=](cudaStream_t st) {
-        k_quantize16<<<grid16, 256, 0, st>>>(xp, yp, count / 16, scale, y2, scale2);
+        launch_plain(k_quantize16, grid16, 256, 0, st, xp, yp, count / 16, scale, y2, scale2);
         return launch_ok();
       };
       steps.push_back(std::move(s));
@@ -650,8 +697,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(vec ? count / 4 : count);
     s.kernel = "k_unary";
     s.run = [=](cudaStream_t st) {
-      if (vec) k_unary<4><<<grid, 256, 0, st>>>(in, out, count, up);
-      else k_unary<1><<<grid, 256, 0, st>>>(in, out, count, up);
+      if (vec) launch_plain(k_unary<4>, grid, 256, 0, st, in, out, count, up);
+      else launch_plain(k_unary<1>, grid, 256, 0, st, in, out, count, up);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -664,7 +711,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(n * sp.lines * 32);
     s.kernel = "k_softmax";
     s.run = [=](cudaStream_t st) {
-      k_softmax<<<grid, 256, 0, st>>>(in, out, sp);
+      launch_plain(k_softmax, grid, 256, 0, st, in, out, sp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -682,7 +729,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const int grid = grid_for(n * cp.in_image_elems);
       c.kernel = "k_concat_copy";
       c.run = [=](cudaStream_t st) {
-        k_concat_copy<<<grid, 256, 0, st>>>(in, out, cp);
+        launch_plain(k_concat_copy, grid, 256, 0, st, in, out, cp);
         return launch_ok();
       };
       steps.push_back(std::move(c));
@@ -696,7 +743,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
     const int grid = grid_for(rp.count * n);
     s.kernel = "k_relayout";
     s.run = [=](cudaStream_t st) {
-      k_relayout<<<grid, 256, 0, st>>>(in, out, rp);
+      launch_plain(k_relayout, grid, 256, 0, st, in, out, rp);
       return launch_ok();
     };
     steps.push_back(std::move(s));
@@ -729,7 +776,7 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
       int8_t* q = dst.q;
       s.kernel = "k_quantize16";
       s.run = [=](cudaStream_t st) {
-        k_quantize16<<<grid, 256, 0, st>>>(src_ptr, q, count16, scale, nullptr, 0.0f);
+        launch_plain(k_quantize16, grid, 256, 0, st, src_ptr, q, count16, scale, nullptr, 0.0f);
         return launch_ok();
       };
     } else if (!flat_in) {
@@ -748,21 +795,21 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
         const dim3 grid(static_cast<unsigned>(std::min(148 * 8, (t.h * t.w / 4 + 255) / 256)), static_cast<unsigned>(n));
         s.kernel = "k_chw_to_nhwc_small_x4";
         s.run = [=](cudaStream_t st) {
-          k_chw_to_nhwc_small_x4<<<grid, 256, 0, st>>>(src_ptr, dst, ep);
+          launch_plain(k_chw_to_nhwc_small_x4, grid, 256, 0, st, src_ptr, dst, ep);
           return launch_ok();
         };
       } else if (t.c <= 4 && (t.Cp == 4 || t.Cp == 16 || (t.Cp == 8 && t.fmt == FMT_I8) || (t.Cp == t.c && t.input_quant_scale <= 0.0f))) {
         const int grid = grid_for(n * t.h * t.w);
         s.kernel = "k_chw_to_nhwc_small";
         s.run = [=](cudaStream_t st) {
-          k_chw_to_nhwc_small<<<grid, 256, 0, st>>>(src_ptr, dst, ep);
+          launch_plain(k_chw_to_nhwc_small, grid, 256, 0, st, src_ptr, dst, ep);
           return launch_ok();
         };
       } else {
         const dim3 grid((t.h * t.w + 31) / 32, (t.c + 31) / 32, static_cast<unsigned>(n));
         s.kernel = "k_chw_to_nhwc_tiled";
         s.run = [=](cudaStream_t st) {
-          k_chw_to_nhwc_tiled<<<grid, dim3(32, 8), 0, st>>>(src_ptr, dst, ep);
+          launch_plain(k_chw_to_nhwc_tiled, grid, dim3(32, 8), 0, st, src_ptr, dst, ep);
           return launch_ok();
         };
       }
@@ -777,8 +824,8 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
       const int grid = grid_for(vec ? count / 4 : count);
       s.kernel = "k_unary";
       s.run = [=](cudaStream_t st) {
-        if (vec) k_unary<4><<<grid, 256, 0, st>>>(src, dst, count, up);
-        else k_unary<1><<<grid, 256, 0, st>>>(src, dst, count, up);
+        if (vec) launch_plain(k_unary<4>, grid, 256, 0, st, src, dst, count, up);
+        else launch_plain(k_unary<1>, grid, 256, 0, st, src, dst, count, up);
         return launch_ok();
       };
     }
@@ -798,7 +845,7 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
       const int C = t.c, HW = t.h * t.w, Cp = t.Cp;
       s.kernel = "k_nhwc_to_chw_tiled";
       s.run = [=](cudaStream_t st) {
-        k_nhwc_to_chw_tiled<<<grid, dim3(32, 8), 0, st>>>(src, dst_ptr, n, C, HW, Cp);
+        launch_plain(k_nhwc_to_chw_tiled, grid, dim3(32, 8), 0, st, src, dst_ptr, n, C, HW, Cp);
         return launch_ok();
       };
     } else {
@@ -812,8 +859,8 @@ void EngineImpl::make_edge_steps(int64_t n, const std::vector<const float*>& d_i
       const int grid = grid_for(vec ? count / 4 : count);
       s.kernel = "k_unary";
       s.run = [=](cudaStream_t st) {
-        if (vec) k_unary<4><<<grid, 256, 0, st>>>(src, dst, count, up);
-        else k_unary<1><<<grid, 256, 0, st>>>(src, dst, count, up);
+        if (vec) launch_plain(k_unary<4>, grid, 256, 0, st, src, dst, count, up);
+        else launch_plain(k_unary<1>, grid, 256, 0, st, src, dst, count, up);
         return launch_ok();
       };
     }

@@ -263,6 +263,7 @@ class EngineImpl {
   bool assemble(const Plan& plan, const std::vector<const float*>& d_in, const std::vector<float*>& d_out, std::vector<Step>* all);
   bool reads_caller_array(int input, int64_t n, const void* ptr) const;
   bool writes_caller_array(int output, const void* ptr) const;
+  bool chw_result(int id) const;
   bool takes_rows(const Node& node, int64_t n) const;
   int absorbed_quantize(const Node& node, int64_t n) const;
   int launch(Plan* plan, const float* const* d_in, float* const* d_out, cudaStream_t st);

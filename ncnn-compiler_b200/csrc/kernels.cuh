@@ -114,6 +114,7 @@ struct EdgeParams {
 };
 
 static __global__ void k_chw_to_nhwc_tiled(const float* __restrict__ src, ActRef dst, EdgeParams p) {
+  ptx::grid_begin();
   __shared__ float tile[32][33];
   const long long img = blockIdx.z;
   const int hw = p.H * p.W;
@@ -140,6 +141,7 @@ static __global__ void k_chw_to_nhwc_tiled(const float* __restrict__ src, ActRef
 // Few channels (C <= 4): one thread per pixel, one 16-byte store per plane (dense pixels of fewer than 4 channels: one
 // store per channel; the 32-channel tiles of the general kernel would be nine tenths empty: 56 -> 8 us for 8 x 3 x 224 x 224).
 static __global__ void k_chw_to_nhwc_small(const float* __restrict__ src, ActRef dst, EdgeParams p) {
+  ptx::grid_begin();
   const long long hw = static_cast<long long>(p.H) * p.W;
   const long long total = p.images * hw;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -168,6 +170,7 @@ static __global__ void k_chw_to_nhwc_small(const float* __restrict__ src, ActRef
 // Channel-last [image][HW][Cp] -> caller's [image][C][HW] fp32.
 static __global__ void k_nhwc_to_chw_tiled(ActRef src, float* __restrict__ dst, long long images, int C,
                                     int HW, int Cp) {
+  ptx::grid_begin();
   __shared__ float tile[32][33];
   const long long img = blockIdx.z;
   const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -187,6 +190,7 @@ static __global__ void k_nhwc_to_chw_tiled(ActRef src, float* __restrict__ dst, 
 // one thread per 4 consecutive pixels of a row, one 128-bit load per channel plane and 64 or
 // 32 contiguous bytes stored per output plane; grid = (row quads, images), 32-bit indices.
 static __global__ void k_chw_to_nhwc_small_x4(const float* __restrict__ src, ActRef dst, EdgeParams p) {
+  ptx::grid_begin();
   const int hw = p.H * p.W;
   const int quads = hw / 4;
   const long long img = blockIdx.y;
@@ -277,6 +281,7 @@ __device__ __forceinline__ float unary_apply(const UnaryParams& u, float v, long
 
 template <int VEC>
 static __global__ void k_unary(ActRef in, ActRef out, long long count, UnaryParams u) {
+  ptx::grid_begin();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * VEC;
   for (long long i = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * VEC;
        i < count; i += stride) {
@@ -302,6 +307,7 @@ __device__ __forceinline__ uint32_t quantize_pack4(const float4& v, float scale)
 }
 static __global__ void k_quantize16(const float* __restrict__ x, int8_t* __restrict__ y, long long count16, float scale,
                                     int8_t* __restrict__ y2, float scale2) {
+  ptx::grid_begin();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count16;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const float4* src = reinterpret_cast<const float4*>(x) + i * 4;
@@ -320,6 +326,7 @@ static __global__ void k_quantize16(const float* __restrict__ x, int8_t* __restr
 // tensor-core path can address them (TMA wants 16-byte row strides): 200 rows of 1001 through a layer of 1537 take
 // 14 us, 155 us on the CUDA cores.  Four results and one 4-byte store per thread.
 static __global__ void k_quantize_rows(ActRef in, int8_t* __restrict__ y, long long rows, int K, int pitch, float scale) {
+  ptx::grid_begin();
   const int quads = pitch / 4;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < rows * quads;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -361,6 +368,7 @@ __device__ __forceinline__ float binary_apply(const BinaryParams& b, float x, fl
 
 template <int VEC>
 static __global__ void k_binary(ActRef a, ActRef b, ActRef out, long long count, BinaryParams p) {
+  ptx::grid_begin();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x * VEC;
   for (long long i = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * VEC;
        i < count; i += stride) {
@@ -403,6 +411,7 @@ __device__ __forceinline__ void pool_store_side4(const PoolParams& p, long long 
 
 template <int VEC>
 static __global__ void k_pool(ActRef in, ActRef out, PoolParams p) {
+  ptx::grid_begin();
   const int cv = p.C / VEC;
   const long long total = p.images * p.OH * p.OW * cv;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -468,6 +477,7 @@ static __global__ void k_pool(ActRef in, ActRef out, PoolParams p) {
 // walks the pixels in the reference's order, seven loads in flight at a time (the generic kernel waits for every
 // pixel in turn: 49 memory latencies for a 7 x 7 image).
 static __global__ void __launch_bounds__(128) k_global_pool4(ActRef in, ActRef out, PoolParams p) {
+  ptx::grid_begin();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   const long long img = blockIdx.y;
   if (c >= p.C) return;
@@ -541,6 +551,7 @@ __device__ __forceinline__ float conv_finish_i8(const ConvEpilogue& e, int acc, 
 template <int VEC, bool INT8>
 static __global__ void k_depthwise(ActRef in, ActRef out, const void* __restrict__ weights, ConvGeom g,
                             ConvEpilogue e) {
+  ptx::grid_begin();
   const int cv = g.C / VEC;
   const long long total = g.images * g.OH * g.OW * cv;
   const float* wf = static_cast<const float*>(weights);
@@ -620,6 +631,7 @@ template <int STRIDE>
 static __global__ void __launch_bounds__(256) k_depthwise3x3_tile(ActRef in, ActRef out,
                                                                   const float* __restrict__ weights,
                                                                   ConvGeom g, ConvEpilogue e) {
+  ptx::grid_begin();
   constexpr int TO = 8;                      // output tile edge
   constexpr int TI = (TO - 1) * STRIDE + 3;  // input patch edge
   constexpr int CG = 8;                      // float4 channel groups per block
@@ -695,6 +707,7 @@ static __global__ void __launch_bounds__(256) k_depthwise3x3_tile(ActRef in, Act
 // fp32 inputs), then every thread takes the maximum over the taps that lie inside the image
 // (padding never wins, ConvertPooling, NCNNToTosa.cpp:1913-1954).
 static __global__ void __launch_bounds__(256) k_maxpool3x3s2_tile(ActRef in, ActRef out, PoolParams p) {
+  ptx::grid_begin();
   constexpr int TO = 8, TI = 17, CG = 8;
   constexpr int LOADS = (TI * TI * CG + 255) / 256;
   __shared__ float4 patch[TI * TI * CG];
@@ -764,6 +777,7 @@ __host__ __device__ __forceinline__ long long f32_weight_at(long long k, int o, 
 template <bool INT8>
 static __global__ void k_conv_direct(ActRef in, ActRef out, const void* __restrict__ weights, ConvGeom g,
                               ConvEpilogue e) {
+  ptx::grid_begin();
   const long long total = g.images * g.OH * g.OW * g.O;
   const float* wf = static_cast<const float*>(weights);
   const int8_t* wq = static_cast<const int8_t*>(weights);
@@ -806,6 +820,7 @@ static __global__ void k_conv_direct(ActRef in, ActRef out, const void* __restri
 template <bool INT8>
 static __global__ void k_matmul_direct(ActRef a, ActRef out, const void* __restrict__ weights,
                                 long long M, int K, int N, ConvEpilogue e, float gemm_beta_unused) {
+  ptx::grid_begin();
   const long long total = M * N;
   const float* wf = static_cast<const float*>(weights);
   const int8_t* wq = static_cast<const int8_t*>(weights);
@@ -841,6 +856,7 @@ static __global__ void k_gemm_i8_rowscale(ActRef a, ActRef out,
                                    const int8_t* __restrict__ wq /*[N][K]*/, int K, int N,
                                    float s_b, const float* __restrict__ c_bias, float alpha,
                                    float beta, int has_c, int scale_alpha) {
+  ptx::grid_begin();
   extern __shared__ int8_t row_q[];
   __shared__ float red[32];
   __shared__ float s_row;
@@ -882,6 +898,7 @@ struct SoftmaxParams {
 };
 
 static __global__ void k_softmax(ActRef in, ActRef out, SoftmaxParams p) {
+  ptx::grid_begin();
   const int lane = threadIdx.x & 31;
   const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   const long long total = p.images * p.lines;
@@ -913,6 +930,7 @@ struct ConcatParams {
 };
 
 static __global__ void k_concat_copy(ActRef in, ActRef out, ConcatParams p) {
+  ptx::grid_begin();
   const long long per = static_cast<long long>(p.outer) * p.len_in * p.inner;
   const long long total = p.images * per;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -957,6 +975,7 @@ __device__ __forceinline__ long long storage_offset(int rank, int c_dim, int h_d
 }
 
 static __global__ void k_relayout(ActRef in, ActRef out, RelayoutParams p) {
+  ptx::grid_begin();
   const long long total = p.images * p.count;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -1006,6 +1025,7 @@ struct DeconvParams {
 
 static __global__ void k_deconv2x2(ActRef in, ActRef out, const float* __restrict__ w,
                                    const float* __restrict__ bias, DeconvParams p) {
+  ptx::grid_begin();
   const long long total = p.images * 4ll * p.H * p.W * p.O;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -1036,6 +1056,7 @@ struct BroadcastParams {
 };
 
 static __global__ void k_binary_broadcast(ActRef a, ActRef b, ActRef out, BroadcastParams p) {
+  ptx::grid_begin();
   const long long total = p.images * p.o_image;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -1089,6 +1110,7 @@ __device__ __forceinline__ void bilinear_coordinate(int index, int in, int out, 
 }
 
 static __global__ void k_remap(ActRef in, ActRef out, RemapParams p) {
+  ptx::grid_begin();
   const long long in_image = static_cast<long long>(p.H) * p.W * p.C;
   const long long out_image = static_cast<long long>(p.OH) * p.OW * p.C;
   const long long total = p.images * out_image;
@@ -1137,6 +1159,7 @@ struct ReduceParams {
 };
 
 static __global__ void k_reduce_mean(ActRef in, ActRef out, ReduceParams p) {
+  ptx::grid_begin();
   const int oc = p.red_c ? 1 : p.C, oh = p.red_h ? 1 : p.H, ow = p.red_w ? 1 : p.W;
   const long long per = static_cast<long long>(oc) * oh * ow;
   const long long in_image = static_cast<long long>(p.C) * p.H * p.W;
@@ -1185,6 +1208,7 @@ struct QuantOpParams {
 };
 
 static __global__ void k_op_quantize(const float* __restrict__ x, int8_t* __restrict__ y, QuantOpParams p) {
+  ptx::grid_begin();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.count;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>((i / p.inner) % p.channels);
@@ -1193,6 +1217,7 @@ static __global__ void k_op_quantize(const float* __restrict__ x, int8_t* __rest
 }
 
 static __global__ void k_op_dequantize(const int* __restrict__ v, float* __restrict__ y, QuantOpParams p) {
+  ptx::grid_begin();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.count;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>((i / p.inner) % p.channels);
@@ -1203,6 +1228,7 @@ static __global__ void k_op_dequantize(const int* __restrict__ v, float* __restr
 }
 
 static __global__ void k_op_requantize(const int* __restrict__ v, int8_t* __restrict__ y, QuantOpParams p) {
+  ptx::grid_begin();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.count;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>((i / p.inner) % p.channels);

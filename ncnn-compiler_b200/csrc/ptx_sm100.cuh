@@ -192,6 +192,11 @@ __device__ __forceinline__ void tmem_alloc(uint32_t smem_result_addr, uint32_t n
                "r"(ncols)
                : "memory");
 }
+// both, for a kernel without a preamble worth the name
+__device__ __forceinline__ void grid_begin() {
+  grid_dependency_trigger();
+  grid_dependency_wait();
+}
 
 __device__ __forceinline__ void tmem_relinquish() {
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");

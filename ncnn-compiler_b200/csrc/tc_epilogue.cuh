@@ -16,6 +16,7 @@
 namespace nb {
 
 constexpr int kDrainWarpBytes = 4096;  // shared memory of one epilogue warp
+constexpr int kDrainSideBytes = 2048;  // and of each int8 copy
 
 // What one warp needs to finish its 32 rows.
 struct TcDirect {
@@ -36,8 +37,10 @@ struct TcDirect {
   int wide;             // residual rows are multiples of 32 bytes and 32-byte aligned: full-sector loads
   long long chw;        // OUT_CHW: elements between channels
   int side_count;       // int8 copies of an fp32 result
-  int8_t* side_q0;      // at this thread's row
-  int8_t* side_q1;
+  uint8_t* side_q0;     // at row 0 of the warp
+  uint8_t* side_q1;
+  long long side_pitch;
+  uint32_t side_stage;  // kDrainSideBytes of the warp's own per copy
   float side_scale0, side_scale1;
   // partial accumulators of other CTAs to add first (split tiles): slots fix_stride words apart, [16-column group][row][16]
   const uint32_t* fix_ws;
@@ -82,6 +85,14 @@ static __device__ __noinline__ void tc_act_many(float* y, int act, float a, floa
 __device__ __forceinline__ void sts_16b(uint32_t at, const uint32_t* w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
+// 16 fp32 results -> 16 int8 with the reference's rounding
+__device__ __forceinline__ void tc_stage_side_quant(uint32_t at, float scale, const float (&y)[16]) {
+  uint32_t w[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+    w[g] = pack_i8x4(quantize_rha(y[4 * g], scale), quantize_rha(y[4 * g + 1], scale), quantize_rha(y[4 * g + 2], scale), quantize_rha(y[4 * g + 3], scale));
+  sts_16b(at, w);
+}
 __device__ __forceinline__ uint4 lds_16b(uint32_t at) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
@@ -94,9 +105,9 @@ template <int CHUNKS>
 struct TcFlushLane {
   long long first;
   uint32_t rows;  // bit i: row i of this lane exists
-  __device__ __forceinline__ void init(const TcDirect& d) {
+  __device__ __forceinline__ void init(const TcDirect& d, long long pitch, long long pitch8) {
     const int r0 = static_cast<int>(threadIdx.x & 31) / CHUNKS;
-    first = (r0 >> 3) * d.pitch8 + (r0 & 7) * d.pitch;
+    first = (r0 >> 3) * pitch8 + (r0 & 7) * pitch;
     rows = (1u << CHUNKS) - 1u;
     if (d.rows >= 32 && d.xs >= 8 && d.ys >= 4) return;
 #pragma unroll
@@ -112,7 +123,8 @@ struct TcFlushLane {
 // and these line-wise reads meet every bank once.  The first `n0` bytes of a row belong to plane 0 at p0, the rest to
 // plane 1 at p1 (two planes: n0 = 64); `have` bytes of each plane's part exist.
 template <int CHUNKS>
-__device__ __forceinline__ void tc_flush(const TcDirect& d, const TcFlushLane<CHUNKS>& fl, uint8_t* p0, uint8_t* p1, int n0, int have) {
+__device__ __forceinline__ void tc_flush(uint32_t stage, long long pitch, long long pitch8, const TcFlushLane<CHUNKS>& fl, uint8_t* p0,
+                                         uint8_t* p1, int n0, int have) {
   __syncwarp();
   const int lane = threadIdx.x & 31;
   const int piece = lane % CHUNKS, r0 = lane / CHUNKS;
@@ -125,12 +137,12 @@ __device__ __forceinline__ void tc_flush(const TcDirect& d, const TcFlushLane<CH
   for (int i = 0; i < CHUNKS; ++i) {
     const int r = r0 + i * (32 / CHUNKS);
     const int swz = CHUNKS == 8 ? piece ^ (r & 7) : piece ^ ((r >> 1) & 3);
-    v[i] = lds_16b(d.stage + static_cast<uint32_t>(r * CHUNKS * 16 + swz * 16));
+    v[i] = lds_16b(stage + static_cast<uint32_t>(r * CHUNKS * 16 + swz * 16));
   }
 #pragma unroll
   for (int i = 0; i < CHUNKS; ++i) {
     // CHUNKS = 8: rows r0 + 4 i; CHUNKS = 4: rows r0 + 8 i
-    const long long off = CHUNKS == 8 ? (i >> 1) * d.pitch8 + (i & 1) * 4 * d.pitch : i * d.pitch8;
+    const long long off = CHUNKS == 8 ? (i >> 1) * pitch8 + (i & 1) * 4 * pitch : i * pitch8;
     if (rows & (1u << i)) *reinterpret_cast<uint4*>(p + off) = v[i];
   }
   __syncwarp();
@@ -160,7 +172,9 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
   const int row = threadIdx.x & 31;
   const uint32_t stage_row = d.stage + static_cast<uint32_t>(row) * 128u;
   TcFlushLane<OUT == OUT_I8 ? 4 : 8> fl;
-  if (OUT != OUT_CHW) fl.init(d);
+  if (OUT != OUT_CHW) fl.init(d, d.pitch, d.pitch8);
+  TcFlushLane<4> side_fl;
+  if (SIDE) side_fl.init(d, d.side_pitch, 8 * d.side_pitch);
   uint32_t nxt[16], r[RW];
   float bias[16], scale[16];
   auto fetch_res = [&](int c) {
@@ -252,7 +266,7 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
       sts_16b(d.stage + static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4)), w);
       if (piece == 3 || !more) {
         const int c64 = c & ~63;
-        if constexpr (OUT == OUT_I8) tc_flush<4>(d, fl, d.o0 + c64, nullptr, 64, min(left - c64, c - c64 + 16));
+        if constexpr (OUT == OUT_I8) tc_flush<4>(d.stage, d.pitch, d.pitch8, fl, d.o0 + c64, nullptr, 64, min(left - c64, c - c64 + 16));
       }
       continue;
     }
@@ -270,9 +284,18 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
 #pragma unroll
       for (int j = 0; j < 16; ++j) y[j] = t[j];
     }
-    if (SIDE && d.side_count > 0 && valid) {
-      tc_store_side_quant(d.side_q0 + c, d.side_scale0, y);
-      if (d.side_count > 1) tc_store_side_quant(d.side_q1 + c, d.side_scale1, y);
+    if (SIDE) {
+      // int8 copies, 64 columns to a flush
+      const int piece = (c >> 4) & 3, c64 = c & ~63;
+      const uint32_t at = d.side_stage + static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
+      tc_stage_side_quant(at, d.side_scale0, y);
+      if (d.side_count > 1) tc_stage_side_quant(at + kDrainSideBytes, d.side_scale1, y);
+      if (piece == 3 || !more) {
+        const int n = min(left - c64, c - c64 + 16);
+        tc_flush<4>(d.side_stage, d.side_pitch, 8 * d.side_pitch, side_fl, d.side_q0 + c64, nullptr, 64, n);
+        if (d.side_count > 1)
+          tc_flush<4>(d.side_stage + kDrainSideBytes, d.side_pitch, 8 * d.side_pitch, side_fl, d.side_q1 + c64, nullptr, 64, n);
+      }
     }
     if (OUT == OUT_CHW) {
       // neighbouring lanes are neighbouring pixels: every store is 128 consecutive bytes of a channel plane
@@ -295,7 +318,7 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
       put(2 * h + 1, hi + 4);
       put(4 + 2 * h, mid);
       put(4 + 2 * h + 1, mid + 4);
-      if (full) tc_flush<8>(d, fl, d.o0 + 2 * c32, d.o1 + 2 * c32, 64, 2 * step_cols);
+      if (full) tc_flush<8>(d.stage, d.pitch, d.pitch8, fl, d.o0 + 2 * c32, d.o1 + 2 * c32, 64, 2 * step_cols);
     } else if constexpr (OUT == OUT_F32_SPLIT) {
       uint32_t w[16], lo[16];
 #pragma unroll
@@ -309,14 +332,14 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
         put(q, w + 4 * q);
         put(4 + q, lo + 4 * q);
       }
-      tc_flush<8>(d, fl, d.o0 + 4 * c, d.o1 + 4 * c, 64, 4 * min(have, 16));
+      tc_flush<8>(d.stage, d.pitch, d.pitch8, fl, d.o0 + 4 * c, d.o1 + 4 * c, 64, 4 * min(have, 16));
     } else if constexpr (OUT == OUT_F32 || OUT == OUT_F32_TF32) {
       uint32_t w[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(OUT == OUT_F32_TF32 ? round_tf32(y[j]) : y[j]);
 #pragma unroll
       for (int q = 0; q < 4; ++q) put(4 * h + q, w + 4 * q);
-      if (full) tc_flush<8>(d, fl, d.o0 + 4 * c32, nullptr, 128, 4 * step_cols);
+      if (full) tc_flush<8>(d.stage, d.pitch, d.pitch8, fl, d.o0 + 4 * c32, nullptr, 128, 4 * step_cols);
     }
   }
 }

@@ -9,6 +9,15 @@
 #include <type_traits>
 
 namespace nb {
+
+bool tc_pdl_enabled() {
+  static const bool on = [] {
+    const char* f = std::getenv("NCNN_B200_PDL");
+    return f == nullptr || f[0] != '0';
+  }();
+  return on;
+}
+
 namespace {
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -194,6 +203,7 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   p.block_n = choose_block_n(p.tiles_m, N, sm_count, 16);
   p.tiles_n = (N + p.block_n - 1) / p.block_n;
   const int kTcSmemBudget = tc_smem_budget(kind);
+  const int drain = kDrainBytes + (e.side_count > 0 ? 8 * 2 * kDrainSideBytes : 0);  // (room for two int8 copies)
   const int planes = tc_planes(kind);
   // a stage holds the A tile(s) and block_n rows of B, every sub-buffer 1 KB aligned
   const int b_bytes = (p.block_n * p.row_bytes + 1023) / 1024 * 1024;
@@ -230,14 +240,14 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
     }
     const long long tiles_mixed = static_cast<long long>(p.tiles_m - best_rows) * p.tiles_n;
     if (best_rows > 0 && best < 0.97 * cost_single && tiles_mixed * 10 >= 9ll * sm_count &&
-        (kTcSmemBudget - kDrainBytes) / pair_stage >= 2) {
+        (kTcSmemBudget - drain) / pair_stage >= 2) {
       p.pair = 1;
       p.pair_rows = best_rows;
       p.tiles_m = p.tiles_m - best_rows;  // tile rows: best_rows pairs, then singles
       p.stage_bytes = pair_stage;
     }
   }
-  const int budget = kTcSmemBudget - kDrainBytes;
+  const int budget = kTcSmemBudget - drain;
   // int8 K blocks are two to four MMAs over 12-32 KB: arming and releasing a ring stage (~450 cycles of barrier
   // hand-shake per block, more than the block's copies and MMAs take) sets the pace.  A stage then holds several
   // K blocks (a divisor of their count, at least three stages deep): one hand-shake for all of them.
@@ -249,7 +259,7 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
         break;
       }
   p.stages = std::max(2, std::min(kTcMaxStages, budget / (p.sub_blocks * p.stage_bytes)));
-  L->smem_bytes = p.stages * p.sub_blocks * p.stage_bytes + kDrainBytes + 1024;
+  L->smem_bytes = p.stages * p.sub_blocks * p.stage_bytes + drain + 1024;
   // never fewer bytes than half an SM's shared memory: two CTAs must not share an
   // SM, each allocates tensor memory for itself
   L->smem_bytes = std::max(L->smem_bytes, 120 * 1024);
@@ -310,12 +320,6 @@ struct PerDeviceOnce {
   }
 };
 
-// NCNN_B200_PDL=0 launches every contraction kernel fully serialised behind its predecessor.
-bool pdl_enabled() {
-  static const bool on = env_int("NCNN_B200_PDL", 1) != 0;
-  return on;
-}
-
 // Launch attributes of the contraction kernels: clusters of two CTAs for the pair form, and programmatic
 // stream serialisation: the kernel's preamble (barriers, tensor memory, descriptor prefetch) may run while
 // the previous kernel of the stream drains; the kernel itself waits (grid_dependency_wait) before it
@@ -337,7 +341,7 @@ struct KernelLaunchConfig {
       attrs[cfg.numAttrs].val.clusterDim.z = 1;
       ++cfg.numAttrs;
     }
-    if (pdl_enabled()) {
+    if (tc_pdl_enabled()) {
       attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attrs[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
       ++cfg.numAttrs;

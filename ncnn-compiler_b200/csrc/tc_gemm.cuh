@@ -527,6 +527,9 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
     d.stage = smem_base + static_cast<uint32_t>(S * SUB) * stage_bytes + static_cast<uint32_t>(group * 4 + quarter) * kDrainWarpBytes;
     if (SIDE) {
       d.side_count = p.side_count;
+      d.side_pitch = p.side_ld;
+      d.side_stage = smem_base + static_cast<uint32_t>(S * SUB) * stage_bytes + 8u * kDrainWarpBytes +
+                     static_cast<uint32_t>(group * 4 + quarter) * 2u * kDrainSideBytes;
       d.side_scale0 = p.side_scale0;
       d.side_scale1 = p.side_scale1;
     }
@@ -571,8 +574,9 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
         d.bias = lp.bias != nullptr ? lp.bias + n_first : nullptr;
         d.scale = lp.scale + n_first;
         if (SIDE) {
-          d.side_q0 = lp.side_q0 + m * lp.side_ld + n_first;
-          d.side_q1 = lp.side_q1 + m * lp.side_ld + n_first;
+          const long long side_at = (m - lane) * lp.side_ld + n_first;
+          d.side_q0 = reinterpret_cast<uint8_t*>(lp.side_q0) + side_at;
+          d.side_q1 = reinterpret_cast<uint8_t*>(lp.side_q1) + side_at;
         }
         tc_drain<KIND, EPI, SIDE, false>(d, t_row, cols, lp.N - n_first, valid);
       } else {

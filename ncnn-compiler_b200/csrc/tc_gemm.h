@@ -97,6 +97,9 @@ std::string tc_plan_gemm(TcLaunch* launch, int kind, const void* a0, const void*
 
 cudaError_t tc_launch(const TcLaunch& launch, cudaStream_t stream);
 
+// NCNN_B200_PDL=0 launches every kernel fully serialised behind its predecessor.
+bool tc_pdl_enabled();
+
 // Packs [O][I][KH][KW] (ncnn order) weights into [O][KH*KW][c_blocks*k_elems] with
 // zero padding, channel innermost.  For fp32 kinds `hi` receives the values
 // rounded to tf32 (GEMM_TF32, GEMM_TF32X3) and `lo` the remainders (GEMM_TF32X3).

@@ -74,3 +74,18 @@ def test_device_arrays_in_place_at_any_alignment(pkg, tmp_path, m, int8):
             else:  # the rows kernel reads fp32 rows in place, bf16 pairs behind an edge launch
                 assert rel_l2(ref, want.reshape(m, n)) <= 1e-5
             assert (got[:shift_out] == 7.0).all() and (got[shift_out + m * n:] == 7.0).all()
+
+
+@pytest.mark.parametrize("cin,cout,k,stride,h,w,n", [
+    (64, 64, 3, 1, 9, 7, 3),    # tiles that span images
+    (32, 37, 1, 1, 5, 11, 2),   # channels in no whole 16-byte pieces
+    (8, 3, 3, 2, 33, 16, 1),
+    (64, 160, 3, 1, 16, 16, 9),
+])
+def test_convolution_writes_the_callers_order(pkg, oracle, tmp_path, cin, cout, k, stride, h, w, n):
+    """A convolution that is a graph output writes [channel][pixel] order from its epilogue."""
+    param, bin_ = pkg.zoo.single_conv(str(tmp_path / "c"), h=h, w=w, cin=cin, cout=cout, k=k, stride=stride, pad=k // 2)
+    x = np.random.default_rng(8).uniform(-1, 1, (n, cin, h, w)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    assert not any(r["kernel"].startswith("k_nhwc_to_chw") for r in m.profile(n, repeat=1))
+    assert rel_l2(m.run(x)[0], oracle_rows(oracle, param, bin_, x)) <= 3e-5
