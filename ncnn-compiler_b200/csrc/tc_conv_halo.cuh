@@ -232,8 +232,10 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
       int s = 0, ab = 0, acc = 0;
       uint32_t ph = 0, a_ph = 0, acc_ph = 0;
       bool ok = true;
+      // the next weight stage or patch is full / the next accumulator is free (see tc_k_block)
+      bool b_seen = false, a_seen = false, empty_seen = false;
       for (int tile = worker; tile < total_tiles && ok; tile += workers) {
-        if (!mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+        if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
           ok = false;
           break;
         }
@@ -241,7 +243,7 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc) * acc_stride;
         uint32_t accumulate = 0u;
         for (int cb = 0; cb < c_blocks && ok; ++cb) {
-          if (!mbar_wait_bounded(smem_u32(&a_full[ab]), a_ph, abort_ptr, kTcWaitLimitNs)) {
+          if (!a_seen && !mbar_wait_bounded(smem_u32(&a_full[ab]), a_ph, abort_ptr, kTcWaitLimitNs)) {
             ok = false;
             break;
           }
@@ -252,7 +254,7 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
           const bool tr = p.trace != nullptr && worker == workers / 2 && tile == worker && cb == 0;
           if (tr) p.trace[0] = clock64();
           for (int tap = 0; tap < taps; ++tap) {
-            if (!mbar_wait_bounded(smem_u32(&b_full[s]), ph, abort_ptr, kTcWaitLimitNs)) {
+            if (!b_seen && !mbar_wait_bounded(smem_u32(&b_full[s]), ph, abort_ptr, kTcWaitLimitNs)) {
               ok = false;
               break;
             }
@@ -260,42 +262,20 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
             if (tr && tap < 16) p.trace[16 + 4 * tap] = clock64();
             const uint64_t a0 = a_patch + static_cast<uint64_t>((kh * PW + kw) * 8);  // 128 B = 8 units
             const uint64_t b0 = b_fixed + (((b_ring + static_cast<uint32_t>(s) * b_stage_bytes) & 0x3ffffu) >> 4);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint64_t ka = a0 + 2u * k;
-              const uint64_t kb = b0 + 2u * k;
-              if (PAIR) {
-                if (KIND == GEMM_TF32) {
-                  mma_tf32_pair(d_tmem, ka, kb, idesc, accumulate);
-                } else if (KIND == GEMM_BF16X3) {
-                  mma_f16_pair(d_tmem, ka + patch_units, kb, idesc, accumulate);  // mid * hi
-                  mma_f16_pair(d_tmem, ka, kb + b_units, idesc, 1u);              // hi * mid
-                  mma_f16_pair(d_tmem, ka, kb, idesc, 1u);                        // hi * hi
-                } else {
-                  mma_tf32_pair(d_tmem, ka + patch_units, kb, idesc, accumulate);
-                  mma_tf32_pair(d_tmem, ka, kb + b_units, idesc, 1u);
-                  mma_tf32_pair(d_tmem, ka, kb, idesc, 1u);
-                }
-              } else if (KIND == GEMM_TF32) {
-                mma_tf32(d_tmem, ka, kb, idesc, accumulate);
-              } else if (KIND == GEMM_BF16X3) {
-                mma_f16(d_tmem, ka + patch_units, kb, idesc, accumulate);  // mid * hi
-                mma_f16(d_tmem, ka, kb + b_units, idesc, 1u);              // hi * mid
-                mma_f16(d_tmem, ka, kb, idesc, 1u);                        // hi * hi
-              } else {
-                mma_tf32(d_tmem, ka + patch_units, kb, idesc, accumulate);  // lo * hi
-                mma_tf32(d_tmem, ka, kb + b_units, idesc, 1u);              // hi * lo
-                mma_tf32(d_tmem, ka, kb, idesc, 1u);                        // hi * hi
-              }
-              accumulate = 1u;
+            tc_k_block<KIND, PAIR>(4, d_tmem, a0, patch_units, b0, b_units, idesc, accumulate);
+            accumulate = 1u;
+            const int next_s = s + 1 == S ? 0 : s + 1;
+            const uint32_t next_ph = s + 1 == S ? ph ^ 1u : ph;
+            b_seen = mbar_test_wait(smem_u32(&b_full[next_s]), next_ph);
+            if (tap + 1 == taps) {
+              a_seen = mbar_test_wait(smem_u32(&a_full[ab ^ 1]), ab == 1 ? a_ph ^ 1u : a_ph);
+              empty_seen = mbar_test_wait(smem_u32(&tempty_bar[acc ^ 1]), acc == 1 ? acc_ph : acc_ph ^ 1u);
             }
             if (PAIR) tc_commit_pair(smem_u32(&b_empty[s]), 3);
             else tc_commit(smem_u32(&b_empty[s]));
             if (tr && tap < 16) p.trace[16 + 4 * tap + 1] = clock64();
-            if (++s == S) {
-              s = 0;
-              ph ^= 1u;
-            }
+            s = next_s;
+            ph = next_ph;
             if (++kw == KW) {
               kw = 0;
               ++kh;

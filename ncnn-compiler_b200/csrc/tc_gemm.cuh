@@ -386,7 +386,6 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       // descriptors are formed by adding small constants to values computed once.
       // (the start-address field counts 16-byte units; a K step is 32 bytes = 2 units)
       const int k_steps = p.row_bytes / 32;
-      const int k_blocks = p.k_blocks;
       const uint64_t desc_fixed = smem_desc_kmajor(0u, static_cast<uint32_t>(p.row_bytes));
       const uint64_t a_first = desc_fixed + ((smem_base & 0x3ffffu) >> 4);
       const uint64_t stage_units = stage_bytes >> 4;
@@ -403,19 +402,19 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       int acc = 0;
       uint32_t acc_ph = 0;
       bool ok = true;
+      bool full_seen = false, empty_seen = false;  // the next stage is full / the next accumulator is free (see tc_k_block)
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        if (!mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, wait_limit)) {
+        if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, wait_limit)) {
           ok = false;
           break;
         }
         tc_fence_after_sync();
         if (tracing) p.trace[(tile / gridDim.x) * 16 + 1] = clock64();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc) * acc_stride;
-        const uint32_t d_tmem1 = d_tmem + 128u;
         const bool pair = tile / tiles_n < pair_rows;
         uint32_t accumulate = 0u;
         for (int kb = 0; kb < k_groups; ++kb) {
-          if (!mbar_wait_bounded(smem_u32(&full_bar[s]), ph, abort_ptr, wait_limit)) {
+          if (!full_seen && !mbar_wait_bounded(smem_u32(&full_bar[s]), ph, abort_ptr, wait_limit)) {
             ok = false;
             break;
           }
@@ -423,66 +422,21 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
           const bool tr = tracing && tile == static_cast<int>(gridDim.x) && kb < 32;
           if (tr) p.trace[1024 + kb * 4 + 2] = clock64();
           for (int sb = 0; sb < SUB; ++sb) {
-          const uint64_t a0 = a_first + static_cast<uint64_t>(s * SUB + sb) * stage_units;
-          const uint64_t b0 = a0 + b_from_a;
-          if (!pair) {
-#pragma unroll 4
-          for (int k = 0; k < k_steps; ++k) {
-            const uint64_t ka = a0 + 2u * k;
-            const uint64_t kbd = b0 + 2u * k;
-            if (KIND == GEMM_TF32) {
-              mma_tf32(d_tmem, ka, kbd, idesc, accumulate);
-            } else if (KIND == GEMM_TF32X3) {
-              mma_tf32(d_tmem, ka + slot_units, kbd, idesc, accumulate);  // lo * hi
-              mma_tf32(d_tmem, ka, kbd + b_slot_units, idesc, 1u);        // hi * lo
-              mma_tf32(d_tmem, ka, kbd, idesc, 1u);                       // hi * hi
-            } else if (KIND == GEMM_BF16X3) {
-              mma_f16(d_tmem, ka + slot_units, kbd, idesc, accumulate);  // mid * hi
-              mma_f16(d_tmem, ka, kbd + b_slot_units, idesc, 1u);        // hi * mid
-              mma_f16(d_tmem, ka, kbd, idesc, 1u);                       // hi * hi
-            } else {
-              mma_i8(d_tmem, ka, kbd, idesc, accumulate);
-            }
+            const uint64_t a0 = a_first + static_cast<uint64_t>(s * SUB + sb) * stage_units;
+            const uint64_t b0 = a0 + b_from_a;
+            if (pair) tc_k_block<KIND, false, true>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate, a1_from_a);
+            else tc_k_block<KIND, false>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate);
             accumulate = 1u;
           }
-          } else {
-            // both halves against the same B tile; each half has its own accumulator columns
-#pragma unroll 4
-            for (int k = 0; k < k_steps; ++k) {
-              const uint64_t ka = a0 + 2u * k;
-              const uint64_t ka1 = ka + a1_from_a;
-              const uint64_t kbd = b0 + 2u * k;
-              if (KIND == GEMM_TF32) {
-                mma_tf32(d_tmem, ka, kbd, idesc, accumulate);
-                mma_tf32(d_tmem1, ka1, kbd, idesc, accumulate);
-              } else if (KIND == GEMM_TF32X3) {
-                mma_tf32(d_tmem, ka + slot_units, kbd, idesc, accumulate);
-                mma_tf32(d_tmem, ka, kbd + b_slot_units, idesc, 1u);
-                mma_tf32(d_tmem, ka, kbd, idesc, 1u);
-                mma_tf32(d_tmem1, ka1 + slot_units, kbd, idesc, accumulate);
-                mma_tf32(d_tmem1, ka1, kbd + b_slot_units, idesc, 1u);
-                mma_tf32(d_tmem1, ka1, kbd, idesc, 1u);
-              } else if (KIND == GEMM_BF16X3) {
-                mma_f16(d_tmem, ka + slot_units, kbd, idesc, accumulate);
-                mma_f16(d_tmem, ka, kbd + b_slot_units, idesc, 1u);
-                mma_f16(d_tmem, ka, kbd, idesc, 1u);
-                mma_f16(d_tmem1, ka1 + slot_units, kbd, idesc, accumulate);
-                mma_f16(d_tmem1, ka1, kbd + b_slot_units, idesc, 1u);
-                mma_f16(d_tmem1, ka1, kbd, idesc, 1u);
-              } else {
-                mma_i8(d_tmem, ka, kbd, idesc, accumulate);
-                mma_i8(d_tmem1, ka1, kbd, idesc, accumulate);
-              }
-              accumulate = 1u;
-            }
-          }
-          }
+          const bool last = kb + 1 == k_groups;
+          const int next_s = s + 1 == S ? 0 : s + 1;
+          const uint32_t next_ph = s + 1 == S ? ph ^ 1u : ph;
+          full_seen = mbar_test_wait(smem_u32(&full_bar[next_s]), next_ph);
+          if (last) empty_seen = mbar_test_wait(smem_u32(&tempty_bar[acc + 1 == accs ? 0 : acc + 1]), acc + 1 == accs ? acc_ph : acc_ph ^ 1u);
           tc_commit(smem_u32(&empty_bar[s]));
           if (tr) p.trace[1024 + kb * 4 + 3] = clock64();
-          if (++s == S) {
-            s = 0;
-            ph ^= 1u;
-          }
+          s = next_s;
+          ph = next_ph;
         }
         if (!ok) break;
         tc_commit(smem_u32(&tfull_bar[acc]));

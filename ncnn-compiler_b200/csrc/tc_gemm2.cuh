@@ -288,10 +288,11 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
       int acc = 0;
       uint32_t acc_ph = 0;
       bool ok = true;
+      bool full_seen = false, empty_seen = false;  // the next stage is full / the next accumulator is free (see tc_k_block)
       for (int i = 0; i < work.nseg && ok; ++i) {
         int tile, kb0, kb1, owned;
         work.seg(i, &tile, &kb0, &kb1, &owned);
-        if (!mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+        if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
           ok = false;
           break;
         }
@@ -306,7 +307,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
         const bool ptr = p.trace != nullptr && blockIdx.x == trace_cta && i < 6;
         if (ptr) p.trace[512 + 8 * i] = clock64();
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait_bounded(smem_u32(&full_bar[s]), ph, abort_ptr, kTcWaitLimitNs)) {
+          if (!full_seen && !mbar_wait_bounded(smem_u32(&full_bar[s]), ph, abort_ptr, kTcWaitLimitNs)) {
             ok = false;
             break;
           }
@@ -314,48 +315,17 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           if (tracing && kb - kb0 < 40) p.trace[16 + 4 * (kb - kb0)] = clock64();
           const uint64_t a0 = a_first + static_cast<uint64_t>(s) * stage_units;
           const uint64_t b0 = a0 + b_from_a;
-#pragma unroll 4
-          for (int k = 0; k < k_steps; ++k) {
-            const uint64_t ka = a0 + 2u * k;
-            const uint64_t kbd = b0 + 2u * k;
-            if (PAIR) {
-              if (KIND == GEMM_TF32) {
-                mma_tf32_pair(d_tmem, ka, kbd, idesc, accumulate);
-              } else if (KIND == GEMM_TF32X3) {
-                mma_tf32_pair(d_tmem, ka + slot_units, kbd, idesc, accumulate);  // lo * hi
-                mma_tf32_pair(d_tmem, ka, kbd + b_slot_units, idesc, 1u);        // hi * lo
-                mma_tf32_pair(d_tmem, ka, kbd, idesc, 1u);                       // hi * hi
-              } else if (KIND == GEMM_BF16X3) {
-                mma_f16_pair(d_tmem, ka + slot_units, kbd, idesc, accumulate);  // mid * hi
-                mma_f16_pair(d_tmem, ka, kbd + b_slot_units, idesc, 1u);        // hi * mid
-                mma_f16_pair(d_tmem, ka, kbd, idesc, 1u);                       // hi * hi
-              } else {
-                mma_i8_pair(d_tmem, ka, kbd, idesc, accumulate);
-              }
-            } else {
-              if (KIND == GEMM_TF32) {
-                mma_tf32(d_tmem, ka, kbd, idesc, accumulate);
-              } else if (KIND == GEMM_TF32X3) {
-                mma_tf32(d_tmem, ka + slot_units, kbd, idesc, accumulate);
-                mma_tf32(d_tmem, ka, kbd + b_slot_units, idesc, 1u);
-                mma_tf32(d_tmem, ka, kbd, idesc, 1u);
-              } else if (KIND == GEMM_BF16X3) {
-                mma_f16(d_tmem, ka + slot_units, kbd, idesc, accumulate);
-                mma_f16(d_tmem, ka, kbd + b_slot_units, idesc, 1u);
-                mma_f16(d_tmem, ka, kbd, idesc, 1u);
-              } else {
-                mma_i8(d_tmem, ka, kbd, idesc, accumulate);
-              }
-            }
-            accumulate = 1u;
-          }
+          tc_k_block<KIND, PAIR>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate);
+          accumulate = 1u;
+          const int next_s = s + 1 == S ? 0 : s + 1;
+          const uint32_t next_ph = s + 1 == S ? ph ^ 1u : ph;
+          full_seen = mbar_test_wait(smem_u32(&full_bar[next_s]), next_ph);
+          if (kb + 1 == kb1) empty_seen = mbar_test_wait(smem_u32(&tempty_bar[acc ^ 1]), acc == 1 ? acc_ph : acc_ph ^ 1u);
           if (PAIR) tc_commit_pair(smem_u32(&empty_bar[s]), 3);  // the stage is free in both CTAs
           else tc_commit(smem_u32(&empty_bar[s]));
           if (tracing && kb - kb0 < 40) p.trace[16 + 4 * (kb - kb0) + 1] = clock64();
-          if (++s == S) {
-            s = 0;
-            ph ^= 1u;
-          }
+          s = next_s;
+          ph = next_ph;
         }
         if (!ok) break;
         if (PAIR) tc_commit_pair(smem_u32(&tfull_bar[acc]), 3);  // both CTAs' halves of the accumulator are complete
