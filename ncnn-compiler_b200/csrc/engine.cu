@@ -260,15 +260,31 @@ int EngineImpl::launch(Plan* plan, const float* const* d_in, float* const* d_out
   return 0;
 }
 
-// Reads back the device status word, waits for the stream and maps the outcome to a status.
-int EngineImpl::finish_host_run(cudaStream_t st) {
-  int status = 0;
-  cudaMemcpyAsync(&status, d_status_, 4, cudaMemcpyDeviceToHost, st);
+// Brings the results and the device status word back, waits for the stream and maps the outcome to a status.
+int EngineImpl::finish_host_run(Plan* plan, float* const* out, cudaStream_t st) {
+  // pinned memory: the status word first, then the results for pageable arrays
+  size_t total = 64;
+  std::vector<size_t> bytes(outputs_.size()), at(outputs_.size(), 0);
+  for (size_t i = 0; i < outputs_.size(); ++i) {
+    bytes[i] = tensors_[resolve(outputs_[i])].logical() * 4 * plan->n;
+    if (!HostStage::pageable(out[i]) || total + bytes[i] > HostStage::kResultBytes) continue;
+    at[i] = total;
+    total += (bytes[i] + 63) / 64 * 64;
+  }
+  uint8_t* pinned = stage_->result(total);
+  int local = 0;
+  for (size_t i = 0; i < outputs_.size(); ++i)
+    cudaMemcpyAsync(pinned != nullptr && at[i] != 0 ? static_cast<void*>(pinned + at[i]) : out[i], plan->d_out[i], bytes[i], cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(pinned != nullptr ? static_cast<void*>(pinned) : &local, d_status_, 4, cudaMemcpyDeviceToHost, st);
   const cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     error_ = std::string("execution failed: ") + cudaGetErrorString(e);
     return 6;
   }
+  if (pinned != nullptr)
+    for (size_t i = 0; i < outputs_.size(); ++i)
+      if (at[i] != 0) std::memcpy(out[i], pinned + at[i], bytes[i]);
+  const int status = pinned != nullptr ? *reinterpret_cast<const int*>(pinned) : local;
   if (status != 0) {
     error_ = "a tensor-core pipeline wait timed out (status " + std::to_string(status) + ")";
     cudaMemset(d_status_, 0, 4);
@@ -389,9 +405,7 @@ int EngineImpl::run_host_pipelined(Plan* plan, const float* const* in, float* co
     cudaStreamSynchronize(stream_);
     return 6;
   }
-  for (size_t i = 0; i < outputs_.size(); ++i)
-    cudaMemcpyAsync(out[i], plan->d_out[i], tensors_[resolve(outputs_[i])].logical() * 4 * n, cudaMemcpyDeviceToHost, stream_);
-  return finish_host_run(stream_);
+  return finish_host_run(plan, out, stream_);
 }
 
 int EngineImpl::run(int64_t n, const float* const* in, float* const* out, bool host, cudaStream_t user_stream) {
@@ -422,13 +436,12 @@ int EngineImpl::run(int64_t n, const float* const* in, float* const* out, bool h
   cudaStream_t st = host ? stream_ : user_stream;
   if (!host) return launch(plan, in, out, st);
   if (!ensure_staging(plan)) return 6;
+  stage_->begin_run();
   for (size_t i = 0; i < inputs_.size(); ++i)
-    cudaMemcpyAsync(plan->d_in[i], in[i], tensors_[resolve(inputs_[i])].logical() * 4 * n, cudaMemcpyHostToDevice, st);
+    stage_->upload(plan->d_in[i], in[i], tensors_[resolve(inputs_[i])].logical() * 4 * n, st);
   const int rc = launch(plan, plan->d_in.data(), plan->d_out.data(), st);
   if (rc != 0) return rc;
-  for (size_t i = 0; i < outputs_.size(); ++i)
-    cudaMemcpyAsync(out[i], plan->d_out[i], tensors_[resolve(outputs_[i])].logical() * 4 * n, cudaMemcpyDeviceToHost, st);
-  return finish_host_run(st);
+  return finish_host_run(plan, out, st);
 }
 
 int EngineImpl::profile(int64_t n, int repeat, std::vector<LayerTiming>* out) {

@@ -11,9 +11,11 @@
 #include <functional>
 #include <limits>
 #include <map>
+#include <memory>
 #include <sstream>
 
 #include "conv_f32.cuh"
+#include "host_stage.h"
 #include "ip_rows.cuh"
 #include "kernels.cuh"
 #include "loader.h"
@@ -246,6 +248,7 @@ class EngineImpl {
     for (auto& kv : plans_) kv.second.release();
     for (void* p : device_allocs_) cudaFree(p);
     if (arena_ != nullptr) cudaFree(arena_);
+    stage_.reset();
     for (cudaEvent_t e : upload_done_)
       if (e != nullptr) cudaEventDestroy(e);
     if (copy_stream_ != nullptr) cudaStreamDestroy(copy_stream_);
@@ -267,7 +270,7 @@ class EngineImpl {
   bool takes_rows(const Node& node, int64_t n) const;
   int absorbed_quantize(const Node& node, int64_t n) const;
   int launch(Plan* plan, const float* const* d_in, float* const* d_out, cudaStream_t st);
-  int finish_host_run(cudaStream_t st);
+  int finish_host_run(Plan* plan, float* const* out, cudaStream_t st);
   void choose_head_limit();
   void fold_channel_concats();
   void fuse_quantize_steps();
@@ -296,6 +299,7 @@ class EngineImpl {
   int* d_split_flags_ = nullptr;
   int sm_count_ = 148;
   cudaStream_t stream_ = nullptr;
+  std::unique_ptr<HostStage> stage_ = std::make_unique<HostStage>();
   cudaStream_t copy_stream_ = nullptr;  // uploads of the pipelined host-pointer path
   cudaEvent_t upload_done_[kMaxChunks] = {};
   // image window applied by ref(): tensors are laid out for layout_n_ images (0: the n
@@ -375,15 +379,12 @@ inline bool stem_rows_enabled() {
   return f == nullptr || f[0] != '0';
 }
 
-// The patch-resident convolution kernel applies to stride-1 filters; measured inside whole
-// networks (batch 64, 3x3 filters at 56/28/14 pixels) it ties with the im2col kernel once the
-// operands are bf16 pairs, and loses a little where its 16x8 tiles overhang the image, so it
-// is opt-in: NCNN_B200_HALO=1 at load time selects it wherever it applies (2: on pairs of CTAs).
+// Where the patch-resident convolution kernel takes a layer (tc_conv_halo.cuh): -1, the default, by measurement (see
+// halo_pays); NCNN_B200_HALO at load time: 0 nowhere, 1 wherever it applies, 2 the same on pairs of CTAs.
 inline int halo_level() {
   const char* f = std::getenv("NCNN_B200_HALO");
-  return f == nullptr || f[0] == 0 ? 0 : std::atoi(f);
+  return f == nullptr || f[0] == 0 ? -1 : std::atoi(f);
 }
-inline bool halo_preferred() { return halo_level() >= 1; }
 
 inline int env_int_or(const char* name, int fallback) {
   const char* f = std::getenv(name);

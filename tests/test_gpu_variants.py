@@ -89,3 +89,33 @@ def test_convolution_writes_the_callers_order(pkg, oracle, tmp_path, cin, cout, 
     m = pkg.Model(param, bin_)
     assert not any(r["kernel"].startswith("k_nhwc_to_chw") for r in m.profile(n, repeat=1))
     assert rel_l2(m.run(x)[0], oracle_rows(oracle, param, bin_, x)) <= 3e-5
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 511, 512])  # inputs of up to 64 KB and results of up to 4 MB go through pinned memory
+def test_small_host_arrays_through_pinned_memory(pkg, tmp_path, m):
+    import torch
+    k, n = 1024, 2048
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n)
+    model = pkg.Model(param, bin_)
+    for seed in range(2):
+        x = np.random.default_rng(seed).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+        got = model.run(x)[0]
+        xd, y = torch.from_numpy(x).cuda(), torch.empty((m, n), device="cuda")
+        model.run_device(m, [xd.data_ptr()], [y.data_ptr()], torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert np.array_equal(got.reshape(m, n), y.cpu().numpy())
+
+
+@pytest.mark.parametrize("h,w,n", [(56, 56, 22), (64, 24, 29), (41, 16, 60)])
+def test_patch_resident_convolution_by_default(pkg, tmp_path, monkeypatch, h, w, n):
+    """64 -> 64 channels: from four tiles per SM on, where the tiles fit the image, with the bits of the im2col kernel."""
+    param, bin_ = pkg.zoo.residual_block(str(tmp_path / "rb"), h=h, w=w, c=64, cout=64)
+    x = np.random.default_rng(9).uniform(-1, 1, (n, 64, h, w)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    halo = any("tc_conv_halo_kernel:pairs" in r["kernel"] for r in m.profile(n, repeat=1))
+    tiles = -(-h // 16) * -(-w // 8)
+    assert halo == (n * tiles >= 4 * 148 and h * w >= 0.85 * 128 * tiles)
+    got = m.run(x)[0]
+    assert np.array_equal(m.run(x[:1])[0], got[:1])
+    monkeypatch.setenv("NCNN_B200_HALO", "0")
+    assert np.array_equal(pkg.Model(param, bin_).run(x)[0], got)
