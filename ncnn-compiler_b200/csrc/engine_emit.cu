@@ -71,6 +71,17 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
 }
 
 
+// Where the patch-resident kernel on CTA pairs beats the im2col kernel: layers of one 64-channel block and at most 64
+// outputs, whose im2col tiles fetch every pixel nine times from L2 for few MMAs (64 -> 64 on 56x56, batch 64: 53.5
+// against 60 us, 59.4 against 63.7 us with a residual; 128 channels tie, one image is 0.5-1.5 us slower), and whose
+// 16x8 tiles overhang the image little and fill the SMs several times over.  With one channel block both kernels add
+// up an output's products in the same order, so the batch may decide.
+static bool halo_pays(int kind, int channels, const Node& node, int64_t n, int sm_count) {
+  if (kind != GEMM_BF16X3 || channels != 64 || node.O > 64 || node.KH * node.KW < 9) return false;
+  const int64_t tiles = static_cast<int64_t>((node.OH + kHaloTileH - 1) / kHaloTileH) * ((node.OW + kHaloTileW - 1) / kHaloTileW);
+  return n * tiles >= 4 * sm_count && static_cast<double>(node.OH) * node.OW >= 0.85 * (tiles * kHaloTileH * kHaloTileW);
+}
+
 // True when an InnerProduct / Gemm of this batch size runs on the kernel for a handful of rows (ip_rows.cuh): one pass
 // over the weights on the CUDA cores instead of mostly empty 128-row tiles.
 bool EngineImpl::takes_rows(const Node& node, int64_t n) const {
@@ -286,7 +297,8 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       }
       // stride-1 filters with spatial extent: the patch-resident kernel loads each input pixel
       // once per tile instead of once per tap
-      if (node.kind == N_CONV && !i8 && !node.stem && node.out_ld == 0 && halo_preferred() &&
+      const bool halo_pairs = halo_level() >= 2 || (halo_level() < 0 && halo_pays(kind, ti.c, node, n, sm_count_));
+      if (node.kind == N_CONV && !i8 && !node.stem && node.out_ld == 0 && (halo_pairs || halo_level() >= 1) &&
           tc_halo_applies(kind, ti.c, node.KH, node.KW, node.sh, node.sw, node.dh, node.dw, node.OH, node.OW, node.O,
                           te.out_mode)) {
         TcHaloConv hc;
@@ -306,7 +318,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         hc.w1 = node.d_w1;
         hc.out_channels = node.O;
         auto hl = std::make_shared<TcHaloLaunch>();
-        if (tc_plan_conv_halo(hl.get(), kind, hc, te, sm_count_, halo_level() >= 2).empty()) {
+        if (tc_plan_conv_halo(hl.get(), kind, hc, te, sm_count_, halo_pairs).empty()) {
           s.kernel = std::string(hl->pair ? "tc_conv_halo_kernel:pairs<" : "tc_conv_halo_kernel<") + kind_name + ">";
           s.run = [hl](cudaStream_t st) { return tc_launch_halo(*hl, st); };
           steps.push_back(std::move(s));
