@@ -74,10 +74,10 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
 // Where the patch-resident kernel on CTA pairs beats the im2col kernel: layers of one 64-channel block and at most 64
 // outputs, whose im2col tiles fetch every pixel nine times from L2 for few MMAs (64 -> 64 on 56x56, batch 64: 53.5
 // against 60 us, 59.4 against 63.7 us with a residual; 128 channels tie, one image is 0.5-1.5 us slower), and whose
-// 16x8 tiles overhang the image little and fill the SMs several times over.  With one channel block both kernels add
-// up an output's products in the same order, so the batch may decide.
+// 16x8 tiles overhang the image little and fill the SMs several times over.  With one channel block (and no chunks) both
+// kernels add up an output's products in the same order, so the batch may decide.
 static bool halo_pays(int kind, int channels, const Node& node, int64_t n, int sm_count) {
-  if (kind != GEMM_BF16X3 || channels != 64 || node.O > 64 || node.KH * node.KW < 9) return false;
+  if (kind != GEMM_BF16X3 || channels != 64 || node.O > 64 || node.KH * node.KW < 9 || node.KH * node.KW >= kTcChunkFrom) return false;
   const int64_t tiles = static_cast<int64_t>((node.OH + kHaloTileH - 1) / kHaloTileH) * ((node.OW + kHaloTileW - 1) / kHaloTileW);
   return n * tiles >= 4 * sm_count && static_cast<double>(node.OH) * node.OW >= 0.85 * (tiles * kHaloTileH * kHaloTileW);
 }

@@ -193,6 +193,41 @@ bool pair_enabled() {
 
 int env_int(const char* name, int fallback);
 
+// The chunks of a contraction's sums, from the layer alone (see kTcChunkFrom); p.k_blocks blocks of p.row_bytes.
+void set_chunks(TcGemmParams& p, int kind, int full_row_bytes) {
+  p.chunks = 1;
+  p.chunk_blocks = p.k_blocks;
+  p.split_k = 0;
+  const int per_block = full_row_bytes / p.row_bytes;  // a pair plan's half-size blocks
+  const int full = p.k_blocks / per_block;
+  if (kind != GEMM_BF16X3 || !p.a_im2col || full < kTcChunkFrom) return;
+  const int chunks = (full + kTcChunkBlocks - 1) / kTcChunkBlocks;
+  const int blocks = (full + chunks - 1) / chunks;
+  p.chunks = (full + blocks - 1) / blocks;
+  p.chunk_blocks = blocks * per_block;
+}
+
+// Chunks side by side: the tile width that does it fastest, or 0 where whole tiles are as fast.  In units of one K block
+// at 16 columns (0.40 us; 128 columns take 1.3 of them, measured): a unit's chunk and its share of the latency of
+// publishing and adding sums, and those sums' way through L2, against the whole tiles' K blocks.
+int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, int sm_count) {
+  if (p.chunks < 2 || e.sk_ws == nullptr || e.sk_flags == nullptr || env_int("NCNN_B200_SPLIT_K", 1) == 0) return 0;
+  auto tiles_of = [&](int bn) { return static_cast<long long>(p.tiles_m) * ((N + bn - 1) / bn); };
+  auto waves = [&](long long units) { return static_cast<double>((units + sm_count - 1) / sm_count); };
+  double best = 0.9 * waves(tiles_of(block_n)) * p.k_blocks * (1.0 + block_n / 400.0);
+  int width = 0;
+  for (int bn = 16; bn <= 128; bn += 16) {
+    const long long tiles = tiles_of(bn), units = tiles * p.chunks;
+    if (tiles * 8 > e.sk_flag_count || static_cast<size_t>(units) * kTcBlockM * bn * 4 > e.sk_ws_bytes) continue;
+    const double cost = waves(units) * (p.chunk_blocks + 3) * (1.0 + bn / 400.0) + 5.0 + static_cast<double>(units) * bn / 1600.0;
+    if (cost < best) {
+      best = cost;
+      width = bn;
+    }
+  }
+  return width;
+}
+
 void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e, int sm_count) {
   TcGemmParams& p = L->p;
   p.M = static_cast<int>(M);
@@ -201,6 +236,13 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   const int res_mode = res_mode_of(e);
   p.direct = direct_rows(kind, e, N, &p.wide) ? 1 : 0;
   p.block_n = choose_block_n(p.tiles_m, N, sm_count, 16);
+  set_chunks(p, kind, p.row_bytes);
+  if (const int width = split_width(p, e, N, p.block_n, sm_count)) {
+    p.block_n = width;
+    p.split_k = 1;
+  }
+  p.sk_ws = e.sk_ws;
+  p.sk_flags = e.sk_flags;
   p.tiles_n = (N + p.block_n - 1) / p.block_n;
   const int kTcSmemBudget = tc_smem_budget(kind);
   const int drain = kDrainBytes + (e.side_count > 0 ? 8 * 2 * kDrainSideBytes : 0);  // (room for two int8 copies)
@@ -216,7 +258,7 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   // (larger) stages.
   p.pair = 0;
   p.pair_rows = 0;
-  if (pair_enabled() && p.k_blocks >= 6 && p.block_n <= 128 && p.row_bytes >= 128) {
+  if (pair_enabled() && p.chunks == 1 && p.k_blocks >= 6 && p.block_n <= 128 && p.row_bytes >= 128) {
     const int pair_stage = planes * (2 * kTcBlockM * p.row_bytes + b_bytes);
     const long long waves_single = (tiles_total + sm_count - 1) / sm_count;
     const double cost_single = static_cast<double>(waves_single) * (kTcBlockM + p.block_n);
@@ -263,8 +305,8 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   // never fewer bytes than half an SM's shared memory: two CTAs must not share an
   // SM, each allocates tensor memory for itself
   L->smem_bytes = std::max(L->smem_bytes, 120 * 1024);
-  const long long tiles = static_cast<long long>(p.tiles_m) * p.tiles_n;
-  L->grid = static_cast<int>(std::min<long long>(tiles, sm_count));
+  const long long units = static_cast<long long>(p.tiles_m) * p.tiles_n * (p.split_k ? p.chunks : 1);
+  L->grid = static_cast<int>(std::min<long long>(units, sm_count));
   L->kind = kind;
   p.bias = e.bias;
   p.scale = e.scale;
@@ -464,6 +506,8 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   } else {
     p.streamk = can_split && may_split && (forced_split == 1 || cost_split < 0.95 * cost_whole) ? 1 : 0;
   }
+  set_chunks(p, kind, full_rb);
+  if (p.streamk) p.chunks = 1;  // (forced: a tile is cut where the workers' shares end)
   if (!p.streamk) workers = static_cast<int>(std::min<long long>(workers, tiles));
   p.sk_ws = e.sk_ws;
   p.sk_flags = e.sk_flags;

@@ -221,10 +221,14 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
   // ~450 cycles of arming and releasing a stage are paid once per SUB blocks
   const int SUB = KIND == GEMM_I8 ? (p.sub_blocks > 1 ? p.sub_blocks : 1) : 1;
   const int k_groups = p.k_blocks / SUB;
-  const int total_tiles = p.tiles_m * p.tiles_n;
-  // 512 TMEM columns: four accumulators (of a shallow contraction several tiles are in the pipeline at once), or two
-  // pairs of them
-  const int accs = p.pair ? 2 : 4;
+  // a unit of work is a tile, or one chunk of its K blocks
+  const int chunks = KIND == GEMM_BF16X3 ? p.chunks : 1;
+  const bool split_k = KIND == GEMM_BF16X3 && p.split_k != 0;
+  const int chunk_groups = chunks > 1 ? p.chunk_blocks : k_groups;  // (such contractions have one K block per stage)
+  const int units = p.tiles_m * p.tiles_n * (split_k ? chunks : 1);
+  // 512 TMEM columns: four accumulators (of a shallow contraction several tiles are in the pipeline at once), two
+  // pairs of them, or three and the running sum of the chunks
+  const int accs = chunks > 1 ? 3 : (p.pair ? 2 : 4);
   volatile int* abort_ptr = &abort_flag;
 
   if (threadIdx.x == 0) {
@@ -278,7 +282,10 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       uint32_t ph = 0;
       long long issued = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+        const int tile = split_k ? unit / chunks : unit;
+        const int kg0 = split_k ? (unit - tile * chunks) * chunk_groups : 0;
+        const int kg1 = split_k ? min(kg0 + chunk_groups, k_groups) : k_groups;
         const int m_blk = tile / p.tiles_n;
         const int n_blk = tile - m_blk * p.tiles_n;
         const bool pair_tile = m_blk < p.pair_rows;
@@ -305,17 +312,23 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
             w_base[half] = ow * p.stride_w - p.pad_l;
           }
         }
-        if (p.trace != nullptr && blockIdx.x == 0 && !is_b) p.trace[(tile / gridDim.x) * 16 + 0] = clock64();
+        if (p.trace != nullptr && blockIdx.x == 0 && !is_b) p.trace[(unit / gridDim.x) * 16 + 0] = clock64();
         // the current K block: channel block, filter row and column
         int cb = 0, kh = 0, kw = 0;
-        for (int kg = 0; kg < k_groups; ++kg) {
+        if (kg0 > 0) {
+          const int tap = kg0 / p.c_blocks;
+          cb = kg0 - tap * p.c_blocks;
+          kh = tap / p.KW;
+          kw = tap - kh * p.KW;
+        }
+        for (int kg = kg0; kg < kg1; ++kg) {
           const uint32_t fb = smem_u32(&full_bar[s]);
-          const bool stall = test_stall && kg == 0 && tile == static_cast<int>(blockIdx.x);
+          const bool stall = test_stall && kg == kg0 && unit == static_cast<int>(blockIdx.x);
           if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, wait_limit)) {
             ok = false;
             break;
           }
-          const bool tr = p.trace != nullptr && blockIdx.x == 0 && !is_b && tile == static_cast<int>(gridDim.x) && kg < 32;
+          const bool tr = p.trace != nullptr && blockIdx.x == 0 && !is_b && unit == static_cast<int>(gridDim.x) && kg < 32;
           if (tr) p.trace[1024 + kg * 4 + 0] = clock64();
           if (!stall) {
             mbar_arrive_expect_tx(fb, my_tx * static_cast<uint32_t>(SUB));
@@ -403,47 +416,55 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       uint32_t acc_ph = 0;
       bool ok = true;
       bool full_seen = false, empty_seen = false;  // the next stage is full / the next accumulator is free (see tc_k_block)
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, wait_limit)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after_sync();
-        if (tracing) p.trace[(tile / gridDim.x) * 16 + 1] = clock64();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc) * acc_stride;
-        const bool pair = tile / tiles_n < pair_rows;
-        uint32_t accumulate = 0u;
-        for (int kb = 0; kb < k_groups; ++kb) {
-          if (!full_seen && !mbar_wait_bounded(smem_u32(&full_bar[s]), ph, abort_ptr, wait_limit)) {
+      for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+        const int tile = split_k ? unit / chunks : unit;
+        // the accumulators of this unit: one, or one per chunk of a whole tile
+        int kb1 = split_k ? (unit - tile * chunks) * chunk_groups : 0;
+        const int kb_end = split_k ? min(kb1 + chunk_groups, k_groups) : k_groups;
+        while (kb1 < kb_end && ok) {
+          const int kb0 = kb1;
+          kb1 = min(kb0 + chunk_groups, kb_end);
+          if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, wait_limit)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const bool tr = tracing && tile == static_cast<int>(gridDim.x) && kb < 32;
-          if (tr) p.trace[1024 + kb * 4 + 2] = clock64();
-          for (int sb = 0; sb < SUB; ++sb) {
-            const uint64_t a0 = a_first + static_cast<uint64_t>(s * SUB + sb) * stage_units;
-            const uint64_t b0 = a0 + b_from_a;
-            if (pair) tc_k_block<KIND, false, true>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate, a1_from_a);
-            else tc_k_block<KIND, false>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate);
-            accumulate = 1u;
+          if (tracing) p.trace[(unit / gridDim.x) * 16 + 1] = clock64();
+          const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc) * acc_stride;
+          const bool pair = tile / tiles_n < pair_rows;
+          uint32_t accumulate = 0u;
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!full_seen && !mbar_wait_bounded(smem_u32(&full_bar[s]), ph, abort_ptr, wait_limit)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after_sync();
+            const bool tr = tracing && unit == static_cast<int>(gridDim.x) && kb < 32;
+            if (tr) p.trace[1024 + kb * 4 + 2] = clock64();
+            for (int sb = 0; sb < SUB; ++sb) {
+              const uint64_t a0 = a_first + static_cast<uint64_t>(s * SUB + sb) * stage_units;
+              const uint64_t b0 = a0 + b_from_a;
+              if (pair) tc_k_block<KIND, false, true>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate, a1_from_a);
+              else tc_k_block<KIND, false>(k_steps, d_tmem, a0, slot_units, b0, b_slot_units, idesc, accumulate);
+              accumulate = 1u;
+            }
+            const bool last = kb + 1 == kb1;
+            const int next_s = s + 1 == S ? 0 : s + 1;
+            const uint32_t next_ph = s + 1 == S ? ph ^ 1u : ph;
+            full_seen = mbar_test_wait(smem_u32(&full_bar[next_s]), next_ph);
+            if (last) empty_seen = mbar_test_wait(smem_u32(&tempty_bar[acc + 1 == accs ? 0 : acc + 1]), acc + 1 == accs ? acc_ph : acc_ph ^ 1u);
+            tc_commit(smem_u32(&empty_bar[s]));
+            if (tr) p.trace[1024 + kb * 4 + 3] = clock64();
+            s = next_s;
+            ph = next_ph;
           }
-          const bool last = kb + 1 == k_groups;
-          const int next_s = s + 1 == S ? 0 : s + 1;
-          const uint32_t next_ph = s + 1 == S ? ph ^ 1u : ph;
-          full_seen = mbar_test_wait(smem_u32(&full_bar[next_s]), next_ph);
-          if (last) empty_seen = mbar_test_wait(smem_u32(&tempty_bar[acc + 1 == accs ? 0 : acc + 1]), acc + 1 == accs ? acc_ph : acc_ph ^ 1u);
-          tc_commit(smem_u32(&empty_bar[s]));
-          if (tr) p.trace[1024 + kb * 4 + 3] = clock64();
-          s = next_s;
-          ph = next_ph;
-        }
-        if (!ok) break;
-        tc_commit(smem_u32(&tfull_bar[acc]));
-        if (tracing) p.trace[(tile / gridDim.x) * 16 + 2] = clock64();
-        if (++acc == accs) {
-          acc = 0;
-          acc_ph ^= 1u;
+          if (!ok) break;
+          tc_commit(smem_u32(&tfull_bar[acc]));
+          if (tracing) p.trace[(unit / gridDim.x) * 16 + 2] = clock64();
+          if (++acc == accs) {
+            acc = 0;
+            acc_ph ^= 1u;
+          }
         }
       }
       if (!ok) {
@@ -488,7 +509,8 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       d.side_scale1 = p.side_scale1;
     }
     const bool tracing = p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 64;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+      const int tile = split_k ? unit / chunks : unit;
       const int m_blk = tile / p.tiles_n;
       const int n_blk = tile - m_blk * p.tiles_n;
       const bool pair_tile = m_blk < p.pair_rows;
@@ -501,14 +523,52 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       const int cols = pair_tile ? p.block_n : (group ? p.block_n - half_cols : half_cols);
       const int n_first = n_blk * p.block_n + c_first;
       const bool valid = m < lp.M;
-      if (tracing) p.trace[(tile / gridDim.x) * 16 + 3] = clock64();
+      if (tracing) p.trace[(unit / gridDim.x) * 16 + 3] = clock64();
       // the vote keeps the warp together: tcgen05.ld below needs all 32 lanes
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, wait_limit) ? 1 : 0) != 0;
       if (!ok) break;
       tc_fence_after_sync();
-      if (tracing) p.trace[(tile / gridDim.x) * 16 + 4] = clock64();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                             static_cast<uint32_t>(acc) * (p.pair ? 256u : 128u) + (pair_tile && group ? 128u : 0u) + static_cast<uint32_t>(c_first);
+      if (tracing) p.trace[(unit / gridDim.x) * 16 + 4] = clock64();
+      uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                       static_cast<uint32_t>(acc) * (p.pair ? 256u : 128u) + (pair_tile && group ? 128u : 0u) + static_cast<uint32_t>(c_first);
+      if (KIND == GEMM_BF16X3 && chunks > 1) {
+        const uint32_t t_first = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c_first);
+        const uint32_t t_sum = t_first + 384u;
+        uint32_t* const ws = lp.sk_ws + static_cast<size_t>(unit) * kTcBlockM * lp.block_n +
+                             static_cast<size_t>(c_first) * kTcBlockM + static_cast<size_t>(row) * 16;
+        for (int c = split_k ? chunks - 1 : 0; c < chunks; ++c) {  // (split: this unit's chunk alone)
+          if (c > 0 && !split_k) {
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, wait_limit) ? 1 : 0) != 0;
+            if (!ok) break;
+            tc_fence_after_sync();
+            t_row = t_first + static_cast<uint32_t>(acc) * 128u;
+          }
+          if (split_k) tc_publish_chunk(t_row, ws, cols);
+          else tc_add_chunk(t_row, t_sum, cols, c == 0);
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
+          if (++acc == accs) {
+            acc = 0;
+            acc_ph ^= 1u;
+          }
+        }
+        if (!ok) break;
+        if (split_k) {
+          // whichever warp publishes these rows and columns last of the tile's chunks adds them up
+          int* const count = lp.sk_flags + tile * 8 + group * 4 + quarter;
+          __threadfence();
+          __syncwarp();
+          int before = 0;
+          if (lane == 0) before = atomicAdd(count, 1);
+          if (__shfl_sync(0xffffffffu, before, 0) != chunks - 1) continue;
+          if (lane == 0) *count = 0;  // for the next launch
+          __threadfence();
+          const size_t slot_words = static_cast<size_t>(kTcBlockM) * lp.block_n;
+          tc_gather_chunks(ws - static_cast<size_t>(unit - tile * chunks) * slot_words, slot_words, chunks, t_sum, cols);
+        }
+        t_row = t_sum;
+      }
       if constexpr (EPI != kEpiAny) {
         if (EPI / 2 == OUT_CHW) {
           const int img = static_cast<int>(m / d.chw);
@@ -547,9 +607,10 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
           }
         }
       }
+      if (tracing) p.trace[(unit / gridDim.x) * 16 + 5] = clock64();
+      if (KIND == GEMM_BF16X3 && chunks > 1) continue;  // (the accumulators were handed back above)
       tc_fence_before_sync();
       __syncwarp();
-      if (tracing) p.trace[(tile / gridDim.x) * 16 + 5] = clock64();
       if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
       if (++acc == accs) {
         acc = 0;

@@ -82,6 +82,13 @@ constexpr int kTcSplitFlagCount = 640;  // two per CTA (one per epilogue group)
 int tc_k_elems(int kind, int channels);
 int tc_row_bytes(int kind, int channels);
 
+// bf16-pair convolutions of at least kTcChunkFrom K blocks are summed in chunks of kTcChunkBlocks (blocks of 64 channels of
+// one filter tap): where a batch leaves SMs idle, the chunks of a tile run side by side, and where it does not, one CTA
+// adds up the same chunks, so that results do not depend on the batch.  A chunk costs a busy GPU ~0.3 us, a K block in a
+// row ~0.45: 7x7x512 -> 512 (72 blocks) 34.8 -> 20.6 us for one image, 35 -> 16 for 4, 36 -> 27 for 16, 44.2 -> 45.5 for 64.
+// (Chunks of 9: 16.6, 20, 54 and 46.7.)  At 36 blocks the few images gain 4 us a layer and batches lose 4 to 5.
+constexpr int kTcChunkFrom = 72, kTcChunkBlocks = 18;
+
 // Convolution: M = view.N*OH*OW pixels, N = out_channels.  `w0`/`w1` are the packed
 // weights [out_channels][KH*KW*c_blocks*k_elems] (see tc_pack_weights).
 // Returns an empty string on success, else the reason.

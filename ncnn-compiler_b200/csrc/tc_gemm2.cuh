@@ -47,6 +47,7 @@ struct Tc2Work {
   int nseg;
   int tail_first;  // the range ends inside a tile: that piece runs first
   int KB, G, worker, streamk;
+  int chunks, chunk_blocks;  // sums in chunks: each chunk of a tile is a piece
   long long tiles, U;
 
   __host__ __device__ __forceinline__ void init(const TcGemmParams& p, int worker_, int G_) {
@@ -54,6 +55,8 @@ struct Tc2Work {
     G = G_;
     worker = worker_;
     streamk = p.streamk;
+    chunks = p.chunks;
+    chunk_blocks = chunks > 1 ? p.chunk_blocks : KB;
     tiles = static_cast<long long>(p.tiles_m) * p.tiles_n;
     U = tiles * KB;
     tail_first = 0;
@@ -71,17 +74,18 @@ struct Tc2Work {
       nseg = t_last - t_first + 1;
       tail_first = (u1 - static_cast<long long>(t_last) * KB) < KB ? 1 : 0;
     } else {
-      nseg = worker < tiles ? static_cast<int>((tiles - worker + G - 1) / G) : 0;
+      nseg = worker < tiles ? static_cast<int>((tiles - worker + G - 1) / G) * chunks : 0;
     }
   }
 
   // piece i: its tile, its K blocks [kb0, kb1), and whether this worker finishes the tile
   __host__ __device__ __forceinline__ void seg(int i, int* tile, int* kb0, int* kb1, int* owned) const {
     if (!streamk) {
-      *tile = worker + i * G;
-      *kb0 = 0;
-      *kb1 = KB;
-      *owned = 1;
+      const int j = i / chunks, c = i - j * chunks;
+      *tile = worker + j * G;
+      *kb0 = c * chunk_blocks;
+      *kb1 = c + 1 == chunks ? KB : *kb0 + chunk_blocks;
+      *owned = c + 1 == chunks ? 1 : 0;
       return;
     }
     const int j = tail_first ? (i == 0 ? nseg - 1 : i - 1) : i;
@@ -130,6 +134,9 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
   const uint32_t b_slot = (stage_bytes / PLANES) - slot;  // this CTA's half of the B tile, rounded to 1 KB
   const int b_rows = p.block_n / CTAS;
   const int S = p.stages;
+  // sums in chunks: the first accumulator for every chunk, the running sum in place of the second (two accumulators of
+  // 256 columns are all of tensor memory)
+  const bool chunked = KIND == GEMM_BF16X3 && p.chunks > 1;
   volatile int* abort_ptr = &abort_flag;
 
   const unsigned trace_cta = (gridDim.x / 4u) * 2u;  // bring-up stamps come from a pair in the middle of the grid
@@ -320,7 +327,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           const int next_s = s + 1 == S ? 0 : s + 1;
           const uint32_t next_ph = s + 1 == S ? ph ^ 1u : ph;
           full_seen = mbar_test_wait(smem_u32(&full_bar[next_s]), next_ph);
-          if (kb + 1 == kb1) empty_seen = mbar_test_wait(smem_u32(&tempty_bar[acc ^ 1]), acc == 1 ? acc_ph : acc_ph ^ 1u);
+          if (kb + 1 == kb1) empty_seen = !chunked && mbar_test_wait(smem_u32(&tempty_bar[acc ^ 1]), acc == 1 ? acc_ph : acc_ph ^ 1u);
           if (PAIR) tc_commit_pair(smem_u32(&empty_bar[s]), 3);  // the stage is free in both CTAs
           else tc_commit(smem_u32(&empty_bar[s]));
           if (tracing && kb - kb0 < 40) p.trace[16 + 4 * (kb - kb0) + 1] = clock64();
@@ -338,7 +345,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           p.trace[512 + 8 * i + 1] = clock64();
           p.trace[512 + 8 * i + 5] = kb1 - kb0;
         }
-        acc ^= 1;
+        if (!chunked) acc ^= 1;
         if (acc == 0) acc_ph ^= 1u;
       }
       if (!ok) {
@@ -397,8 +404,20 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
         p.trace[512 + 8 * i + 2] = clock64();
         p.trace[512 + 8 * i + 6] = owned;
       }
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                             static_cast<uint32_t>(acc) * kTc2AccStride + static_cast<uint32_t>(col0);
+      uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                       static_cast<uint32_t>(acc) * kTc2AccStride + static_cast<uint32_t>(col0);
+      if (chunked) {
+        tc_add_chunk(t_row, t_row + kTc2AccStride, half, kb0 == 0);
+        t_row += kTc2AccStride;
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_cluster(tempty0);
+          else mbar_arrive(tempty0);
+        }
+        acc_ph ^= 1u;
+        if (!owned) continue;
+      }
       // this group's columns of a CTA's workspace slot: [16-column group][row][16]
       const size_t ws_group = static_cast<size_t>(col0 >> 4) * 128 * 16;
       if (!owned) {
@@ -487,6 +506,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
       __syncwarp();
       if (etr) p.trace[5] = clock64();
       if (eptr) p.trace[512 + 8 * i + 3] = clock64();
+      if (chunked) continue;  // (the accumulator was handed back above)
       if (lane == 0) {
         if (PAIR) mbar_arrive_cluster(acc ? tempty1 : tempty0);
         else mbar_arrive(acc ? tempty1 : tempty0);

@@ -98,6 +98,10 @@ struct TcGemmParams {
   int8_t* side_q1;
   float side_scale0, side_scale1;
   long long side_ld;   // row stride of the int8 copies in elements
+  // bf16-pair convolutions of deep contractions: the K blocks are summed in `chunks` groups of chunk_blocks each and the
+  // groups' sums added in order (tc_chunks: by the layer alone, so that every batch size rounds the same).  split_k = 1:
+  // the chunks of a tile run on different CTAs (tc_gemm_kernel).
+  int chunks, chunk_blocks, split_k;
   uint32_t* sk_ws;     // one slot of 128 x block_n accumulator words per CTA
   int* sk_flags;       // one word per CTA: 1 while its slot holds a partial that nobody has consumed
 };
@@ -152,6 +156,59 @@ __device__ __forceinline__ void tc_k_block(int steps, uint32_t d, uint64_t a, ui
   if (steps == 4) tc_k_steps<KIND, CTA_PAIR, 4, HALVES>(d, a, a_plane, b, b_plane, idesc, accumulate, a_half);
   else if (steps == 2) tc_k_steps<KIND, CTA_PAIR, 2, HALVES>(d, a, a_plane, b, b_plane, idesc, accumulate, a_half);
   else tc_k_steps<KIND, CTA_PAIR, 1, HALVES>(d, a, a_plane, b, b_plane, idesc, accumulate, a_half);
+}
+
+// ---- sums in chunks (see TcGemmParams::chunks)
+// Adds the accumulator of one chunk to the running sum of this warp's 32 rows, both in tensor memory (an epilogue thread
+// has no registers for the sums of a whole tile); `first`: starts the sum.  Every lane of the warp must call it.
+__device__ __forceinline__ void tc_add_chunk(uint32_t t_acc, uint32_t t_sum, int cols, bool first) {
+#pragma unroll 1
+  for (int c = 0; c < cols; c += 16) {
+    uint32_t v[16], s[16];
+    ptx::tmem_ld16(t_acc + static_cast<uint32_t>(c), v);
+    if (!first) ptx::tmem_ld16(t_sum + static_cast<uint32_t>(c), s);
+    ptx::tmem_ld_wait();
+    if (!first)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(s[j]), __uint_as_float(v[j])));
+    ptx::tmem_st16(t_sum + static_cast<uint32_t>(c), v);
+  }
+  ptx::tmem_st_wait();
+}
+// The same sum of chunks that different CTAs computed.  `ws` is this thread's row in the slot of a chunk
+// ([16-column group][row][16] words); the slots of a tile's chunks follow each other.
+__device__ __forceinline__ void tc_publish_chunk(uint32_t t_acc, uint32_t* ws, int cols) {
+#pragma unroll 1
+  for (int c = 0; c < cols; c += 16) {
+    uint32_t v[16];
+    ptx::tmem_ld16(t_acc + static_cast<uint32_t>(c), v);
+    ptx::tmem_ld_wait();
+    uint4* d = reinterpret_cast<uint4*>(ws + static_cast<size_t>(c) * 128);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) __stcg(d + q, make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+  }
+}
+__device__ __forceinline__ void tc_gather_chunks(const uint32_t* ws, size_t slot_words, int chunks, uint32_t t_sum, int cols) {
+#pragma unroll 1
+  for (int c = 0; c < cols; c += 16) {
+    float y[16];
+#pragma unroll 4
+    for (int k = 0; k < chunks; ++k) {
+      const float4* s = reinterpret_cast<const float4*>(ws + static_cast<size_t>(k) * slot_words + static_cast<size_t>(c) * 128);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 f = __ldcg(s + q);
+        const float w[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[4 * q + j] = k == 0 ? w[j] : __fadd_rn(y[4 * q + j], w[j]);
+      }
+    }
+    uint32_t v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(y[j]);
+    ptx::tmem_st16(t_sum + static_cast<uint32_t>(c), v);
+  }
+  ptx::tmem_st_wait();
 }
 
 // round-half-away-from-zero exactly as the reference evaluates it in fp32:

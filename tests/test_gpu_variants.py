@@ -119,3 +119,20 @@ def test_patch_resident_convolution_by_default(pkg, tmp_path, monkeypatch, h, w,
     assert np.array_equal(m.run(x[:1])[0], got[:1])
     monkeypatch.setenv("NCNN_B200_HALO", "0")
     assert np.array_equal(pkg.Model(param, bin_).run(x)[0], got)
+
+
+@pytest.mark.parametrize("cin,cout,k,h,w,many", [
+    (512, 80, 3, 7, 7, 30),    # 72 K blocks = 4 chunks; several tiles per image row block, a ragged last column tile
+    (328, 24, 5, 5, 9, 3),     # 64-byte operand rows, 275 blocks: chunks that do not divide them
+    (1160, 256, 3, 8, 16, 100) # whole tiles, and tiles of CTA pairs, that add up the same chunks
+])
+def test_deep_convolutions_sum_in_chunks(pkg, oracle, tmp_path, cin, cout, k, h, w, many):
+    """The chunks of a deep contraction run side by side for few images and one after the other for many: the same bits."""
+    param, bin_ = pkg.zoo.single_conv(str(tmp_path / "c"), h=h, w=w, cin=cin, cout=cout, k=k, stride=1, pad=k // 2)
+    x = np.random.default_rng(10).uniform(-1, 1, (many, cin, h, w)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    one = m.run(x[:1])[0]
+    assert rel_l2(one, oracle_rows(oracle, param, bin_, x[:1])) <= 3e-5
+    for n in (2, many):
+        for _ in range(2):
+            assert np.array_equal(m.run(x[:n])[0][:1], one)
