@@ -82,6 +82,15 @@ static bool halo_pays(int kind, int channels, const Node& node, int64_t n, int s
   return n * tiles >= 4 * sm_count && static_cast<double>(node.OH) * node.OW >= 0.85 * (tiles * kHaloTileH * kHaloTileW);
 }
 
+// Where the depthwise layer inside a projection is a launch of its own again: maps of at most 256 pixels in all.  The
+// fused kernel walks the channels in blocks of 32, ~1.2 us each and one after the other, on as many CTAs as there are
+// 128-pixel tiles; with one or two of those two launches are faster (one 14x14 image, 576 channels: 23 -> 9 us, 384: 17 ->
+// 8).  The same products in the same order (below the depth that is summed in chunks), so the batch may decide.
+static bool depthwise_apart(const Node& node, int64_t n) {
+  if (env_int_or("NCNN_B200_FUSE_DW", 1) >= 2) return false;  // in one kernel wherever it applies
+  return !node.ex_fused && n * node.OH * node.OW <= 256 && tc_row_bytes(GEMM_BF16X3, node.dw_c) != 0 && node.dw_c < kTcChunkFrom * 32;
+}
+
 // True when an InnerProduct / Gemm of this batch size runs on the kernel for a handful of rows (ip_rows.cuh): one pass
 // over the weights on the CUDA cores instead of mostly empty 128-row tiles.
 bool EngineImpl::takes_rows(const Node& node, int64_t n) const {
@@ -255,6 +264,58 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const char* kind_name = kind == GEMM_I8 ? "i8" : (kind == GEMM_TF32 ? "tf32" : (kind == GEMM_BF16X3 ? "bf16x3" : "tf32x3"));
       auto launch = std::make_shared<TcLaunch>();
       std::string perr;
+      if (node.dw_fused && depthwise_apart(node, n)) {
+        // the depthwise result as bf16 pairs in the workspace of split contractions (this one has too few K blocks to split)
+        const size_t plane = (static_cast<size_t>(n) * node.OH * node.OW * node.dw_c * 2 + 255) / 256 * 256;
+        ActRef mid;
+        mid.fmt = FMT_BF16X2;
+        mid.p0 = reinterpret_cast<float*>(d_split_ws_);
+        mid.p1 = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(d_split_ws_) + plane);
+        ConvGeom g{};
+        g.images = n;
+        g.H = g.OH = node.OH;
+        g.W = g.OW = node.OW;
+        g.C = g.O = node.dw_c;
+        g.KH = g.KW = 3;
+        g.sh = g.sw = g.dh = g.dw = 1;
+        g.pt = node.dw_pt;
+        g.pl = node.dw_pl;
+        ConvEpilogue de{};
+        de.bias = node.dw_bias;
+        de.act = node.dw_act;
+        de.act_a = node.dw_act_a;
+        de.act_b = node.dw_act_b;
+        const dim3 grid(((node.OH + 7) / 8) * ((node.OW + 7) / 8), (node.dw_c / 4 + 7) / 8, static_cast<unsigned>(n));
+        const float* dw = node.dw_w;
+        Step d = s;
+        d.name = node.dw_name;
+        d.kernel = "k_depthwise3x3_tile";
+        d.run = [=](cudaStream_t st) {
+          launch_plain(k_depthwise3x3_tile<1>, grid, 256, 0, st, in, mid, dw, g, de);
+          return launch_ok();
+        };
+        TcIm2colView v;
+        v.plane0 = mid.p0;
+        v.plane1 = mid.p1;
+        v.C = node.dw_c;
+        v.W = node.OW;
+        v.H = node.OH;
+        v.N = n;
+        v.stride_w = static_cast<uint64_t>(node.dw_c) * 2;
+        v.stride_h = v.stride_w * node.OW;
+        v.stride_n = v.stride_h * node.OH;
+        v.OH = node.OH;
+        v.OW = node.OW;
+        perr = tc_plan_conv(launch.get(), GEMM_BF16X3, v, node.d_w0, node.d_w1, node.O, te, sm_count_);
+        if (!perr.empty()) return fail(err, "layer " + node.name + ": " + perr);
+        d.flops = 18.0 * node.dw_c * node.OH * node.OW * n;
+        s.flops -= d.flops;
+        s.kernel = "tc_gemm_kernel<bf16x3>";
+        s.run = [launch](cudaStream_t st) { return tc_launch(*launch, st); };
+        steps.push_back(std::move(d));
+        steps.push_back(std::move(s));
+        return true;
+      }
       if (node.dw_fused) {
         TcDwProjConv dc;
         dc.x = in.p0;

@@ -136,3 +136,16 @@ def test_deep_convolutions_sum_in_chunks(pkg, oracle, tmp_path, cin, cout, k, h,
     for n in (2, many):
         for _ in range(2):
             assert np.array_equal(m.run(x[:n])[0][:1], one)
+
+
+@pytest.mark.parametrize("size,n", [(32, 64), (32, 65), (64, 4), (64, 5), (224, 1)])
+def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkeypatch, size, n):
+    """Maps of up to 256 pixels run the two layers apart: the bits of a batch that runs them in one kernel."""
+    param, bin_ = pkg.zoo.mobilenet_v2(str(tmp_path / "m"), size=size)
+    x = np.random.default_rng(11).uniform(-1, 1, (n + 8, 3, size, size)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    got = m.run(x[:n])[0]
+    assert np.array_equal(m.run(x)[0][:n], got)
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    monkeypatch.setenv("NCNN_B200_FUSE_EXPAND", "0")
+    assert rel_l2(got, pkg.Model(param, bin_).run(x[:n])[0]) <= 1e-5
