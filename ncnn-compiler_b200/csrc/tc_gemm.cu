@@ -343,25 +343,6 @@ int env_int(const char* name, int fallback) {
 
 int max_pairs_resident(int kind, int smem_bytes, int sm_count);
 
-// Function attributes (the opt-in to more than 48 KB of dynamic shared memory) belong to a device's
-// context: they are set once per device, with that device current, not once per process.
-struct PerDeviceOnce {
-  std::mutex mutex;
-  bool done[64] = {};
-  cudaError_t result[64] = {};
-  template <class F>
-  cudaError_t run(F&& setup) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!done[device]) {
-      result[device] = setup();
-      done[device] = true;
-    }
-    return result[device];
-  }
-};
-
 // Launch attributes of the contraction kernels: clusters of two CTAs for the pair form, and programmatic
 // stream serialisation: the kernel's preamble (barriers, tensor memory, descriptor prefetch) may run while
 // the previous kernel of the stream drains; the kernel itself waits (grid_dependency_wait) before it
@@ -682,7 +663,7 @@ cudaError_t with_form(int out_mode, bool res, F&& f) {
   return cudaErrorInvalidValue;
 }
 
-// Opts a kernel in to `smem` bytes of dynamic shared memory, once per device.
+// Opts a kernel in to `smem` bytes of dynamic shared memory, once per device (the attribute belongs to a device's context).
 template <class K>
 cudaError_t opt_in(K kernel, int smem) {
   static std::mutex mutex;
@@ -1320,14 +1301,11 @@ std::string tc_plan_stem_pool(TcStemPoolLaunch* L, const TcStemConv& c, const Tc
   pp.POH = pooled_h;
   pp.POW = pooled_w;
   pp.ring_row_bytes = (c.OW * N * 4 + 1023) / 1024 * 1024;
-  pp.stage_tile_bytes = (pooled_w * 64 + 1023) / 1024 * 1024;
-  pp.has_side = e_in.side_count;
+  pp.side_q = e_in.side_count ? e_in.side_q[0] : nullptr;
   pp.side_scale = e_in.side_count ? e_in.side_scale[0] : 0.0f;
   const int weights = c.KH * planes * conv.p.b_slot;
   const int stage = planes * conv.p.a_plane_bytes;
-  // staging tiles of 64-byte rows: bf16 pairs 2 planes x N / 32, fp32 N / 16 (+ one for the int8 copy)
-  const int tiles = i8 ? N / 16 + pp.has_side : 2 * (N / 32);
-  const int fixed = weights + pp.ring_row_bytes + tiles * pp.stage_tile_bytes + 1024;
+  const int fixed = weights + pp.ring_row_bytes + 1024;
   pp.row_stages = fixed + 4 * stage <= kStemPoolMaxSmem ? 4 : 2;
   L->smem_bytes = fixed + pp.row_stages * stage;
   if (L->smem_bytes > kStemPoolMaxSmem) return "shared memory cannot hold the weights, two row stages and a result row";
@@ -1340,35 +1318,13 @@ std::string tc_plan_stem_pool(TcStemPoolLaunch* L, const TcStemConv& c, const Tc
   L->map_a1 = conv.map_a1;
   L->map_b0 = conv.map_b0;
   L->map_b1 = conv.map_b1;
-  const uint64_t pixels = static_cast<uint64_t>(pooled_rows) * pooled_w;
-  if (i8) {
-    // pooled result: [pooled pixels][N] fp32, boxes of 16 channels x one pooled row; the int8 copy in one box
-    err = encode_tiled_2d(&L->map_o0, GEMM_TF32, e.out0, N, pixels, static_cast<uint64_t>(N) * 4, 16, static_cast<uint32_t>(pooled_w), 64);
-    if (err.empty() && pp.has_side)
-      err = encode_tiled_2d(&L->map_o1, GEMM_I8, e_in.side_q[0], N, pixels, static_cast<uint64_t>(N), 64, static_cast<uint32_t>(pooled_w), 64);
-    return err;
-  }
-  // pooled result: [pooled pixels][N] bf16 per plane, boxes of 32 channels x one pooled row, 64-byte swizzle
-  err = encode_tiled_2d(&L->map_o0, GEMM_BF16X3, e.out0, N, pixels, static_cast<uint64_t>(N) * 2, 32, static_cast<uint32_t>(pooled_w), 64);
-  if (err.empty())
-    err = encode_tiled_2d(&L->map_o1, GEMM_BF16X3, e.out1, N, pixels, static_cast<uint64_t>(N) * 2, 32, static_cast<uint32_t>(pooled_w), 64);
-  return err;
+  return {};
 }
 
 cudaError_t tc_launch_stem_pool(const TcStemPoolLaunch& L, cudaStream_t stream) {
-  static PerDeviceOnce attr_once;
-  const cudaError_t attr_err = attr_once.run([] {
-    cudaError_t e = cudaFuncSetAttribute(tc_stem_pool_kernel<GEMM_BF16X3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStemPoolMaxSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tc_stem_pool_kernel<GEMM_I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStemPoolMaxSmem);
-    return e;
-  });
-  if (attr_err != cudaSuccess) return attr_err;
   KernelLaunchConfig lc(L.grid, kStemPoolThreads, L.smem_bytes, false, stream);
-  const cudaError_t e =
-      L.kind == GEMM_I8 ? cudaLaunchKernelEx(&lc.cfg, tc_stem_pool_kernel<GEMM_I8>, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0, L.map_o1)
-                        : cudaLaunchKernelEx(&lc.cfg, tc_stem_pool_kernel<GEMM_BF16X3>, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1, L.map_o0,
-                                             L.map_o1);
+  const cudaError_t e = L.kind == GEMM_I8 ? launch_opted(tc_stem_pool_kernel<GEMM_I8>, kStemPoolMaxSmem, lc, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1)
+                                          : launch_opted(tc_stem_pool_kernel<GEMM_BF16X3>, kStemPoolMaxSmem, lc, L.pp, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -234,8 +234,6 @@ struct TcStemPoolLaunch {
   alignas(64) CUtensorMap map_a1{};
   alignas(64) CUtensorMap map_b0{};
   alignas(64) CUtensorMap map_b1{};
-  alignas(64) CUtensorMap map_o0{};  // pooled result: bf16 hi / mid planes, or fp32 and its int8 copy
-  alignas(64) CUtensorMap map_o1{};
   int grid = 0;
   int smem_bytes = 0;
   int kind = GEMM_BF16X3;

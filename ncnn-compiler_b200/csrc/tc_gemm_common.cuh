@@ -286,7 +286,7 @@ __device__ __forceinline__ void tc_store_side_quant(int8_t* q, float scale, cons
   *reinterpret_cast<uint4*>(q) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Operand and staging rows of 64 bytes with the 64-byte TMA swizzle: the 16-byte chunk j of row r lives at
+// Operand rows of 64 bytes with the 64-byte TMA swizzle: the 16-byte chunk j of row r lives at
 // r*64 + ((j ^ ((r >> 1) & 3)) * 16).
 __device__ __forceinline__ uint32_t stage_chunk_offset(int row, int j) {
   return static_cast<uint32_t>(row * 64 + ((j ^ ((row >> 1) & 3)) << 4));

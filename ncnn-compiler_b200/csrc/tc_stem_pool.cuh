@@ -5,15 +5,18 @@
 // order: 2j-1, 2j, 2j+1 for the first pooled row j of the range (or of an image), then two new rows per pooled
 // row, because row 2j+1 is also row 2(j+1)-1.  Every convolution row is computed like a tile of tc_stem_kernel
 // (input rows by TMA, windows read in place, three bf16 MMAs or one int8 MMA per K step; two MMA-issuing warps
-// take alternate rows).  Eight epilogue warps drain it from TMEM with bias and activation; a thread meets the
-// same pixel column and channels in every row, so the maximum over the three rows is kept in registers, and
-// the row that completes a pooled row writes it into one row of shared memory, from which the warps take the
-// maxima over pixels 2x-1 .. 2x+1, convert them and store the pooled row with TMA.  The stem's own result never
-// reaches HBM.  One convolution row per range is computed twice (2 % at 148 ranges over 64 x 56 pooled rows).
+// take alternate rows).  Eight epilogue warps drain it from TMEM; a thread meets the same pixel column and channels
+// in every row, so the maximum over the three rows is kept in registers, and the row that completes a pooled row
+// writes it into one row of shared memory, from which the warps take the maxima over pixels 2x-1 .. 2x+1, apply
+// scale, bias and activation, convert and store: a warp's 16- or 8-byte pieces are whole lines (as TMA stores of
+// 64-byte box rows they took 21 clocks a row).  The stem's own result never reaches HBM.
+// One convolution row per range is computed twice (2 % at 148 ranges over 64 x 56 pooled rows).
 // The values are those of the two separate kernels: the same bits.  Results: bf16 pairs (hi and mid planes)
 // for the bf16 form; fp32, and optionally an int8 copy Q(value, side_scale) for the int8 convolution that reads
 // the pooled tensor next, for the int8 form.
 #pragma once
+
+#include <type_traits>
 
 #include "tc_stem.cuh"
 
@@ -27,9 +30,8 @@ struct TcStemPoolParams {
   int images;
   int POH, POW;         // pooled extent: OH / 2, OW / 2 (3x3 windows, stride 2, one pixel of padding)
   int ring_row_bytes;   // the row of vertical maxima: OW x N fp32, rounded to 1 KB
-  int stage_tile_bytes; // one staging tile of the pooled row: POW rows x 64 bytes, rounded to 1 KB
   int row_stages;       // input row stages in shared memory: 4, or 2 where 4 do not fit
-  int has_side;         // fp32 results: an int8 copy leaves through the second output map
+  int8_t* side_q;       // fp32 results: their int8 copy, or null
   float side_scale;
 };
 
@@ -54,8 +56,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kStemPoolThreads, 1)
 tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_constant__ CUtensorMap map_a0,
                     const __grid_constant__ CUtensorMap map_a1, const __grid_constant__ CUtensorMap map_b0,
-                    const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_o0,
-                    const __grid_constant__ CUtensorMap map_o1) {
+                    const __grid_constant__ CUtensorMap map_b1) {
   using namespace ptx;
   const TcStemParams& p = pp.s;
   constexpr int PLANES = KIND == GEMM_I8 ? 1 : 2;
@@ -66,6 +67,7 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
   __shared__ __align__(8) uint64_t tfull_bar[4];   // four accumulators of 64 columns: two per MMA issuer
   __shared__ __align__(8) uint64_t tempty_bar[4];
   __shared__ __align__(8) uint64_t weights_bar;
+  __shared__ __align__(8) uint64_t ring_bar;  // the row of vertical maxima has been read
   __shared__ __align__(16) float tile_bias[128];
   __shared__ __align__(16) float tile_scale[128];
   __shared__ uint32_t tmem_slot;
@@ -79,7 +81,6 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
   const uint32_t a_region = b_region + static_cast<uint32_t>(p.KH * PLANES) * static_cast<uint32_t>(p.b_slot);
   const uint32_t stage_bytes = static_cast<uint32_t>(PLANES) * static_cast<uint32_t>(p.a_plane_bytes);
   const uint32_t ring = a_region + static_cast<uint32_t>(S) * stage_bytes;      // one row of vertical maxima, fp32
-  const uint32_t staging = ring + static_cast<uint32_t>(pp.ring_row_bytes);    // pooled row: tiles of [POW][64 B]
   volatile int* abort_ptr = &abort_flag;
 
   if (threadIdx.x == 0) {
@@ -91,6 +92,7 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
       mbar_init(smem_u32(&tempty_bar[i]), kStemPoolEpiThreads / 32);
     }
     mbar_init(smem_u32(&weights_bar), 1);
+    mbar_init(smem_u32(&ring_bar), kStemPoolEpiThreads / 32);
     fence_mbar_init();
     prefetch_tensormap(&map_a0);
     prefetch_tensormap(&map_b0);
@@ -98,8 +100,6 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
       prefetch_tensormap(&map_a1);
       prefetch_tensormap(&map_b1);
     }
-    prefetch_tensormap(&map_o0);
-    if (PLANES == 2 || pp.has_side) prefetch_tensormap(&map_o1);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&tmem_slot), 256);
@@ -232,27 +232,42 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
     const uint32_t mask = static_cast<uint32_t>(chunks > 16 ? 15 : chunks - 1);  // chunk ^ (pixel & mask): spreads the banks
     const uint32_t entry = static_cast<uint32_t>(p.N) * 4u;
     const int chunk_shift = p.N == 64 ? 4 : 3;
-    // none, ReLU and clip as one clamp (the planner admits no other activation): one copy of a many-way
-    // activation per value made this loop stall on instruction fetch
-    const float act_lo = p.act == ACT_RELU ? 0.0f : (p.act == ACT_CLIP ? p.act_a : -INFINITY);
-    const float act_hi = p.act == ACT_CLIP ? p.act_b : INFINITY;
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
-    // Vertical maxima stay in registers: this thread drains the same pixel column and the same channels of every
-    // convolution row, so the maximum over rows 2j-1, 2j, 2j+1 needs no shared memory.  `odd_row` holds this
-    // thread's values of the last odd row (row 2j+1 is also row 2(j+1)-1), `upper` the maximum of rows 2j-1 and 2j;
-    // the odd row that completes a pooled row writes max(upper, row) into the one row of shared memory from which
-    // the horizontal maxima are taken: a third of the shared-memory reads and half of the writes of pooling out
-    // of three stored rows, next to MMAs that read their operands from the same memory.
-    float odd_row[32], upper[32];
+    // What bounds this kernel is these warps' work per convolution row, so what can wait until a row is pooled does.
+    // Dequantisation, bias, activation and their roundings are monotone: the largest result is the result of the largest
+    // accumulator (the loader admits no negative scales), and a quarter of the values is left when they are applied:
+    // 64 images of 224x224, bf16 pairs 87 -> 73 us (256 images: 315 -> 234, now the MMAs' pace), int8 256: 320 -> 208.
+    // Vertical maxima stay in registers: this thread drains the same pixel column and the same channels of every row.
+    // `odd_row` holds its accumulators of the last odd row (row 2j+1 is also row 2(j+1)-1), `upper` the maximum of rows
+    // 2j-1 and 2j; the odd row that completes a pooled row writes max(upper, row) into the one row of shared memory from
+    // which the horizontal maxima are taken.
+    using Raw = std::conditional_t<KIND == GEMM_I8, int, float>;
+    auto raw_max = [](Raw a, Raw b) {
+      if constexpr (KIND == GEMM_I8) return max(a, b);
+      else return fmaxf(a, b);
+    };
+    Raw odd_row[32], upper[32];
+    int pooled = 0;  // pooled rows finished by this CTA
+    // the horizontal stage: this thread's four channels (the same for all its pixels)
+    const int hc = t & (chunks - 1);
+    const float4 bias4 = *reinterpret_cast<const float4*>(&tile_bias[4 * hc]);
+    const float4 scale4 = *reinterpret_cast<const float4*>(&tile_scale[4 * hc]);
+    // none, ReLU and clip as one clamp (the planner admits no other activation)
+    const float act_lo = p.act == ACT_RELU ? 0.0f : (p.act == ACT_CLIP ? p.act_a : -INFINITY);
+    const float act_hi = p.act == ACT_CLIP ? p.act_b : INFINITY;
+    auto finish = [&](Raw m, float scale, float bias) {
+      const float y = KIND == GEMM_I8 ? __fmul_rn(static_cast<float>(m), scale) : static_cast<float>(m);
+      return fminf(fmaxf(__fadd_rn(__fadd_rn(y, bias), 0.0f), act_lo), act_hi);
+    };
 #pragma unroll
-    for (int i = 0; i < 32; ++i) odd_row[i] = upper[i] = -INFINITY;
+    for (int i = 0; i < 32; ++i) odd_row[i] = upper[i] = Raw(0);
     stem_pool_rows(pp, [&](int img, int oh, int j, bool last, long long q) {
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
       if (!ok) return false;
       tc_fence_after_sync();
-      // ---- drain: bias and activation as the stand-alone epilogue
+      // ---- drain
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * 64u;
       const bool odd = (oh & 1) != 0;
       const bool row_above = oh > 0;  // an even row has row oh - 1 above it in `odd_row` unless it is the image's first
@@ -268,46 +283,39 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
       if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
       acc = (acc + 1) & 3;
       if (acc == 0) acc_ph ^= 1u;
+      if (last && !(ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&ring_bar), static_cast<uint32_t>(pooled & 1) ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0))
+        return false;
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         if (cc == 0 || two_chunks) {
           const int c0 = c_first + cc * 16;
-          const uint32_t (&v)[16] = vv[cc];
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            const float4 b4 = *reinterpret_cast<const float4*>(&tile_bias[c0 + 4 * g]);
-            float y[4];
-            if (KIND == GEMM_I8) {
-              // dequantise: float(accumulator) * scale[channel], then bias (the order of the stand-alone epilogue)
-              const float4 s4 = *reinterpret_cast<const float4*>(&tile_scale[c0 + 4 * g]);
-              y[0] = __fmul_rn(static_cast<float>(static_cast<int>(v[4 * g + 0])), s4.x);
-              y[1] = __fmul_rn(static_cast<float>(static_cast<int>(v[4 * g + 1])), s4.y);
-              y[2] = __fmul_rn(static_cast<float>(static_cast<int>(v[4 * g + 2])), s4.z);
-              y[3] = __fmul_rn(static_cast<float>(static_cast<int>(v[4 * g + 3])), s4.w);
-            } else {
-              y[0] = __uint_as_float(v[4 * g + 0]);
-              y[1] = __uint_as_float(v[4 * g + 1]);
-              y[2] = __uint_as_float(v[4 * g + 2]);
-              y[3] = __uint_as_float(v[4 * g + 3]);
+            Raw y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if constexpr (KIND == GEMM_I8) y[e] = static_cast<int>(vv[cc][4 * g + e]);
+              else y[e] = __uint_as_float(vv[cc][4 * g + e]);
             }
-            y[0] = fminf(fmaxf(__fadd_rn(__fadd_rn(y[0], b4.x), 0.0f), act_lo), act_hi);
-            y[1] = fminf(fmaxf(__fadd_rn(__fadd_rn(y[1], b4.y), 0.0f), act_lo), act_hi);
-            y[2] = fminf(fmaxf(__fadd_rn(__fadd_rn(y[2], b4.z), 0.0f), act_lo), act_hi);
-            y[3] = fminf(fmaxf(__fadd_rn(__fadd_rn(y[3], b4.w), 0.0f), act_lo), act_hi);
-            float* up = &upper[cc * 16 + 4 * g];
-            float* od = &odd_row[cc * 16 + 4 * g];
+            Raw* up = &upper[cc * 16 + 4 * g];
+            Raw* od = &odd_row[cc * 16 + 4 * g];
             if (!odd) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) up[e] = row_above ? fmaxf(od[e], y[e]) : y[e];
+              for (int e = 0; e < 4; ++e) up[e] = row_above ? raw_max(od[e], y[e]) : y[e];
             } else {
 #pragma unroll
               for (int e = 0; e < 4; ++e) od[e] = y[e];
               if (last && px < p.OW) {
                 const uint32_t chunk = static_cast<uint32_t>(c0 / 4 + g);
                 const uint32_t at = ring + static_cast<uint32_t>(px) * entry + ((chunk ^ (static_cast<uint32_t>(px) & mask)) << 4);
-                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(fmaxf(up[0], y[0])), "f"(fmaxf(up[1], y[1])),
-                             "f"(fmaxf(up[2], y[2])), "f"(fmaxf(up[3], y[3]))
-                             : "memory");
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const Raw r = raw_max(up[e], y[e]);
+                  if constexpr (KIND == GEMM_I8) w[e] = static_cast<uint32_t>(r);
+                  else w[e] = __float_as_uint(r);
+                }
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
               }
             }
           }
@@ -315,72 +323,51 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
       }
       if (last) {
         // ---- pooled row j: horizontal maxima over pixels 2x-1 .. 2x+1 of the row of vertical maxima
-        if (t == 0) tma_store_wait_read(0);  // the staging tiles of the pooled row before have been read out
         named_barrier_sync(1, kStemPoolEpiThreads);  // the row of vertical maxima is complete
         const int items = pp.POW * chunks;
-#pragma unroll 1
+#pragma unroll 2
         for (int item = t; item < items; item += kStemPoolEpiThreads) {
-          const int x = item >> chunk_shift, c = item & (chunks - 1);
+          const int x = item >> chunk_shift, c = hc;
           // (pixel -1 is replaced by pixel 0: a maximum does not change when an element is taken twice)
-          float4 v[3];
+          Raw v[3][4];
 #pragma unroll
           for (int dx = 0; dx < 3; ++dx) {
             const int sx = max(2 * x + dx - 1, 0);
             const uint32_t off = static_cast<uint32_t>(sx) * entry + ((static_cast<uint32_t>(c) ^ (static_cast<uint32_t>(sx) & mask)) << 4);
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[dx].x), "=f"(v[dx].y), "=f"(v[dx].z), "=f"(v[dx].w) : "r"(ring + off));
-          }
-          float4 m = v[0];
+            uint32_t w[4];
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(ring + off));
 #pragma unroll
-          for (int i = 1; i < 3; ++i) m = make_float4(fmaxf(m.x, v[i].x), fmaxf(m.y, v[i].y), fmaxf(m.z, v[i].z), fmaxf(m.w, v[i].w));
-          if (KIND == GEMM_I8) {
-            // fp32 results: staging [16-channel box][POW rows][64 bytes]; then the int8 copy, one tile of POW rows x N bytes
-            const uint32_t at = staging + static_cast<uint32_t>(c >> 2) * static_cast<uint32_t>(pp.stage_tile_bytes) + stage_chunk_offset(x, c & 3);
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(m.x), "f"(m.y), "f"(m.z), "f"(m.w) : "memory");
-            if (pp.has_side) {
-              const uint32_t word = (static_cast<uint32_t>(quantize_rha(m.x, pp.side_scale)) & 0xffu) |
-                                    ((static_cast<uint32_t>(quantize_rha(m.y, pp.side_scale)) & 0xffu) << 8) |
-                                    ((static_cast<uint32_t>(quantize_rha(m.z, pp.side_scale)) & 0xffu) << 16) |
-                                    ((static_cast<uint32_t>(quantize_rha(m.w, pp.side_scale)) & 0xffu) << 24);
-              const uint32_t side_at = staging + static_cast<uint32_t>(p.N / 16) * static_cast<uint32_t>(pp.stage_tile_bytes) +
-                                       stage_chunk_offset(x, c >> 2) + static_cast<uint32_t>((c & 3) * 4);
-              asm volatile("st.shared.b32 [%0], %1;" ::"r"(side_at), "r"(word) : "memory");
-            }
-          } else {
-            uint32_t hi0, mid0, hi1, mid1;
-            split_bf16x2(m.x, m.y, hi0, mid0);
-            split_bf16x2(m.z, m.w, hi1, mid1);
-            // staging: [plane][32-channel half][POW rows][64 bytes], 64-byte swizzle as the store expects
-            const int half = c >> 3, c8 = c & 7;
-            const uint32_t at = staging + static_cast<uint32_t>(half) * static_cast<uint32_t>(pp.stage_tile_bytes) +
-                                stage_chunk_offset(x, c8 >> 1) + static_cast<uint32_t>((c8 & 1) * 8);
-            const uint32_t plane = static_cast<uint32_t>((p.N + 31) / 32) * static_cast<uint32_t>(pp.stage_tile_bytes);
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(hi0), "r"(hi1) : "memory");
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + plane), "r"(mid0), "r"(mid1) : "memory");
-          }
-        }
-        fence_proxy_async_smem();
-        named_barrier_sync(1, kStemPoolEpiThreads);  // staged; and every read of the ring for this pooled row is done
-        if (t == 0) {
-          const int m_first = static_cast<int>(q) * pp.POW;  // pooled pixels before this row
-          if (KIND == GEMM_I8) {
-            const int boxes = p.N / 16;
-            for (int b = 0; b < boxes; ++b) tma_store_2d(&map_o0, staging + static_cast<uint32_t>(b) * pp.stage_tile_bytes, 16 * b, m_first);
-            if (pp.has_side) tma_store_2d(&map_o1, staging + static_cast<uint32_t>(boxes) * pp.stage_tile_bytes, 0, m_first);
-          } else {
-            const int halves = (p.N + 31) / 32;
-            for (int h = 0; h < halves; ++h) {
-              tma_store_2d(&map_o0, staging + static_cast<uint32_t>(h) * pp.stage_tile_bytes, 32 * h, m_first);
-              tma_store_2d(&map_o1, staging + static_cast<uint32_t>(halves + h) * pp.stage_tile_bytes, 32 * h, m_first);
+            for (int e = 0; e < 4; ++e) {
+              if constexpr (KIND == GEMM_I8) v[dx][e] = static_cast<int>(w[e]);
+              else v[dx][e] = __uint_as_float(w[e]);
             }
           }
-          tma_store_commit();
+          const float4 m = make_float4(finish(raw_max(raw_max(v[0][0], v[1][0]), v[2][0]), scale4.x, bias4.x),
+                                       finish(raw_max(raw_max(v[0][1], v[1][1]), v[2][1]), scale4.y, bias4.y),
+                                       finish(raw_max(raw_max(v[0][2], v[1][2]), v[2][2]), scale4.z, bias4.z),
+                                       finish(raw_max(raw_max(v[0][3], v[1][3]), v[2][3]), scale4.w, bias4.w));
+          const long long at = (q * pp.POW + x) * p.N + 4 * c;
+          if (KIND == GEMM_I8) {
+            *reinterpret_cast<float4*>(p.out0 + at) = m;
+            if (pp.side_q != nullptr)
+              *reinterpret_cast<uint32_t*>(pp.side_q + at) = pack_i8x4(quantize_rha(m.x, pp.side_scale), quantize_rha(m.y, pp.side_scale),
+                                                                       quantize_rha(m.z, pp.side_scale), quantize_rha(m.w, pp.side_scale));
+          } else {
+            uint2 hi, mid;
+            split_bf16x2(m.x, m.y, hi.x, mid.x);
+            split_bf16x2(m.z, m.w, hi.y, mid.y);
+            *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out0) + at) = hi;
+            *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out1) + at) = mid;
+          }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ring_bar));
+        ++pooled;
       }
       (void)img;
       return true;
     });
     if (!ok && lane == 0 && atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_EPILOGUE);
-    if (t == 0) tma_store_wait_all();
   }
 
   tc_fence_before_sync();
