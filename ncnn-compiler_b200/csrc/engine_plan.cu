@@ -186,7 +186,7 @@ bool EngineImpl::choose_impl(std::string* err) {
 
 // A channel Concat whose inputs are all single-use results of tensor-core convolutions needs no
 // copy: each convolution's epilogue already takes an output row stride, so it writes its
-// channels straight into the Concat's tensor (TMA stores clip at the convolution's own width).
+// channels straight into the Concat's tensor.
 // Offsets and the total width must keep every row 16-byte aligned in any format (multiples of 8).
 void EngineImpl::fold_channel_concats() {
   for (size_t k = 0; k < nodes_.size(); ++k) {

@@ -23,8 +23,8 @@ class HostStage {
   HostStage(const HostStage&) = delete;
   HostStage& operator=(const HostStage&) = delete;
   ~HostStage() {
-    if (input_ != nullptr) cudaFreeHost(input_);
-    if (result_ != nullptr) cudaFreeHost(result_);
+    if (first_ != nullptr) cudaFreeHost(first_);
+    if (large_ != nullptr) cudaFreeHost(large_);
   }
 
   static bool pageable(const void* p) {
@@ -42,8 +42,8 @@ class HostStage {
   // Queues the copy of one input to the device.
   cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     const size_t room = (bytes + 63) / 64 * 64;
-    if (used_ + room <= kInputBytes && pageable(src) && reserve(&input_, &input_bytes_, kInputBytes)) {
-      uint8_t* at = input_ + used_;
+    if (used_ + room <= kInputBytes && pageable(src) && open()) {
+      uint8_t* at = first_ + used_;
       used_ += room;
       std::memcpy(at, src, bytes);
       src = at;
@@ -53,30 +53,34 @@ class HostStage {
 
   // Pinned memory for the results of one run, or null when it cannot be had.
   uint8_t* result(size_t bytes) {
-    size_t want = 64u << 10;
+    if (bytes <= kSmallResult) return open() ? first_ + kInputBytes : nullptr;
+    if (bytes <= large_bytes_) return large_;
+    size_t want = 2 * kSmallResult;
     while (want < bytes) want *= 2;
-    return want <= kResultBytes && reserve(&result_, &result_bytes_, want) ? result_ : nullptr;
+    if (want > kResultBytes) return nullptr;
+    if (large_ != nullptr) cudaFreeHost(large_);
+    large_ = allocate(want);
+    large_bytes_ = large_ != nullptr ? want : 0;
+    return large_;
   }
 
  private:
-  static bool reserve(uint8_t** p, size_t* have, size_t want) {
-    if (*have >= want) return true;
-    if (*p != nullptr) cudaFreeHost(*p);
-    *p = nullptr;
-    *have = 0;
-    void* fresh = nullptr;
-    if (cudaHostAlloc(&fresh, want, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    *p = static_cast<uint8_t*>(fresh);
-    *have = want;
-    return true;
+  static constexpr size_t kSmallResult = 64u << 10;
+  static uint8_t* allocate(size_t bytes) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return static_cast<uint8_t*>(p);
+    cudaGetLastError();
+    return nullptr;
+  }
+  // (inputs and small results in one piece: an allocation is a large part of a model's first run)
+  bool open() {
+    if (first_ == nullptr) first_ = allocate(kInputBytes + kSmallResult);
+    return first_ != nullptr;
   }
 
-  uint8_t* input_ = nullptr;
-  uint8_t* result_ = nullptr;
-  size_t input_bytes_ = 0, result_bytes_ = 0, used_ = 0;
+  uint8_t* first_ = nullptr;
+  uint8_t* large_ = nullptr;
+  size_t large_bytes_ = 0, used_ = 0;
 };
 
 }  // namespace nb

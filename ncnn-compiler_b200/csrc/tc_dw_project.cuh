@@ -19,7 +19,7 @@
 //     64-byte-swizzled operand tile that tcgen05.mma reads,
 //   * one thread issues the projection's MMAs (mid*hi + hi*mid + hi*hi, as tc_gemm_kernel does) against
 //     that channel block's weights, which TMA streams through a small ring,
-// and the usual epilogue warps drain the accumulator (bias, residual, activation, TMA stores).
+// and the usual epilogue warps drain the accumulator (bias, residual, activation).
 // Without EXPAND the operands, their order and the accumulation are those of the two separate kernels, so the
 // results are the same bits.  With EXPAND the expand layer's products are the same too; only its bias is added
 // after the accumulation instead of by the epilogue of a separate kernel, which is the same fp32 addition.

@@ -375,7 +375,7 @@ struct KernelLaunchConfig {
 // True when tc_gemm2_kernel takes this contraction (on CTA pairs, or on single CTAs with tiles split
 // between them); fills the plan like finish_plan does.
 // `half_blocks_ok`: K blocks of half the size (64-byte rows) address the same packed operands, so
-// the plan may trade K-block size for staging tiles.
+// the plan may trade K-block size for ring stages.
 bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e, int sm_count,
                          bool half_blocks_ok) {
   TcGemmParams& p = L->p;

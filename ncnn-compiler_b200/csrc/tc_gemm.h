@@ -194,7 +194,7 @@ struct TcDwProjConv {
 };
 
 // True when the fused kernel takes the pair of layers: 3x3, stride 1, dilation 1, output extent equal to the
-// input's, channels in fours; projection 1x1 stride 1 with bf16-pair operands and a staged epilogue.
+// input's, channels in fours; projection 1x1 stride 1 with bf16-pair operands.
 bool tc_dw_project_applies(int C, int N, int H, int W, int out_mode, bool has_res, bool res_bf16);
 // True when the whole inverted-residual block (1x1 expand Cin -> C with at most 32 input channels, 3x3 depthwise of
 // stride 1 or 2 with output OH x OW, 1x1 projection C -> N) fits the fused kernel, whatever formats its output and
