@@ -509,20 +509,44 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       d.side_scale1 = p.side_scale1;
     }
     const bool tracing = p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 64;
+    // this thread's row and columns of a tile: rows of one half of a pair, or half of the columns
+    struct Share {
+      long long m;
+      int n_first, c_first, cols;
+      bool pair;
+    };
+    // An int8 layer's fp32 residual that has left L2 since it was written (126 MB) starts on its way back one tile ahead;
+    // the drain itself asks one step ahead only.  56x56x64, 256 images: 169 -> 156 us.  (28x28x128, which is still in L2,
+    // went from 84 to 88, and bf16-pair layers with long main loops gained nothing.)
+    const bool far_residual = KIND == GEMM_I8 && EPI != kEpiAny && EPI % 2 == 1 && lp.res_mode == RES_F32 &&
+                              static_cast<long long>(lp.M) * lp.ldo * 4 > (126ll << 20);
+    auto share = [&](int tile) {
+      const int m_blk = tile / p.tiles_n;
+      Share w;
+      w.pair = m_blk < p.pair_rows;
+      const long long m_tile = w.pair ? static_cast<long long>(m_blk) * (2 * kTcBlockM)
+                                      : static_cast<long long>(p.pair_rows) * (2 * kTcBlockM) +
+                                            static_cast<long long>(m_blk - p.pair_rows) * kTcBlockM;
+      w.m = m_tile + (w.pair && group ? kTcBlockM : 0) + row;
+      w.c_first = !w.pair && group ? half_cols : 0;
+      w.cols = w.pair ? p.block_n : (group ? p.block_n - half_cols : half_cols);
+      w.n_first = (tile - m_blk * p.tiles_n) * p.block_n + w.c_first;
+      return w;
+    };
     for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
       const int tile = split_k ? unit / chunks : unit;
-      const int m_blk = tile / p.tiles_n;
-      const int n_blk = tile - m_blk * p.tiles_n;
-      const bool pair_tile = m_blk < p.pair_rows;
-      const long long m_tile = pair_tile ? static_cast<long long>(m_blk) * (2 * kTcBlockM)
-                                         : static_cast<long long>(p.pair_rows) * (2 * kTcBlockM) +
-                                               static_cast<long long>(m_blk - p.pair_rows) * kTcBlockM;
-      // this group's share: rows of one half of a pair, or half of the columns
-      const long long m = m_tile + (pair_tile && group ? kTcBlockM : 0) + row;
-      const int c_first = !pair_tile && group ? half_cols : 0;
-      const int cols = pair_tile ? p.block_n : (group ? p.block_n - half_cols : half_cols);
-      const int n_first = n_blk * p.block_n + c_first;
+      const Share here = share(tile);
+      const bool pair_tile = here.pair;
+      const long long m = here.m;
+      const int c_first = here.c_first, cols = here.cols, n_first = here.n_first;
       const bool valid = m < lp.M;
+      if (far_residual && unit + static_cast<int>(gridDim.x) < units) {
+        const Share next = share(unit + static_cast<int>(gridDim.x));
+        const long long bytes = 4ll * min(next.cols, lp.N - next.n_first);
+        const uint8_t* r0 = reinterpret_cast<const uint8_t*>(lp.res0 + next.m * lp.ldo + next.n_first);
+        if (next.m < lp.M)
+          for (long long b = 0; b < bytes; b += 128) prefetch_l2(r0 + b);
+      }
       if (tracing) p.trace[(unit / gridDim.x) * 16 + 3] = clock64();
       // the vote keeps the warp together: tcgen05.ld below needs all 32 lanes
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, wait_limit) ? 1 : 0) != 0;

@@ -149,3 +149,13 @@ def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkey
     monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
     monkeypatch.setenv("NCNN_B200_FUSE_EXPAND", "0")
     assert rel_l2(got, pkg.Model(param, bin_).run(x[:n])[0]) <= 1e-5
+
+
+def test_int8_residuals_beyond_the_l2_cache(pkg, tmp_path):
+    """165 images: layer 1's fp32 residuals exceed 126 MB and are requested a tile ahead, up to the last, partial tile."""
+    param, bin_ = pkg.zoo.resnet18(str(tmp_path / "r"), int8=True, classes=16)
+    x = np.random.default_rng(13).uniform(-1, 1, (165, 3, 224, 224)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    got = m.run(x)[0]
+    for rows in (slice(0, 3), slice(80, 82), slice(162, 165)):
+        assert np.array_equal(m.run(x[rows])[0], got[rows])
