@@ -265,7 +265,10 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       auto launch = std::make_shared<TcLaunch>();
       std::string perr;
       if (node.dw_fused && depthwise_apart(node, n)) {
-        // the depthwise result as bf16 pairs in the workspace of split contractions (this one has too few K blocks to split)
+        // the depthwise result as bf16 pairs in the workspace of split contractions, which this projection therefore goes
+        // without: its tiles stay whole, also where every other convolution is split (NCNN_B200_STREAMK=1)
+        te.sk_ws = nullptr;
+        te.sk_flags = nullptr;
         const size_t plane = (static_cast<size_t>(n) * node.OH * node.OW * node.dw_c * 2 + 255) / 256 * 256;
         ActRef mid;
         mid.fmt = FMT_BF16X2;

@@ -151,6 +151,23 @@ def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkey
     assert rel_l2(got, pkg.Model(param, bin_).run(x[:n])[0]) <= 1e-5
 
 
+def test_depthwise_apart_keeps_its_result_while_other_convolutions_split(pkg, oracle, tmp_path, monkeypatch):
+    """NCNN_B200_STREAMK=1 splits convolutions through the workspace that holds the depthwise result of small maps: the
+    projections behind those depthwise layers must not be split, the others are."""
+    param, bin_ = pkg.zoo.mobilenet_v2(str(tmp_path / "m"))
+    x = np.random.default_rng(14).uniform(-1, 1, (1, 3, 224, 224)).astype(np.float32)
+    monkeypatch.setenv("NCNN_B200_STREAMK", "1")
+    m = pkg.Model(param, bin_)
+    fused = {r["layer"].split("+")[-1] for r in m.profile(256, repeat=1) if r["layer"].count("+") == 1}
+    kernels = {r["layer"]: r["kernel"] for r in m.profile(1, repeat=1)}
+    apart = fused & kernels.keys()
+    assert any("split" in k for k in kernels.values())
+    assert apart and all(kernels[name] == "tc_gemm_kernel<bf16x3>" for name in apart)
+    want = oracle_rows(oracle, param, bin_, x)
+    for _ in range(20):
+        assert rel_l2(m.run(x)[0], want) <= 2e-4
+
+
 def test_int8_residuals_beyond_the_l2_cache(pkg, tmp_path):
     """165 images: layer 1's fp32 residuals exceed 126 MB and are requested a tile ahead, up to the last, partial tile."""
     param, bin_ = pkg.zoo.resnet18(str(tmp_path / "r"), int8=True, classes=16)
