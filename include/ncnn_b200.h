@@ -106,6 +106,9 @@ int ncnn_b200_run_batch(ncnn_b200_model *model, int64_t n, const float *const *i
  * not seen before, which lay the arena out anew) belongs after the previous one has finished.
  * The first use of a new batch size synchronises the device for that reason.  Plans (CUDA
  * graphs, staging buffers) are cached for the eight most recently used batch sizes.
+ * Arrays may share memory: the results are those of a call that reads every input before it
+ * writes any output, and writes the outputs in order.  (A flat input that meets an output costs
+ * a copy; arrays apart from one another are read and written in place.)
  * Every entry point makes the model's device (options.device) current for the call and puts
  * the caller's device back before it returns. */
 int ncnn_b200_run_batch_device(ncnn_b200_model *model, int64_t n, const float *const *inputs,

@@ -189,14 +189,23 @@ cudaGraphExec_t EngineImpl::capture_steps(const std::vector<Step>& steps) {
 
 // Every launch of one pass of `plan` over the given caller arrays: input edges, layers, output edges.  Arrays whose
 // layout is the tensor's own are used in place, so their edge steps fall away and the layers that touch them are
-// emitted with the caller's pointers.
+// emitted with the caller's pointers.  Layers write results while others still read inputs: an input that shares memory
+// with an output is copied before the first layer, and outputs that share memory are written at the end, in order.
 bool EngineImpl::assemble(const Plan& plan, const std::vector<const float*>& d_in, const std::vector<float*>& d_out, std::vector<Step>* all) {
   const int64_t n = plan.n;
   caller_array_.assign(tensors_.size(), nullptr);
+  auto meets_output = [&](const float* p, int tensor, size_t self) {
+    for (size_t o = 0; o < outputs_.size(); ++o)
+      if (o != self && std::less<const float*>()(p, d_out[o] + tensors_[resolve(outputs_[o])].logical() * n) &&
+          std::less<const float*>()(d_out[o], p + tensors_[resolve(tensor)].logical() * n))
+        return true;
+    return false;
+  };
   for (size_t i = 0; i < inputs_.size(); ++i)
-    if (reads_caller_array(static_cast<int>(i), n, d_in[i])) caller_array_[resolve(inputs_[i])] = const_cast<float*>(d_in[i]);
+    if (reads_caller_array(static_cast<int>(i), n, d_in[i]) && !meets_output(d_in[i], inputs_[i], outputs_.size()))
+      caller_array_[resolve(inputs_[i])] = const_cast<float*>(d_in[i]);
   for (size_t i = 0; i < outputs_.size(); ++i)
-    if (caller_array_[resolve(outputs_[i])] == nullptr && writes_caller_array(static_cast<int>(i), d_out[i]))
+    if (caller_array_[resolve(outputs_[i])] == nullptr && writes_caller_array(static_cast<int>(i), d_out[i]) && !meets_output(d_out[i], outputs_[i], i))
       caller_array_[resolve(outputs_[i])] = d_out[i];
   std::vector<Step> post;
   make_edge_steps(n, d_in, d_out, all, &post);
@@ -578,10 +587,19 @@ int Engine::launches_per_run(int64_t n) {
   DeviceGuard guard(impl_->device_);
   Plan* p = impl_->plan_for(n);
   if (p == nullptr) return -1;
-  // (the arena stands in for the caller's arrays: aligned, as a caller's allocation is)
+  // (addresses from the arena on stand in for the caller's arrays: aligned and apart, as a caller's allocations are)
   std::vector<Step> all;
-  float* any = reinterpret_cast<float*>(impl_->arena_);
-  if (!impl_->assemble(*p, std::vector<const float*>(impl_->inputs_.size(), any), std::vector<float*>(impl_->outputs_.size(), any), &all)) return -1;
+  uint8_t* at = impl_->arena_;
+  auto stand_in = [&](const TensorShape& shape) {
+    float* array = reinterpret_cast<float*>(at);
+    at += round_up(static_cast<size_t>(shape.elements()) * 4 * n, 256);
+    return array;
+  };
+  std::vector<const float*> in;
+  std::vector<float*> out;
+  for (int i = 0; i < input_count(); ++i) in.push_back(stand_in(input_shape(i)));
+  for (int i = 0; i < output_count(); ++i) out.push_back(stand_in(output_shape(i)));
+  if (!impl_->assemble(*p, in, out, &all)) return -1;
   return static_cast<int>(all.size());
 }
 const std::string& Engine::last_error() const { return impl_->error_; }

@@ -76,6 +76,48 @@ def test_device_arrays_in_place_at_any_alignment(pkg, tmp_path, m, int8):
             assert (got[:shift_out] == 7.0).all() and (got[shift_out + m * n:] == 7.0).all()
 
 
+@pytest.mark.parametrize("mode,int8,k,m", [(0, False, 4096, 1), (0, False, 4096, 8), (0, True, 4096, 8), (2, False, 300, 1), (2, False, 300, 70)])
+def test_device_arrays_may_share_memory(pkg, tmp_path, mode, int8, k, m):
+    """An output in the memory of an input, wholly and in part: the results of arrays that lie apart."""
+    import torch
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, k, int8=int8)
+    model = pkg.Model(param, bin_, accuracy_mode=mode)
+    x = np.random.default_rng(15).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    want = model.run(x)[0].reshape(-1)
+    src, room = torch.from_numpy(x.reshape(-1)).cuda(), torch.empty(2 * m * k, device="cuda")
+    launches = model.launch_count(m)
+    for at_in, at_out in [(0, 0), (0, 4 * (k // 8)), (m * k - 4, 0)]:
+        for _ in range(10):
+            room[at_in:at_in + m * k] = src
+            model.run_device(m, [room.data_ptr() + 4 * at_in], [room.data_ptr() + 4 * at_out], torch.cuda.current_stream().cuda_stream)
+            got = room[at_out:at_out + m * k].cpu().numpy()
+            assert rel_l2(got, want) <= 1e-5 and (not int8 or np.array_equal(got, want))
+    assert launches == model.launch_count(m)
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+def test_an_output_may_take_the_memory_of_an_input_that_is_read_again(pkg, tmp_path, mode):
+    """Two layers read one flat input and the first one's result lies over it; two results in one array: the last stays."""
+    import torch
+    k = 1536
+    net = pkg.zoo._Net(16)
+    net.w.layer("Input", "input", [], ["data"], f"0=1 1=1 2={k}")
+    net.w.layer("Split", "split", ["data"], ["a", "b"])
+    net.inner_product("ip1", "a", "y1", k, k)
+    net.inner_product("ip2", "b", "y2", k, k)
+    model = pkg.Model(*net.w.save(str(tmp_path / "two")), accuracy_mode=mode)
+    x = np.random.default_rng(17).uniform(-1, 1, (2, k, 1, 1)).astype(np.float32)
+    want = [y.reshape(2, k) for y in model.run(x)]
+    src, first, second = torch.from_numpy(x.reshape(2, k)).cuda(), torch.empty(2, k, device="cuda"), torch.empty(2, k, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(10):
+        first.copy_(src)
+        model.run_device(2, [first.data_ptr()], [first.data_ptr(), second.data_ptr()], stream)
+        assert rel_l2(first.cpu(), want[0]) <= 1e-5 and rel_l2(second.cpu(), want[1]) <= 1e-5
+    model.run_device(2, [src.data_ptr()], [second.data_ptr(), second.data_ptr()], stream)
+    assert rel_l2(second.cpu(), want[1]) <= 1e-5
+
+
 @pytest.mark.parametrize("cin,cout,k,stride,h,w,n", [
     (64, 64, 3, 1, 9, 7, 3),    # tiles that span images
     (32, 37, 1, 1, 5, 11, 2),   # channels in no whole 16-byte pieces
