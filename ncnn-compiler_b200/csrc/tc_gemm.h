@@ -82,12 +82,21 @@ constexpr int kTcSplitFlagCount = 640;  // two per CTA (one per epilogue group)
 int tc_k_elems(int kind, int channels);
 int tc_row_bytes(int kind, int channels);
 
-// bf16-pair convolutions of at least kTcChunkFrom K blocks are summed in chunks of kTcChunkBlocks (blocks of 64 channels of
-// one filter tap): where a batch leaves SMs idle, the chunks of a tile run side by side, and where it does not, one CTA
-// adds up the same chunks, so that results do not depend on the batch.  A chunk costs a busy GPU ~0.3 us, a K block in a
-// row ~0.45: 7x7x512 -> 512 (72 blocks) 34.8 -> 20.6 us for one image, 35 -> 16 for 4, 36 -> 27 for 16, 44.2 -> 45.5 for 64.
-// (Chunks of 9: 16.6, 20, 54 and 46.7.)  At 36 blocks the few images gain 4 us a layer and batches lose 4 to 5.
-constexpr int kTcChunkFrom = 72, kTcChunkBlocks = 18;
+// bf16-pair convolutions of at least kTcChunkFrom K blocks are summed in chunks of kTcChunkBlocks: where a batch leaves SMs
+// idle, the chunks of a tile run side by side, and where it does not, one CTA adds up the same chunks, so that results do
+// not depend on the batch.  Both count K blocks of either width: in a row a block of 64 channels of a filter tap costs the
+// chain ~0.57 us, one of 32 channels (channel counts that are no multiple of 64) ~0.45.  3x3 layers, whole -> in chunks, us:
+//   blocks       7x7, 1 image     16 images       64 images        14x14, 64 images
+//   36 of 64     25.5 -> 19.7     25.4 -> 21.4    27.5 -> 28.2     47.7 -> 52.1 (gives up its paired tiles)
+//   45           29.0 -> 19.4     29.7 -> 23.5    32.8 -> 33.5     58.4 -> 64.5 (the same)
+//   54           33.2 -> 21.0     33.8 -> 25.6    38.4 -> 39.6     86.8 -> 95.2 (CTA pairs, here and below)
+//   63           36.8 -> 21.4     40.6 -> 30.5    44.4 -> 45.8    113.7 -> 123.9
+//   72           41.2 -> 21.4     42.0 -> 33.7    51.2 -> 52.1    142.4 -> 154.6
+//   63 of 32     29.0 -> 16.7     29.2 -> 25.0    32.2 -> 32.0     61.5 -> 61.8
+//   81           34.5 -> 18.6     35.0 -> 28.8    39.4 -> 39.6     79.8 -> 79.9
+// Whole batches lose the same few per cent at every depth, so there is no crossover to draw the line at.  It lies at four
+// chunks: one image then takes about half its time, with three two thirds and with two four fifths.
+constexpr int kTcChunkBlocks = 18, kTcChunkFrom = 3 * kTcChunkBlocks + 1;
 
 // Convolution: M = view.N*OH*OW pixels, N = out_channels.  `w0`/`w1` are the packed
 // weights [out_channels][KH*KW*c_blocks*k_elems] (see tc_pack_weights).

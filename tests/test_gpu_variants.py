@@ -166,7 +166,9 @@ def test_patch_resident_convolution_by_default(pkg, tmp_path, monkeypatch, h, w,
 @pytest.mark.parametrize("cin,cout,k,h,w,many", [
     (512, 80, 3, 7, 7, 30),    # 72 K blocks = 4 chunks; several tiles per image row block, a ragged last column tile
     (328, 24, 5, 5, 9, 3),     # 64-byte operand rows, 275 blocks: chunks that do not divide them
-    (1160, 256, 3, 8, 16, 100) # whole tiles, and tiles of CTA pairs, that add up the same chunks
+    (1160, 256, 3, 8, 16, 100), # many images: whole tiles that add up the same chunks
+    (448, 24, 3, 7, 7, 30),    # 63 blocks of 64 channels: four chunks, the last one short
+    (56, 40, 8, 11, 9, 20),    # 128 blocks of 32 channels, the second of every tap half empty
 ])
 def test_deep_convolutions_sum_in_chunks(pkg, oracle, tmp_path, cin, cout, k, h, w, many):
     """The chunks of a deep contraction run side by side for few images and one after the other for many: the same bits."""
