@@ -184,7 +184,7 @@ def test_deep_convolutions_sum_in_chunks(pkg, oracle, tmp_path, cin, cout, k, h,
 
 @pytest.mark.parametrize("size,n", [(32, 64), (32, 65), (64, 4), (64, 5), (224, 1)])
 def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkeypatch, size, n):
-    """Small maps run the two layers apart: the bits of a batch that runs them in one kernel."""
+    """Maps of up to 256 pixels run the two layers apart: the bits of a batch that runs them in one kernel."""
     param, bin_ = pkg.zoo.mobilenet_v2(str(tmp_path / "m"), size=size)
     x = np.random.default_rng(11).uniform(-1, 1, (n + 8, 3, size, size)).astype(np.float32)
     m = pkg.Model(param, bin_)
@@ -193,21 +193,6 @@ def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkey
     monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
     monkeypatch.setenv("NCNN_B200_FUSE_EXPAND", "0")
     assert rel_l2(got, pkg.Model(param, bin_).run(x[:n])[0]) <= 1e-5
-
-
-@pytest.mark.parametrize("h,hidden,n", [
-    (14, 384, 11),    # 12 blocks of channels: up to 2 304 pixels
-    (16, 240, 3),     # 8 blocks, the last one half full: up to 768, met exactly
-    (16, 1536, 13),   # 48 blocks: the workspace ends before the line does
-])
-def test_depthwise_apart_up_to_its_line(pkg, tmp_path, h, hidden, n):
-    """The two layers apart for n images and in one kernel for n + 1, with the same bits."""
-    param, bin_ = pkg.zoo.inverted_residual(str(tmp_path / "b"), h, h, 64, hidden, 64)
-    x = np.random.default_rng(18).uniform(-1, 1, (n + 1, 64, h, h)).astype(np.float32)
-    m = pkg.Model(param, bin_)
-    assert not any("tc_dw_project" in r["kernel"] for r in m.profile(n, repeat=1))
-    assert any("tc_dw_project" in r["kernel"] for r in m.profile(n + 1, repeat=1))
-    assert np.array_equal(m.run(x[:n])[0], m.run(x)[0][:n])
 
 
 def test_depthwise_apart_keeps_its_result_while_other_convolutions_split(pkg, oracle, tmp_path, monkeypatch):
