@@ -400,12 +400,21 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   // more barrier hand-shakes per output.  Taken when whole tiles fill at least one wave of pairs.
   const int pair_bn = even_width(kTc2MaxBlockN);
   const long long pair_tiles = ((M + kTc2TileM - 1) / kTc2TileM) * ((N + pair_bn - 1) / pair_bn);
-  const bool pair_form = pair_bn >= env_int("NCNN_B200_CTA2_MIN_BN", 192) &&
-                         (pair_tiles >= sm_count / 2 || env_int("NCNN_B200_CTA2_ALWAYS", 0) != 0);
-  // Form 2, single CTAs with split tiles: tiles of 128 rows x up to 128 columns, every SM an equal share of
-  // the K blocks.  Taken when whole tiles would leave SMs idle (few, deep tiles) and the workspace allows.
   const int one_bn = even_width(128);
   const long long one_tiles = ((M + kTcBlockM - 1) / kTcBlockM) * ((N + one_bn - 1) / one_bn);
+  // Sums in chunks (the same in every form, so the batch may decide): tiles of 256 columns have no second accumulator
+  // while the running sum takes its place, so the MMAs of a pair wait for every chunk to be added, and a wave of pair
+  // tiles takes ~1.6 waves of the one-CTA kernel's, which has room for both.  Pairs where they still come out ahead: two
+  // layers of 7x7x512 -> 512 and their edges, pairs / one CTA in us, with the waves of each: 192 images (1, 2) 207 / 228,
+  // 208 (2, 3) 353 / 318, 256 (2, 3) 347 / 334, 296 (2, 4) 354 / 432, 448 (3, 5) 549 / 611, 512 (3, 6) 557 / 659; 768
+  // channels, 128 images (2, 2) 483 / 318, 192 (2, 3) 493 / 512.  Operand rows of 64 bytes stay on pairs, which fetch
+  // half of the weights each (14x14x392 -> 392, 64 images (2, 3) 303 / 379).
+  const bool chunked = kind == GEMM_BF16X3 && p.a_im2col && p.row_bytes == 128 && full_kb >= kTcChunkFrom;
+  const long long pair_waves = (pair_tiles + sm_count / 2 - 1) / (sm_count / 2), one_waves = (one_tiles + sm_count - 1) / sm_count;
+  const bool pairs_win = pair_tiles >= sm_count / 2 && (!chunked || 3 * pair_waves < 2 * one_waves);
+  const bool pair_form = pair_bn >= env_int("NCNN_B200_CTA2_MIN_BN", 192) && (pairs_win || env_int("NCNN_B200_CTA2_ALWAYS", 0) != 0);
+  // Form 2, single CTAs with split tiles: tiles of 128 rows x up to 128 columns, every SM an equal share of
+  // the K blocks.  Taken when whole tiles would leave SMs idle (few, deep tiles) and the workspace allows.
   const long long one_units = one_tiles * full_kb;
   const int one_workers = static_cast<int>(std::min<long long>(sm_count, one_units / 4));
   bool split_form = false;

@@ -89,9 +89,9 @@ int tc_row_bytes(int kind, int channels);
 //   blocks       7x7, 1 image     16 images       64 images        14x14, 64 images
 //   36 of 64     25.5 -> 19.7     25.4 -> 21.4    27.5 -> 28.2     47.7 -> 52.1 (gives up its paired tiles)
 //   45           29.0 -> 19.4     29.7 -> 23.5    32.8 -> 33.5     58.4 -> 64.5 (the same)
-//   54           33.2 -> 21.0     33.8 -> 25.6    38.4 -> 39.6     86.8 -> 95.2 (CTA pairs, here and below)
-//   63           36.8 -> 21.4     40.6 -> 30.5    44.4 -> 45.8    113.7 -> 123.9
-//   72           41.2 -> 21.4     42.0 -> 33.7    51.2 -> 52.1    142.4 -> 154.6
+//   54           33.2 -> 21.0     33.8 -> 25.6    38.4 -> 39.6     86.8 -> 95.2 (both on CTA pairs)
+//   63           36.8 -> 21.4     40.6 -> 30.5    44.4 -> 45.8    113.7 -> 121 (whole on pairs, chunks on one CTA)
+//   72           41.2 -> 21.4     42.0 -> 33.7    51.2 -> 52.1    142.4 -> 145 (the same; 192 images of 7x7, both on pairs: 83 -> 93)
 //   63 of 32     29.0 -> 16.7     29.2 -> 25.0    32.2 -> 32.0     61.5 -> 61.8
 //   81           34.5 -> 18.6     35.0 -> 28.8    39.4 -> 39.6     79.8 -> 79.9
 // Whole batches lose the same few per cent at every depth, so there is no crossover to draw the line at.  It lies at four

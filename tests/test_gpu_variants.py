@@ -182,6 +182,23 @@ def test_deep_convolutions_sum_in_chunks(pkg, oracle, tmp_path, cin, cout, k, h,
             assert np.array_equal(m.run(x[:n])[0][:1], one)
 
 
+@pytest.mark.parametrize("c,h,n,pairs", [
+    (512, 7, 192, True),   # one wave of pair tiles against two of the one-CTA kernel's
+    (512, 7, 208, False),  # two against three
+    (392, 14, 64, True),   # two against three, operand rows of 64 bytes
+])
+def test_chunks_on_pairs_of_ctas(pkg, tmp_path, c, h, n, pairs):
+    """Deep layers of large batches on CTA pairs, where these win, sum the chunks of a lone image."""
+    param, bin_ = pkg.zoo.residual_block(str(tmp_path / "rb"), h=h, w=h, c=c, cout=64)
+    x = np.random.default_rng(19).uniform(-1, 1, (n, c, h, h)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    kernels = {r["layer"]: r["kernel"] for r in m.profile(n, repeat=1)}
+    assert ("tc_gemm2_kernel:pairs" in kernels["conv1"]) == pairs
+    got = m.run(x)[0]
+    for i in (0, n // 2, n - 1):
+        assert np.array_equal(m.run(x[i:i + 1])[0], got[i:i + 1])
+
+
 @pytest.mark.parametrize("size,n", [(32, 64), (32, 65), (64, 4), (64, 5), (224, 1)])
 def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkeypatch, size, n):
     """Maps of up to 256 pixels run the two layers apart: the bits of a batch that runs them in one kernel."""
