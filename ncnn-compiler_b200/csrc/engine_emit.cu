@@ -82,13 +82,21 @@ static bool halo_pays(int kind, int channels, const Node& node, int64_t n, int s
   return n * tiles >= 4 * sm_count && static_cast<double>(node.OH) * node.OW >= 0.85 * (tiles * kHaloTileH * kHaloTileW);
 }
 
-// Where the depthwise layer inside a projection is a launch of its own again: maps of at most 256 pixels in all.  The
-// fused kernel walks the channels in blocks of 32, ~1.2 us each and one after the other, on as many CTAs as there are
-// 128-pixel tiles; with one or two of those two launches are faster (one 14x14 image, 576 channels: 23 -> 9 us, 384: 17 ->
-// 8).  The same products in the same order (below the depth that is summed in chunks), so the batch may decide.
+// Where the depthwise layer inside a projection is a launch of its own again.  The fused kernel walks the channels in
+// blocks of 32, ~1 us each and one after the other however few tiles there are; two launches cost ~5 us and a trip of the
+// depthwise result through L2 that grows with the pixels.  Whole calls of one block, fused -> apart in us, on 14x14 maps
+// but for the last column (16x16):
+//   channels   192 (16x16)      240                384                576                768
+//   images     1: 18.7 -> 19.0   1: 21.8 -> 20.7    1: 24.8 -> 20.7    1: 30.9 -> 22.8    1: 37.2 -> 24.8
+//              2: 18.6 -> 19.3   4: 22.7 -> 23.0    6: 26.8 -> 24.8   16: 38.1 -> 34.6   16: 47.4 -> 43.0
+//              4: 18.7 -> 20.7   8: 24.4 -> 26.5   16: 29.6 -> 30.4   32: 43.4 -> 45.3   24: 53.3 -> 51.5
+// So it takes more than six blocks, and from there on few pixels.  The limit of two tiles of 128 lies below every crossover
+// measured (700 pixels with 8 blocks, 2 500 with 12, 4 700 with 18): it keeps the small batches between in one kernel.
+// The same products in the same order (below the depth that is summed in chunks), so the batch may decide.
 static bool depthwise_apart(const Node& node, int64_t n) {
   if (env_int_or("NCNN_B200_FUSE_DW", 1) >= 2) return false;  // in one kernel wherever it applies
-  return !node.ex_fused && n * node.OH * node.OW <= 256 && tc_row_bytes(GEMM_BF16X3, node.dw_c) != 0 && node.dw_c < kTcChunkFrom * 32;
+  const int blocks = (node.dw_c + 31) / 32;
+  return !node.ex_fused && blocks > 6 && blocks < kTcChunkFrom && n * node.OH * node.OW <= 256 && tc_row_bytes(GEMM_BF16X3, node.dw_c) != 0;
 }
 
 // True when an InnerProduct / Gemm of this batch size runs on the kernel for a handful of rows (ip_rows.cuh): one pass

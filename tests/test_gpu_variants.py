@@ -201,7 +201,7 @@ def test_chunks_on_pairs_of_ctas(pkg, tmp_path, c, h, n, pairs):
 
 @pytest.mark.parametrize("size,n", [(32, 64), (32, 65), (64, 4), (64, 5), (224, 1)])
 def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkeypatch, size, n):
-    """Maps of up to 256 pixels run the two layers apart: the bits of a batch that runs them in one kernel."""
+    """Deep blocks on maps of up to 256 pixels run the two layers apart: the bits of a batch that runs them in one kernel."""
     param, bin_ = pkg.zoo.mobilenet_v2(str(tmp_path / "m"), size=size)
     x = np.random.default_rng(11).uniform(-1, 1, (n + 8, 3, size, size)).astype(np.float32)
     m = pkg.Model(param, bin_)
@@ -210,6 +210,16 @@ def test_depthwise_apart_from_the_projection_on_small_maps(pkg, tmp_path, monkey
     monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
     monkeypatch.setenv("NCNN_B200_FUSE_EXPAND", "0")
     assert rel_l2(got, pkg.Model(param, bin_).run(x[:n])[0]) <= 1e-5
+
+
+@pytest.mark.parametrize("hidden,n,apart", [(192, 1, False), (200, 1, True), (200, 2, False)])
+def test_depthwise_apart_from_seven_blocks_of_channels(pkg, tmp_path, hidden, n, apart):
+    """16x16 pixels are the most; whichever form runs, the bits of the images in a larger batch."""
+    param, bin_ = pkg.zoo.inverted_residual(str(tmp_path / "b"), 16, 16, 64, hidden, 64)
+    x = np.random.default_rng(18).uniform(-1, 1, (5, 64, 16, 16)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    assert any("tc_dw_project" in r["kernel"] for r in m.profile(n, repeat=1)) != apart
+    assert np.array_equal(m.run(x[:n])[0], m.run(x)[0][:n])
 
 
 def test_depthwise_apart_keeps_its_result_while_other_convolutions_split(pkg, oracle, tmp_path, monkeypatch):
