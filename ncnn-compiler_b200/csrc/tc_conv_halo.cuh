@@ -306,7 +306,6 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
     const int c_first = group ? half_cols : 0, cols = group ? p.block_n - half_cols : half_cols;
     const TcHaloParams lp = p;
     TcDirect d{};
-    d.out_mode = p.out_mode;
     d.res_mode = p.res_mode;
     d.act = p.act;
     d.act_a = p.act_a;

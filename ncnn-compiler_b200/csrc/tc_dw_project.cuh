@@ -399,7 +399,6 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
     const int row = quarter * 32 + lane;  // accumulator row = pixel (row / 8, row % 8) of the tile
     const TcDwProjParams lp = p;
     TcDirect d{};
-    d.out_mode = p.out_mode;
     d.res_mode = p.res_mode;
     d.act = p.act;
     d.act_a = p.act_a;

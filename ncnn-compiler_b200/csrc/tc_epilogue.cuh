@@ -31,7 +31,7 @@ struct TcDirect {
   const uint8_t* r1;
   const float* bias;    // at the first column, or null
   const float* scale;   // GEMM_I8
-  int out_mode, res_mode;
+  int res_mode;
   int act;
   float act_a, act_b, out_scale;
   int wide;             // residual rows are multiples of 32 bytes and 32-byte aligned: full-sector loads

@@ -484,7 +484,6 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
     bool ok = true;
     const TcGemmParams lp = p;  // a register copy (a reference to the kernel parameter makes every access a generic load)
     TcDirect d{};
-    d.out_mode = p.out_mode;
     d.res_mode = p.res_mode;
     d.act = p.act;
     d.act_a = p.act_a;

@@ -371,7 +371,6 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
     bool ok = true;
     const TcGemmParams lp = p;
     TcDirect d{};
-    d.out_mode = p.out_mode;
     d.res_mode = p.res_mode;
     d.act = p.act;
     d.act_a = p.act_a;

@@ -228,7 +228,6 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
       bool ok = true;
       const TcStemParams lp = p;
       TcDirect d{};
-      d.out_mode = p.out_mode;
       d.act = p.act;
       d.act_a = p.act_a;
       d.act_b = p.act_b;
