@@ -117,10 +117,9 @@ std::string encode_im2col(CUtensorMap* map, int kind, const void* base, const Tc
   return {};
 }
 
-// Dynamic shared memory a CTA may fill: 227 KB per block, minus the kernel's static shared
-// memory (barriers and per-tile constants: 1.2 KB, 2.2 KB for the int8 kernel with its
-// dequantisation factors), minus 1 KB of alignment slack.
-constexpr int tc_smem_budget(int kind) { return (kind == GEMM_I8 ? 223 : 224) * 1024; }
+// Shared memory that the rings and buffers of a CTA may fill: 227 KB per block, minus 1 KB of alignment slack, minus the
+// kernels' static shared memory (barriers and flags, 208 to 272 bytes), and 1 KB of room for that to grow.
+constexpr int kTcSmemBudget = 224 * 1024;
 constexpr int kDrainBytes = 8 * kDrainWarpBytes;  // shared memory of the eight epilogue warps
 
 int res_mode_of(const TcEpilogue& e) {
@@ -244,7 +243,6 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   p.sk_ws = e.sk_ws;
   p.sk_flags = e.sk_flags;
   p.tiles_n = (N + p.block_n - 1) / p.block_n;
-  const int kTcSmemBudget = tc_smem_budget(kind);
   const int drain = kDrainBytes + (e.side_count > 0 ? 8 * 2 * kDrainSideBytes : 0);  // (room for two int8 copies)
   const int planes = tc_planes(kind);
   // a stage holds the A tile(s) and block_n rows of B, every sub-buffer 1 KB aligned
@@ -440,7 +438,7 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
   p.tiles_m = static_cast<int>((M + tile_m - 1) / tile_m);
   p.block_n = pair_form ? pair_bn : one_bn;
   p.tiles_n = (N + p.block_n - 1) / p.block_n;
-  const int budget_all = tc_smem_budget(kind);
+  const int budget_all = kTcSmemBudget;
   const int planes = tc_planes(kind);
   // Full-size K blocks with a ring deep enough to cover the copy latency, else half-size ones.
   const int full_rb = p.row_bytes, full_cb = p.c_blocks, full_ke = p.k_elems;
@@ -699,7 +697,7 @@ int pairs_resident(int smem_bytes, int sm_count) {
   KernelLaunchConfig wc(sm_count / 2 * 2, kTc2Threads, smem_bytes, true, nullptr);
   int clusters = 0;
   const auto kernel = tc_gemm2_kernel<KIND, true, epi_form(OUT_F32, false)>;
-  if (opt_in(kernel, tc_smem_budget(KIND) + 1024) != cudaSuccess || cudaOccupancyMaxActiveClusters(&clusters, kernel, &wc.cfg) != cudaSuccess) {
+  if (opt_in(kernel, kTcSmemBudget + 1024) != cudaSuccess || cudaOccupancyMaxActiveClusters(&clusters, kernel, &wc.cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -727,8 +725,8 @@ cudaError_t launch_workers(const TcLaunch& L, cudaStream_t stream) {
   KernelLaunchConfig wc(L.grid, kTc2Threads, L.smem_bytes, pair, stream);
   return with_form<KIND, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
     constexpr int EPI = decltype(form)::value;
-    if (pair) return launch_opted(tc_gemm2_kernel<KIND, true, EPI>, tc_smem_budget(KIND) + 1024, wc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-    return launch_opted(tc_gemm2_kernel<KIND, false, EPI>, tc_smem_budget(KIND) + 1024, wc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+    if (pair) return launch_opted(tc_gemm2_kernel<KIND, true, EPI>, kTcSmemBudget + 1024, wc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+    return launch_opted(tc_gemm2_kernel<KIND, false, EPI>, kTcSmemBudget + 1024, wc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
   });
 }
 
@@ -746,7 +744,7 @@ cudaError_t tc_launch_workers(const TcLaunch& L, cudaStream_t stream) {
 template <int KIND>
 cudaError_t launch_gemm(const TcLaunch& L, cudaStream_t stream) {
   KernelLaunchConfig lc(L.grid, kTcThreads, L.smem_bytes, false, stream);
-  const int max_smem = tc_smem_budget(KIND) + 1024;  // contents + alignment slack
+  const int max_smem = kTcSmemBudget + 1024;  // contents + alignment slack
   // (int8 copies of an fp32 result are written by instantiations of their own)
   if constexpr (KIND == GEMM_I8) {
     if (L.p.side_count > 0) {
@@ -864,7 +862,6 @@ std::string tc_plan_conv_halo(TcHaloLaunch* L, int kind, const TcHaloConv& c, co
   p.status = e.status;
   p.trace = e.trace;
   const int fixed = 2 * planes * p.patch_bytes + kDrainBytes;
-  const int kTcSmemBudget = 224 * 1024;
   p.stages = (kTcSmemBudget - fixed) / (planes * p.b_bytes);
   p.stages = std::min(p.stages, kTcMaxStages);
   if (p.stages < 2) return "shared memory cannot hold the patch buffers and two weight stages";
@@ -898,8 +895,8 @@ cudaError_t tc_launch_halo(const TcHaloLaunch& L, cudaStream_t stream) {
     constexpr int KIND = decltype(kind)::value;
     return with_form<KIND, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
       constexpr int EPI = decltype(form)::value;
-      if (L.pair) return launch_opted(tc_conv_halo_kernel<KIND, true, EPI>, 225 * 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
-      return launch_opted(tc_conv_halo_kernel<KIND, false, EPI>, 225 * 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+      if (L.pair) return launch_opted(tc_conv_halo_kernel<KIND, true, EPI>, kTcSmemBudget + 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+      return launch_opted(tc_conv_halo_kernel<KIND, false, EPI>, kTcSmemBudget + 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
     });
   };
   cudaError_t e;
@@ -933,7 +930,7 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int strid
   if (expand && r.block_n > 128) return r;  // (the expand accumulators take the TMEM columns past two 128-column ones)
   r.tiles_n = (N + r.block_n - 1) / r.block_n;
   r.b_bytes = (r.block_n * 64 + 1023) / 1024 * 1024;
-  const int budget = 224 * 1024;  // the kernel's own static shared memory is ~2 KB
+  const int budget = kTcSmemBudget;
   const int c_pad = (C + kDwpChannels - 1) / kDwpChannels * kDwpChannels;
   const int table = (c_pad * (expand ? 11 : 10) * 4 + 1023) / 1024 * 1024;  // depthwise filter and bias (+ expand bias)
   const int stage = 2 * r.b_bytes + (expand ? 4096 : 0);
@@ -1091,7 +1088,7 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
 
 cudaError_t tc_launch_dw_project(const TcDwProjLaunch& L, cudaStream_t stream) {
   KernelLaunchConfig lc(L.grid, kDwpThreads, L.smem_bytes, false, stream);
-  constexpr int max_smem = 225 * 1024;
+  constexpr int max_smem = kTcSmemBudget + 1024;
   const cudaError_t e = with_form<GEMM_BF16X3, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
     constexpr int EPI = decltype(form)::value;
     if (!L.expand) return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 1, false, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
@@ -1229,7 +1226,7 @@ std::string tc_plan_stem(TcStemLaunch* L, const TcStemConv& c, const TcEpilogue&
   p.out1 = e.out1;
   p.outq = e.outq;
   if (!direct_rows(c.kind, e, N, &p.wide)) return "the stem kernel writes rows of 16-byte pieces";
-  const int budget = tc_smem_budget(c.kind);
+  const int budget = kTcSmemBudget;
   const int weights = c.KH * planes * p.b_slot;
   const int stage = planes * p.a_plane_bytes;
   // (a stage holds a whole tile's input: two are a double buffer)
@@ -1278,7 +1275,7 @@ cudaError_t tc_launch_stem(const TcStemLaunch& L, cudaStream_t stream) {
     constexpr int KIND = decltype(kind)::value;
     return with_form<KIND, false>(L.p.out_mode, false, [&](auto form) {
       if constexpr (decltype(form)::value % 2 == 1) return cudaErrorInvalidValue;  // (a stem has no residual)
-      else return launch_opted(tc_stem_kernel<KIND, decltype(form)::value>, tc_smem_budget(KIND) + 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+      else return launch_opted(tc_stem_kernel<KIND, decltype(form)::value>, kTcSmemBudget + 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
     });
   };
   const cudaError_t e = L.kind == GEMM_I8 ? launch(std::integral_constant<int, GEMM_I8>{}) : launch(std::integral_constant<int, GEMM_BF16X3>{});
