@@ -2,9 +2,12 @@
 //
 // Ordinary (pageable) arrays cost a synchronising copy of the driver's each, 10-15 us whatever their size.  Small
 // inputs, the results and the status word go through this memory instead: a memcpy here, an asynchronous copy there,
-// one synchronisation for the whole run (ResNet-18 int8, one 64x64 image: 226 -> 208 us).  Inputs beyond 64 KB stay
-// with the driver, whose own staging was faster at 0.6-10 MB than pieces of 64-512 KB filled here, by one thread
-// (240 against 254-290 us for 0.6 MB) as well as by four (480 against 700 us for 3.7 MB).
+// one synchronisation for the whole run (ResNet-18 int8, one 64x64 image: 226 -> 208 us).  Larger inputs stay with the
+// driver, which copies a piece while the GPU fetches the one before it.  Whole calls of one small convolution, driver
+// against this memory, us: 75 KB 59.0 / 57.1, 127 KB 63.4 / 60.1, 192 KB 68.8 / 66.5, 243 KB 74.3 / 72.5, 363 KB
+// 85.6 / 85.4, 432 KB 92.8 / 102.9, 631 KB 114.6 / 135.4, 2 MB 306 / 337.  So the lines cross near 350 KB; up to there 2-3 us
+// are left on the table for a quarter of the pinned memory per model.  Pieces of 64-512 KB filled by one to four threads were
+// slower than the driver too (0.6 MB: 240 against 254-290 us, 3.7 MB: 480 against 700 us).
 #pragma once
 
 #include <cstdint>

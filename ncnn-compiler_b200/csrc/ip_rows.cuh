@@ -49,10 +49,18 @@ inline size_t ip_rows_smem_bytes(int M, int K, bool int8) {
   return static_cast<size_t>(M) * K * (int8 ? 1 : 4);
 }
 
-// True when the launch fits: few rows, rows of whole vectors, all rows in shared memory at once, and weights
-// large enough (8 MB as stored) for the call to be a pass over them.  Smaller layers stay on the tensor-core path
-// at every M, so that their results do not change with the batch size; for the large ones the last bits of a row
-// differ between M <= 8 and M > 8 (another order of summation), never between calls of the same M.
+// True when the launch fits: few rows, rows of whole vectors, all rows in shared memory at once, and weights large enough
+// (8 MB as stored) for the call to be a pass over them.  fp32: smaller layers stay on the tensor-core path at every M, so
+// that their results do not change with the batch size; for the large ones the last bits of a row differ between M <= 8 and
+// M > 8 (another order of summation), never between calls of the same M.  int8 sums are exact in any order; it shares the
+// line without that reason, and below it up to four rows would be faster here, eight not (whole calls, tensor cores and
+// their Quantize step against this kernel, us):
+//   weights        1 row           2 rows          4 rows          8 rows
+//   512 x 512      8.4 / 6.3       8.4 / 6.4       8.4 / 8.3       8.4 / 8.5
+//   1024 x 1024    8.4 / 6.3       8.4 / 6.3       8.4 / 8.4       9.0 / 10.4
+//   2048 x 2048   12.5 / 6.4      12.5 / 8.4      12.5 / 10.3     12.5 / 12.5
+//   2816 x 2816   14.5 / 8.4      14.5 / 8.4      14.5 / 10.4     13.6 / 14.5
+//   4096 x 4096   22.5 / 8.4      21.4 / 10.4     21.8 / 12.5     21.4 / 18.6 (above the line)
 inline bool ip_rows_applies(long long M, int K, int N, bool int8, int out_mode, bool has_res, bool has_side) {
   if (M < 1 || M > kIpRowsMaxM || N < 1 || has_res || has_side) return false;
   if (static_cast<long long>(K) * N * (int8 ? 1 : 4) < (8ll << 20)) return false;
