@@ -299,9 +299,10 @@ def test_handles_on_their_own_device_leave_the_callers_device_alone(pkg, tmp_pat
 # ------------------------------------------------------------------ Quantize folded into the producer
 def test_quantize_steps_fold_into_their_producers(pkg, oracle, tmp_path, monkeypatch):
     """The int8 network's Quantize steps (NCNNToTosa.cpp:4802-4824, one in front of every int8 contraction whose
-    input is fp32) can be written by the layer that produces the fp32 tensor.  By default the pooling layers do
-    (two launches fewer; three more where two steps read the same tensor and become one pass); with NCNN_B200_FUSE_QUANT=2 the residual convolutions emit the int8 copies for the next
-    block as well (two where a strided block has a projection): twelve launches fewer.  Either way the same bits
+    input is fp32) can be written by the layer that produces the fp32 tensor.  With NCNN_B200_FUSE_QUANT=1 the pooling layers do
+    (two launches fewer; three more where two steps read the same tensor and become one pass); by default (2) the residual
+    convolutions emit the int8 copies for the next block as well (two where a strided block has a projection): twelve launches
+    fewer, no Quantize step left.  Either way the same bits
     as the separate steps, and bit exact against the oracle."""
     param, bin_ = pkg.zoo.resnet18(str(tmp_path / "r18q"), int8=True)
     x = np.random.default_rng(402).uniform(-1, 1, (4, 3, 224, 224)).astype(np.float32)
