@@ -432,7 +432,10 @@ int EngineImpl::run(int64_t n, const float* const* in, float* const* out, bool h
   // unfilled, so its bounded waits run out (nothing faults or hangs; the run returns status 7).
   const bool stall = std::getenv("NCNN_B200_TEST_STALL") != nullptr;
   if (stall != stall_injected_) {
+    // (the kernels read the word before they wait for the launch before them)
+    cudaStreamSynchronize(host ? stream_ : user_stream);
     cudaMemsetAsync(d_status_ + 1, stall ? 1 : 0, sizeof(int), host ? stream_ : user_stream);
+    cudaStreamSynchronize(host ? stream_ : user_stream);
     stall_injected_ = stall;
   }
   const char* pipe_env = std::getenv("NCNN_B200_PIPELINE");

@@ -322,14 +322,8 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
       int img, oy0, ox0, n0;
       bool valid;
       decode(tile, &img, &oy0, &ox0, &n0, &valid);
-      ok = __all_sync(0xffffffffu,
-                      mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
-      if (!ok) break;
-      tc_fence_after_sync();
       const uint32_t t_row =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * acc_stride;
-      const bool etr = p.trace != nullptr && worker == workers / 2 && rank == 0 && tile == worker && threadIdx.x == 64;
-      if (etr) p.trace[4] = clock64();
       const int oy = oy0 + (row >> 3), ox = ox0 + (row & 7);
       const bool inside = valid && oy < lp.OH && ox < lp.OW;
       const long long at = (((static_cast<long long>(img) * lp.OH + oy) * lp.OW + ox)) * lp.N + n0 + c_first;
@@ -346,7 +340,15 @@ tc_conv_halo_kernel(const __grid_constant__ TcHaloParams p, const __grid_constan
       d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + at * rs;
       d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + at * rs;
       d.bias = lp.bias != nullptr ? lp.bias + n0 + c_first : nullptr;
-      tc_drain<KIND, EPI, false, false>(d, t_row + static_cast<uint32_t>(c_first), cols, lp.N - n0 - c_first, inside);
+      TcOperands<KIND, EPI % 2 == 1> ops;
+      ops.fetch(d, 0, cols > 0 ? lp.N - n0 - c_first : 0, inside);
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
+      if (!ok) break;
+      tc_fence_after_sync();
+      const bool etr = p.trace != nullptr && worker == workers / 2 && rank == 0 && tile == worker && threadIdx.x == 64;
+      if (etr) p.trace[4] = clock64();
+      tc_drain<KIND, EPI, false, false>(d, t_row + static_cast<uint32_t>(c_first), cols, lp.N - n0 - c_first, inside, ops);
       if (etr) p.trace[5] = clock64();
       tc_fence_before_sync();
       __syncwarp();

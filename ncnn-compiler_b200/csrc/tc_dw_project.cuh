@@ -184,7 +184,7 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  grid_dependency_wait();
+  if (warp != 0) grid_dependency_wait();  // (the producer waits once its first copies of weights are under way)
 
   // channel blocks of one pixel tile are neighbours, so CTAs working side by side share the patch in L2
   auto decode = [&](int tile, int* img, int* oy0, int* ox0, int* n0) {
@@ -211,6 +211,27 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
       uint32_t ph = 0, p_ph = 0;
       long long patches = 0, weights = 0, tiles_done = 0, x_issued = 0;
       bool ok = true;
+      // a block's weights into ring stage `st`
+      auto load_weights = [&](int st, int cb, int n0) {
+        const uint32_t fb = smem_u32(&b_full[st]);
+        mbar_arrive_expect_tx(fb, b_tx);
+        const uint32_t stage = b_base + static_cast<uint32_t>(st) * b_stage_bytes;
+        tma_load_2d(stage, &map_b0, fb, cb * kDwpChannels, n0);
+        tma_load_2d(stage + b_bytes, &map_b1, fb, cb * kDwpChannels, n0);
+        if (EXPAND) {
+          tma_load_2d(stage + 2u * b_bytes, &map_e0, fb, 0, cb * kDwpChannels);
+          tma_load_2d(stage + 2u * b_bytes + kExWeightBytes, &map_e1, fb, 0, cb * kDwpChannels);
+        }
+        ++weights;
+      };
+      // no kernel writes weights: those of the first tile's first blocks come in while the kernel before this one runs
+      const int ahead = static_cast<int>(blockIdx.x) < total_tiles ? min(S, p.c_blocks) : 0;
+      if (ahead > 0) {
+        int img, oy0, ox0, n0;
+        decode(static_cast<int>(blockIdx.x), &img, &oy0, &ox0, &n0);
+        for (int cb = 0; cb < ahead; ++cb) load_weights(cb, cb, n0);
+      }
+      grid_dependency_wait();
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++tiles_done) {
         int img, oy0, ox0, n0;
         decode(tile, &img, &oy0, &ox0, &n0);
@@ -254,20 +275,13 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
               p_ph ^= 1u;
             }
           }
-          if (!mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
-            ok = false;
-            break;
+          if (tiles_done > 0 || cb >= ahead) {
+            if (!mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+              ok = false;
+              break;
+            }
+            load_weights(s, cb, n0);
           }
-          const uint32_t fb = smem_u32(&b_full[s]);
-          mbar_arrive_expect_tx(fb, b_tx);
-          const uint32_t stage = b_base + static_cast<uint32_t>(s) * b_stage_bytes;
-          tma_load_2d(stage, &map_b0, fb, cb * kDwpChannels, n0);
-          tma_load_2d(stage + b_bytes, &map_b1, fb, cb * kDwpChannels, n0);
-          if (EXPAND) {
-            tma_load_2d(stage + 2u * b_bytes, &map_e0, fb, 0, cb * kDwpChannels);
-            tma_load_2d(stage + 2u * b_bytes + kExWeightBytes, &map_e1, fb, 0, cb * kDwpChannels);
-          }
-          ++weights;
           if (++s == S) {
             s = 0;
             ph ^= 1u;
@@ -411,10 +425,6 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       int img, oy0, ox0, n0;
       decode(tile, &img, &oy0, &ox0, &n0);
-      ok = __all_sync(0xffffffffu,
-                      mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
-      if (!ok) break;
-      tc_fence_after_sync();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * acc_stride;
       // (of a stride-2 tile only the first 64 rows are pixels)
       const int oy = oy0 + (row >> 3), ox = ox0 + (row & 7);
@@ -433,7 +443,13 @@ tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_cons
       d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + at * rs;
       d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + at * rs;
       d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
-      tc_drain<KIND, EPI, false, false>(d, t_row, lp.block_n, lp.N - n0, inside);
+      TcOperands<KIND, EPI % 2 == 1> ops;
+      ops.fetch(d, 0, lp.N - n0, inside);
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
+      if (!ok) break;
+      tc_fence_after_sync();
+      tc_drain<KIND, EPI, false, false>(d, t_row, lp.block_n, lp.N - n0, inside, ops);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

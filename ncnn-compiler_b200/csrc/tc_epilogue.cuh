@@ -165,35 +165,44 @@ __device__ __forceinline__ void tc_load16(const float* p, int have, float (&b)[1
   }
 }
 
+// What 16 columns of a row meet besides their accumulator: bias, dequantisation factor and residual.
+template <int KIND, bool RES>
+struct TcOperands {
+  static constexpr int RW = !RES ? 1 : (KIND == GEMM_TF32X3 ? 32 : 16);  // residual words: 16 fp32, 8 + 8 of a bf16 pair, or 16 + 16 of a split pair
+  uint32_t r[RW];
+  float bias[16], scale[16];
+  // those of columns c to c + 15, of which `have` exist (none: nothing is read)
+  __device__ __forceinline__ void fetch(const TcDirect& d, int c, int have, bool valid) {
+    tc_load16(d.bias != nullptr ? d.bias + c : nullptr, have, bias);
+    if (KIND == GEMM_I8) tc_load16(d.scale + c, have, scale);
+    if (!RES) return;
+    if (!valid) {
+#pragma unroll
+      for (int j = 0; j < RW; ++j) r[j] = 0u;
+    } else if (d.res_mode == RES_BF16X2) {
+      tc_row_load<32>(d.r0 + 2 * c, r, 2 * have, d.wide);
+      tc_row_load<32>(d.r1 + 2 * c, r + (RES ? 8 : 0), 2 * have, d.wide);
+    } else {
+      tc_row_load<64>(d.r0 + 4 * c, r, 4 * have, d.wide);
+      if (KIND == GEMM_TF32X3 && d.res_mode == RES_SPLIT) tc_row_load<64>(d.r1 + 4 * c, r + (RW == 32 ? 16 : 0), 4 * have, d.wide);
+    }
+  }
+};
+
 template <int KIND, int OUT, bool RES, bool SIDE, bool FIX>
-__device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, int cols, int left, bool valid) {
+__device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, int cols, int left, bool valid, TcOperands<KIND, RES>& ops) {
   using namespace ptx;
-  constexpr int RW = !RES ? 1 : (KIND == GEMM_TF32X3 ? 32 : 16);  // residual words: 16 fp32, 8 + 8 of a bf16 pair, or 16 + 16 of a split pair
+  constexpr int RW = TcOperands<KIND, RES>::RW;
   const int row = threadIdx.x & 31;
   const uint32_t stage_row = d.stage + static_cast<uint32_t>(row) * 128u;
   TcFlushLane<OUT == OUT_I8 ? 4 : 8> fl;
   if (OUT != OUT_CHW) fl.init(d, d.pitch, d.pitch8);
   TcFlushLane<4> side_fl;
   if (SIDE) side_fl.init(d, d.side_pitch, 8 * d.side_pitch);
-  uint32_t nxt[16], r[RW];
-  float bias[16], scale[16];
-  auto fetch_res = [&](int c) {
-    if (!RES) return;
-    if (!valid) {
-#pragma unroll
-      for (int j = 0; j < RW; ++j) r[j] = 0u;
-    } else if (d.res_mode == RES_BF16X2) {
-      tc_row_load<32>(d.r0 + 2 * c, r, 2 * (left - c), d.wide);
-      tc_row_load<32>(d.r1 + 2 * c, r + (RES ? 8 : 0), 2 * (left - c), d.wide);
-    } else {
-      tc_row_load<64>(d.r0 + 4 * c, r, 4 * (left - c), d.wide);
-      if (KIND == GEMM_TF32X3 && d.res_mode == RES_SPLIT) tc_row_load<64>(d.r1 + 4 * c, r + (RW == 32 ? 16 : 0), 4 * (left - c), d.wide);
-    }
-  };
+  uint32_t nxt[16];
+  uint32_t(&r)[RW] = ops.r;
+  float(&bias)[16] = ops.bias, (&scale)[16] = ops.scale;
   tmem_ld16(t_row, nxt);
-  tc_load16(d.bias, left, bias);
-  if (KIND == GEMM_I8) tc_load16(d.scale, left, scale);
-  fetch_res(0);
 #pragma unroll 1
   for (int c = 0; c < cols; c += 16) {
     const int have = left - c;  // columns from here on
@@ -250,9 +259,7 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
     if (more) {
       // the next 16 columns' operands are on their way while these are finished and stored
       tmem_ld16(t_row + static_cast<uint32_t>(c + 16), nxt);
-      tc_load16(d.bias != nullptr ? d.bias + c + 16 : nullptr, have - 16, bias);
-      if (KIND == GEMM_I8) tc_load16(d.scale + c + 16, have - 16, scale);
-      fetch_res(c + 16);
+      ops.fetch(d, c + 16, have - 16, valid);
     }
     if (OUT == OUT_I8) {
       // requantise, clamp at zero for a fused ReLU (the order of the reference's int8 path)
@@ -352,12 +359,20 @@ constexpr int kEpiAny = -1;  // element by element, any format and alignment
 
 // Drains `cols` accumulator columns (a multiple of 16) of this warp's 32 rows, of which `left` exist in the result (a
 // multiple of the 16-byte piece of every format involved).  `valid`: this thread's row exists.  Every lane of the warp
-// must call it.  SIDE: int8 copies may take part; FIX: partial accumulators may.
+// must call it.  SIDE: int8 copies may take part; FIX: partial accumulators may.  `ops`: the first 16 columns' operands,
+// which a caller fetches before it waits for the accumulator (a tile alone in the pipeline otherwise pays their way from
+// L2 or HBM after its last product).
 template <int KIND, int EPI, bool SIDE, bool FIX>
-__device__ __forceinline__ void tc_drain(const TcDirect& d, uint32_t t_row, int cols, int left, bool valid) {
+__device__ __forceinline__ void tc_drain(const TcDirect& d, uint32_t t_row, int cols, int left, bool valid, TcOperands<KIND, EPI % 2 == 1>& ops) {
   if (cols > left) cols = (left + 15) & ~15;
   if (cols <= 0) return;
-  tc_drain_as<KIND, EPI / 2, EPI % 2 == 1, SIDE, FIX>(d, t_row, cols, left, valid);
+  tc_drain_as<KIND, EPI / 2, EPI % 2 == 1, SIDE, FIX>(d, t_row, cols, left, valid, ops);
+}
+template <int KIND, int EPI, bool SIDE, bool FIX>
+__device__ __forceinline__ void tc_drain(const TcDirect& d, uint32_t t_row, int cols, int left, bool valid) {
+  TcOperands<KIND, EPI % 2 == 1> ops;
+  ops.fetch(d, 0, left, valid);
+  tc_drain<KIND, EPI, SIDE, FIX>(d, t_row, cols, left, valid, ops);
 }
 
 }  // namespace nb

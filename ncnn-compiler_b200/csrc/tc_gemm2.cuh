@@ -176,8 +176,8 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   // barriers, tensor memory and descriptors are ready: from here on the kernel touches tensors that the
-  // kernel before it in the stream may still be writing
-  grid_dependency_wait();
+  // kernel before it in the stream may still be writing (the producers wait later: see tc_gemm.cuh)
+  if (warp != 0 && warp != 6) grid_dependency_wait();
 
   if (warp == 0 || warp == 6) {
     // ------------------------------------------------------------ producers
@@ -191,7 +191,7 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
       int s = 0;
       uint32_t ph = 0;
       long long issued = 0;
-      bool ok = true;
+      bool ok = true, waited = false;
       for (int i = 0; i < work.nseg && ok; ++i) {
         int tile, kb0, kb1, owned;
         work.seg(i, &tile, &kb0, &kb1, &owned);
@@ -203,9 +203,10 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
         const int n0 = n_blk * p.block_n + static_cast<int>(rank) * b_rows;
         int img = 0, h_base = 0, w_base = 0;
         if (p.a_im2col) {
-          const long long per_img = static_cast<long long>(p.OH) * p.OW;
-          img = static_cast<int>(m0 / per_img);
-          const int r = static_cast<int>(m0 - img * per_img);
+          const unsigned per_img = static_cast<unsigned>(p.OH) * static_cast<unsigned>(p.OW);
+          const unsigned m = static_cast<unsigned>(m0);  // (below M, which is an int)
+          img = static_cast<int>(m / per_img);
+          const int r = static_cast<int>(m - static_cast<unsigned>(img) * per_img);
           const int oh = r / p.OW;
           const int ow = r - oh * p.OW;
           h_base = oh * p.stride_h - p.pad_t;
@@ -217,6 +218,10 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
         int kw = tap0 - kh * p.KW;
         for (int kb = kb0; kb < kb1; ++kb) {
           const uint32_t fb = PAIR ? map_to_cta(smem_u32(&full_bar[s]), 0u) : smem_u32(&full_bar[s]);
+          if (!waited && (!is_b || issued == S)) {
+            grid_dependency_wait();
+            waited = true;
+          }
           if (!mbar_wait_bounded(smem_u32(&empty_bar[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
             ok = false;
             break;
@@ -391,6 +396,26 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
       const long long m_first = static_cast<long long>(m_blk) * TILE_M + static_cast<long long>(rank) * kTcBlockM;
       const bool row_valid = m_first + row < p.M;  // rows past the end hold nothing worth exchanging
       const int n0 = n_blk * p.block_n + col0;
+      const long long m = m_first + row;
+      constexpr int es = EPI / 2 == OUT_I8 ? 1 : (EPI / 2 == OUT_BF16X2 ? 2 : 4);
+      TcOperands<KIND, EPI % 2 == 1> ops;
+      if (owned) {
+        const long long at = ((m - lane) * lp.ldo + n0) * es;
+        d.o0 = (EPI / 2 == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + at;
+        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at;
+        d.pitch = lp.ldo * es;
+        d.pitch8 = 8 * d.pitch;
+        const long long rows_left = lp.M - (m - lane);
+        d.rows = rows_left > 32 ? 32 : static_cast<int>(rows_left);
+        if (EPI % 2 == 1) {
+          const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
+          d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n0) * rs;
+          d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n0) * rs;
+        }
+        d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
+        d.scale = lp.scale + n0;
+        ops.fetch(d, 0, half > 0 ? lp.N - n0 : 0, row_valid);
+      }
       // the vote keeps the warp together: tcgen05.ld below needs all 32 lanes
       ok = __all_sync(0xffffffffu,
                       mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
@@ -474,26 +499,10 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
             p.trace[512 + 8 * i + 7] = fix;
           }
         }
-        const long long m = m_first + row;
-        constexpr int es = EPI / 2 == OUT_I8 ? 1 : (EPI / 2 == OUT_BF16X2 ? 2 : 4);
-        const long long at = ((m - lane) * lp.ldo + n0) * es;
-        d.o0 = (EPI / 2 == OUT_I8 ? reinterpret_cast<uint8_t*>(lp.outq) : reinterpret_cast<uint8_t*>(lp.out0)) + at;
-        d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at;
-        d.pitch = lp.ldo * es;
-        d.pitch8 = 8 * d.pitch;
-        const long long rows_left = lp.M - (m - lane);
-        d.rows = rows_left > 32 ? 32 : static_cast<int>(rows_left);
-        if (EPI % 2 == 1) {
-          const int rs = lp.res_mode == RES_BF16X2 ? 2 : 4;
-          d.r0 = reinterpret_cast<const uint8_t*>(lp.res0) + (m * lp.ldo + n0) * rs;
-          d.r1 = reinterpret_cast<const uint8_t*>(lp.res1) + (m * lp.ldo + n0) * rs;
-        }
-        d.bias = lp.bias != nullptr ? lp.bias + n0 : nullptr;
-        d.scale = lp.scale + n0;
         d.fix_count = fix;
         d.fix_ws = lp.sk_ws + static_cast<long long>(static_cast<int>(blockIdx.x) - CTAS) * static_cast<long long>(slot_words) +
                    ws_group + static_cast<size_t>(row) * 16;
-        tc_drain<KIND, EPI, false, true>(d, t_row, half, lp.N - n0, row_valid);
+        tc_drain<KIND, EPI, false, true>(d, t_row, half, lp.N - n0, row_valid, ops);
         if (fix > 0) {
           // every warp of the group has read the slots: free them
           named_barrier_sync(bar_base, 128);

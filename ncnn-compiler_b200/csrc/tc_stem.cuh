@@ -116,8 +116,8 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   // barriers, tensor memory and descriptors are ready: from here on the kernel touches tensors that the
-  // kernel before it in the stream may still be writing
-  grid_dependency_wait();
+  // kernel before it in the stream may still be writing (the producer waits once its copies of the weights are under way)
+  if (warp != 0) grid_dependency_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer: weights once, then rows
@@ -130,6 +130,7 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
         tma_load_2d(dst, &map_b0, wb, kh * (KIND == GEMM_I8 ? 64 : 32), 0);
         if (PLANES == 2) tma_load_2d(dst + static_cast<uint32_t>(p.b_slot), &map_b1, wb, kh * 32, 0);
       }
+      grid_dependency_wait();
       int s = 0;
       uint32_t ph = 0;
       long long issued = 0;
@@ -244,6 +245,8 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
            tile += tile_step, i += groups) {
         const int acc = i % accs;
         const uint32_t acc_ph = static_cast<uint32_t>((i / accs) & 1);
+        TcOperands<KIND, EPI % 2 == 1> ops;
+        ops.fetch(d, 0, lp.N, row < lp.OW);
         ok = __all_sync(0xffffffffu,
                         mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
         if (!ok) break;
@@ -256,7 +259,7 @@ tc_stem_kernel(const __grid_constant__ TcStemParams p, const __grid_constant__ C
         d.o1 = reinterpret_cast<uint8_t*>(lp.out1) + at * es;
         d.pitch = static_cast<long long>(lp.N) * es;
         d.pitch8 = 8 * d.pitch;
-        tc_drain<KIND, EPI, false, false>(d, t_row, lp.N, lp.N, row < lp.OW);
+        tc_drain<KIND, EPI, false, false>(d, t_row, lp.N, lp.N, row < lp.OW, ops);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

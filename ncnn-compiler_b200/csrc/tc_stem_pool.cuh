@@ -116,7 +116,7 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  grid_dependency_wait();
+  if (warp != 0) grid_dependency_wait();  // (the producer waits once its copies of the weights are under way)
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer: weights once, then rows
@@ -129,6 +129,7 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
         tma_load_2d(dst, &map_b0, wb, kh * (KIND == GEMM_I8 ? 64 : 32), 0);
         if (PLANES == 2) tma_load_2d(dst + static_cast<uint32_t>(p.b_slot), &map_b1, wb, kh * 32, 0);
       }
+      grid_dependency_wait();
       int s = 0;
       uint32_t ph = 0;
       long long issued = 0;
