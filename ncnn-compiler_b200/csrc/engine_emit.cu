@@ -472,6 +472,17 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         v.OH = node.OH;
         v.OW = node.OW;
         perr = tc_plan_conv(launch.get(), kind, v, node.d_w0, node.d_w1, node.O, te, sm_count_);
+        // few pixels: small tiles out of input patches (unless a switch asks for pairs of CTAs or split tiles)
+        const bool forced = launch->cta2 != 0 && (env_int_or("NCNN_B200_CTA2_ALWAYS", 0) != 0 || env_int_or("NCNN_B200_STREAMK", 0) == 1);
+        if (perr.empty() && !node.stem && patch_level() != 0 && !forced) {
+          auto pl = std::make_shared<TcPatchLaunch>();
+          if (tc_plan_conv_patch(pl.get(), kind, v, node.d_w0, node.d_w1, node.O, te, sm_count_, *launch, patch_level() > 0).empty()) {
+            s.kernel = std::string("tc_conv_patch_kernel<") + kind_name + ">";
+            s.run = [pl](cudaStream_t st) { return tc_launch_patch(*pl, st); };
+            steps.push_back(std::move(s));
+            return true;
+          }
+        }
       } else {
         const long long M = (to.rank == 2 ? static_cast<long long>(ti.h) : 1) * n;
         const void* a0 = i8 ? static_cast<const void*>(in.q) : static_cast<const void*>(in.p0);

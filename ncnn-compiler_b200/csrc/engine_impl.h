@@ -381,6 +381,11 @@ inline bool stem_rows_enabled() {
 
 // Where the patch-resident convolution kernel takes a layer (tc_conv_halo.cuh): -1, the default, by measurement (see
 // halo_pays); NCNN_B200_HALO at load time: 0 nowhere, 1 wherever it applies, 2 the same on pairs of CTAs.
+// NCNN_B200_PATCH: 0 never runs a convolution on tc_conv_patch_kernel, 1 wherever it applies
+inline int patch_level() {
+  const char* f = std::getenv("NCNN_B200_PATCH");
+  return f == nullptr ? -1 : std::atoi(f);
+}
 inline int halo_level() {
   const char* f = std::getenv("NCNN_B200_HALO");
   return f == nullptr || f[0] == 0 ? -1 : std::atoi(f);

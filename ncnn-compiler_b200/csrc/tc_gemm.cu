@@ -452,6 +452,7 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
     p.k_elems = half_blocks ? full_ke / 2 : full_ke;
     p.c_blocks = half_blocks ? full_cb * 2 : full_cb;
     p.k_blocks = half_blocks ? full_kb * 2 : full_kb;
+    p.half_blocks = half_blocks ? 1 : 0;
     p.stage_bytes = stage;
     p.stages = stages;
     return true;
@@ -488,6 +489,7 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
       p.k_elems = full_ke;
       p.c_blocks = full_cb;
       p.k_blocks = full_kb;
+      p.half_blocks = 0;
       L->cta2 = 0;
       return false;
     }
@@ -903,6 +905,189 @@ cudaError_t tc_launch_halo(const TcHaloLaunch& L, cudaStream_t stream) {
   if (L.kind == GEMM_BF16X3) e = launch(std::integral_constant<int, GEMM_BF16X3>{});
   else if (L.kind == GEMM_TF32X3) e = launch(std::integral_constant<int, GEMM_TF32X3>{});
   else e = launch(std::integral_constant<int, GEMM_TF32>{});
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ convolution of few pixels
+namespace {
+
+// Expected clocks of a layer's launch.  A K block takes what its MMAs take (128 bytes of operands a clock, or the tensor
+// rate) or what its copies take (~3 clocks a row of 128 bytes, ~2 of 64), whichever is longer.
+double mma_clocks(int m, int n) { return std::max({m == 64 ? 23.0 : 39.0, (m + n) / 4.0, n * m / (m == 64 ? 128.0 : 256.0)}); }
+double k_block_clocks(int row_bytes, int m, int n, double rows) {
+  return std::max(row_bytes / 32 * 3 * mma_clocks(m, n), rows * (row_bytes == 128 ? 3.0 : 2.0)) + 20.0;
+}
+
+double gemm_clocks(const TcLaunch& L, int sm_count) {
+  const TcGemmParams& p = L.p;
+  const double fixed = 3000.0 + 12.0 * p.block_n + (p.split_k || p.streamk ? 3000.0 : 0.0);
+  if (L.cta2 == 2) {
+    const double block = k_block_clocks(p.row_bytes, 128, p.block_n, 2.0 * (kTcBlockM + p.block_n / 2));
+    const long long tiles = static_cast<long long>(p.tiles_m) * p.tiles_n, workers = L.grid / 2;
+    return fixed + static_cast<double>((tiles + workers - 1) / workers) * p.k_blocks * block;
+  }
+  // (what lies between two blocks is hidden behind wide MMAs only)
+  const double block = std::max(k_block_clocks(p.row_bytes, 128, p.block_n, 2.0 * (kTcBlockM + p.block_n)),
+                                p.row_bytes / 32 * 3 * mma_clocks(128, p.block_n) + 330.0);
+  const long long singles = static_cast<long long>(p.tiles_m - p.pair_rows) * p.tiles_n * (p.split_k ? p.chunks : 1);
+  const long long pairs = static_cast<long long>(p.pair_rows) * p.tiles_n;
+  const double pair_block = p.pair ? std::max(2.0 * p.row_bytes / 32 * 3 * mma_clocks(128, p.block_n), 6.0 * (2 * kTcBlockM + p.block_n)) : 0.0;
+  const int blocks = p.split_k ? p.chunk_blocks : p.k_blocks;
+  return fixed + blocks * (static_cast<double>((singles + sm_count - 1) / sm_count) * block + static_cast<double>((pairs + sm_count - 1) / sm_count) * pair_block);
+}
+
+}  // namespace
+
+std::string tc_plan_conv_patch(TcPatchLaunch* L, int kind, const TcIm2colView& v, const void* w0, const void* w1,
+                               int out_channels, const TcEpilogue& e, int sm_count, const TcLaunch& gemm, bool always) {
+  const int stride = v.stride_conv_h;
+  if (kind != GEMM_BF16X3 || v.stride_conv_w != stride || (stride != 1 && stride != 2) || v.dil_h != 1 || v.dil_w != 1 || v.KH > 16 || v.KW > 16)
+    return "the patch kernel takes bf16 pairs, strides of 1 or 2 and no dilation";
+  int wide = 0;
+  if (e.out_mode == OUT_I8 || e.side_count > 0 || !direct_rows(kind, e, out_channels, &wide)) return "the patch kernel writes rows of 16-byte pieces";
+  const int rb = tc_row_bytes(kind, static_cast<int>(v.C));
+  if (rb == 0) return "channel count is not addressable by TMA";
+  TcGemmParams g{};  // K blocks and chunks as tc_gemm_kernel has them
+  g.row_bytes = rb;
+  g.k_elems = rb / 2;
+  g.c_blocks = static_cast<int>((v.C + g.k_elems - 1) / g.k_elems);
+  g.k_blocks = v.KH * v.KW * g.c_blocks;
+  g.a_im2col = 1;
+  set_chunks(g, kind, rb);
+  const int taps = v.KH * v.KW;
+  if (taps < 2) return "a 1x1 filter has nothing to reuse";
+  // (a single tile of few K blocks would gain ~1.5 us; the test of the waits that run out, whose stall is made in
+  // tc_gemm_kernel, asks for it there)
+  if (!always && gemm.cta2 == 0 && gemm.p.tiles_m == 1 && g.k_blocks <= 9) return "a single short tile";
+  // The model ranks tile shapes well and both kernels' tiles roughly: with operand rows of 128 bytes this kernel came out
+  // ahead up to 0.68 of the other's clocks, with rows of 64 bytes (channel counts that are no multiple of 64) up to 0.81.
+  // 3x3 layers, launches by events (~8 us of which are the events'), other kernel -> this one:
+  //   64 channels, 56x56     1 image 13.3 -> 11.6    4: 15.4 -> 15.3      8: 21.6 -> 19.5    16: 24.2 -> 27.7 (0.97)
+  //   128, 28x28             1: 17.4 -> 13.4         3: 17.5 -> 17.3      6: 17.6 -> 19.5 (0.75)
+  //   256, 14x14             1: 25.5 -> 17.4         8: 25.6 -> 23.0     16: 27.7 -> 26.9    24: 27.6 -> 39.9 (1.13)
+  //   512, 7x7 (in chunks)   1: 21.6 -> 17.3         2: 21.2 -> 19.6      4: 21.5 -> 25.1 (0.82)
+  //   256 -> 512, stride 2   1: 25.6 -> 19.5         8: 25.6 -> 20.1     12: 25.6 -> 30.4 (1.09)
+  //   96, 28x28              1: 19.4 -> 13.3        16: 29.7 -> 19.5     32: 40.2 -> 27.7    64: 42.0 -> 48.2 (0.87)
+  //   168, 50x50             1: 30.8 -> 21.5         8: 97.4 -> 66.6     12: 125 -> 87       16: 128 -> 119 (0.87)
+  TcPatchParams best{};
+  double best_clocks = always ? 1e300 : (rb == 128 ? 0.68 : 0.81) * gemm_clocks(gemm, sm_count);
+  // one tile shape: 8 or 16 rows of 8 pixels, `bn` columns, groups of all taps of a channel block or of a filter row
+  auto consider = [&](int th, int bn, bool whole_groups) {
+    TcPatchParams p{};
+    p.images = static_cast<int>(v.N);
+    p.tile_h = th;
+    p.tiles_y = (v.OH + th - 1) / th;
+    p.tiles_x = (v.OW + kPatchTileW - 1) / kPatchTileW;
+    p.block_n = bn;
+    p.tiles_n = (out_channels + bn - 1) / bn;
+    const long long tiles = static_cast<long long>(v.N) * p.tiles_y * p.tiles_x * p.tiles_n;
+    if (tiles > (1 << 24)) return;
+    p.subs = stride;
+    p.row_step = stride;
+    p.patch_h = (th - 1) * stride + v.KH;
+    p.patch_w = ((kPatchTileW - 1) * stride + v.KW + stride - 1) / stride;
+    p.sub_bytes = (p.patch_w * p.patch_h * rb + 1023) / 1024 * 1024;
+    p.step_even = stride == 2 ? p.sub_bytes : rb;
+    p.step_odd = stride == 2 ? rb - p.sub_bytes : rb;
+    p.group = whole_groups ? taps : v.KW;
+    if (g.chunks > 1 && g.chunk_blocks % p.group != 0) return;  // (a chunk holds whole groups)
+    p.group_rows = p.group / v.KW;
+    p.patch_groups = v.KH / p.group_rows;
+    p.groups = g.k_blocks / p.group;
+    p.chunk_groups = g.chunks > 1 ? g.chunk_blocks / p.group : p.groups;
+    p.b_bytes = (bn * rb + 1023) / 1024 * 1024;
+    p.acc_cols = (bn + 31) / 32 * 32;
+    const int buf = 2 * p.subs * p.sub_bytes, stage = p.group * 2 * p.b_bytes, drain = 4 * kDrainWarpBytes;
+    // two CTAs to an SM (of this kernel only: anything less than 110 KB would let in the others, which take all of
+    // tensor memory), or one with deeper rings
+    auto fits = [&](int budget, int bufs, int least) {
+      p.patch_bufs = bufs;
+      p.stages = std::min({kTcMaxStages, p.groups, (budget - drain - bufs * buf) / stage});
+      return p.stages >= std::min(least, p.groups);
+    };
+    if (!fits(111 * 1024, 2, 2) && !fits(kTcSmemBudget, 3, 3) && !fits(kTcSmemBudget, 2, 2)) return;
+    const double block = k_block_clocks(rb, 8 * th, bn, 2.0 * p.subs * p.patch_w * p.patch_h / taps + 2.0 * bn) + 350.0 / p.group;
+    for (int split = 0; split <= (g.chunks > 1 ? 1 : 0); ++split) {
+      const long long units = tiles * (split ? g.chunks : 1);
+      if (split && (e.sk_ws == nullptr || e.sk_flags == nullptr || tiles * 4 > e.sk_flag_count ||
+                    static_cast<size_t>(units) * kTcBlockM * bn * 4 > e.sk_ws_bytes))
+        continue;
+      const double waves = static_cast<double>((units + sm_count - 1) / sm_count);
+      const double clocks = 3000.0 + 12.0 * bn + (split ? 3000.0 + static_cast<double>(units) * bn / 4.0 : 0.0) +
+                            waves * ((split ? g.chunk_blocks : g.k_blocks) * block + 300.0);
+      if (clocks >= best_clocks) continue;
+      best_clocks = clocks;
+      best = p;
+      best.split_k = split;
+    }
+  };
+  for (int th : {8, 16})
+    for (int bn = 16; bn <= 128 && bn < out_channels + 16; bn += 16)
+      for (bool whole_groups : {true, false}) consider(th, bn, whole_groups);
+  if (best.tile_h == 0) return "other kernels are expected to be as fast";
+  TcPatchParams& p = L->p;
+  p = best;
+  p.OH = v.OH;
+  p.OW = v.OW;
+  p.N = out_channels;
+  p.c_blocks = g.c_blocks;
+  p.k_elems = g.k_elems;
+  p.row_bytes = rb;
+  p.taps = taps;
+  p.KW = v.KW;
+  p.k_blocks = g.k_blocks;
+  p.stride = stride;
+  p.pad_t = v.pad_t;
+  p.pad_l = v.pad_l;
+  p.chunks = g.chunks;
+  const int cols = p.acc_cols * (p.chunks > 1 && !p.split_k ? 3 : 2);
+  p.tmem_cols = 32;
+  while (p.tmem_cols < cols) p.tmem_cols *= 2;
+  p.sk_ws = e.sk_ws;
+  p.sk_flags = e.sk_flags;
+  p.wide = wide;
+  p.bias = e.bias;
+  p.out0 = e.out0;
+  p.out1 = e.out1;
+  p.res0 = e.res0;
+  p.res1 = e.res1;
+  p.ldo = e.ldo;
+  p.res_mode = res_mode_of(e);
+  p.out_mode = e.out_mode;
+  p.act = e.act;
+  p.act_a = e.act_a;
+  p.act_b = e.act_b;
+  p.status = e.status;
+  const int contents = p.patch_bufs * 2 * p.subs * p.sub_bytes + p.stages * p.group * 2 * p.b_bytes + 4 * kDrainWarpBytes;
+  L->smem_bytes = std::max(contents + 1024, 110 * 1024);
+  if (p.tmem_cols > 256) L->smem_bytes = std::max(L->smem_bytes, 120 * 1024);
+  L->kind = kind;
+  const long long units = static_cast<long long>(p.images) * p.tiles_y * p.tiles_x * p.tiles_n * (p.split_k ? p.chunks : 1);
+  L->grid = static_cast<int>(std::min<long long>(units, sm_count));
+
+  const cuuint64_t dims[4] = {v.C, v.W, v.H, v.N};
+  const cuuint64_t strides[3] = {v.stride_w, v.stride_h, v.stride_n};
+  const cuuint32_t step = static_cast<cuuint32_t>(stride);  // (a copy skips every other column at stride 2)
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(p.k_elems), (static_cast<cuuint32_t>(p.patch_w) - 1) * step + 1, static_cast<cuuint32_t>(p.patch_h), 1};
+  const cuuint32_t elem_strides[4] = {1, step, 1, 1};
+  if (box[1] > 256 || box[2] > 256) return "the patch does not fit a TMA box";
+  for (int plane = 0; plane < 2; ++plane) {
+    const CUresult r = g_encode_tiled(plane ? &L->map_a1 : &L->map_a0, dtype_for(kind), 4, const_cast<void*>(plane ? v.plane1 : v.plane0), dims,
+                                      strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(rb),
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled (patch) failed with code " + std::to_string(static_cast<int>(r));
+  }
+  const uint64_t k_total = static_cast<uint64_t>(p.k_blocks) * p.k_elems;
+  std::string err = encode_tiled_2d(&L->map_b0, kind, w0, k_total, out_channels, k_total * 2, p.k_elems, p.block_n, rb);
+  if (err.empty()) err = encode_tiled_2d(&L->map_b1, kind, w1, k_total, out_channels, k_total * 2, p.k_elems, p.block_n, rb);
+  return err;
+}
+
+cudaError_t tc_launch_patch(const TcPatchLaunch& L, cudaStream_t stream) {
+  KernelLaunchConfig lc(L.grid, kPatchThreads, L.smem_bytes, false, stream);
+  const cudaError_t e = with_form<GEMM_BF16X3, true>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
+    return launch_opted(tc_conv_patch_kernel<GEMM_BF16X3, decltype(form)::value>, kTcSmemBudget + 1024, lc, L.p, L.map_a0, L.map_a1, L.map_b0, L.map_b1);
+  });
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -221,6 +221,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
   // ~450 cycles of arming and releasing a stage are paid once per SUB blocks
   const int SUB = KIND == GEMM_I8 ? (p.sub_blocks > 1 ? p.sub_blocks : 1) : 1;
   const int k_groups = p.k_blocks / SUB;
+  const int taps = p.k_blocks / p.c_blocks;  // K runs over channel blocks, then the taps of one (plain matrices: one tap)
   // a unit of work is a tile, or one chunk of its K blocks
   const int chunks = KIND == GEMM_BF16X3 ? p.chunks : 1;
   const bool split_k = KIND == GEMM_BF16X3 && p.split_k != 0;
@@ -318,11 +319,11 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
           }
         }
         if (p.trace != nullptr && blockIdx.x == 0 && !is_b) p.trace[(unit / gridDim.x) * 16 + 0] = clock64();
-        // the current K block: channel block, filter row and column
-        int cb = 0, kh = 0, kw = 0;
+        // the current K block: channel block, tap, and the tap's filter row and column
+        int cb = 0, tap = 0, kh = 0, kw = 0;
         if (kg0 > 0) {
-          const int tap = kg0 / p.c_blocks;
-          cb = kg0 - tap * p.c_blocks;
+          cb = kg0 / taps;
+          tap = kg0 - cb * taps;
           kh = tap / p.KW;
           kw = tap - kh * p.KW;
         }
@@ -344,7 +345,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
             for (int sb = 0; sb < SUB; ++sb) {
               const uint32_t dst = smem_base + static_cast<uint32_t>(s * SUB + sb) * stage_bytes;
               if (is_b) {
-                const int k = (kg * SUB + sb) * p.k_elems;
+                const int k = (tap * p.c_blocks + cb) * p.k_elems;
                 tma_load_2d(dst + b_off, &map_b0, fb, k, n0);
                 if (PLANES == 2) tma_load_2d(dst + b_off + b_slot, &map_b1, fb, k, n0);
               } else {
@@ -358,18 +359,19 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
                     if (PLANES == 2)
                       tma_load_im2col_4d(at + slot, &map_a1, fb, cb * p.k_elems, w_base[half], h_base[half], img[half], dw, dh);
                   } else {
-                    const int k = (kg * SUB + sb) * p.k_elems;
+                    const int k = cb * p.k_elems;
                     tma_load_2d(at, &map_a0, fb, k, static_cast<int>(half ? m1 : m0));
                     if (PLANES == 2) tma_load_2d(at + slot, &map_a1, fb, k, static_cast<int>(half ? m1 : m0));
                   }
                 }
-                if (++cb == p.c_blocks) {
-                  cb = 0;
-                  if (++kw == p.KW) {
-                    kw = 0;
-                    ++kh;
-                  }
-                }
+              }
+              if (++kw == p.KW) {
+                kw = 0;
+                ++kh;
+              }
+              if (++tap == taps) {
+                tap = kh = kw = 0;
+                ++cb;
               }
             }
           }

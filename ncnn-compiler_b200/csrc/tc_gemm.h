@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "tc_conv_halo.cuh"
+#include "tc_conv_patch.cuh"
 #include "tc_dw_project.cuh"
 #include "tc_gemm.cuh"
 #include "tc_gemm2.cuh"
@@ -163,6 +164,24 @@ bool tc_halo_applies(int kind, int C, int KH, int KW, int stride_h, int stride_w
 std::string tc_plan_conv_halo(TcHaloLaunch* launch, int kind, const TcHaloConv& conv, const TcEpilogue& epilogue,
                               int sm_count, bool pair = false);
 cudaError_t tc_launch_halo(const TcHaloLaunch& launch, cudaStream_t stream);
+
+// ---- convolution of few pixels out of input patches (tc_conv_patch.cuh)
+struct TcPatchLaunch {
+  TcPatchParams p{};
+  alignas(64) CUtensorMap map_a0{};
+  alignas(64) CUtensorMap map_a1{};
+  alignas(64) CUtensorMap map_b0{};
+  alignas(64) CUtensorMap map_b1{};
+  int kind = GEMM_BF16X3;
+  int grid = 0;
+  int smem_bytes = 0;
+};
+// Plans the convolution of tc_plan_conv's arguments on tc_conv_patch_kernel, in the tile shape that is expected to take
+// the least time.  Returns the reason where the kernel does not apply (bf16 pairs, stride 1 or 2, no dilation), or, unless
+// `always`, where `gemm`, the same layer's plan on the other kernels, is expected to be about as fast.
+std::string tc_plan_conv_patch(TcPatchLaunch* launch, int kind, const TcIm2colView& view, const void* w0, const void* w1,
+                               int out_channels, const TcEpilogue& epilogue, int sm_count, const TcLaunch& gemm, bool always);
+cudaError_t tc_launch_patch(const TcPatchLaunch& launch, cudaStream_t stream);
 
 // ---- 3x3 depthwise convolution fused into the following 1x1 convolution (tc_dw_project.cuh)
 struct TcDwProjLaunch {

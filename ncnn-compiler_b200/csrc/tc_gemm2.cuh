@@ -212,10 +212,11 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           h_base = oh * p.stride_h - p.pad_t;
           w_base = ow * p.stride_w - p.pad_l;
         }
-        const int tap0 = kb0 / p.c_blocks;
-        int cb = kb0 - tap0 * p.c_blocks;
-        int kh = tap0 / p.KW;
-        int kw = tap0 - kh * p.KW;
+        // K runs over channel blocks, then taps; half-size blocks follow each other inside a tap (the same order of products)
+        const int taps = p.k_blocks / p.c_blocks, halves = p.half_blocks ? 2 : 1;
+        int cb = kb0 / (taps * halves), half = kb0 % halves, tap = kb0 / halves - cb * taps;
+        int kh = tap / p.KW;
+        int kw = tap - kh * p.KW;
         for (int kb = kb0; kb < kb1; ++kb) {
           const uint32_t fb = PAIR ? map_to_cta(smem_u32(&full_bar[s]), 0u) : smem_u32(&full_bar[s]);
           if (!waited && (!is_b || issued == S)) {
@@ -230,32 +231,37 @@ tc_gemm2_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ 
           const bool tr = p.trace != nullptr && blockIdx.x == trace_cta && !is_b && i == 0 && kb - kb0 < 40;
           if (tr) p.trace[16 + 4 * (kb - kb0) + 2] = clock64();
           const uint32_t dst0 = smem_base + s * stage_bytes + my_off;
+          const int c_at = (cb * halves + half) * p.k_elems, k_at = tap * p.c_blocks * p.k_elems + c_at;
 #pragma unroll
           for (int plane = 0; plane < PLANES; ++plane) {
             const uint32_t dst = dst0 + static_cast<uint32_t>(plane) * my_plane;
             if (is_b) {
               const CUtensorMap* map = plane ? &map_b1 : &map_b0;
-              if (PAIR) tma_load_2d_pair(dst, map, fb, kb * p.k_elems, n0);
-              else tma_load_2d(dst, map, fb, kb * p.k_elems, n0);
+              if (PAIR) tma_load_2d_pair(dst, map, fb, k_at, n0);
+              else tma_load_2d(dst, map, fb, k_at, n0);
             } else {
               const CUtensorMap* map = plane ? &map_a1 : &map_a0;
               const uint16_t dw = static_cast<uint16_t>(kw * p.dil_w), dh = static_cast<uint16_t>(kh * p.dil_h);
               if (p.a_im2col) {
-                if (PAIR) tma_load_im2col_4d_pair(dst, map, fb, cb * p.k_elems, w_base, h_base, img, dw, dh);
-                else tma_load_im2col_4d(dst, map, fb, cb * p.k_elems, w_base, h_base, img, dw, dh);
+                if (PAIR) tma_load_im2col_4d_pair(dst, map, fb, c_at, w_base, h_base, img, dw, dh);
+                else tma_load_im2col_4d(dst, map, fb, c_at, w_base, h_base, img, dw, dh);
               } else {
-                if (PAIR) tma_load_2d_pair(dst, map, fb, kb * p.k_elems, static_cast<int>(m0));
-                else tma_load_2d(dst, map, fb, kb * p.k_elems, static_cast<int>(m0));
+                if (PAIR) tma_load_2d_pair(dst, map, fb, c_at, static_cast<int>(m0));
+                else tma_load_2d(dst, map, fb, c_at, static_cast<int>(m0));
               }
             }
           }
           if (tr) p.trace[16 + 4 * (kb - kb0) + 3] = clock64();
           ++issued;
-          if (++cb == p.c_blocks) {
-            cb = 0;
+          if (++half == halves) {
+            half = 0;
             if (++kw == p.KW) {
               kw = 0;
               ++kh;
+            }
+            if (++tap == taps) {
+              tap = kh = kw = 0;
+              ++cb;
             }
           }
           if (++s == S) {

@@ -52,6 +52,7 @@ struct TcGemmParams {
   int tiles_m, tiles_n, block_n;
   int k_blocks;   // K iterations per tile = taps * c_blocks
   int c_blocks;   // channel blocks per filter tap (K blocks for a plain GEMM)
+  int half_blocks;  // tc_gemm2_kernel: K blocks are halves of the usual size, c_blocks and k_blocks count halves
   int k_elems;    // elements per K block
   int row_bytes;  // bytes per shared-memory operand row: 128 or 64
   int stages;

@@ -247,3 +247,61 @@ def test_int8_residuals_beyond_the_l2_cache(pkg, tmp_path):
     got = m.run(x)[0]
     for rows in (slice(0, 3), slice(80, 82), slice(162, 165)):
         assert np.array_equal(m.run(x[rows])[0], got[rows])
+
+
+@pytest.mark.parametrize("cin,cout,k,stride,h,w,n", [
+    (64, 64, 3, 1, 56, 56, 2),    # whole tiles
+    (64, 48, 3, 1, 9, 13, 3),     # tiles that overhang both ways
+    (8, 24, 3, 1, 17, 8, 1),      # one block of channels, most of it zero fill
+    (40, 20, 2, 1, 11, 10, 5),    # 64-byte rows, a second block that is a quarter full, rows of 80 bytes out
+    (96, 160, 3, 2, 15, 14, 2),   # stride 2 from odd and even columns
+    (96, 128, 5, 2, 12, 21, 1),
+    (64, 16, 7, 1, 7, 7, 2),      # groups of a filter row
+    (256, 256, 3, 1, 14, 14, 40), # more tiles than SMs
+    (512, 40, 3, 1, 5, 6, 1),     # chunks on different blocks
+    (512, 512, 3, 2, 8, 8, 70),   # and one after the other
+    (200, 64, 4, 1, 6, 40, 2),    # an even filter
+])
+def test_patch_kernel_equals_im2col_kernel(pkg, oracle, tmp_path, monkeypatch, cin, cout, k, stride, h, w, n):
+    """Small tiles out of input patches: the same products in the same order as the im2col kernel, so the same bits."""
+    param, bin_ = pkg.zoo.single_conv(str(tmp_path / "c"), h=h, w=w, cin=cin, cout=cout, k=k, stride=stride, pad=k // 2)
+    x = np.random.default_rng(23).uniform(-1, 1, (n, cin, h, w)).astype(np.float32)
+    got = {}
+    for level in ("0", "1"):
+        monkeypatch.setenv("NCNN_B200_PATCH", level)
+        m = pkg.Model(param, bin_)
+        got[level] = m.run(x)[0]
+        assert any("tc_conv_patch_kernel" in r["kernel"] for r in m.profile(n, repeat=1)) == (level == "1")
+        m.close()
+    assert np.array_equal(got["1"], got["0"])
+    assert rel_l2(got["1"][:1], oracle_rows(oracle, param, bin_, x[:1])) <= 3e-5
+
+
+@pytest.mark.parametrize("c,cout,h,n", [(64, 96, 15, 2), (128, 64, 7, 9), (96, 32, 10, 3)])
+def test_patch_kernel_with_residuals(pkg, tmp_path, monkeypatch, c, cout, h, n):
+    """bf16-pair results and residuals of tiles that overhang the image."""
+    param, bin_ = pkg.zoo.residual_block(str(tmp_path / "rb"), h=h, w=h, c=c, cout=cout)
+    x = np.random.default_rng(24).uniform(-1, 1, (n, c, h, h)).astype(np.float32)
+    monkeypatch.setenv("NCNN_B200_PATCH", "1")
+    m = pkg.Model(param, bin_)
+    got = m.run(x)[0]
+    kernels = {r["layer"]: r["kernel"] for r in m.profile(n, repeat=1)}
+    assert "tc_conv_patch_kernel" in kernels["conv1"] and "tc_conv_patch_kernel" in kernels["conv2"]
+    monkeypatch.setenv("NCNN_B200_PATCH", "0")
+    assert np.array_equal(pkg.Model(param, bin_).run(x)[0], got)
+
+
+def test_patch_kernel_waits_that_run_out(pkg, tmp_path, monkeypatch):
+    """A first patch that never comes: the bounded waits give up, the call answers 7, the handle recovers."""
+    param, bin_ = pkg.zoo.single_conv(str(tmp_path / "c"), h=20, w=20, cin=128)
+    x = np.random.default_rng(25).uniform(-1, 1, (1, 128, 20, 20)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    assert any("tc_conv_patch_kernel" in r["kernel"] for r in m.profile(1, repeat=1))
+    good = m.run(x)[0].copy()
+    monkeypatch.setenv("NCNN_B200_TEST_STALL", "1")
+    with pytest.raises(pkg.NcnnB200Error) as err:
+        m.run(x)
+    assert err.value.status == 7
+    monkeypatch.delenv("NCNN_B200_TEST_STALL")
+    assert np.array_equal(m.run(x)[0], good)
+    m.check_status()
