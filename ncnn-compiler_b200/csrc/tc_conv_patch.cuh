@@ -395,7 +395,7 @@ tc_conv_patch_kernel(const __grid_constant__ TcPatchParams p, const __grid_const
         // the chunks of a tile run on different CTAs; whichever warp publishes its rows last adds them up (tc_gemm.cuh)
         const size_t slot_words = static_cast<size_t>(kTcBlockM) * lp.block_n;
         uint32_t* const ws = lp.sk_ws + static_cast<size_t>(unit) * slot_words + static_cast<size_t>(quarter * 32 + lane) * 16;
-        tc_publish_chunk(t_row, ws, lp.block_n);
+        tc_publish_chunk(t_row, ws, lp.block_n, inside);
         int* const count = lp.sk_flags + u.tile * 4 + quarter;
         __threadfence();
         __syncwarp();
@@ -407,7 +407,7 @@ tc_conv_patch_kernel(const __grid_constant__ TcPatchParams p, const __grid_const
         }
         if (lane == 0) *count = 0;  // for the next launch
         __threadfence();
-        tc_gather_chunks(ws - static_cast<size_t>(unit - u.tile * chunks) * slot_words, slot_words, chunks, t_row, lp.block_n);
+        tc_gather_chunks<KIND>(ws - static_cast<size_t>(unit - u.tile * chunks) * slot_words, slot_words, chunks, t_row, lp.block_n, inside);
       } else if (chunks > 1) {
         const uint32_t t_sum = t_quarter + static_cast<uint32_t>(2 * lp.acc_cols);
         for (int c = 0; c < chunks && ok; ++c) {

@@ -227,6 +227,50 @@ int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, 
   return width;
 }
 
+// InnerProduct and Gemm of too few rows to fill the SMs: the tile width and the chunks of K that are expected to take the
+// least time, the chunks of a tile on different CTAs.  Clocks as in gemm_clocks (a block's copies, or its MMAs and the gap
+// between blocks), and for the chunks' sums their way through L2.  Contractions of up to 22 blocks of bf16 pairs (1408
+// values) stay whole: a network's last layer then gives a batch the bits of its images run one by one.
+// Whole calls in us, before (workers that share tiles, tc_gemm2.cuh, or whole tiles) -> in chunks:
+//            2048 -> 1024          3000 -> 700           2816 -> 2816           4096 -> 4096
+//   fp32     64 rows 24.7 -> 16.4  64 rows 34.6 -> 14.4  64 rows 30.8 -> 20.5   64 rows 32.8 -> 28.7
+//            128     34.2 -> 14.4  128     48.4 -> 16.5  128     39.7 -> 22.7   128     39.4 -> 33.9
+//            300     33.7 -> 20.5  300     40.9 -> 22.7  300     30.9 -> 32.8   300     46.9 -> 45.6
+//            1000    26.7 -> 30.8  1000    36.8 -> 34.9  1000    49.3 -> 54.2   1000    87.4 -> 84.3
+//   int8     128     11.0 -> 12.8  300     12.9 -> 18.5  64      12.3 -> 14.5   64      23.4 -> 19.1, 128 30.7 -> 18.5
+// so it takes up to three tiles of rows; int8, whose blocks are short, from 28 blocks on and up to two.
+struct RowsSplit {
+  int block_n = 0, chunk_blocks = 0, chunks = 1;
+  double clocks = 1e300;
+};
+RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, int N, int sm_count) {
+  RowsSplit best;
+  if ((kind != GEMM_BF16X3 && kind != GEMM_I8) || e.sk_ws == nullptr || e.sk_flags == nullptr) return best;
+  const bool i8 = kind == GEMM_I8;
+  if (k_blocks < (i8 ? 28 : 23) || M > (i8 ? 2 : 3) * kTcBlockM || env_int("NCNN_B200_SPLIT_K", 1) == 0) return best;
+  const long long tiles_m = (M + kTcBlockM - 1) / kTcBlockM;
+  for (int bn = 16; bn <= 128 && bn < N + 16; bn += 16) {
+    const long long tiles = tiles_m * ((N + bn - 1) / bn);
+    const double mmas = i8 ? 4.0 : 12.0;
+    const double block = std::max(tc_planes(kind) * 3.0 * (kTcBlockM + bn), mmas * std::max(39.0, (kTcBlockM + bn) / 4.0) + 330.0);
+    for (int chunks = 1; chunks <= std::min(32, k_blocks / 2); ++chunks) {
+      const int blocks = (k_blocks + chunks - 1) / chunks;
+      if ((k_blocks + blocks - 1) / blocks != chunks) continue;
+      const long long units = tiles * chunks;
+      if (chunks > 1 && (tiles * 8 > e.sk_flag_count || static_cast<size_t>(units) * kTcBlockM * bn * 4 > e.sk_ws_bytes)) continue;
+      // (a warp adds four chunks of 16 columns in ~700 clocks)
+      const double sums = 2500.0 + 700.0 * ((chunks + 3) / 4) * ((bn + 31) / 32) + static_cast<double>(tiles) * std::min<long long>(M, kTcBlockM) * chunks * bn / 500.0;
+      const double clocks = static_cast<double>((units + sm_count - 1) / sm_count) * blocks * block + 3000.0 + 12.0 * bn + (chunks > 1 ? sums : 0.0);
+      if (clocks >= best.clocks) continue;
+      best.clocks = clocks;
+      best.block_n = bn;
+      best.chunk_blocks = blocks;
+      best.chunks = chunks;
+    }
+  }
+  return best;
+}
+
 void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e, int sm_count) {
   TcGemmParams& p = L->p;
   p.M = static_cast<int>(M);
@@ -239,6 +283,15 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   if (const int width = split_width(p, e, N, p.block_n, sm_count)) {
     p.block_n = width;
     p.split_k = 1;
+  }
+  if (!p.a_im2col) {
+    const RowsSplit rows = split_rows(kind, M, p.k_blocks, e, N, sm_count);
+    if (rows.chunks > 1) {
+      p.block_n = rows.block_n;
+      p.chunk_blocks = rows.chunk_blocks;
+      p.chunks = rows.chunks;
+      p.split_k = 1;
+    }
   }
   p.sk_ws = e.sk_ws;
   p.sk_flags = e.sk_flags;
@@ -292,7 +345,7 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   // hand-shake per block, more than the block's copies and MMAs take) sets the pace.  A stage then holds several
   // K blocks (a divisor of their count, at least three stages deep): one hand-shake for all of them.
   p.sub_blocks = 1;
-  if (kind == GEMM_I8 && !p.pair && env_int("NCNN_B200_SUB_BLOCKS", 1) != 0)
+  if (kind == GEMM_I8 && !p.pair && !p.split_k && env_int("NCNN_B200_SUB_BLOCKS", 1) != 0)
     for (int sub : {4, 3, 2})
       if (p.k_blocks % sub == 0 && budget / (sub * p.stage_bytes) >= 3) {
         p.sub_blocks = sub;
@@ -428,6 +481,9 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
     const double cost_whole = static_cast<double>((one_tiles + sm_count - 1) / sm_count) * full_kb;
     const double cost_split = static_cast<double>((one_units + one_workers - 1) / one_workers) + 20.0;
     split_form = forced_split == 1 || cost_split < 0.9 * cost_whole;
+    // (chunks of K on different CTAs do the same without workers that wait, and win where rows are few)
+    const double block = std::max(tc_planes(kind) * 3.0 * (kTcBlockM + one_bn), (kind == GEMM_I8 ? 4.0 : 12.0) * (kTcBlockM + one_bn) / 4.0);
+    if (forced_split != 1 && split_rows(kind, M, full_kb, e, N, sm_count).clocks < cost_split * block + 3000.0) split_form = false;
   }
   if (!pair_form && !split_form) return false;
   const int ctas = pair_form ? 2 : 1;

@@ -223,8 +223,9 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
   const int k_groups = p.k_blocks / SUB;
   const int taps = p.k_blocks / p.c_blocks;  // K runs over channel blocks, then the taps of one (plain matrices: one tap)
   // a unit of work is a tile, or one chunk of its K blocks
-  const int chunks = KIND == GEMM_BF16X3 ? p.chunks : 1;
-  const bool split_k = KIND == GEMM_BF16X3 && p.split_k != 0;
+  constexpr bool CHUNKS = KIND == GEMM_BF16X3 || KIND == GEMM_I8;  // (int8: on different CTAs only)
+  const int chunks = CHUNKS ? p.chunks : 1;
+  const bool split_k = CHUNKS && p.split_k != 0;
   const int chunk_groups = chunks > 1 ? p.chunk_blocks : k_groups;  // (such contractions have one K block per stage)
   const int units = p.tiles_m * p.tiles_n * (split_k ? chunks : 1);
   // 512 TMEM columns: four accumulators (of a shallow contraction several tiles are in the pipeline at once), two
@@ -592,7 +593,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
       if (tracing) p.trace[(unit / gridDim.x) * 16 + 4] = clock64();
       uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                        static_cast<uint32_t>(acc) * (p.pair ? 256u : 128u) + (pair_tile && group ? 128u : 0u) + static_cast<uint32_t>(c_first);
-      if (KIND == GEMM_BF16X3 && chunks > 1) {
+      if (CHUNKS && chunks > 1) {
         const uint32_t t_first = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(c_first);
         const uint32_t t_sum = t_first + 384u;
         uint32_t* const ws = lp.sk_ws + static_cast<size_t>(unit) * kTcBlockM * lp.block_n +
@@ -604,8 +605,8 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
             tc_fence_after_sync();
             t_row = t_first + static_cast<uint32_t>(acc) * 128u;
           }
-          if (split_k) tc_publish_chunk(t_row, ws, cols);
-          else tc_add_chunk(t_row, t_sum, cols, c == 0);
+          if (split_k) tc_publish_chunk(t_row, ws, cols, valid);
+          else if (KIND == GEMM_BF16X3) tc_add_chunk(t_row, t_sum, cols, c == 0);
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
@@ -626,7 +627,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
           if (lane == 0) *count = 0;  // for the next launch
           __threadfence();
           const size_t slot_words = static_cast<size_t>(kTcBlockM) * lp.block_n;
-          tc_gather_chunks(ws - static_cast<size_t>(unit - tile * chunks) * slot_words, slot_words, chunks, t_sum, cols);
+          tc_gather_chunks<KIND>(ws - static_cast<size_t>(unit - tile * chunks) * slot_words, slot_words, chunks, t_sum, cols, valid);
         }
         t_row = t_sum;
       }
@@ -647,7 +648,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
         }
       }
       if (tracing) p.trace[(unit / gridDim.x) * 16 + 5] = clock64();
-      if (KIND == GEMM_BF16X3 && chunks > 1) continue;  // (the accumulators were handed back above)
+      if (CHUNKS && chunks > 1) continue;  // (the accumulators were handed back above)
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));

@@ -99,9 +99,9 @@ struct TcGemmParams {
   int8_t* side_q1;
   float side_scale0, side_scale1;
   long long side_ld;   // row stride of the int8 copies in elements
-  // bf16-pair convolutions of deep contractions: the K blocks are summed in `chunks` groups of chunk_blocks each and the
-  // groups' sums added in order (tc_chunks: by the layer alone, so that every batch size rounds the same).  split_k = 1:
-  // the chunks of a tile run on different CTAs (tc_gemm_kernel).
+  // The K blocks are summed in `chunks` groups of chunk_blocks each and the groups' sums added in order: deep bf16-pair
+  // convolutions (set_chunks: by the layer alone, so that every batch size rounds the same), and InnerProducts of few rows
+  // (split_rows).  split_k = 1: the chunks of a tile run on different CTAs (tc_gemm_kernel).
   int chunks, chunk_blocks, split_k;
   uint32_t* sk_ws;     // one slot of 128 x block_n accumulator words per CTA
   int* sk_flags;       // one word per CTA: 1 while its slot holds a partial that nobody has consumed
@@ -178,35 +178,42 @@ __device__ __forceinline__ void tc_add_chunk(uint32_t t_acc, uint32_t t_sum, int
 }
 // The same sum of chunks that different CTAs computed.  `ws` is this thread's row in the slot of a chunk
 // ([16-column group][row][16] words); the slots of a tile's chunks follow each other.
-__device__ __forceinline__ void tc_publish_chunk(uint32_t t_acc, uint32_t* ws, int cols) {
+// (`valid`: the row exists; every lane of the warp must call it)
+__device__ __forceinline__ void tc_publish_chunk(uint32_t t_acc, uint32_t* ws, int cols, bool valid) {
 #pragma unroll 1
   for (int c = 0; c < cols; c += 16) {
     uint32_t v[16];
     ptx::tmem_ld16(t_acc + static_cast<uint32_t>(c), v);
     ptx::tmem_ld_wait();
+    if (!valid) continue;
     uint4* d = reinterpret_cast<uint4*>(ws + static_cast<size_t>(c) * 128);
 #pragma unroll
     for (int q = 0; q < 4; ++q) __stcg(d + q, make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
   }
 }
-__device__ __forceinline__ void tc_gather_chunks(const uint32_t* ws, size_t slot_words, int chunks, uint32_t t_sum, int cols) {
+template <int KIND>
+__device__ __forceinline__ void tc_gather_chunks(const uint32_t* ws, size_t slot_words, int chunks, uint32_t t_sum, int cols, bool valid) {
 #pragma unroll 1
   for (int c = 0; c < cols; c += 16) {
-    float y[16];
-#pragma unroll 4
-    for (int k = 0; k < chunks; ++k) {
-      const float4* s = reinterpret_cast<const float4*>(ws + static_cast<size_t>(k) * slot_words + static_cast<size_t>(c) * 128);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 f = __ldcg(s + q);
-        const float w[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) y[4 * q + j] = k == 0 ? w[j] : __fadd_rn(y[4 * q + j], w[j]);
-      }
-    }
     uint32_t v[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(y[j]);
+    for (int j = 0; j < 16; ++j) v[j] = 0u;
+    if (valid) {
+#pragma unroll 4
+      for (int k = 0; k < chunks; ++k) {
+        const uint4* s = reinterpret_cast<const uint4*>(ws + static_cast<size_t>(k) * slot_words + static_cast<size_t>(c) * 128);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint4 f = __ldcg(s + q);
+          const uint32_t w[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (KIND == GEMM_I8) v[4 * q + j] += w[j];
+            else v[4 * q + j] = k == 0 ? w[j] : __float_as_uint(__fadd_rn(__uint_as_float(v[4 * q + j]), __uint_as_float(w[j])));
+          }
+        }
+      }
+    }
     ptx::tmem_st16(t_sum + static_cast<uint32_t>(c), v);
   }
   ptx::tmem_st_wait();

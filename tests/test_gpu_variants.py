@@ -305,3 +305,30 @@ def test_patch_kernel_waits_that_run_out(pkg, tmp_path, monkeypatch):
     monkeypatch.delenv("NCNN_B200_TEST_STALL")
     assert np.array_equal(m.run(x)[0], good)
     m.check_status()
+
+
+@pytest.mark.parametrize("m,k,n,int8", [
+    (9, 1472, 24, False),    # 23 K blocks: the shallowest, one narrow tile column
+    (100, 2048, 1000, False),
+    (128, 3000, 40, False),  # a last K block and a last chunk that are not full
+    (129, 1536, 72, False),  # a second tile of one row
+    (384, 1600, 136, False),
+    (385, 1600, 136, False), # past the line
+    (3, 4096, 80, True),
+    (256, 3600, 48, True),
+    (12, 3584, 2000, True),
+])
+def test_inner_product_of_few_rows_in_chunks(pkg, oracle, tmp_path, m, k, n, int8):
+    """Chunks of K on different blocks, added by whichever finishes last: the same bits call after call; int8 exact."""
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n, int8=int8)
+    x = np.random.default_rng(26).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    model = pkg.Model(param, bin_)
+    got = model.run(x)[0]
+    for _ in range(20):
+        assert np.array_equal(model.run(x)[0], got)
+    rows = sorted({0, m // 2, m - 1})
+    want = oracle_rows(oracle, param, bin_, x[rows]).reshape(got[rows].shape)
+    if int8:
+        assert np.array_equal(got[rows], want)
+    else:
+        assert rel_l2(got[rows], want) <= 3e-5
