@@ -246,7 +246,12 @@ int EngineImpl::launch(Plan* plan, const float* const* d_in, float* const* d_out
     fresh.ptrs.assign(d_in, d_in + ni);
     fresh.ptrs.insert(fresh.ptrs.end(), d_out, d_out + no);
     if (!assemble(*plan, std::vector<const float*>(d_in, d_in + ni), std::vector<float*>(d_out, d_out + no), &fresh.steps)) return 6;
-    if (opt_.use_cuda_graph) {
+    // A pass that is one launch of the rows kernel goes to the stream as it is: a graph's replay costs the GPU 3 to 4 us
+    // between calls (they come in steps of 2.05 us), a launch overlaps the one before it (InnerProduct 4096 x 4096, one row:
+    // 18.5 -> 15.5 us a call, 1024 x 2048: 8.2 -> 7.7).  Two launches take the host 10.6 us a call against 8.2 for a graph,
+    // and win only from ~9 us of GPU time on (12.3 -> 10.7, 14.4 -> 11.9; 512 x 512 8.2 -> 10.7): they stay a graph.  So does
+    // k_conv_f32, whose blocks come in several waves and mix with the next call's (1001 x 1537, one row: 45 -> 56).
+    if (opt_.use_cuda_graph && !(fresh.steps.size() == 1 && fresh.steps[0].direct)) {
       fresh.graph = capture_steps(fresh.steps);
       if (fresh.graph == nullptr) return 6;
       fresh.steps.clear();
@@ -260,7 +265,7 @@ int EngineImpl::launch(Plan* plan, const float* const* d_in, float* const* d_out
     pass = &plan->passes.back();
   }
   pass->last_used = ++use_counter_;
-  if (!opt_.use_cuda_graph) return issue_steps(pass->steps, st) ? 0 : 6;
+  if (pass->graph == nullptr) return issue_steps(pass->steps, st) ? 0 : 6;
   const cudaError_t e = cudaGraphLaunch(pass->graph, st);
   if (e != cudaSuccess) {
     error_ = std::string("launch failed: ") + cudaGetErrorString(e);

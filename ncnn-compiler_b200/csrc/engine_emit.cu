@@ -526,6 +526,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
           const int tasks = (ip.N + kIpRowsCols - 1) / kIpRowsCols;
           const int grid = std::max(1, std::min(sm_count_, tasks));
           s.kernel = i8 ? "k_ip_rows<i8>" : "k_ip_rows<bf16x2>";
+          s.direct = true;
           s.run = [=](cudaStream_t st) {
             if (i8) launch_plain(k_ip_rows<true>, grid, kIpRowsThreads, smem, st, ip);
             else launch_plain(k_ip_rows<false>, grid, kIpRowsThreads, smem, st, ip);

@@ -136,6 +136,7 @@ struct Step {
   std::string name, kernel;
   std::function<cudaError_t(cudaStream_t)> run;
   double flops = 0.0, bytes = 0.0;
+  bool direct = false;  // alone in a pass, it is launched without a graph (EngineImpl::launch)
 };
 
 constexpr int kMaxChunks = 4;
