@@ -472,8 +472,18 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         v.OH = node.OH;
         v.OW = node.OW;
         perr = tc_plan_conv(launch.get(), kind, v, node.d_w0, node.d_w1, node.O, te, sm_count_);
-        // few pixels: small tiles out of input patches (unless a switch asks for pairs of CTAs or split tiles)
         const bool forced = launch->cta2 != 0 && (env_int_or("NCNN_B200_CTA2_ALWAYS", 0) != 0 || env_int_or("NCNN_B200_STREAMK", 0) == 1);
+        // int8 filters of several taps that fit shared memory (unless a switch asks for pairs of CTAs or split tiles)
+        if (perr.empty() && i8 && !node.stem && conv_i8_level() != 0 && !forced) {
+          auto cl = std::make_shared<TcConvI8Launch>();
+          if (tc_plan_conv_i8(cl.get(), v, node.d_w0, node.O, te, sm_count_, conv_i8_level() > 0).empty()) {
+            s.kernel = "tc_conv_i8_kernel<i8>";
+            s.run = [cl](cudaStream_t st) { return tc_launch_conv_i8(*cl, st); };
+            steps.push_back(std::move(s));
+            return true;
+          }
+        }
+        // few pixels: small tiles out of input patches (unless a switch asks for pairs of CTAs or split tiles)
         if (perr.empty() && !node.stem && patch_level() != 0 && !forced) {
           auto pl = std::make_shared<TcPatchLaunch>();
           if (tc_plan_conv_patch(pl.get(), kind, v, node.d_w0, node.d_w1, node.O, te, sm_count_, *launch, patch_level() > 0).empty()) {

@@ -387,6 +387,11 @@ inline int patch_level() {
   const char* f = std::getenv("NCNN_B200_PATCH");
   return f == nullptr ? -1 : std::atoi(f);
 }
+// NCNN_B200_CONV_I8: the same for tc_conv_i8_kernel
+inline int conv_i8_level() {
+  const char* f = std::getenv("NCNN_B200_CONV_I8");
+  return f == nullptr || f[0] == 0 ? -1 : std::atoi(f);
+}
 inline int halo_level() {
   const char* f = std::getenv("NCNN_B200_HALO");
   return f == nullptr || f[0] == 0 ? -1 : std::atoi(f);

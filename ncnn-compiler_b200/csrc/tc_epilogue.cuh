@@ -39,7 +39,7 @@ struct TcDirect {
   int side_count;       // int8 copies of an fp32 result
   uint8_t* side_q0;     // at row 0 of the warp
   uint8_t* side_q1;
-  long long side_pitch;
+  long long side_pitch, side_pitch8;
   uint32_t side_stage;  // kDrainSideBytes of the warp's own per copy
   float side_scale0, side_scale1;
   // partial accumulators of other CTAs to add first (split tiles): slots fix_stride words apart, [16-column group][row][16]
@@ -85,12 +85,16 @@ static __device__ __noinline__ void tc_act_many(float* y, int act, float a, floa
 __device__ __forceinline__ void sts_16b(uint32_t at, const uint32_t* w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
-// 16 fp32 results -> 16 int8 with the reference's rounding
-__device__ __forceinline__ void tc_stage_side_quant(uint32_t at, float scale, const float (&y)[16]) {
+// 16 fp32 results -> 16 int8 with the reference's rounding; `positive`: neither results nor scale are below zero
+__device__ __forceinline__ void tc_stage_side_quant(uint32_t at, float scale, bool positive, const float (&y)[16]) {
   uint32_t w[4];
+  if (positive) {
 #pragma unroll
-  for (int g = 0; g < 4; ++g)
-    w[g] = pack_i8x4(quantize_rha(y[4 * g], scale), quantize_rha(y[4 * g + 1], scale), quantize_rha(y[4 * g + 2], scale), quantize_rha(y[4 * g + 3], scale));
+    for (int g = 0; g < 4; ++g) w[g] = quantize4_at_zero(y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3], scale);
+  } else {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) w[g] = quantize4(y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3], scale);
+  }
   sts_16b(at, w);
 }
 __device__ __forceinline__ uint4 lds_16b(uint32_t at) {
@@ -198,7 +202,7 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
   TcFlushLane<OUT == OUT_I8 ? 4 : 8> fl;
   if (OUT != OUT_CHW) fl.init(d, d.pitch, d.pitch8);
   TcFlushLane<4> side_fl;
-  if (SIDE) side_fl.init(d, d.side_pitch, 8 * d.side_pitch);
+  if (SIDE) side_fl.init(d, d.side_pitch, d.side_pitch8);
   uint32_t nxt[16];
   uint32_t(&r)[RW] = ops.r;
   float(&bias)[16] = ops.bias, (&scale)[16] = ops.scale;
@@ -263,12 +267,14 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
     }
     if (OUT == OUT_I8) {
       // requantise, clamp at zero for a fused ReLU (the order of the reference's int8 path)
-      const int floor_q = d.act == ACT_RELU ? 0 : -127;
       uint32_t w[4];
+      if (d.act == ACT_RELU) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
-        w[g] = pack_i8x4(max(quantize_rha(y[4 * g], d.out_scale), floor_q), max(quantize_rha(y[4 * g + 1], d.out_scale), floor_q),
-                         max(quantize_rha(y[4 * g + 2], d.out_scale), floor_q), max(quantize_rha(y[4 * g + 3], d.out_scale), floor_q));
+        for (int g = 0; g < 4; ++g) w[g] = quantize4_at_zero(y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3], d.out_scale);
+      } else {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) w[g] = quantize4(y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3], d.out_scale);
+      }
       const int piece = (c >> 4) & 3;
       sts_16b(d.stage + static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4)), w);
       if (piece == 3 || !more) {
@@ -295,13 +301,13 @@ __device__ __forceinline__ void tc_drain_as(const TcDirect& d, uint32_t t_row, i
       // int8 copies, 64 columns to a flush
       const int piece = (c >> 4) & 3, c64 = c & ~63;
       const uint32_t at = d.side_stage + static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
-      tc_stage_side_quant(at, d.side_scale0, y);
-      if (d.side_count > 1) tc_stage_side_quant(at + kDrainSideBytes, d.side_scale1, y);
+      tc_stage_side_quant(at, d.side_scale0, d.act == ACT_RELU && d.side_scale0 >= 0.0f, y);
+      if (d.side_count > 1) tc_stage_side_quant(at + kDrainSideBytes, d.side_scale1, d.act == ACT_RELU && d.side_scale1 >= 0.0f, y);
       if (piece == 3 || !more) {
         const int n = min(left - c64, c - c64 + 16);
-        tc_flush<4>(d.side_stage, d.side_pitch, 8 * d.side_pitch, side_fl, d.side_q0 + c64, nullptr, 64, n);
+        tc_flush<4>(d.side_stage, d.side_pitch, d.side_pitch8, side_fl, d.side_q0 + c64, nullptr, 64, n);
         if (d.side_count > 1)
-          tc_flush<4>(d.side_stage + kDrainSideBytes, d.side_pitch, 8 * d.side_pitch, side_fl, d.side_q1 + c64, nullptr, 64, n);
+          tc_flush<4>(d.side_stage + kDrainSideBytes, d.side_pitch, d.side_pitch8, side_fl, d.side_q1 + c64, nullptr, 64, n);
       }
     }
     if (OUT == OUT_CHW) {

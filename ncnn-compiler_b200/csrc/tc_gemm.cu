@@ -1147,6 +1147,123 @@ cudaError_t tc_launch_patch(const TcPatchLaunch& L, cudaStream_t stream) {
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+// ------------------------------------------------------------------ int8 convolution with its filter resident
+std::string tc_plan_conv_i8(TcConvI8Launch* L, const TcIm2colView& v, const void* w, int out_channels, const TcEpilogue& e, int sm_count,
+                            bool always) {
+  load_driver_entry_points();
+  if (!g_driver_error.empty()) return g_driver_error;
+  const int taps = v.KH * v.KW;
+  if (v.stride_conv_h != 1 || v.stride_conv_w != 1 || v.dil_h != 1 || v.dil_w != 1 || taps < 2 || v.KH > 16 || v.KW > 16)
+    return "the kernel takes filters of several taps, stride 1 and no dilation";
+  const int rb = tc_row_bytes(GEMM_I8, static_cast<int>(v.C));
+  if (rb < 64) return "rows of 32 bytes or none";
+  TcConvI8Params& p = L->p;
+  std::memset(&p, 0, sizeof(p));
+  const int res_mode = res_mode_of(e);
+  if ((e.out_mode != OUT_I8 && e.out_mode != OUT_F32) || (e.side_count > 0 && e.out_mode != OUT_F32) || (res_mode != RES_NONE && res_mode != RES_F32) ||
+      !direct_rows(GEMM_I8, e, out_channels, &p.wide))
+    return "the kernel writes channel-last rows of 16-byte pieces";
+  p.images = static_cast<int>(v.N);
+  p.OH = v.OH;
+  p.OW = v.OW;
+  p.N = out_channels;
+  p.tiles_y = (v.OH + kI8TileH - 1) / kI8TileH;
+  p.tiles_x = (v.OW + kI8TileW - 1) / kI8TileW;
+  const long long tiles = static_cast<long long>(v.N) * p.tiles_y * p.tiles_x;
+  if (tiles > (1 << 28)) return "too many tiles for one launch";
+  p.row_bytes = p.k_elems = rb;
+  p.c_blocks = (static_cast<int>(v.C) + rb - 1) / rb;
+  p.KH = v.KH;
+  p.KW = v.KW;
+  p.pad_t = v.pad_t;
+  p.pad_l = v.pad_l;
+  p.patch_h = kI8TileH + v.KH - 1;
+  p.patch_w = kI8TileW + v.KW - 1;
+  p.patch_bytes = (p.patch_h * p.patch_w * rb + 1023) / 1024 * 1024;
+  p.drain_bytes = (e.out_mode == OUT_I8 ? kDrainSideBytes : kDrainWarpBytes) + e.side_count * kDrainSideBytes;
+  const int blocks = taps * p.c_blocks;
+  // the widest column block that leaves room for two patches and an epilogue group, then more groups, then more patches
+  for (int parts = 1; parts <= (out_channels + 15) / 16; ++parts) {
+    p.block_n = ((out_channels + parts - 1) / parts + 15) / 16 * 16;
+    if (p.block_n > 256) continue;
+    p.b_bytes = (p.block_n * rb + 1023) / 1024 * 1024;
+    p.acc_cols = (p.block_n + 31) / 32 * 32;
+    for (p.groups = kI8MaxGroups; p.groups >= 1; --p.groups) {
+      if (p.groups * p.acc_cols > static_cast<int>(kTcTmemCols)) continue;
+      p.patches = std::min(kI8MaxPatches, (kTcSmemBudget - blocks * p.b_bytes - 4 * p.groups * p.drain_bytes) / p.patch_bytes);
+      if (p.patches >= 2) break;
+    }
+    if (p.groups >= 2) break;
+  }
+  if (p.groups < 2) return "the filter does not fit shared memory";
+  p.accs = p.groups * std::min({static_cast<int>(kTcTmemCols) / (p.groups * p.acc_cols), kI8MaxAccs / p.groups, 2});
+  p.tiles_n = (out_channels + p.block_n - 1) / p.block_n;
+  if (p.tiles_n > sm_count) return "more column blocks than SMs";
+  // Launches of ResNet-18's layers by events (~8 us of which are the events'), tc_gemm_kernel (or pairs of CTAs) -> this one; the
+  // second figure of a pair is a layer that adds an fp32 residual and writes fp32 and an int8 copy:
+  //   64 channels, 56x56           1 image 10.4, 12.6 -> 10.6, 13.3   4: 11.8, 14.1 -> 10.3, 13.7   64: 37, 51 -> 21, 41   256: 120, 160 -> 53, 116
+  //       33x33 (57 % of the tiles filled), 256 images 47, 69 -> 33, 64;  16x16, 16 images (one wave) 12.0, 12.6 -> 10.4, 13.5
+  //   128, 28x28 (77 %)            4: 11.2 -> 12.7   16: 14.4, 16.3 -> 13.5, 14.5   64: 20.5, 22.5 -> 18.5, 22.5   256: 43, 48 -> 39, 51
+  //       17x17 (38 %), 256 images 22.5, 24.7 -> 31, 41
+  //   256 (four column blocks), 14x14   4: 12.6, 15.2 -> 12.0, 14.3   16 (one wave): 14.4, 16.8 -> 12.5, 16.3   256: 38, 59 -> 43, 80
+  //   512 (16), 7x7                1: 16.4 -> 12.5   4 (one wave): 16.4 -> 12.7   16: 16.6 -> 18.4
+  // With one tile to a CTA nothing is reused, and what is left is a shorter chain: from 18 K blocks on.  With several the filter's
+  // reuse wins, unless tiles are mostly empty or the pixels are read again for each of many column blocks.
+  const long long waves = (tiles + sm_count / p.tiles_n - 1) / (sm_count / p.tiles_n);
+  const double filled = static_cast<double>(v.OH) * v.OW / (static_cast<double>(p.tiles_y) * p.tiles_x * kI8TileH * kI8TileW);
+  const bool pays = waves == 1 ? blocks >= 18 : p.tiles_n <= 2 && filled >= (rb == 64 ? 0.5 : 0.7);
+  if (!always && !pays) return "other kernels are expected to be as fast";
+  p.bias = e.bias;
+  p.scale = e.scale;
+  p.out0 = e.out0;
+  p.outq = e.outq;
+  p.res0 = e.res0;
+  p.ldo = e.ldo;
+  p.res_mode = res_mode;
+  p.far_res = p.res_mode == RES_F32 && static_cast<long long>(v.N) * v.OH * v.OW * e.ldo * 4 > (126ll << 20);
+  p.act = e.act;
+  p.act_a = e.act_a;
+  p.act_b = e.act_b;
+  p.out_scale = e.out_scale;
+  p.side_count = e.side_count;
+  p.side_q0 = e.side_q[0];
+  p.side_q1 = e.side_q[1];
+  p.side_scale0 = e.side_scale[0];
+  p.side_scale1 = e.side_scale[1];
+  p.status = e.status;
+  L->out_mode = e.out_mode;
+  L->threads = 64 + 128 * p.groups;
+  // never fewer bytes than half an SM's shared memory: each CTA takes all of tensor memory
+  L->smem_bytes = std::max(blocks * p.b_bytes + p.patches * p.patch_bytes + 4 * p.groups * p.drain_bytes + 1024, 120 * 1024);
+  L->grid = p.tiles_n * static_cast<int>(std::min<long long>(tiles, sm_count / p.tiles_n));
+
+  const cuuint64_t dims[4] = {v.C, v.W, v.H, v.N};
+  const cuuint64_t strides[3] = {v.stride_w, v.stride_h, v.stride_n};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(p.k_elems), static_cast<cuuint32_t>(p.patch_w), static_cast<cuuint32_t>(p.patch_h), 1};
+  const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
+  const CUresult r = g_encode_tiled(&L->map_a, dtype_for(GEMM_I8), 4, const_cast<void*>(v.plane0), dims, strides, box, elem_strides,
+                                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(rb), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return "cuTensorMapEncodeTiled (int8 patch) failed with code " + std::to_string(static_cast<int>(r));
+  const uint64_t k_total = static_cast<uint64_t>(blocks) * p.k_elems;
+  return encode_tiled_2d(&L->map_b, GEMM_I8, w, k_total, out_channels, k_total, p.k_elems, p.block_n, rb);
+}
+
+cudaError_t tc_launch_conv_i8(const TcConvI8Launch& L, cudaStream_t stream) {
+  KernelLaunchConfig lc(L.grid, L.threads, L.smem_bytes, false, stream);
+  const int max_smem = kTcSmemBudget + 1024;
+  cudaError_t e;
+  if (L.p.side_count > 0) {
+    if (L.p.res_mode != RES_NONE) e = launch_opted(tc_conv_i8_kernel<epi_form(OUT_F32, true), true>, max_smem, lc, L.p, L.map_a, L.map_b);
+    else e = launch_opted(tc_conv_i8_kernel<epi_form(OUT_F32, false), true>, max_smem, lc, L.p, L.map_a, L.map_b);
+  } else {
+    e = with_form<GEMM_I8, false>(L.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
+      return launch_opted(tc_conv_i8_kernel<decltype(form)::value, false>, max_smem, lc, L.p, L.map_a, L.map_b);
+    });
+  }
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 // ------------------------------------------------------------------ depthwise + projection
 namespace {
 

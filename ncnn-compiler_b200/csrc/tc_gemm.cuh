@@ -514,6 +514,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
     if (SIDE) {
       d.side_count = p.side_count;
       d.side_pitch = p.side_ld;
+      d.side_pitch8 = 8 * p.side_ld;
       d.side_stage = smem_base + static_cast<uint32_t>(S * SUB) * stage_bytes + 8u * kDrainWarpBytes +
                      static_cast<uint32_t>(group * 4 + quarter) * 2u * kDrainSideBytes;
       d.side_scale0 = p.side_scale0;

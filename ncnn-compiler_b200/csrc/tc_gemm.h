@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "tc_conv_halo.cuh"
+#include "tc_conv_i8.cuh"
 #include "tc_conv_patch.cuh"
 #include "tc_dw_project.cuh"
 #include "tc_gemm.cuh"
@@ -182,6 +183,23 @@ struct TcPatchLaunch {
 std::string tc_plan_conv_patch(TcPatchLaunch* launch, int kind, const TcIm2colView& view, const void* w0, const void* w1,
                                int out_channels, const TcEpilogue& epilogue, int sm_count, const TcLaunch& gemm, bool always);
 cudaError_t tc_launch_patch(const TcPatchLaunch& launch, cudaStream_t stream);
+
+// ---- int8 convolution with its filter resident in shared memory (tc_conv_i8.cuh)
+struct TcConvI8Launch {
+  TcConvI8Params p{};
+  alignas(64) CUtensorMap map_a{};
+  alignas(64) CUtensorMap map_b{};
+  int out_mode = OUT_I8;
+  int grid = 0;
+  int threads = 0;
+  int smem_bytes = 0;
+};
+// Plans the convolution of tc_plan_conv's arguments on tc_conv_i8_kernel.  Returns the reason where the kernel does not apply
+// (stride and dilation 1, more than 32 channels, a filter that fits shared memory), or, unless `always`, where the other
+// kernels are expected to be as fast.
+std::string tc_plan_conv_i8(TcConvI8Launch* launch, const TcIm2colView& view, const void* w, int out_channels,
+                            const TcEpilogue& epilogue, int sm_count, bool always);
+cudaError_t tc_launch_conv_i8(const TcConvI8Launch& launch, cudaStream_t stream);
 
 // ---- 3x3 depthwise convolution fused into the following 1x1 convolution (tc_dw_project.cuh)
 struct TcDwProjLaunch {

@@ -234,6 +234,19 @@ __device__ __forceinline__ uint32_t pack_i8x4(int a, int b, int c, int d) {
   asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(b), "r"(a), "r"(hi));
   return r;
 }
+__device__ __forceinline__ uint32_t quantize4(float a, float b, float c, float d, float s) {
+  return pack_i8x4(quantize_rha(a, s), quantize_rha(b, s), quantize_rha(c, s), quantize_rha(d, s));
+}
+// The same with a clamp at zero in place of -127 (a fused ReLU, or values and a scale that are not negative): what is negative
+// ends as zero however it is rounded, and cutting off a fraction is an addition, 2^23 plus the value rounded towards zero,
+// whose low bits are the whole part.  Conversions to int run at an eighth of the rate of additions.
+// (The form with a sign takes more instructions than it saves: 56x56x64 with an int8 copy 128 -> 141 us.)
+__device__ __forceinline__ uint32_t quantize4_at_zero(float a, float b, float c, float d, float s) {
+  auto bits = [s](float x) {
+    return __float_as_uint(__fadd_rz(fmaxf(fminf(__fadd_rn(__fmul_rn(x, s), 0.5f), 127.0f), 0.0f), 8388608.0f));
+  };
+  return __byte_perm(__byte_perm(bits(a), bits(b), 0x0040), __byte_perm(bits(c), bits(d), 0x0040), 0x5410);
+}
 
 __device__ __forceinline__ float round_tf32(float x) {
   uint32_t r;
@@ -288,9 +301,7 @@ __device__ __forceinline__ float apply_act(float y, int act, float a, float b) {
 __device__ __forceinline__ void tc_store_side_quant(int8_t* q, float scale, const float (&y)[16]) {
   uint32_t w[4];
 #pragma unroll
-  for (int g = 0; g < 4; ++g)
-    w[g] = pack_i8x4(quantize_rha(y[4 * g + 0], scale), quantize_rha(y[4 * g + 1], scale), quantize_rha(y[4 * g + 2], scale),
-                     quantize_rha(y[4 * g + 3], scale));
+  for (int g = 0; g < 4; ++g) w[g] = quantize4(y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3], scale);
   *reinterpret_cast<uint4*>(q) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 

@@ -351,8 +351,7 @@ tc_stem_pool_kernel(const __grid_constant__ TcStemPoolParams pp, const __grid_co
           if (KIND == GEMM_I8) {
             *reinterpret_cast<float4*>(p.out0 + at) = m;
             if (pp.side_q != nullptr)
-              *reinterpret_cast<uint32_t*>(pp.side_q + at) = pack_i8x4(quantize_rha(m.x, pp.side_scale), quantize_rha(m.y, pp.side_scale),
-                                                                       quantize_rha(m.z, pp.side_scale), quantize_rha(m.w, pp.side_scale));
+              *reinterpret_cast<uint32_t*>(pp.side_q + at) = quantize4(m.x, m.y, m.z, m.w, pp.side_scale);
           } else {
             uint2 hi, mid;
             split_bf16x2(m.x, m.y, hi.x, mid.x);

@@ -332,3 +332,58 @@ def test_inner_product_of_few_rows_in_chunks(pkg, oracle, tmp_path, m, k, n, int
         assert np.array_equal(got[rows], want)
     else:
         assert rel_l2(got[rows], want) <= 3e-5
+
+
+def _int8_pair(zoo, prefix, cin, mid, cout, k, h, w, act):
+    """Two int8 Convolutions in a row: the first writes int8 (term 101), the second fp32."""
+    net = zoo._Net(41, int8=True)
+    net.w.layer("Input", "input", [], ["data"], f"0={w} 1={h} 2={cin}")
+    net.conv("a", "data", "x", cin, mid, k, 1, k // 2, act=act, zero_bias=False, term=101)
+    net.conv("b", "x", "output", mid, cout, k, 1, k // 2, zero_bias=False, term=1)
+    return net.w.save(prefix)
+
+
+@pytest.mark.parametrize("cin,mid,cout,k,h,w,act,n", [
+    (64, 64, 64, 3, 16, 8, 1, 1),      # one whole tile
+    (64, 80, 48, 3, 17, 9, 1, 3),      # tiles that overhang both ways, rows that are no multiple of 64 bytes
+    (48, 96, 16, 3, 33, 20, 0, 2),     # a channel block that is three quarters full; results below zero
+    (80, 128, 128, 3, 28, 28, 1, 21),  # 128-byte rows, a filter that leaves room for few patches, more tiles than SMs
+    (192, 64, 272, 3, 15, 7, 0, 2),    # two channel blocks; several column blocks, the last one narrower
+    (256, 256, 256, 3, 7, 7, 1, 40),   # four column blocks of all taps of two channel blocks
+    (64, 64, 64, 2, 11, 12, 1, 2),     # filters that are no 3x3
+    (128, 48, 64, 5, 13, 16, 0, 2),
+])
+def test_int8_convolution_with_its_filter_resident(pkg, oracle, tmp_path, monkeypatch, cin, mid, cout, k, h, w, act, n):
+    """Whole-number sums: the same bits as the im2col kernel and the oracle."""
+    param, bin_ = _int8_pair(pkg.zoo, str(tmp_path / "c"), cin, mid, cout, k, h, w, act)
+    x = np.random.default_rng(42).uniform(-1, 1, (n, cin, h, w)).astype(np.float32)
+    got = {}
+    for level in ("0", "1"):
+        monkeypatch.setenv("NCNN_B200_CONV_I8", level)
+        m = pkg.Model(param, bin_)
+        got[level] = m.run(x)[0]
+        kernels = {r["layer"]: r["kernel"] for r in m.profile(n, repeat=1)}
+        assert ("tc_conv_i8_kernel" in kernels["a"]) == (level == "1")
+        m.close()
+    assert np.array_equal(got["1"], got["0"])
+    assert np.array_equal(got["1"][-1:], oracle_rows(oracle, param, bin_, x[-1:]))
+
+
+@pytest.mark.parametrize("size,n", [(64, 5), (97, 2), (224, 20)])
+def test_int8_network_with_resident_filters(pkg, oracle, tmp_path, monkeypatch, size, n):
+    """fp32 residuals and results with one or two int8 copies, tiles that overhang; by default (None) on the layers it suits."""
+    param, bin_ = pkg.zoo.resnet18(str(tmp_path / "r8"), int8=True, size=size, classes=40)
+    x = np.random.default_rng(size).uniform(-1, 1, (n, 3, size, size)).astype(np.float32)
+    got, used = {}, {}
+    for level in ("0", "1", None):
+        if level is None:
+            monkeypatch.delenv("NCNN_B200_CONV_I8")
+        else:
+            monkeypatch.setenv("NCNN_B200_CONV_I8", level)
+        m = pkg.Model(param, bin_)
+        got[level] = m.run(x)[0]
+        used[level] = sum("tc_conv_i8_kernel" in r["kernel"] for r in m.profile(n, repeat=1))
+        m.close()
+    assert used["0"] == 0 and used["1"] == 13 and used[None] > 0
+    assert np.array_equal(got["1"], got["0"]) and np.array_equal(got[None], got["0"])
+    assert np.array_equal(got["1"][:1], oracle_rows(oracle, param, bin_, x[:1]))
