@@ -339,6 +339,106 @@ static __global__ void __launch_bounds__(BM, 256 / BM) k_conv_f32(const float* _
   }
 }
 
+// ---- InnerProduct / Gemm of at most 16 rows, fp32 on the CUDA cores: one pass over the weights.
+//
+// k_conv_f32's tiles of 64 rows read every weight once too, but a block's 16 k at a time, and multiply mostly zeros.  Here a
+// warp takes 32 columns of one chunk of K and requests all its weights (up to 32 KB) before it waits for the first; ROWS
+// running pairs of sums per column, the rows of x broadcast from shared memory.  The chunks and the order of every sum are
+// k_conv_f32's, so the results are its bits.
+// Whole calls in us, tiles -> this kernel (the same bits, so the batch may decide):
+//            512 -> 1000     1001 -> 1537    3001 -> 2501    4095 -> 4091    4097 -> 515     255 -> 33
+//   1 row    22.6 -> 8.4     45.1 -> 10.3    65.6 -> 13.6   120.5 -> 19.7    49.3 -> 12.4    41.1 -> 8.3
+//   8 rows   22.6 -> 12.4    45.2 -> 14.4    65.6 -> 22.1   120.9 -> 28.8    51.3 -> 16.5    41.1 -> 12.4
+//   16 rows  22.6 -> 16.5    47.2 -> 20.6    67.7 -> 30.9   122.9 -> 51.5    51.3 -> 20.6    43.1 -> 14.5
+// (7 -> 5: 8 rows 8.3 -> 6.2, 16 rows 8.4 -> 10.3: short rows take it up to eight.)
+// What bounds it: one row, the weights' way from HBM (4095 -> 4091: 67 MB at 3.4 TB/s, launch included); many rows, the 48 KB
+// of a warp, of which an SM holds four, and the broadcasts (one 16-byte read for two packed FMAs).
+constexpr int kRowsF32Cols = 32;
+constexpr int kRowsF32Max = 16;
+
+__device__ __forceinline__ void cp_async_8(uint32_t smem_dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+
+template <int ROWS>
+static __global__ void __launch_bounds__(kRowsF32Cols) k_rows_f32(const float* __restrict__ x, ActRef out, const F32ConvParams p) {
+  ptx::grid_dependency_trigger();
+  constexpr int PAIRS = kF32Chunk / 2;
+  __shared__ __align__(16) uint64_t sw[PAIRS][kRowsF32Cols];
+  __shared__ __align__(16) float sx[ROWS][kF32Chunk];
+  const int lane = threadIdx.x, tile = blockIdx.x, chunk = blockIdx.y;
+  const int o = tile * kRowsF32Cols + lane, O = p.g.O, M = static_cast<int>(p.g.images);
+  const int k_begin = chunk * p.chunk_k, k_end = min(p.K, k_begin + p.chunk_k);
+  const int pairs = (k_end - k_begin + 1) / 2;
+  const bool in = o < O;
+  // (no kernel writes weights: they come while the kernel before this one runs)
+  const float* w = p.weights + (static_cast<long long>(k_begin / 2) * O + (in ? o : 0)) * 2;
+  const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(&sw[0][lane]));
+#pragma unroll 16
+  for (int j = 0; j < pairs; ++j) cp_async_8(dst + static_cast<uint32_t>(j) * (kRowsF32Cols * 8), w + static_cast<long long>(j) * O * 2);
+  if (pairs & 1) sw[pairs][lane] = 0ull;  // (pairs are taken two at a time; a chunk holds an even number unless it is the last)
+  ptx::grid_dependency_wait();
+  const uint32_t xdst = static_cast<uint32_t>(__cvta_generic_to_shared(&sx[0][lane]));
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const float* row = x + static_cast<long long>(r) * p.K + k_begin;
+#pragma unroll 8
+    for (int k = lane; k < 4 * ((pairs + 1) / 2); k += kRowsF32Cols) {
+      const bool there = r < M && k_begin + k < k_end;
+      cp_async_4(xdst + static_cast<uint32_t>(r * kF32Chunk + k - lane) * 4u, there ? row + k : x, there ? 4 : 0);
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+  uint64_t acc[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) acc[r] = 0ull;
+#pragma unroll 4
+  for (int j = 0; j < pairs; j += 2) {
+    const uint64_t w0 = sw[j][lane], w1 = sw[j + 1][lane];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&sx[r][2 * j]);
+      f32x2_fma(acc[r], a.x, w0);
+      f32x2_fma(acc[r], a.y, w1);
+    }
+  }
+  float y[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const float2 t = f32x2_get(acc[r]);
+    y[r] = __fadd_rn(t.x, t.y);
+  }
+  if (p.chunks > 1) {
+    // the block that finishes a tile last adds its chunks in order
+    float* const ws = p.partials + static_cast<size_t>(tile) * p.chunks * ROWS * kRowsF32Cols + lane;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) __stcg(ws + (chunk * ROWS + r) * kRowsF32Cols, y[r]);
+    __threadfence();
+    __syncwarp();
+    int before = 0;
+    if (lane == 0) before = atomicAdd(p.counters + tile, 1);
+    if (__shfl_sync(0xffffffffu, before, 0) != p.chunks - 1) return;
+    if (lane == 0) p.counters[tile] = 0;  // as the next launch expects it
+    __threadfence();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) y[r] = __ldcg(ws + r * kRowsF32Cols);
+#pragma unroll 2
+    for (int c = 1; c < p.chunks; ++c)
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) y[r] = __fadd_rn(y[r], __ldcg(ws + (c * ROWS + r) * kRowsF32Cols));
+  }
+  if (!in) return;
+  const float b = p.e.bias != nullptr ? __ldg(p.e.bias + o) : 0.0f;
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    if (r >= M) break;
+    const long long at = static_cast<long long>(r) * O + o;
+    act_store(out, at, conv_finish_f32(p.e, __fadd_rn(y[r], b), p.e.has_res ? act_load(p.e.res, at) : 0.0f));
+  }
+}
+
 constexpr int f32_smem_bytes(int bm) { return (kF32Stages * (bm * kF32Ak + kF32Bk * kF32Bn) + bm * kF32Bn) * 4; }
 
 }  // namespace nb

@@ -57,6 +57,24 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
   p.clamp_lo = e.act == ACT_RELU ? 0.0f : (e.act == ACT_CLIP ? e.act_a : -std::numeric_limits<float>::infinity());
   p.clamp_hi = e.act == ACT_CLIP ? e.act_b : std::numeric_limits<float>::infinity();
   const float* x = in.p0;
+  // a handful of rows: a pass over the weights (k_rows_f32, which says where; NCNN_B200_ROWS_F32=0: tiles everywhere)
+  const int cols = (g.O + kRowsF32Cols - 1) / kRowsF32Cols;
+  const int most = env_flag_off("NCNN_B200_ROWS_F32") ? 0 : (p.K >= 128 ? kRowsF32Max : kRowsF32Max / 2);
+  const bool flat = g.H == 1 && g.W == 1 && g.OH == 1 && g.OW == 1 && g.KH == 1 && g.KW == 1;
+  if (flat && rows <= most && p.chunks < 65536 &&
+      (p.chunks == 1 || (cols <= kTcSplitFlagCount && static_cast<size_t>(cols) * p.chunks * kRowsF32Max * kRowsF32Cols * 4 <= kTcSplitWorkspaceBytes))) {
+    const dim3 rgrid(static_cast<unsigned>(cols), static_cast<unsigned>(p.chunks));
+    s->kernel = "k_rows_f32";
+    s->run = [=](cudaStream_t st) {
+      if (rows <= 1) launch_plain(k_rows_f32<1>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else if (rows <= 2) launch_plain(k_rows_f32<2>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else if (rows <= 4) launch_plain(k_rows_f32<4>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else if (rows <= 8) launch_plain(k_rows_f32<8>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else launch_plain(k_rows_f32<kRowsF32Max>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      return launch_ok();
+    };
+    return {};
+  }
   const dim3 grid(static_cast<unsigned>(tiles), p.split ? p.chunks : 1);
   const cudaError_t ae = large ? cudaFuncSetAttribute(k_conv_f32<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem_bytes(128))
                                : cudaFuncSetAttribute(k_conv_f32<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem_bytes(64));

@@ -387,3 +387,26 @@ def test_int8_network_with_resident_filters(pkg, oracle, tmp_path, monkeypatch, 
     assert used["0"] == 0 and used["1"] == 13 and used[None] > 0
     assert np.array_equal(got["1"], got["0"]) and np.array_equal(got[None], got["0"])
     assert np.array_equal(got["1"][:1], oracle_rows(oracle, param, bin_, x[:1]))
+
+
+@pytest.mark.parametrize("m,k,n", [
+    (1, 7, 5),       # one short chunk, most lanes without a column
+    (3, 1001, 33),   # an odd K: its last pair is half there; one column past a block
+    (8, 512, 64),    # whole chunks
+    (9, 257, 31),    # two chunks, the second one shorter
+    (16, 4097, 515), # as many rows as the kernel takes, seventeen chunks
+])
+def test_fp32_inner_product_of_few_rows(pkg, oracle, tmp_path, monkeypatch, m, k, n):
+    """A pass over the weights sums in the tiles' chunks and order: the same bits, so more rows change none."""
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n)
+    x = np.random.default_rng(43).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    model = pkg.Model(param, bin_, accuracy_mode=pkg.FP32_CUDA)
+    got = model.run(x)[0]
+    assert any(r["kernel"] == "k_rows_f32" for r in model.profile(m, repeat=1))
+    many = model.run(np.concatenate([x] * (16 // m + 1)))[0]  # more rows than the kernel takes
+    assert np.array_equal(many[:m], got) and np.array_equal(many[-m:], got)
+    monkeypatch.setenv("NCNN_B200_ROWS_F32", "0")
+    tiles = pkg.Model(param, bin_, accuracy_mode=pkg.FP32_CUDA)
+    assert np.array_equal(tiles.run(x)[0], got)
+    assert not any(r["kernel"] == "k_rows_f32" for r in tiles.profile(m, repeat=1))
+    assert rel_l2(got, oracle_rows(oracle, param, bin_, x)) <= 2e-6
