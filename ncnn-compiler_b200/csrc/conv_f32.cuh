@@ -339,7 +339,7 @@ static __global__ void __launch_bounds__(BM, 256 / BM) k_conv_f32(const float* _
   }
 }
 
-// ---- InnerProduct / Gemm of at most 16 rows, fp32 on the CUDA cores: one pass over the weights.
+// ---- InnerProduct / Gemm of few rows, fp32 on the CUDA cores: one pass over the weights for every 16 rows.
 //
 // k_conv_f32's tiles of 64 rows read every weight once too, but a block's 16 k at a time, and multiply mostly zeros.  Here a
 // warp takes 32 columns of one chunk of K and requests all its weights (up to 32 KB) before it waits for the first; ROWS
@@ -350,11 +350,18 @@ static __global__ void __launch_bounds__(BM, 256 / BM) k_conv_f32(const float* _
 //   1 row    22.6 -> 8.4     45.1 -> 10.3    65.6 -> 13.6   120.5 -> 19.7    49.3 -> 12.4    41.1 -> 8.3
 //   8 rows   22.6 -> 12.4    45.2 -> 14.4    65.6 -> 22.1   120.9 -> 28.8    51.3 -> 16.5    41.1 -> 12.4
 //   16 rows  22.6 -> 16.5    47.2 -> 20.6    67.7 -> 30.9   122.9 -> 51.5    51.3 -> 20.6    43.1 -> 14.5
-// (7 -> 5: 8 rows 8.3 -> 6.2, 16 rows 8.4 -> 10.3: short rows take it up to eight.)
+//   32       22.6 -> 16.7    49.3 -> 20.6    69.7 -> 49.8   126.9 -> 90.1    55.4 -> 22.6    45.3 -> 16.5
+//   48       22.6 -> 18.5    53.2 -> 22.6    73.8 -> 65.6   131.1 -> 127.3   57.5 -> 32.9    49.3 -> 16.5
+//   64       22.6 -> 18.5    55.4 -> 32.5    76.1 -> 82.4   134.6 -> 163.8   61.4 -> 34.5    51.3 -> 16.5
+// So up to three groups of 16 rows, and up to kRowsF32Most where seven warps an SM (which holds four at a time) do it
+// (96 rows: 513 -> 600 30.8 -> 16.5, 700 -> 2001, 7.7 warps an SM, 37.0 -> 38.5): from there on the weights' repeated way out of L2
+// costs more than the tiles' empty rows.  7 -> 5: 8 rows 8.3 -> 6.2, 16 rows 8.4 -> 10.3: short
+// rows take it up to eight.
 // What bounds it: one row, the weights' way from HBM (4095 -> 4091: 67 MB at 3.4 TB/s, launch included); many rows, the 48 KB
 // of a warp, of which an SM holds four, and the broadcasts (one 16-byte read for two packed FMAs).
 constexpr int kRowsF32Cols = 32;
-constexpr int kRowsF32Max = 16;
+constexpr int kRowsF32Max = 16;    // rows of a warp
+constexpr int kRowsF32Most = 128;  // rows of a call
 
 __device__ __forceinline__ void cp_async_8(uint32_t smem_dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_dst), "l"(src) : "memory");
@@ -366,8 +373,9 @@ static __global__ void __launch_bounds__(kRowsF32Cols) k_rows_f32(const float* _
   constexpr int PAIRS = kF32Chunk / 2;
   __shared__ __align__(16) uint64_t sw[PAIRS][kRowsF32Cols];
   __shared__ __align__(16) float sx[ROWS][kF32Chunk];
-  const int lane = threadIdx.x, tile = blockIdx.x, chunk = blockIdx.y;
-  const int o = tile * kRowsF32Cols + lane, O = p.g.O, M = static_cast<int>(p.g.images);
+  const int lane = threadIdx.x, chunk = blockIdx.y, row0 = blockIdx.z * ROWS;
+  const int tile = blockIdx.x + blockIdx.z * gridDim.x;
+  const int o = blockIdx.x * kRowsF32Cols + lane, O = p.g.O, M = static_cast<int>(p.g.images) - row0;
   const int k_begin = chunk * p.chunk_k, k_end = min(p.K, k_begin + p.chunk_k);
   const int pairs = (k_end - k_begin + 1) / 2;
   const bool in = o < O;
@@ -381,7 +389,7 @@ static __global__ void __launch_bounds__(kRowsF32Cols) k_rows_f32(const float* _
   const uint32_t xdst = static_cast<uint32_t>(__cvta_generic_to_shared(&sx[0][lane]));
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    const float* row = x + static_cast<long long>(r) * p.K + k_begin;
+    const float* row = x + static_cast<long long>(row0 + r) * p.K + k_begin;
 #pragma unroll 8
     for (int k = lane; k < 4 * ((pairs + 1) / 2); k += kRowsF32Cols) {
       const bool there = r < M && k_begin + k < k_end;
@@ -434,7 +442,7 @@ static __global__ void __launch_bounds__(kRowsF32Cols) k_rows_f32(const float* _
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     if (r >= M) break;
-    const long long at = static_cast<long long>(r) * O + o;
+    const long long at = static_cast<long long>(row0 + r) * O + o;
     act_store(out, at, conv_finish_f32(p.e, __fadd_rn(y[r], b), p.e.has_res ? act_load(p.e.res, at) : 0.0f));
   }
 }

@@ -59,11 +59,12 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
   const float* x = in.p0;
   // a handful of rows: a pass over the weights (k_rows_f32, which says where; NCNN_B200_ROWS_F32=0: tiles everywhere)
   const int cols = (g.O + kRowsF32Cols - 1) / kRowsF32Cols;
-  const int most = env_flag_off("NCNN_B200_ROWS_F32") ? 0 : (p.K >= 128 ? kRowsF32Max : kRowsF32Max / 2);
+  const long long groups = (rows + kRowsF32Max - 1) / kRowsF32Max, warps = cols * groups * p.chunks;
   const bool flat = g.H == 1 && g.W == 1 && g.OH == 1 && g.OW == 1 && g.KH == 1 && g.KW == 1;
-  if (flat && rows <= most && p.chunks < 65536 &&
-      (p.chunks == 1 || (cols <= kTcSplitFlagCount && static_cast<size_t>(cols) * p.chunks * kRowsF32Max * kRowsF32Cols * 4 <= kTcSplitWorkspaceBytes))) {
-    const dim3 rgrid(static_cast<unsigned>(cols), static_cast<unsigned>(p.chunks));
+  const bool few = p.K >= 128 ? groups <= 3 || (rows <= kRowsF32Most && warps <= 7ll * sm_count_) : rows <= 8;
+  if (flat && few && p.chunks < 65536 && !env_flag_off("NCNN_B200_ROWS_F32") &&
+      (p.chunks == 1 || (cols * groups <= kTcSplitFlagCount && static_cast<size_t>(warps) * kRowsF32Max * kRowsF32Cols * 4 <= kTcSplitWorkspaceBytes))) {
+    const dim3 rgrid(static_cast<unsigned>(cols), static_cast<unsigned>(p.chunks), static_cast<unsigned>(groups));
     s->kernel = "k_rows_f32";
     s->run = [=](cudaStream_t st) {
       if (rows <= 1) launch_plain(k_rows_f32<1>, rgrid, kRowsF32Cols, 0, st, x, out, p);

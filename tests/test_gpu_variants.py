@@ -394,7 +394,9 @@ def test_int8_network_with_resident_filters(pkg, oracle, tmp_path, monkeypatch, 
     (3, 1001, 33),   # an odd K: its last pair is half there; one column past a block
     (8, 512, 64),    # whole chunks
     (9, 257, 31),    # two chunks, the second one shorter
-    (16, 4097, 515), # as many rows as the kernel takes, seventeen chunks
+    (16, 4097, 515), # as many rows as a warp takes, seventeen chunks
+    (17, 300, 70),   # a second group of one row
+    (128, 130, 40),  # as many rows as a call may have
 ])
 def test_fp32_inner_product_of_few_rows(pkg, oracle, tmp_path, monkeypatch, m, k, n):
     """A pass over the weights sums in the tiles' chunks and order: the same bits, so more rows change none."""
@@ -403,7 +405,7 @@ def test_fp32_inner_product_of_few_rows(pkg, oracle, tmp_path, monkeypatch, m, k
     model = pkg.Model(param, bin_, accuracy_mode=pkg.FP32_CUDA)
     got = model.run(x)[0]
     assert any(r["kernel"] == "k_rows_f32" for r in model.profile(m, repeat=1))
-    many = model.run(np.concatenate([x] * (16 // m + 1)))[0]  # more rows than the kernel takes
+    many = model.run(np.concatenate([x] * (128 // m + 1)))[0]  # more rows than the kernel takes
     assert np.array_equal(many[:m], got) and np.array_equal(many[-m:], got)
     monkeypatch.setenv("NCNN_B200_ROWS_F32", "0")
     tiles = pkg.Model(param, bin_, accuracy_mode=pkg.FP32_CUDA)
