@@ -229,8 +229,12 @@ int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, 
 
 // InnerProduct and Gemm of too few rows to fill the SMs: the tile width and the chunks of K that are expected to take the
 // least time, the chunks of a tile on different CTAs.  Clocks as in gemm_clocks (a block's copies, or its MMAs and the gap
-// between blocks), and for the chunks' sums their way through L2.  Contractions of up to 22 blocks of bf16 pairs (1408
-// values) stay whole: a network's last layer then gives a batch the bits of its images run one by one.
+// between blocks), and for the chunks' sums their way through L2.
+// fp32 sums round by where K is cut, so a layer has one way to cut it: the chunks that are best for a full tile of 128 rows
+// (with fewer rows others would be up to 4 % better by these clocks), for every call that is cut at all, and calls of 1 to
+// 128 rows are all cut or all whole; the rows choose the tile width, which no bit depends on.  Contractions of up to 26 blocks of bf16
+// pairs (1664 values) are never cut: a network's last layer then gives a batch the bits of its images run one by one
+// (1536 -> 1000, 33 rows: 16.5 us whole, 12.7 in chunks).  Whole numbers are exact however they are cut.
 // Whole calls in us, before (workers that share tiles, tc_gemm2.cuh, or whole tiles) -> in chunks:
 //            2048 -> 1024          3000 -> 700           2816 -> 2816           4096 -> 4096
 //   fp32     64 rows 24.7 -> 16.4  64 rows 34.6 -> 14.4  64 rows 30.8 -> 20.5   64 rows 32.8 -> 28.7
@@ -243,17 +247,17 @@ struct RowsSplit {
   int block_n = 0, chunk_blocks = 0, chunks = 1;
   double clocks = 1e300;
 };
-RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, int N, int sm_count) {
+// The best of whole tiles and tiles in `only` chunks (0: in any number of them).
+RowsSplit best_rows_split(int kind, long long M, int k_blocks, const TcEpilogue& e, int N, int sm_count, int only) {
   RowsSplit best;
-  if ((kind != GEMM_BF16X3 && kind != GEMM_I8) || e.sk_ws == nullptr || e.sk_flags == nullptr) return best;
   const bool i8 = kind == GEMM_I8;
-  if (k_blocks < (i8 ? 28 : 23) || M > (i8 ? 2 : 3) * kTcBlockM || env_int("NCNN_B200_SPLIT_K", 1) == 0) return best;
   const long long tiles_m = (M + kTcBlockM - 1) / kTcBlockM;
   for (int bn = 16; bn <= 128 && bn < N + 16; bn += 16) {
     const long long tiles = tiles_m * ((N + bn - 1) / bn);
     const double mmas = i8 ? 4.0 : 12.0;
     const double block = std::max(tc_planes(kind) * 3.0 * (kTcBlockM + bn), mmas * std::max(39.0, (kTcBlockM + bn) / 4.0) + 330.0);
     for (int chunks = 1; chunks <= std::min(32, k_blocks / 2); ++chunks) {
+      if (only != 0 && chunks != 1 && chunks != only) continue;
       const int blocks = (k_blocks + chunks - 1) / chunks;
       if ((k_blocks + blocks - 1) / blocks != chunks) continue;
       const long long units = tiles * chunks;
@@ -269,6 +273,19 @@ RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, i
     }
   }
   return best;
+}
+RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, int N, int sm_count) {
+  if ((kind != GEMM_BF16X3 && kind != GEMM_I8) || e.sk_ws == nullptr || e.sk_flags == nullptr) return {};
+  const bool i8 = kind == GEMM_I8;
+  if (k_blocks < (i8 ? 28 : 27) || M > (i8 ? 2 : 3) * kTcBlockM || env_int("NCNN_B200_SPLIT_K", 1) == 0) return {};
+  if (i8) return best_rows_split(kind, M, k_blocks, e, N, sm_count, 0);
+  const RowsSplit layer = best_rows_split(kind, kTcBlockM, k_blocks, e, N, sm_count, 0);
+  RowsSplit rows = best_rows_split(kind, M, k_blocks, e, N, sm_count, layer.chunks);
+  if (M <= kTcBlockM) {
+    if (rows.chunks != layer.chunks) rows = layer;
+    rows.clocks = layer.clocks;  // (what other forms are compared with: the same for all calls of one tile)
+  }
+  return rows;
 }
 
 void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e, int sm_count) {

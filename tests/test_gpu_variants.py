@@ -308,12 +308,16 @@ def test_patch_kernel_waits_that_run_out(pkg, tmp_path, monkeypatch):
 
 
 @pytest.mark.parametrize("m,k,n,int8", [
-    (9, 1472, 24, False),    # 23 K blocks: the shallowest, one narrow tile column
+    (9, 1472, 24, False),    # 23 K blocks: whole
+    (9, 1728, 24, False),    # 27: the shallowest in chunks, one narrow tile column
     (100, 2048, 1000, False),
     (128, 3000, 40, False),  # a last K block and a last chunk that are not full
-    (129, 1536, 72, False),  # a second tile of one row
+    (129, 1536, 72, False),
+    (129, 1792, 72, False),  # a second tile of one row
     (384, 1600, 136, False),
-    (385, 1600, 136, False), # past the line
+    (384, 1984, 136, False),
+    (385, 1600, 136, False),
+    (385, 1984, 136, False), # past the line
     (3, 4096, 80, True),
     (256, 3600, 48, True),
     (12, 3584, 2000, True),
@@ -332,6 +336,28 @@ def test_inner_product_of_few_rows_in_chunks(pkg, oracle, tmp_path, m, k, n, int
         assert np.array_equal(got[rows], want)
     else:
         assert rel_l2(got[rows], want) <= 3e-5
+
+
+@pytest.mark.parametrize("k,n", [
+    (1472, 1000),  # 23 K blocks: whole in every call
+    (1664, 1000),  # 26: the deepest of these
+    (1728, 1000),  # 27: in chunks
+    (1792, 1000),
+    (2048, 1000),
+    (4094, 520),   # a last K block that is not full
+    (2816, 2816),
+])
+def test_inner_product_sums_alike_whatever_the_rows_of_a_tile(pkg, tmp_path, k, n):
+    """Chunks of K follow from the layer: a row has the bits that it has among 128; where nothing is cut, those of any call."""
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n)
+    most = 400 if k <= 1664 else 128
+    x = np.random.default_rng(27).uniform(-1, 1, (most, 1, 1, k)).astype(np.float32)
+    model = pkg.Model(param, bin_)
+    want = model.run(x)[0]
+    first = 9 if 4 * k * n >= 8 << 20 else 1  # (up to eight rows of such weights take the rows kernel)
+    for m in (first, 16, 32, 33, 64, 65, 100, 127, 128, 384):
+        if m <= most:
+            assert np.array_equal(model.run(x[:m])[0], want[:m]), m
 
 
 def _int8_pair(zoo, prefix, cin, mid, cout, k, h, w, act):
