@@ -192,6 +192,9 @@ bool pair_enabled() {
 
 int env_int(const char* name, int fallback);
 
+// NCNN_B200_SPLIT_K=0 in the environment never puts the chunks of a tile on different CTAs: one CTA adds up the same chunks.
+bool split_k_enabled() { return env_int("NCNN_B200_SPLIT_K", 1) != 0; }
+
 // The chunks of a contraction's sums, from the layer alone (see kTcChunkFrom); p.k_blocks blocks of p.row_bytes.
 void set_chunks(TcGemmParams& p, int kind, int full_row_bytes) {
   p.chunks = 1;
@@ -210,7 +213,7 @@ void set_chunks(TcGemmParams& p, int kind, int full_row_bytes) {
 // at 16 columns (0.40 us; 128 columns take 1.3 of them, measured): a unit's chunk and its share of the latency of
 // publishing and adding sums, and those sums' way through L2, against the whole tiles' K blocks.
 int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, int sm_count) {
-  if (p.chunks < 2 || e.sk_ws == nullptr || e.sk_flags == nullptr || env_int("NCNN_B200_SPLIT_K", 1) == 0) return 0;
+  if (p.chunks < 2 || e.sk_ws == nullptr || e.sk_flags == nullptr || !split_k_enabled()) return 0;
   auto tiles_of = [&](int bn) { return static_cast<long long>(p.tiles_m) * ((N + bn - 1) / bn); };
   auto waves = [&](long long units) { return static_cast<double>((units + sm_count - 1) / sm_count); };
   double best = 0.9 * waves(tiles_of(block_n)) * p.k_blocks * (1.0 + block_n / 400.0);
@@ -277,8 +280,8 @@ RowsSplit best_rows_split(int kind, long long M, int k_blocks, const TcEpilogue&
 RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, int N, int sm_count) {
   if ((kind != GEMM_BF16X3 && kind != GEMM_I8) || e.sk_ws == nullptr || e.sk_flags == nullptr) return {};
   const bool i8 = kind == GEMM_I8;
-  if (k_blocks < (i8 ? 28 : 27) || M > (i8 ? 2 : 3) * kTcBlockM || env_int("NCNN_B200_SPLIT_K", 1) == 0) return {};
-  if (i8) return best_rows_split(kind, M, k_blocks, e, N, sm_count, 0);
+  if (k_blocks < (i8 ? 28 : 27) || M > (i8 ? 2 : 3) * kTcBlockM) return {};
+  if (i8) return split_k_enabled() ? best_rows_split(kind, M, k_blocks, e, N, sm_count, 0) : RowsSplit{};
   const RowsSplit layer = best_rows_split(kind, kTcBlockM, k_blocks, e, N, sm_count, 0);
   RowsSplit rows = best_rows_split(kind, M, k_blocks, e, N, sm_count, layer.chunks);
   if (M <= kTcBlockM) {
@@ -304,10 +307,12 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
   if (!p.a_im2col) {
     const RowsSplit rows = split_rows(kind, M, p.k_blocks, e, N, sm_count);
     if (rows.chunks > 1) {
-      p.block_n = rows.block_n;
       p.chunk_blocks = rows.chunk_blocks;
       p.chunks = rows.chunks;
-      p.split_k = 1;
+      if (split_k_enabled()) {
+        p.block_n = rows.block_n;
+        p.split_k = 1;
+      }
     }
   }
   p.sk_ws = e.sk_ws;

@@ -360,6 +360,24 @@ def test_inner_product_sums_alike_whatever_the_rows_of_a_tile(pkg, tmp_path, k, 
             assert np.array_equal(model.run(x[:m])[0], want[:m]), m
 
 
+@pytest.mark.parametrize("m,k,n", [
+    (1, 2048, 1000),
+    (33, 2048, 1000),
+    (128, 3000, 40),   # a last K block and a last chunk that are not full, one narrow tile column
+    (129, 3000, 700),  # a second tile of one row
+    (300, 2048, 512),
+    (300, 2816, 2816),
+    (100, 3600, 48),
+])
+def test_chunks_in_one_cta_change_no_bit_of_an_inner_product(pkg, tmp_path, monkeypatch, m, k, n):
+    """NCNN_B200_SPLIT_K=0 puts the chunks of a tile one after the other; the sums stay what they are."""
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n)
+    x = np.random.default_rng(28).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    want = pkg.Model(param, bin_).run(x)[0]
+    monkeypatch.setenv("NCNN_B200_SPLIT_K", "0")
+    assert np.array_equal(pkg.Model(param, bin_).run(x)[0], want)
+
+
 def _int8_pair(zoo, prefix, cin, mid, cout, k, h, w, act):
     """Two int8 Convolutions in a row: the first writes int8 (term 101), the second fp32."""
     net = zoo._Net(41, int8=True)
