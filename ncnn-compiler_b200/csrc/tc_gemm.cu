@@ -242,10 +242,14 @@ int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, 
 //            2048 -> 1024          3000 -> 700           2816 -> 2816           4096 -> 4096
 //   fp32     64 rows 24.7 -> 16.4  64 rows 34.6 -> 14.4  64 rows 30.8 -> 20.5   64 rows 32.8 -> 28.7
 //            128     34.2 -> 14.4  128     48.4 -> 16.5  128     39.7 -> 22.7   128     39.4 -> 33.9
-//            300     33.7 -> 20.5  300     40.9 -> 22.7  300     30.9 -> 32.8   300     46.9 -> 45.6
 //            1000    26.7 -> 30.8  1000    36.8 -> 34.9  1000    49.3 -> 54.2   1000    87.4 -> 84.3
 //   int8     128     11.0 -> 12.8  300     12.9 -> 18.5  64      12.3 -> 14.5   64      23.4 -> 19.1, 128 30.7 -> 18.5
-// so it takes up to three tiles of rows; int8, whose blocks are short, from 28 blocks on and up to two.
+// and of more than one tile of rows, whole tiles against the layer's chunks (their number behind the layer; ! is not taken):
+//            2048 -> 1024 (4)      3000 -> 700 (6)       2816 -> 2816 (4)       4096 -> 1000 (8)       2048 -> 2048 (4)
+//   fp32     200 rows 22.6 / 18.8  200 rows 28.8 / 22.3  200 rows 28.6 / 28.9!  200 rows 36.2 / 32.7   200 rows 22.0 / 26.8!
+//            384      22.7 / 23.8! 384      29.0 / 28.8! 384      30.9 / 45.9!  384      37.0 / 48.6!  384      22.7 / 35.6!
+// so it takes up to three tiles of rows, where the clocks below say so (of three, 4096 -> 512 37.1 -> 31.2); int8, whose blocks are short, from 28 blocks on and up
+// to two.
 struct RowsSplit {
   int block_n = 0, chunk_blocks = 0, chunks = 1;
   double clocks = 1e300;
@@ -265,8 +269,11 @@ RowsSplit best_rows_split(int kind, long long M, int k_blocks, const TcEpilogue&
       if ((k_blocks + blocks - 1) / blocks != chunks) continue;
       const long long units = tiles * chunks;
       if (chunks > 1 && (tiles * 8 > e.sk_flag_count || static_cast<size_t>(units) * kTcBlockM * bn * 4 > e.sk_ws_bytes)) continue;
-      // (a warp adds four chunks of 16 columns in ~700 clocks)
-      const double sums = 2500.0 + 700.0 * ((chunks + 3) / 4) * ((bn + 31) / 32) + static_cast<double>(tiles) * std::min<long long>(M, kTcBlockM) * chunks * bn / 500.0;
+      // (a warp adds four chunks of 16 columns in ~700 clocks.  Two and three tiles of rows, fp32: fitted to 65 of the calls
+      // above; the sums of that many tiles get in one another's way)
+      const double sums = i8 || tiles_m == 1
+                              ? 2500.0 + 700.0 * ((chunks + 3) / 4) * ((bn + 31) / 32) + static_cast<double>(tiles) * std::min<long long>(M, kTcBlockM) * chunks * bn / 500.0
+                              : 44.0 * chunks * bn + static_cast<double>(M) * N * chunks / 130.0 - 5300.0;
       const double clocks = static_cast<double>((units + sm_count - 1) / sm_count) * blocks * block + 3000.0 + 12.0 * bn + (chunks > 1 ? sums : 0.0);
       if (clocks >= best.clocks) continue;
       best.clocks = clocks;
@@ -287,6 +294,10 @@ RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, i
   if (M <= kTcBlockM) {
     if (rows.chunks != layer.chunks) rows = layer;
     rows.clocks = layer.clocks;  // (what other forms are compared with: the same for all calls of one tile)
+  } else if (M > 2 * kTcBlockM && rows.chunks > 1) {
+    // (up to a tenth of the clocks' gain did not come: 2048 -> 1024, 300 rows 25.2 in chunks, 22.7 whole)
+    const RowsSplit whole = best_rows_split(kind, M, k_blocks, e, N, sm_count, 1);
+    if (rows.clocks > 0.8 * whole.clocks) rows = whole;
   }
   return rows;
 }
@@ -503,9 +514,11 @@ bool finish_plan_workers(TcLaunch* L, int kind, long long M, int N, const TcEpil
     const double cost_whole = static_cast<double>((one_tiles + sm_count - 1) / sm_count) * full_kb;
     const double cost_split = static_cast<double>((one_units + one_workers - 1) / one_workers) + 20.0;
     split_form = forced_split == 1 || cost_split < 0.9 * cost_whole;
-    // (chunks of K on different CTAs do the same without workers that wait, and win where rows are few)
+    // (chunks of K on different CTAs do the same without workers that wait, and win where rows are few.  A tile of many
+    // workers waits for each of them: 4096 -> 512, 200 rows, 18 to a tile 55 us, whole 41; 4096 -> 4096, 2 to a tile 39.5 and 40.9)
     const double block = std::max(tc_planes(kind) * 3.0 * (kTcBlockM + one_bn), (kind == GEMM_I8 ? 4.0 : 12.0) * (kTcBlockM + one_bn) / 4.0);
-    if (forced_split != 1 && split_rows(kind, M, full_kb, e, N, sm_count).clocks < cost_split * block + 3000.0) split_form = false;
+    const double waits = kind == GEMM_BF16X3 ? 4000.0 * std::max(0.0, static_cast<double>(one_workers) / one_tiles - 2.5) : 0.0;
+    if (forced_split != 1 && split_rows(kind, M, full_kb, e, N, sm_count).clocks < cost_split * block + 3000.0 + waits) split_form = false;
   }
   if (!pair_form && !split_form) return false;
   const int ctas = pair_form ? 2 : 1;

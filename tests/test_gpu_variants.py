@@ -378,6 +378,19 @@ def test_chunks_in_one_cta_change_no_bit_of_an_inner_product(pkg, tmp_path, monk
     assert np.array_equal(pkg.Model(param, bin_).run(x)[0], want)
 
 
+@pytest.mark.parametrize("m,k,n,other", [
+    (200, 3000, 700, 128),   # in chunks: those of calls of up to 128 rows
+    (300, 2816, 2816, 600),  # more than 128 rows of a wide layer: whole, like a call of many rows
+    (129, 2048, 2048, 600),
+])
+def test_inner_product_of_two_and_three_tiles_of_rows(pkg, tmp_path, m, k, n, other):
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n)
+    x = np.random.default_rng(29).uniform(-1, 1, (max(m, other), 1, 1, k)).astype(np.float32)
+    model = pkg.Model(param, bin_)
+    least = min(m, other)
+    assert np.array_equal(model.run(x[:m])[0][:least], model.run(x[:other])[0][:least])
+
+
 def _int8_pair(zoo, prefix, cin, mid, cout, k, h, w, act):
     """Two int8 Convolutions in a row: the first writes int8 (term 101), the second fp32."""
     net = zoo._Net(41, int8=True)
