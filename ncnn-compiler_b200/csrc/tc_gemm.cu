@@ -1238,15 +1238,19 @@ std::string tc_plan_conv_i8(TcConvI8Launch* L, const TcIm2colView& v, const void
   // second figure of a pair is a layer that adds an fp32 residual and writes fp32 and an int8 copy:
   //   64 channels, 56x56           1 image 10.4, 12.6 -> 10.6, 13.3   4: 11.8, 14.1 -> 10.3, 13.7   64: 37, 51 -> 21, 41   256: 120, 160 -> 53, 116
   //       33x33 (57 % of the tiles filled), 256 images 47, 69 -> 33, 64;  16x16, 16 images (one wave) 12.0, 12.6 -> 10.4, 13.5
-  //   128, 28x28 (77 %)            4: 11.2 -> 12.7   16: 14.4, 16.3 -> 13.5, 14.5   64: 20.5, 22.5 -> 18.5, 22.5   256: 43, 48 -> 39, 51
+  //   128, 28x28 (77 %)            4: 11.2 -> 12.7   16: 14.4, 16.3 -> 13.5, 14.5   64: 20.5, 30.8 -> 18.5, 29.8   96: 22.6, 39.4 -> 22.4, 40.1
+  //       256: 43, 86 -> 38, 88;  fp32 results without a residual  64: 22.5 -> 22.2   96: 24.5 -> 26.7   192: 38 -> 43   256: 47 -> 51
   //       17x17 (38 %), 256 images 22.5, 24.7 -> 31, 41
   //   256 (four column blocks), 14x14   4: 12.6, 15.2 -> 12.0, 14.3   16 (one wave): 14.4, 16.8 -> 12.5, 16.3   256: 38, 59 -> 43, 80
   //   512 (16), 7x7                1: 16.4 -> 12.5   4 (one wave): 16.4 -> 12.7   16: 16.6 -> 18.4
   // With one tile to a CTA nothing is reused, and what is left is a shorter chain: from 18 K blocks on.  With several the filter's
-  // reuse wins, unless tiles are mostly empty or the pixels are read again for each of many column blocks.
+  // reuse wins, unless tiles are mostly empty or the pixels are read again for each of many column blocks.  Beside a filter of
+  // 128-byte rows fp32 results have room for two epilogue groups, or for three and half of the columns, and the drain falls
+  // behind: up to four tiles an SM (128 images, residual: 52.6 and 49.3, where the other kernel's last wave is short).
   const long long waves = (tiles + sm_count / p.tiles_n - 1) / (sm_count / p.tiles_n);
   const double filled = static_cast<double>(v.OH) * v.OW / (static_cast<double>(p.tiles_y) * p.tiles_x * kI8TileH * kI8TileW);
-  const bool pays = waves == 1 ? blocks >= 18 : p.tiles_n <= 2 && filled >= (rb == 64 ? 0.5 : 0.7);
+  const bool slow_drain = rb == 128 && e.out_mode == OUT_F32 && tiles > 4ll * sm_count;
+  const bool pays = waves == 1 ? blocks >= 18 : p.tiles_n <= 2 && !slow_drain && filled >= (rb == 64 ? 0.5 : 0.7);
   if (!always && !pays) return "other kernels are expected to be as fast";
   p.bias = e.bias;
   p.scale = e.scale;

@@ -446,6 +446,16 @@ def test_int8_network_with_resident_filters(pkg, oracle, tmp_path, monkeypatch, 
     assert np.array_equal(got["1"][:1], oracle_rows(oracle, param, bin_, x[:1]))
 
 
+@pytest.mark.parametrize("n,pays", [(74, True), (75, False)])
+def test_int8_filters_of_128_channels_stay_resident_for_few_fp32_tiles(pkg, tmp_path, n, pays):
+    """fp32 results, with a residual or not: up to four tiles of 16 x 8 pixels an SM; int8 results on either side."""
+    param, bin_ = pkg.zoo.resnet18(str(tmp_path / "r8"), int8=True, classes=8)
+    kernels = {r["layer"]: r["kernel"] for r in pkg.Model(param, bin_).profile(n, repeat=1)}
+    for layer in ("l2b0_conv2", "l2b1_conv2"):
+        assert ("tc_conv_i8_kernel" in kernels[layer]) == pays
+    assert "tc_conv_i8_kernel" in kernels["l2b1_conv1"] and "tc_conv_i8_kernel" in kernels["l1b1_conv2"]
+
+
 @pytest.mark.parametrize("m,k,n", [
     (1, 7, 5),       # one short chunk, most lanes without a column
     (3, 1001, 33),   # an odd K: its last pair is half there; one column past a block
