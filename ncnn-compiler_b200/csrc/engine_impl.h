@@ -380,27 +380,19 @@ inline bool stem_rows_enabled() {
   return f == nullptr || f[0] != '0';
 }
 
-// Where the patch-resident convolution kernel takes a layer (tc_conv_halo.cuh): -1, the default, by measurement (see
-// halo_pays); NCNN_B200_HALO at load time: 0 nowhere, 1 wherever it applies, 2 the same on pairs of CTAs.
-// NCNN_B200_PATCH: 0 never runs a convolution on tc_conv_patch_kernel, 1 wherever it applies
-inline int patch_level() {
-  const char* f = std::getenv("NCNN_B200_PATCH");
-  return f == nullptr ? -1 : std::atoi(f);
-}
-// NCNN_B200_CONV_I8: the same for tc_conv_i8_kernel
-inline int conv_i8_level() {
-  const char* f = std::getenv("NCNN_B200_CONV_I8");
-  return f == nullptr || f[0] == 0 ? -1 : std::atoi(f);
-}
-inline int halo_level() {
-  const char* f = std::getenv("NCNN_B200_HALO");
-  return f == nullptr || f[0] == 0 ? -1 : std::atoi(f);
-}
-
+// A whole number from the environment; a name that is not set, or set to nothing, is the fallback.
 inline int env_int_or(const char* name, int fallback) {
   const char* f = std::getenv(name);
   return f == nullptr || f[0] == 0 ? fallback : std::atoi(f);
 }
+
+// Where the patch-resident convolution kernel takes a layer (tc_conv_halo.cuh): -1, the default, by measurement (see
+// halo_pays); NCNN_B200_HALO at load time: 0 nowhere, 1 wherever it applies, 2 the same on pairs of CTAs.
+inline int halo_level() { return env_int_or("NCNN_B200_HALO", -1); }
+// tc_conv_patch_kernel: -1, the default, by measurement; NCNN_B200_PATCH: 0 nowhere, 1 wherever it applies.
+inline int patch_level() { return env_int_or("NCNN_B200_PATCH", -1); }
+// tc_conv_i8_kernel: the same with NCNN_B200_CONV_I8.
+inline int conv_i8_level() { return env_int_or("NCNN_B200_CONV_I8", -1); }
 
 // NAME=0 in the environment switches an optional pass off
 inline bool env_flag_off(const char* name) {

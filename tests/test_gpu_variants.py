@@ -307,6 +307,24 @@ def test_patch_kernel_waits_that_run_out(pkg, tmp_path, monkeypatch):
     m.check_status()
 
 
+@pytest.mark.parametrize("switch,net,n", [
+    ("NCNN_B200_PATCH", "conv128", 1),
+    ("NCNN_B200_HALO", "conv64", 22),
+    ("NCNN_B200_CONV_I8", "resnet18", 16),
+])
+def test_an_empty_switch_is_no_switch(pkg, tmp_path, monkeypatch, switch, net, n):
+    path = str(tmp_path / net)
+    files = (pkg.zoo.single_conv(path, h=20, w=20, cin=128) if net == "conv128" else
+             pkg.zoo.residual_block(path, h=56, w=56, c=64, cout=64) if net == "conv64" else
+             pkg.zoo.resnet18(path, int8=True, classes=8))
+    used = []
+    for value in (None, "", "0"):
+        if value is not None:
+            monkeypatch.setenv(switch, value)
+        used.append([r["kernel"] for r in pkg.Model(*files).profile(n, repeat=1)])
+    assert used[1] == used[0] and used[2] != used[0]
+
+
 @pytest.mark.parametrize("m,k,n,int8", [
     (9, 1472, 24, False),    # 23 K blocks: whole
     (9, 1728, 24, False),    # 27: the shallowest in chunks, one narrow tile column
