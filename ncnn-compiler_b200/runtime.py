@@ -121,10 +121,14 @@ _PACK_ONE = struct.Struct("P").pack
 
 def _pointers(values):
     """The addresses as one table in memory, for calls that only read it: a call of one input and one output spends 0.9 us
-    in ctypes this way and 2.1 with arrays of c_void_p, of ~8.5 that a small call takes on the host."""
-    if len(values) == 1:
-        return _PACK_ONE(values[0] or 0)
-    return struct.pack("%dP" % len(values), *[v or 0 for v in values])
+    in ctypes this way and 2.1 with arrays of c_void_p, of ~8.5 that a small call takes on the host.  What is no whole
+    number (a c_void_p, say) goes into such an array, which also says what it does not take."""
+    try:
+        if len(values) == 1:
+            return _PACK_ONE(0 if values[0] is None else values[0])
+        return struct.pack("%dP" % len(values), *[0 if v is None else v for v in values])
+    except struct.error:
+        return _ptr_array(values)
 
 
 class Model:

@@ -44,6 +44,22 @@ def test_null_arguments_are_rejected_without_a_gpu(pkg):
 
 
 @pytest.mark.skipif(os.path.exists("/dev/nvidia0"), reason="checks the behaviour of a box without a GPU")
+@pytest.mark.parametrize("values,addresses", [
+    ([64], [64]), ([None], [0]), ([64, None, np.int64(128)], [64, 0, 128]),
+    ([ctypes.c_void_p(64)], [64]), ([ctypes.c_void_p(None), 128, None, ctypes.c_void_p(1 << 47)], [0, 128, 0, 1 << 47]),
+])
+def test_pointer_tables_take_what_a_pointer_argument_takes(pkg, values, addresses):
+    table = pkg.runtime._pointers(values)
+    assert ctypes.c_void_p.from_param(table) is not None
+    assert list((ctypes.c_uint64 * len(values)).from_buffer_copy(table)) == addresses
+
+
+def test_pointer_tables_refuse_what_is_no_address(pkg):
+    for values in (["x"], [""], [1.5, 64], [0.0, 64]):
+        with pytest.raises(TypeError):
+            pkg.runtime._pointers(values)
+
+
 def test_load_fails_loudly_without_a_gpu(pkg):
     param, bin_ = fixture("convolution")
     with pytest.raises(pkg.NcnnB200Error) as e:
