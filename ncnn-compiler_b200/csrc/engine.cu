@@ -433,8 +433,8 @@ int EngineImpl::run(int64_t n, const float* const* in, float* const* out, bool h
   }
   Plan* plan = plan_for(n);
   if (plan == nullptr) return 6;
-  // Host tests of the time-out path: NCNN_B200_TEST_STALL makes the one-CTA contraction kernel leave one stage
-  // unfilled, so its bounded waits run out (nothing faults or hangs; the run returns status 7).
+  // Host tests of the time-out path: NCNN_B200_TEST_STALL makes tc_gemm_kernel leave one stage unfilled, tc_conv_patch_kernel
+  // and tc_conv_i8_kernel one patch, so their bounded waits run out (nothing faults or hangs; the run returns status 7).
   const bool stall = std::getenv("NCNN_B200_TEST_STALL") != nullptr;
   if (stall != stall_injected_) {
     // (the kernels read the word before they wait for the launch before them)

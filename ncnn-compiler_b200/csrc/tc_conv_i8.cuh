@@ -105,6 +105,9 @@ tc_conv_i8_kernel(const __grid_constant__ TcConvI8Params p, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  // (host tests of the time-out path: see tc_gemm.cuh)
+  const int test_stall = p.status[1];
+  const uint64_t wait_limit = test_stall ? 2000000ull : kTcWaitLimitNs;
   if (warp != 0) grid_dependency_wait();
 
   auto decode = [&](int t, int* img, int* oy0, int* ox0) {
@@ -134,13 +137,15 @@ tc_conv_i8_kernel(const __grid_constant__ TcConvI8Params p, const __grid_constan
         int img, oy0, ox0;
         decode(tile, &img, &oy0, &ox0);
         for (int cb = 0; cb < p.c_blocks; ++cb) {
-          if (!mbar_wait_bounded(smem_u32(&a_empty[ab]), ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+          if (!mbar_wait_bounded(smem_u32(&a_empty[ab]), ph ^ 1u, abort_ptr, wait_limit)) {
             ok = false;
             break;
           }
-          const uint32_t fb = smem_u32(&a_full[ab]);
-          mbar_arrive_expect_tx(fb, tx);
-          tma_load_4d(ring + static_cast<uint32_t>(ab) * patch_bytes, &map_a, fb, cb * p.k_elems, ox0 - p.pad_l, oy0 - p.pad_t, img);
+          if (!test_stall || issued > 0) {  // (a test's first patch is never armed: the waits for it run out)
+            const uint32_t fb = smem_u32(&a_full[ab]);
+            mbar_arrive_expect_tx(fb, tx);
+            tma_load_4d(ring + static_cast<uint32_t>(ab) * patch_bytes, &map_a, fb, cb * p.k_elems, ox0 - p.pad_l, oy0 - p.pad_t, img);
+          }
           ++issued;
           if (++ab == p.patches) {
             ab = 0;
@@ -154,7 +159,7 @@ tc_conv_i8_kernel(const __grid_constant__ TcConvI8Params p, const __grid_constan
         int zero = 0;
         mbar_wait_bounded(wb, 0u, &zero, 200000000ull);
         for (long long i = issued > p.patches ? issued - p.patches : 0; i < issued; ++i)
-          mbar_wait_bounded(smem_u32(&a_full[i % p.patches]), static_cast<uint32_t>((i / p.patches) & 1), &zero, 200000000ull);
+          mbar_wait_bounded(smem_u32(&a_full[i % p.patches]), static_cast<uint32_t>((i / p.patches) & 1), &zero, test_stall ? 2000000ull : 200000000ull);
       }
     }
   } else if (warp == 1) {
@@ -172,10 +177,10 @@ tc_conv_i8_kernel(const __grid_constant__ TcConvI8Params p, const __grid_constan
       int ab = 0, acc = 0;
       uint32_t a_ph = 0, acc_ph = 0;
       // the next patch is here / the next accumulator is free (asked before a commit: see tc_gemm_common.cuh)
-      bool ok = mbar_wait_bounded(smem_u32(&b_full), 0u, abort_ptr, kTcWaitLimitNs), a_seen = false, empty_seen = false;
+      bool ok = mbar_wait_bounded(smem_u32(&b_full), 0u, abort_ptr, wait_limit), a_seen = false, empty_seen = false;
       auto run = [&](auto steps, auto three) {
         for (int tile = first; tile < tiles && ok; tile += step) {
-          if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
+          if (!empty_seen && !mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, wait_limit)) {
             ok = false;
             break;
           }
@@ -185,7 +190,7 @@ tc_conv_i8_kernel(const __grid_constant__ TcConvI8Params p, const __grid_constan
           uint32_t accumulate = 0u;
           uint64_t b = b_first;
           for (int cb = 0; cb < c_blocks; ++cb) {
-            if (!a_seen && !mbar_wait_bounded(smem_u32(&a_full[ab]), a_ph, abort_ptr, kTcWaitLimitNs)) {
+            if (!a_seen && !mbar_wait_bounded(smem_u32(&a_full[ab]), a_ph, abort_ptr, wait_limit)) {
               ok = false;
               break;
             }
@@ -290,7 +295,7 @@ tc_conv_i8_kernel(const __grid_constant__ TcConvI8Params p, const __grid_constan
           for (int b = 0; b < 4 * min(lp.block_n, left); b += 128) prefetch_l2(r + b);
       }
       // the vote keeps the warp together: tcgen05.ld needs all 32 lanes
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&tfull_bar[acc]), acc_ph, abort_ptr, wait_limit) ? 1 : 0) != 0;
       if (!ok) break;
       tc_fence_after_sync();
       tc_drain<GEMM_I8, EPI, SIDE, false>(d, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * lp.acc_cols),

@@ -464,6 +464,31 @@ def test_int8_network_with_resident_filters(pkg, oracle, tmp_path, monkeypatch, 
     assert np.array_equal(got["1"][:1], oracle_rows(oracle, param, bin_, x[:1]))
 
 
+@pytest.mark.parametrize("cin,n", [
+    (256, 2),   # two channel blocks, one tile to a CTA
+    (64, 21),   # more tiles than CTAs
+])
+def test_int8_resident_filters_waits_that_run_out(pkg, tmp_path, monkeypatch, cin, n):
+    """A first patch that never comes, in the one tensor-core kernel of the net: the waits give up, the call answers 7, the
+    handle recovers."""
+    net = pkg.zoo._Net(44, int8=True)
+    net.w.layer("Input", "input", [], ["data"], f"0=28 1=28 2={cin}")
+    net.conv("a", "data", "x", cin, 64, 3, 1, 1, act=1, zero_bias=False, term=1)
+    net.w.layer("Pooling", "gap", ["x"], ["output"], "0=1 4=1")
+    monkeypatch.setenv("NCNN_B200_CONV_I8", "1")
+    m = pkg.Model(*net.w.save(str(tmp_path / "c")))
+    x = np.random.default_rng(45).uniform(-1, 1, (n, cin, 28, 28)).astype(np.float32)
+    assert [r["kernel"] for r in m.profile(n, repeat=1) if r["kernel"].startswith("tc_")] == ["tc_conv_i8_kernel<i8>"]
+    good = m.run(x)[0].copy()
+    monkeypatch.setenv("NCNN_B200_TEST_STALL", "1")
+    with pytest.raises(pkg.NcnnB200Error) as err:
+        m.run(x)
+    assert err.value.status == 7
+    monkeypatch.delenv("NCNN_B200_TEST_STALL")
+    assert np.array_equal(m.run(x)[0], good)
+    m.check_status()
+
+
 @pytest.mark.parametrize("n,pays", [(74, True), (75, False)])
 def test_int8_filters_of_128_channels_stay_resident_for_few_fp32_tiles(pkg, tmp_path, n, pays):
     """fp32 results, with a residual or not: up to four tiles of 16 x 8 pixels an SM; int8 results on either side."""
