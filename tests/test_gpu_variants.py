@@ -522,3 +522,78 @@ def test_fp32_inner_product_of_few_rows(pkg, oracle, tmp_path, monkeypatch, m, k
     assert np.array_equal(tiles.run(x)[0], got)
     assert not any(r["kernel"] == "k_rows_f32" for r in tiles.profile(m, repeat=1))
     assert rel_l2(got, oracle_rows(oracle, param, bin_, x)) <= 2e-6
+
+
+def _one_launch(pkg, tmp_path, int8):
+    """An InnerProduct whose call is one launch of the rows kernel, which goes to the caller's stream without a graph."""
+    model = pkg.Model(*pkg.zoo.inner_product(str(tmp_path / "ip"), 4096, 2048, int8=int8))
+    x = np.random.default_rng(51).uniform(-1, 1, (7, 1, 1, 4096)).astype(np.float32)
+    want = np.stack([model.run(xi[None])[0].reshape(-1) for xi in x])
+    assert model.launch_count(1) == 1
+    return model, x.reshape(7, 4096), want
+
+
+@pytest.mark.parametrize("int8", [False, True])
+def test_one_launch_follows_what_precedes_it_on_the_stream(pkg, tmp_path, int8):
+    """The input is written just before the call and again just after it; the result is read just after it."""
+    import torch
+    model, x, want = _one_launch(pkg, tmp_path, int8)
+    source, busy, stream = torch.from_numpy(x).cuda(), torch.rand(1 << 25, device="cuda"), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        row, y, got = torch.zeros(4096, device="cuda"), torch.zeros(2048, device="cuda"), []
+        for _ in range(5):
+            for i in range(len(x)):
+                busy.mul_(1.0)
+                row.copy_(source[i])
+                model.run_device(1, [row.data_ptr()], [y.data_ptr()], stream.cuda_stream)
+                row.fill_(9.0)
+                got.append(y.clone())
+                y.fill_(5.0)
+    stream.synchronize()
+    assert np.array_equal(torch.stack(got).cpu().numpy(), np.concatenate([want] * 5))
+
+
+@pytest.mark.parametrize("int8", [False, True])
+def test_one_launch_with_arrays_in_turn(pkg, tmp_path, int8):
+    """Back to back, each call's input the array that the call before wrote into; more sets of arrays than a plan remembers."""
+    import torch
+    model, x, want = _one_launch(pkg, tmp_path, int8)
+    stream = torch.cuda.current_stream().cuda_stream
+    xs, ys = torch.from_numpy(x).cuda(), torch.zeros(len(x), 2048, device="cuda")
+    for order in (range(7), (0, 1) * 8, (6, 0, 5, 1, 4, 2, 3), range(7)):
+        ys.zero_()
+        for i in order:
+            model.run_device(1, [xs[i].data_ptr()], [ys[i].data_ptr()], stream)
+        used = sorted(set(order))
+        assert np.array_equal(ys.cpu().numpy()[used], want[used])
+    square = pkg.Model(*pkg.zoo.inner_product(str(tmp_path / "sq"), 4096, 4096, int8=int8))
+    first = square.run(x[0].reshape(1, 1, 4096))[0].reshape(-1)
+    second = square.run(first.reshape(1, 1, 4096))[0].reshape(-1)
+    a, b, c = xs[0].clone(), torch.zeros(4096, device="cuda"), torch.zeros(4096, device="cuda")
+    for _ in range(20):
+        square.run_device(1, [a.data_ptr()], [b.data_ptr()], stream)
+        square.run_device(1, [b.data_ptr()], [c.data_ptr()], stream)
+    assert np.array_equal(b.cpu().numpy(), first) and np.array_equal(c.cpu().numpy(), second)
+
+
+@pytest.mark.parametrize("int8", [False, True])
+def test_one_launch_under_the_callers_capture(pkg, tmp_path, int8):
+    """Captured between two kernels of the caller's; new values in the arrays for every replay, also after the pass was dropped."""
+    import torch
+    model, x, want = _one_launch(pkg, tmp_path, int8)
+    source = torch.from_numpy(x).cuda()
+    half, row, y, z = (torch.zeros(n, device="cuda") for n in (4096, 4096, 2048, 2048))
+    model.run_device(1, [row.data_ptr()], [y.data_ptr()], torch.cuda.current_stream().cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        torch.mul(half, 2.0, out=row)
+        model.run_device(1, [row.data_ptr()], [y.data_ptr()], torch.cuda.current_stream().cuda_stream)
+        z.copy_(y)
+    for i in range(len(x)):
+        torch.mul(source[i], 0.5, out=half)  # (exact)
+        graph.replay()
+        assert np.array_equal(z.cpu().numpy(), want[i])
+        other = torch.zeros(2048, device="cuda")
+        model.run_device(1, [source[i].data_ptr()], [other.data_ptr()], torch.cuda.current_stream().cuda_stream)
+        assert np.array_equal(other.cpu().numpy(), want[i])
