@@ -353,10 +353,15 @@ static __global__ void __launch_bounds__(BM, 256 / BM) k_conv_f32(const float* _
 //   32       22.6 -> 16.7    49.3 -> 20.6    69.7 -> 49.8   126.9 -> 90.1    55.4 -> 22.6    45.3 -> 16.5
 //   48       22.6 -> 18.5    53.2 -> 22.6    73.8 -> 65.6   131.1 -> 127.3   57.5 -> 32.9    49.3 -> 16.5
 //   64       22.6 -> 18.5    55.4 -> 32.5    76.1 -> 82.4   134.6 -> 163.8   61.4 -> 34.5    51.3 -> 16.5
-// So up to three groups of 16 rows, and up to kRowsF32Most where seven warps an SM (which holds four at a time) do it
-// (96 rows: 513 -> 600 30.8 -> 16.5, 700 -> 2001, 7.7 warps an SM, 37.0 -> 38.5): from there on the weights' repeated way out of L2
-// costs more than the tiles' empty rows.  7 -> 5: 8 rows 8.3 -> 6.2, 16 rows 8.4 -> 10.3: short
-// rows take it up to eight.
+// One group of 16 rows always takes it.  More groups bring every weight out of L2 again, and the tiles are slower where their
+// operands come element by element (K, or the columns, no multiple of 4); so from 17 rows to kRowsF32Most the two are compared
+// by an estimate fitted to 299 calls (K 130 to 4095, 33 to 12000 columns, 17 to 128 rows), of which it picks the slower form in
+// 17, by 4 to 18 %:
+//            300 -> 12000    513 -> 7000     700 -> 7000     1001 -> 2501    1001 -> 12000   4095 -> 2501
+//   17       25.0 / 35.5!    39.3 -> 33.0    33.1 / 39.3!    47.6 -> 27.0    80.3 -> 69.4   102.8 -> 60.3    (! tiles stay)
+//   48       24.9 / 51.7!    40.2 / 47.6!    33.2 / 57.7!    53.6 -> 33.0    82.4 / 102.8!  108.9 -> 85.0
+//   96                       61.8 / 83.3!                    70.0 -> 53.7                   162.2 / 153.2!
+// 7 -> 5: 8 rows 8.3 -> 6.2, 16 rows 8.4 -> 10.3: short rows take it up to eight.
 // What bounds it: one row, the weights' way from HBM (4095 -> 4091: 67 MB at 3.4 TB/s, launch included); many rows, the 48 KB
 // of a warp, of which an SM holds four, and the broadcasts (one 16-byte read for two packed FMAs).
 constexpr int kRowsF32Cols = 32;

@@ -61,7 +61,12 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
   const int cols = (g.O + kRowsF32Cols - 1) / kRowsF32Cols;
   const long long groups = (rows + kRowsF32Max - 1) / kRowsF32Max, warps = cols * groups * p.chunks;
   const bool flat = g.H == 1 && g.W == 1 && g.OH == 1 && g.OW == 1 && g.KH == 1 && g.KW == 1;
-  const bool few = p.K >= 128 ? groups <= 3 || (rows <= kRowsF32Most && warps <= 7ll * sm_count_) : rows <= 8;
+  // expected us (conv_f32.cuh): waves of warps or of 64-row tiles, each in chunks of up to 256 k
+  const double places = 4.0 * sm_count_, chunk = p.chunk_k / 256.0;
+  const double rows_us = chunk * (13.0 * static_cast<double>(warps) / places + 3.0) + 0.35 * static_cast<double>(groups);
+  const double tile_waves = static_cast<double>(tiles) * (p.split ? p.chunks : 1) / places;
+  const double tiles_us = chunk * (p.split ? 1 : p.chunks) * ((p.vec_a ? 12.0 : 28.0) * std::ceil(tile_waves) + 20.0 * tile_waves) + (p.vec_o ? 0.0 : 10.0);
+  const bool few = p.K >= 128 ? groups == 1 || (rows <= kRowsF32Most && rows_us < tiles_us) : rows <= 8;
   if (flat && few && p.chunks < 65536 && !env_flag_off("NCNN_B200_ROWS_F32") &&
       (p.chunks == 1 || (cols * groups <= kTcSplitFlagCount && static_cast<size_t>(warps) * kRowsF32Max * kRowsF32Cols * 4 <= kTcSplitWorkspaceBytes))) {
     const dim3 rgrid(static_cast<unsigned>(cols), static_cast<unsigned>(p.chunks), static_cast<unsigned>(groups));

@@ -524,6 +524,19 @@ def test_fp32_inner_product_of_few_rows(pkg, oracle, tmp_path, monkeypatch, m, k
     assert rel_l2(got, oracle_rows(oracle, param, bin_, x)) <= 2e-6
 
 
+@pytest.mark.parametrize("m,k,n,takes", [
+    (16, 300, 12000, True),    # one group of rows, always
+    (17, 300, 12000, False),   # more: many columns of short chunks that come in whole pieces
+    (48, 513, 7000, False),
+    (48, 1001, 2501, True),    # operands of the tiles come element by element
+    (128, 1001, 600, True),
+    (129, 1001, 600, False),
+])
+def test_which_fp32_inner_products_are_a_pass_over_the_weights(pkg, tmp_path, m, k, n, takes):
+    model = pkg.Model(*pkg.zoo.inner_product(str(tmp_path / "ip"), k, n), accuracy_mode=pkg.FP32_CUDA)
+    assert any(r["kernel"] == "k_rows_f32" for r in model.profile(m, repeat=1)) == takes
+
+
 def _one_launch(pkg, tmp_path, int8):
     """An InnerProduct whose call is one launch of the rows kernel, which goes to the caller's stream without a graph."""
     model = pkg.Model(*pkg.zoo.inner_product(str(tmp_path / "ip"), 4096, 2048, int8=int8))
