@@ -362,6 +362,9 @@ static __global__ void __launch_bounds__(BM, 256 / BM) k_conv_f32(const float* _
 //   48       24.9 / 51.7!    40.2 / 47.6!    33.2 / 57.7!    53.6 -> 33.0    82.4 / 102.8!  108.9 -> 85.0
 //   96                       61.8 / 83.3!                    70.0 -> 53.7                   162.2 / 153.2!
 // 7 -> 5: 8 rows 8.3 -> 6.2, 16 rows 8.4 -> 10.3: short rows take it up to eight.
+// The chunks of all 32-column blocks meet in the workspace of split contractions (21 MB, 16384 counters): with 4096 inputs that is
+// one row through 327680 columns, 8 through 40960, 16 through 20480; wider calls stay on tiles.  Beyond the 640 counters that
+// other kernels share: 513 -> 20512, one row 71.9 -> 14.5, 16 rows 73.9 -> 49.3; 4096 -> 32000, one row 445 -> 139, 8 rows 445 -> 199.
 // What bounds it: one row, the weights' way from HBM (4095 -> 4091: 67 MB at 3.4 TB/s, launch included); many rows, the 48 KB
 // of a warp, of which an SM holds four, and the broadcasts (one 16-byte read for two packed FMAs).
 constexpr int kRowsF32Cols = 32;

@@ -53,8 +53,9 @@ bool EngineImpl::build(const std::string& param, const std::string& bin, const E
   // workspace of the contraction kernel that splits tiles between CTA pairs: partial accumulators
   // and one flag word per CTA (zero between launches); all launches of a model run on one stream
   void* ws = nullptr;
-  if (device_alloc(&ws, kTcSplitWorkspaceBytes + 4096) != cudaSuccess) return fail(err, "out of device memory");
-  cudaMemset(ws, 0, kTcSplitWorkspaceBytes + 4096);
+  constexpr size_t ws_bytes = kTcSplitWorkspaceBytes + kTcFlagWords * sizeof(int);
+  if (device_alloc(&ws, ws_bytes) != cudaSuccess) return fail(err, "out of device memory");
+  cudaMemset(ws, 0, ws_bytes);
   device_allocs_.push_back(ws);
   d_split_ws_ = static_cast<uint32_t*>(ws);
   d_split_flags_ = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + kTcSplitWorkspaceBytes);
@@ -302,7 +303,7 @@ int EngineImpl::finish_host_run(Plan* plan, float* const* out, cudaStream_t st) 
   if (status != 0) {
     error_ = "a tensor-core pipeline wait timed out (status " + std::to_string(status) + ")";
     cudaMemset(d_status_, 0, 4);
-    cudaMemset(d_split_flags_, 0, kTcSplitFlagCount * sizeof(int));  // pieces nobody consumed
+    cudaMemset(d_split_flags_, 0, kTcFlagWords * sizeof(int));  // pieces nobody consumed
     return 7;
   }
   return 0;
@@ -586,7 +587,7 @@ int Engine::check_status() {
   if (status != 0) {
     impl_->error_ = "a tensor-core pipeline wait timed out (status " + std::to_string(status) + ")";
     cudaMemset(impl_->d_status_, 0, 4);
-    cudaMemset(impl_->d_split_flags_, 0, kTcSplitFlagCount * sizeof(int));
+    cudaMemset(impl_->d_split_flags_, 0, kTcFlagWords * sizeof(int));
     return 7;
   }
   return 0;

@@ -60,6 +60,7 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
   // a handful of rows: a pass over the weights (k_rows_f32, which says where; NCNN_B200_ROWS_F32=0: tiles everywhere)
   const int cols = (g.O + kRowsF32Cols - 1) / kRowsF32Cols;
   const long long groups = (rows + kRowsF32Max - 1) / kRowsF32Max, warps = cols * groups * p.chunks;
+  const int warp_rows = rows <= 1 ? 1 : (rows <= 2 ? 2 : (rows <= 4 ? 4 : (rows <= 8 ? 8 : kRowsF32Max)));
   const bool flat = g.H == 1 && g.W == 1 && g.OH == 1 && g.OW == 1 && g.KH == 1 && g.KW == 1;
   // expected us (conv_f32.cuh): waves of warps or of 64-row tiles, each in chunks of up to 256 k
   const double places = 4.0 * sm_count_, chunk = p.chunk_k / 256.0;
@@ -68,14 +69,14 @@ std::string EngineImpl::emit_conv_f32(Step* s, const ActRef& in, const ActRef& o
   const double tiles_us = chunk * (p.split ? 1 : p.chunks) * ((p.vec_a ? 12.0 : 28.0) * std::ceil(tile_waves) + 20.0 * tile_waves) + (p.vec_o ? 0.0 : 10.0);
   const bool few = p.K >= 128 ? groups == 1 || (rows <= kRowsF32Most && rows_us < tiles_us) : rows <= 8;
   if (flat && few && p.chunks < 65536 && !env_flag_off("NCNN_B200_ROWS_F32") &&
-      (p.chunks == 1 || (cols * groups <= kTcSplitFlagCount && static_cast<size_t>(warps) * kRowsF32Max * kRowsF32Cols * 4 <= kTcSplitWorkspaceBytes))) {
+      (p.chunks == 1 || (cols * groups <= kTcFlagWords && static_cast<size_t>(warps) * warp_rows * kRowsF32Cols * 4 <= kTcSplitWorkspaceBytes))) {
     const dim3 rgrid(static_cast<unsigned>(cols), static_cast<unsigned>(p.chunks), static_cast<unsigned>(groups));
     s->kernel = "k_rows_f32";
     s->run = [=](cudaStream_t st) {
-      if (rows <= 1) launch_plain(k_rows_f32<1>, rgrid, kRowsF32Cols, 0, st, x, out, p);
-      else if (rows <= 2) launch_plain(k_rows_f32<2>, rgrid, kRowsF32Cols, 0, st, x, out, p);
-      else if (rows <= 4) launch_plain(k_rows_f32<4>, rgrid, kRowsF32Cols, 0, st, x, out, p);
-      else if (rows <= 8) launch_plain(k_rows_f32<8>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      if (warp_rows == 1) launch_plain(k_rows_f32<1>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else if (warp_rows == 2) launch_plain(k_rows_f32<2>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else if (warp_rows == 4) launch_plain(k_rows_f32<4>, rgrid, kRowsF32Cols, 0, st, x, out, p);
+      else if (warp_rows == 8) launch_plain(k_rows_f32<8>, rgrid, kRowsF32Cols, 0, st, x, out, p);
       else launch_plain(k_rows_f32<kRowsF32Max>, rgrid, kRowsF32Cols, 0, st, x, out, p);
       return launch_ok();
     };

@@ -78,6 +78,8 @@ struct TcEpilogue {
 // bytes of partial-accumulator workspace and flag words that let every layer split tiles
 constexpr size_t kTcSplitWorkspaceBytes = 160ull * kTcBlockM * kTc2MaxBlockN * 4;
 constexpr int kTcSplitFlagCount = 640;  // two per CTA (one per epilogue group)
+// words that are there: k_rows_f32 counts the finished chunks of every 32 columns (conv_f32.cuh)
+constexpr int kTcFlagWords = 16384;
 
 // Elements per K block for a kind and a channel count; 0 when the tensor-core
 // path cannot address that channel count (rows must be multiples of 16 bytes).

@@ -507,6 +507,8 @@ def test_int8_filters_of_128_channels_stay_resident_for_few_fp32_tiles(pkg, tmp_
     (16, 4097, 515), # as many rows as a warp takes, seventeen chunks
     (17, 300, 70),   # a second group of one row
     (128, 130, 40),  # as many rows as a call may have
+    (1, 513, 20512), # 641 blocks of columns of three chunks
+    (17, 1001, 10272), # 642 in two groups of rows
 ])
 def test_fp32_inner_product_of_few_rows(pkg, oracle, tmp_path, monkeypatch, m, k, n):
     """A pass over the weights sums in the tiles' chunks and order: the same bits, so more rows change none."""
