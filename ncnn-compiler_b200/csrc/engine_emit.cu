@@ -496,7 +496,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         }
         v.OH = node.OH;
         v.OW = node.OW;
-        perr = tc_plan_conv(launch.get(), kind, v, node.d_w0, node.d_w1, node.O, te, sm_count_);
+        perr = tc_plan_conv_tiles(launch.get(), kind, v, node.O, te, sm_count_);
         const bool forced = launch->cta2 != 0 && (env_int_or("NCNN_B200_CTA2_ALWAYS", 0) != 0 || env_int_or("NCNN_B200_STREAMK", 0) == 1);
         // int8 filters of several taps that fit shared memory (unless a switch asks for pairs of CTAs or split tiles)
         if (perr.empty() && i8 && !node.stem && conv_i8_level() != 0 && !forced) {
@@ -518,6 +518,7 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
             return true;
           }
         }
+        if (perr.empty()) perr = tc_encode_conv(launch.get(), kind, v, node.d_w0, node.d_w1, node.O);
       } else {
         const long long M = (to.rank == 2 ? static_cast<long long>(ti.h) : 1) * n;
         const void* a0 = i8 ? static_cast<const void*>(in.q) : static_cast<const void*>(in.p0);

@@ -638,8 +638,7 @@ int tc_k_elems(int kind, int channels) {
   return rb / tc_elem_bytes(kind);
 }
 
-std::string tc_plan_conv(TcLaunch* L, int kind, const TcIm2colView& v, const void* w0,
-                         const void* w1, int out_channels, const TcEpilogue& e, int sm_count) {
+std::string tc_plan_conv_tiles(TcLaunch* L, int kind, const TcIm2colView& v, int out_channels, const TcEpilogue& e, int sm_count) {
   load_driver_entry_points();
   if (!g_driver_error.empty()) return g_driver_error;
   const int rb = tc_row_bytes(kind, static_cast<int>(v.C));
@@ -665,6 +664,11 @@ std::string tc_plan_conv(TcLaunch* L, int kind, const TcIm2colView& v, const voi
   L->cta2 = 0;
   if (!finish_plan_workers(L, kind, M, out_channels, e, sm_count, v.C % 64 == 0))
     finish_plan(L, kind, M, out_channels, e, sm_count);
+  return {};
+}
+
+std::string tc_encode_conv(TcLaunch* L, int kind, const TcIm2colView& v, const void* w0, const void* w1, int out_channels) {
+  const TcGemmParams& p = L->p;
   const uint32_t b_box_rows = static_cast<uint32_t>(L->cta2 == 2 ? p.block_n / 2 : p.block_n);
   const int prb = p.row_bytes;  // the pair plan may have halved the K blocks
 
@@ -688,6 +692,12 @@ std::string tc_plan_conv(TcLaunch* L, int kind, const TcIm2colView& v, const voi
     L->map_b1 = L->map_b0;
   }
   return {};
+}
+
+std::string tc_plan_conv(TcLaunch* L, int kind, const TcIm2colView& v, const void* w0, const void* w1, int out_channels, const TcEpilogue& e,
+                         int sm_count) {
+  const std::string err = tc_plan_conv_tiles(L, kind, v, out_channels, e, sm_count);
+  return err.empty() ? tc_encode_conv(L, kind, v, w0, w1, out_channels) : err;
 }
 
 std::string tc_plan_gemm(TcLaunch* L, int kind, const void* a0, const void* a1, long long M, int K,

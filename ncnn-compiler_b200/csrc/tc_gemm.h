@@ -108,6 +108,10 @@ constexpr int kTcChunkBlocks = 18, kTcChunkFrom = 3 * kTcChunkBlocks + 1;
 std::string tc_plan_conv(TcLaunch* launch, int kind, const TcIm2colView& view, const void* w0,
                          const void* w1, int out_channels, const TcEpilogue& epilogue,
                          int sm_count);
+// The two halves of it: whether and how tc_gemm_kernel or tc_gemm2_kernel would run the layer, which other kernels are
+// compared with, and the tensor maps, which only the kernel that runs needs.
+std::string tc_plan_conv_tiles(TcLaunch* launch, int kind, const TcIm2colView& view, int out_channels, const TcEpilogue& epilogue, int sm_count);
+std::string tc_encode_conv(TcLaunch* launch, int kind, const TcIm2colView& view, const void* w0, const void* w1, int out_channels);
 
 // Plain GEMM: A is [M][K] row-major with row stride lda elements (planes a0/a1),
 // weights packed [N][Kpad].
