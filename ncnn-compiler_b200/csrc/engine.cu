@@ -50,8 +50,8 @@ bool EngineImpl::build(const std::string& param, const std::string& bin, const E
   cudaMemset(st, 0, 256);
   device_allocs_.push_back(st);
   d_status_ = static_cast<int*>(st);
-  // workspace of the contraction kernel that splits tiles between CTA pairs: partial accumulators
-  // and one flag word per CTA (zero between launches); all launches of a model run on one stream
+  // workspace of the kernels that split sums between blocks: partial sums, and flags and counters (zero between launches);
+  // all launches of a model run on one stream
   void* ws = nullptr;
   constexpr size_t ws_bytes = kTcSplitWorkspaceBytes + kTcFlagWords * sizeof(int);
   if (device_alloc(&ws, ws_bytes) != cudaSuccess) return fail(err, "out of device memory");

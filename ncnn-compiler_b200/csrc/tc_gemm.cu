@@ -1057,8 +1057,8 @@ std::string tc_plan_conv_patch(TcPatchLaunch* L, int kind, const TcIm2colView& v
   set_chunks(g, kind, rb);
   const int taps = v.KH * v.KW;
   if (taps < 2) return "a 1x1 filter has nothing to reuse";
-  // (a single tile of few K blocks would gain ~1.5 us; the test of the waits that run out, whose stall is made in
-  // tc_gemm_kernel, asks for it there)
+  // (a single tile of few K blocks stays with tc_gemm_kernel because the test of that kernel's waits asks for it there, not
+  // because it is faster: whole calls of 64 -> 64, 4x4 to 11x11 pixels, and of 64 -> 256, 11x11, take 10.4 us there and 8.3 here)
   if (!always && gemm.cta2 == 0 && gemm.p.tiles_m == 1 && g.k_blocks <= 9) return "a single short tile";
   // The model ranks tile shapes well and both kernels' tiles roughly: with operand rows of 128 bytes this kernel came out
   // ahead up to 0.68 of the other's clocks, with rows of 64 bytes (channel counts that are no multiple of 64) up to 0.81.
