@@ -234,27 +234,31 @@ int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, 
 // least time, the chunks of a tile on different CTAs.  Clocks as in gemm_clocks (a block's copies, or its MMAs and the gap
 // between blocks), and for the chunks' sums their way through L2.
 // fp32 sums round by where K is cut, so a layer has one way to cut it: the chunks that are best for a full tile of 128 rows
-// (with fewer rows others would be up to 4 % better by these clocks), for every call that is cut at all, and calls of 1 to
-// 128 rows are all cut or all whole; the rows choose the tile width, which no bit depends on.  Contractions of up to 26 blocks of bf16
-// pairs (1664 values) are never cut: a network's last layer then gives a batch the bits of its images run one by one
-// (1536 -> 1000, 33 rows: 16.5 us whole, 12.7 in chunks).  Whole numbers are exact however they are cut.
+// (with fewer rows others would be up to 4 % better by these clocks).  Calls of up to three tiles of rows are all cut so, or
+// (where chunks gain nothing) all whole; the rows choose the tile width, which no bit depends on, and whether a tile's chunks
+// lie apart or follow one another in one CTA, which costs 0 to 5 % over whole tiles and rounds like chunks apart (4096 -> 1000,
+// 300 rows: 4.4e-6 of the result's norm off in chunks, 1.4e-5 whole).  Contractions of up to 26 blocks of bf16 pairs (1664 values)
+// are never cut: a network's last layer then gives a batch of any size the bits of its images run one by one (1536 -> 1000,
+// 33 rows: 16.5 us whole, 12.7 in chunks; chunks for every batch would cost calls of thousands of rows 8 to 20 %).  Whole
+// numbers are exact however they are cut.
 // Whole calls in us, before (workers that share tiles, tc_gemm2.cuh, or whole tiles) -> in chunks:
 //            2048 -> 1024          3000 -> 700           2816 -> 2816           4096 -> 4096
 //   fp32     64 rows 24.7 -> 16.4  64 rows 34.6 -> 14.4  64 rows 30.8 -> 20.5   64 rows 32.8 -> 28.7
 //            128     34.2 -> 14.4  128     48.4 -> 16.5  128     39.7 -> 22.7   128     39.4 -> 33.9
 //            1000    26.7 -> 30.8  1000    36.8 -> 34.9  1000    49.3 -> 54.2   1000    87.4 -> 84.3
 //   int8     128     11.0 -> 12.8  300     12.9 -> 18.5  64      12.3 -> 14.5   64      23.4 -> 19.1, 128 30.7 -> 18.5
-// and of more than one tile of rows, whole tiles against the layer's chunks (their number behind the layer; ! is not taken):
+// and of more than one tile of rows, chunks in one CTA against chunks apart (their number behind the layer; ! is not taken):
 //            2048 -> 1024 (4)      3000 -> 700 (6)       2816 -> 2816 (4)       4096 -> 1000 (8)       2048 -> 2048 (4)
-//   fp32     200 rows 22.6 / 18.8  200 rows 28.8 / 22.3  200 rows 28.6 / 28.9!  200 rows 36.2 / 32.7   200 rows 22.0 / 26.8!
-//            384      22.7 / 23.8! 384      29.0 / 28.8! 384      30.9 / 45.9!  384      37.0 / 48.6!  384      22.7 / 35.6!
-// so it takes up to three tiles of rows, where the clocks below say so (of three, 4096 -> 512 37.1 -> 31.2); int8, whose blocks are short, from 28 blocks on and up
-// to two.
+//   fp32     200 rows 22.7 / 18.7  200 rows 30.1 / 22.5  200 rows 28.8 / 28.9!  200 rows 37.9 / 32.8   200 rows 22.7 / 26.8!
+//            384      22.8 / 23.8! 384      30.9 / 28.8! 384      30.9 / 45.9!  384      39.2 / 48.6!  384      24.7 / 35.6!
+// so they lie apart where the clocks below say so (of three tiles, 4096 -> 512 37.1 / 31.2); int8, whose blocks are short, is
+// cut from 28 blocks on and up to two tiles.
 struct RowsSplit {
   int block_n = 0, chunk_blocks = 0, chunks = 1;
+  bool apart = false;  // the chunks of a tile on different CTAs
   double clocks = 1e300;
 };
-// The best of whole tiles and tiles in `only` chunks (0: in any number of them).
+// The best of whole tiles and tiles in `only` chunks apart (0: in any number of them).
 RowsSplit best_rows_split(int kind, long long M, int k_blocks, const TcEpilogue& e, int N, int sm_count, int only) {
   RowsSplit best;
   const bool i8 = kind == GEMM_I8;
@@ -288,16 +292,28 @@ RowsSplit split_rows(int kind, long long M, int k_blocks, const TcEpilogue& e, i
   if ((kind != GEMM_BF16X3 && kind != GEMM_I8) || e.sk_ws == nullptr || e.sk_flags == nullptr) return {};
   const bool i8 = kind == GEMM_I8;
   if (k_blocks < (i8 ? 28 : 27) || M > (i8 ? 2 : 3) * kTcBlockM) return {};
-  if (i8) return split_k_enabled() ? best_rows_split(kind, M, k_blocks, e, N, sm_count, 0) : RowsSplit{};
-  const RowsSplit layer = best_rows_split(kind, kTcBlockM, k_blocks, e, N, sm_count, 0);
+  if (i8) {
+    RowsSplit rows = split_k_enabled() ? best_rows_split(kind, M, k_blocks, e, N, sm_count, 0) : RowsSplit{};
+    rows.apart = rows.chunks > 1;
+    return rows;
+  }
+  RowsSplit layer = best_rows_split(kind, kTcBlockM, k_blocks, e, N, sm_count, 0);
+  layer.apart = layer.chunks > 1;
+  if (layer.chunks == 1) return best_rows_split(kind, M, k_blocks, e, N, sm_count, 1);
   RowsSplit rows = best_rows_split(kind, M, k_blocks, e, N, sm_count, layer.chunks);
+  rows.apart = rows.chunks > 1;
   if (M <= kTcBlockM) {
-    if (rows.chunks != layer.chunks) rows = layer;
+    if (!rows.apart) rows = layer;
     rows.clocks = layer.clocks;  // (what other forms are compared with: the same for all calls of one tile)
-  } else if (M > 2 * kTcBlockM && rows.chunks > 1) {
-    // (up to a tenth of the clocks' gain did not come: 2048 -> 1024, 300 rows 25.2 in chunks, 22.7 whole)
-    const RowsSplit whole = best_rows_split(kind, M, k_blocks, e, N, sm_count, 1);
-    if (rows.clocks > 0.8 * whole.clocks) rows = whole;
+    return rows;
+  }
+  // (up to a tenth of the clocks' gain did not come: 2048 -> 1024, 300 rows 25.2 in chunks, 22.7 whole)
+  const RowsSplit whole = best_rows_split(kind, M, k_blocks, e, N, sm_count, 1);
+  if (M > 2 * kTcBlockM && rows.clocks > 0.8 * whole.clocks) rows = whole;
+  if (rows.chunks == 1) {
+    rows.chunks = layer.chunks;
+    rows.chunk_blocks = layer.chunk_blocks;
+    rows.apart = false;
   }
   return rows;
 }
@@ -320,7 +336,7 @@ void finish_plan(TcLaunch* L, int kind, long long M, int N, const TcEpilogue& e,
     if (rows.chunks > 1) {
       p.chunk_blocks = rows.chunk_blocks;
       p.chunks = rows.chunks;
-      if (split_k_enabled()) {
+      if (rows.apart && split_k_enabled()) {
         p.block_n = rows.block_n;
         p.split_k = 1;
       }

@@ -396,17 +396,19 @@ def test_chunks_in_one_cta_change_no_bit_of_an_inner_product(pkg, tmp_path, monk
     assert np.array_equal(pkg.Model(param, bin_).run(x)[0], want)
 
 
-@pytest.mark.parametrize("m,k,n,other", [
-    (200, 3000, 700, 128),   # in chunks: those of calls of up to 128 rows
-    (300, 2816, 2816, 600),  # more than 128 rows of a wide layer: whole, like a call of many rows
-    (129, 2048, 2048, 600),
+@pytest.mark.parametrize("m,k,n", [
+    (200, 3000, 700),   # chunks on different CTAs
+    (300, 2816, 2816),  # one after the other
+    (129, 2048, 2048),
+    (384, 4096, 1000),
+    (384, 1728, 1000),
 ])
-def test_inner_product_of_two_and_three_tiles_of_rows(pkg, tmp_path, m, k, n, other):
+def test_inner_product_of_two_and_three_tiles_of_rows(pkg, tmp_path, m, k, n):
+    """Wherever its chunks run, a row has the bits that it has in a call of one tile."""
     param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n)
-    x = np.random.default_rng(29).uniform(-1, 1, (max(m, other), 1, 1, k)).astype(np.float32)
+    x = np.random.default_rng(29).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
     model = pkg.Model(param, bin_)
-    least = min(m, other)
-    assert np.array_equal(model.run(x[:m])[0][:least], model.run(x[:other])[0][:least])
+    assert np.array_equal(model.run(x)[0][m - 128:], model.run(x[m - 128:])[0])
 
 
 def _int8_pair(zoo, prefix, cin, mid, cout, k, h, w, act):
