@@ -234,8 +234,8 @@ int split_width(const TcGemmParams& p, const TcEpilogue& e, int N, int block_n, 
 // least time, the chunks of a tile on different CTAs.  Clocks as in gemm_clocks (a block's copies, or its MMAs and the gap
 // between blocks), and for the chunks' sums their way through L2.
 // fp32 sums round by where K is cut, so a layer has one way to cut it: the chunks that are best for a full tile of 128 rows
-// (with fewer rows others would be up to 4 % better by these clocks).  Calls of up to three tiles of rows are all cut so, or
-// (where chunks gain nothing) all whole; the rows choose the tile width, which no bit depends on, and whether a tile's chunks
+// (with fewer rows others would be up to 4 % better by these clocks).  Calls of up to three tiles of rows that come here are all
+// cut so, or (where chunks gain nothing) all whole; the rows choose the tile width, which no bit depends on, and whether a tile's chunks
 // lie apart or follow one another in one CTA, which costs 0 to 5 % over whole tiles and rounds like chunks apart (4096 -> 1000,
 // 300 rows: 4.4e-6 of the result's norm off in chunks, 1.4e-5 whole).  Contractions of up to 26 blocks of bf16 pairs (1664 values)
 // are never cut: a network's last layer then gives a batch of any size the bits of its images run one by one (1536 -> 1000,
