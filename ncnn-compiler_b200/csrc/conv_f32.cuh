@@ -51,14 +51,6 @@ inline void f32_chunks(int K, int* chunks, int* chunk_k) {
   *chunks = (K + *chunk_k - 1) / *chunk_k;
 }
 
-__device__ __forceinline__ void f32x2_fma(uint64_t& d, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float2 f32x2_get(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
 __device__ __forceinline__ void cp_async_4(uint32_t smem_dst, const void* src, int src_bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_dst), "l"(src), "r"(src_bytes) : "memory");
 }

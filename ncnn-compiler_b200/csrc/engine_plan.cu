@@ -328,11 +328,10 @@ void EngineImpl::fuse_depthwise_projection() {
           ex.k_elems == 32 && ex.d_w0 != nullptr && ex.d_w1 != nullptr)
         je = static_cast<int>(j);
     }
-    // Measured on MobileNetV2 at batch 256: with the expand layer inside, stride-2 blocks are 10-16 % faster than
-    // their three layers (the expanded tensor is four times the block's output), stride-1 blocks 35 % slower than
-    // expand + fused pair (per block of 32 channels the kernel then runs 12 more MMAs and a TMEM read-back on top of
-    // the depthwise arithmetic).  So stride-1 blocks join only with NCNN_B200_FUSE_EXPAND=2.
-    if (je >= 0 && dw.sh == 1 && env_int_or("NCNN_B200_FUSE_EXPAND", 1) < 2) je = -1;
+    // Measured on MobileNetV2 at batch 256, the block's three layers (stride 2) or expand layer and fused pair (stride 1)
+    // against the whole block: 112x112x96 at stride 2 0.80 -> 0.29 ms, 56x56x144 0.38 -> 0.29 (stride 1) and 0.40 -> 0.18,
+    // 28x28x192 0.134 -> 0.104 and 0.137 -> 0.065.  NCNN_B200_FUSE_EXPAND=1 keeps the stride-1 blocks apart.
+    if (je >= 0 && dw.sh == 1 && env_int_or("NCNN_B200_FUSE_EXPAND", 2) < 2) je = -1;
     if (je < 0 && dw.sh != 1) continue;
     if (dw.sh != 1 && dw.sh != 2) continue;
     if (uses[mid] != 1 || tin.rank != 3 || tin.fmt != FMT_F32 || tin.Cp != tin.c || tin.Wp != tin.w || tin.w_off != 0 ||

@@ -379,6 +379,17 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Registers a thread of this warpgroup (four warps that all execute it) holds from here on: gives some back, or waits until
+// other warpgroups of the block gave back as many.  A multiple of 8 from 24 to 256.
+template <int REGS>
+__device__ __forceinline__ void reg_dealloc() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
+}
+template <int REGS>
+__device__ __forceinline__ void reg_alloc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
+}
+
 // Shared-memory matrix descriptor for a K-major operand tile whose rows are
 // `row_bytes` long (32, 64 or 128) and stored with the matching TMA swizzle:
 // eight rows form one swizzle atom, atoms follow each other every 8*row_bytes.

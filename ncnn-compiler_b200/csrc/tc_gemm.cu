@@ -1373,8 +1373,8 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int strid
       // patch, about once in 10^5 loads with the L2 flushed)
       for (int patches : {4, 2}) {
         if (expand && patches != 2) continue;
-        const int fixed = (expand ? x_bufs * 2 * r.x_plane_bytes : 0) + patches * dwp_patch_bytes(stride) +
-                          2 * 2 * dwp_a_plane_bytes(stride) + 4 * kDrainWarpBytes + table;
+        const int fixed = (expand ? x_bufs * 2 * r.x_plane_bytes : 0) + patches * dwp_patch_bytes(stride, expand) +
+                          2 * 2 * dwp_a_plane_bytes(stride) + dwp_drain_warps(stride) * kDrainWarpBytes + table;
         const int stages = std::min(kDwpMaxStages, (budget - fixed) / stage);
         if (stages >= min_stages) {
           r.stages = stages;

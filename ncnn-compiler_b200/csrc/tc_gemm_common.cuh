@@ -268,6 +268,29 @@ __device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uin
   mid = pack_bf16x2(__fadd_rn(a, -bf16_low(hi)), __fadd_rn(b, -bf16_high(hi)));
 }
 
+// two fp32 values in one register pair
+__device__ __forceinline__ void f32x2_fma(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void f32x2_add(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t f32x2_make(uint32_t lo, uint32_t hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 f32x2_get(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t lds_b64(uint32_t at) {
+  uint64_t v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(at));
+  return v;
+}
+
 // The activations a network seldom uses live in one function that is called, not inlined: an epilogue applies its
 // activation to 16 or 32 values in a row, and a copy of every branch per value made the loops large enough to
 // stall on instruction fetch (a 3x3 depthwise block spent 5000 cycles there instead of 400).
