@@ -215,7 +215,6 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
   const uint32_t stage_bytes = static_cast<uint32_t>(p.stage_bytes);
   const int AS = p.pair ? 2 : 1;  // A tiles per stage
   const uint32_t b_slot = (stage_bytes / PLANES) - static_cast<uint32_t>(AS) * slot;  // B tile, rounded to 1 KB
-  const uint32_t tx_bytes = PLANES * (slot + static_cast<uint32_t>(p.block_n) * p.row_bytes);
   const int S = p.stages;
   // int8 K blocks are small (two MMAs over 12 KB for 64 channels): a stage holds SUB of them, so that the
   // ~450 cycles of arming and releasing a stage are paid once per SUB blocks
@@ -302,7 +301,7 @@ tc_gemm_kernel(const __grid_constant__ TcGemmParams p, const __grid_constant__ C
         const int halves = pair_tile ? 2 : 1;
         // a second half that starts past the last row repeats the first (its results are never stored)
         const long long m1 = pair_tile && m0 + kTcBlockM < p.M ? m0 + kTcBlockM : m0;
-        const uint32_t my_tx = is_b ? b_tx : static_cast<uint32_t>(PLANES * halves) * slot;
+        const uint32_t my_tx = is_b ? b_tx : static_cast<uint32_t>(PLANES * halves * p.a_rows) * p.row_bytes;
         const int n0 = n_blk * p.block_n;
         int img[2] = {0, 0}, h_base[2] = {0, 0}, w_base[2] = {0, 0};
         if (p.a_im2col && !is_b) {

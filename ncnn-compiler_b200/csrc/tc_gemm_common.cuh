@@ -56,6 +56,7 @@ struct TcGemmParams {
   int k_elems;    // elements per K block
   int row_bytes;  // bytes per shared-memory operand row: 128 or 64
   int stages;
+  int a_rows;       // rows of A that a copy brings: 128, or what a single tile of fewer rows has (a multiple of 8)
   int stage_bytes;  // bytes of one ring stage: planes * (A tile + B tile rounded to 1 KB)
   int a_im2col;  // A addressing: 0 plain matrix (tiled TMA), 1 im2col TMA
   int OH, OW, KW;

@@ -378,6 +378,30 @@ def test_inner_product_sums_alike_whatever_the_rows_of_a_tile(pkg, tmp_path, k, 
             assert np.array_equal(model.run(x[:m])[0], want[:m]), m
 
 
+@pytest.mark.parametrize("h,w,cin", [(1, 1, 64), (1, 7, 96), (3, 3, 32), (7, 9, 64), (8, 8, 40), (5, 13, 64), (11, 11, 64), (8, 16, 64)])
+def test_lone_tile_of_few_pixels(pkg, tmp_path, monkeypatch, h, w, cin):
+    """A tile that is alone brings only the rows it has (1 to 128 of them): the bits of the same image in front of others."""
+    monkeypatch.setenv("NCNN_B200_PATCH", "0")
+    param, bin_ = pkg.zoo.single_conv(str(tmp_path / "c"), h=h, w=w, cin=cin, cout=72, k=1, stride=1, pad=0)
+    x = np.random.default_rng(h * w).uniform(-1, 1, (300 // (h * w) + 2, cin, h, w)).astype(np.float32)
+    model = pkg.Model(param, bin_)
+    assert any(r["kernel"].startswith("tc_gemm_kernel") for r in model.profile(1, 1))
+    want = model.run(x)[0]
+    assert np.array_equal(model.run(x[:1])[0], want[:1])
+    assert rel_l2(want, pkg.Model(param, bin_, accuracy_mode=pkg.FP32_CUDA).run(x)[0]) <= 3e-5
+
+
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 63, 64, 65, 121, 128])
+@pytest.mark.parametrize("k,n", [(1001, 130), (512, 64)])
+def test_lone_tile_of_few_int8_rows(pkg, oracle, tmp_path, m, k, n):
+    param, bin_ = pkg.zoo.inner_product(str(tmp_path / "ip"), k, n, int8=True)
+    x = np.random.default_rng(m).uniform(-1, 1, (m, 1, 1, k)).astype(np.float32)
+    got = pkg.Model(param, bin_).run(x)[0]
+    ref = oracle.Model(param, bin_)
+    for i in sorted({0, m // 2, m - 1}):
+        assert np.array_equal(got[i], ref.run([x[i]])[0])
+
+
 @pytest.mark.parametrize("m,k,n", [
     (1, 2048, 1000),
     (33, 2048, 1000),
