@@ -362,6 +362,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "memory");
 }
 
+// 8, 2 and 1 of them
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld1(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v[0]) : "r"(taddr) : "memory");
+}
+
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
@@ -402,6 +416,19 @@ __device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t smem_addr, uint32_
   d |= layout << 61;
   return d;
 }
+
+// The same for an operand whose rows (M or N) are contiguous: 64 bf16 values of one k are 128 bytes, eight k make a swizzle
+// atom of 1 KB; the next eight k lie `k_stride` bytes further, the next 64 rows `row_stride`.
+__device__ __forceinline__ uint64_t smem_desc_mnmajor(uint32_t smem_addr, uint32_t row_stride, uint32_t k_stride) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4);
+  d |= static_cast<uint64_t>(row_stride >> 4) << 16;
+  d |= static_cast<uint64_t>(k_stride >> 4) << 32;
+  d |= 1ull << 46;
+  d |= 2ull << 61;
+  return d;
+}
+constexpr uint32_t kInstrAMnMajor = 1u << 15;  // instruction descriptor: A's rows are contiguous
 
 // Instruction descriptor: dense, no negate, both operands K-major.
 //   c_format: 1 = f32, 2 = s32;  ab_format: 2 = tf32 (kind::tf32), 1 = s8 (kind::i8)

@@ -1340,60 +1340,75 @@ cudaError_t tc_launch_conv_i8(const TcConvI8Launch& L, cudaStream_t stream) {
 namespace {
 
 struct DwProjShape {
-  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, smem = 0;
+  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, e_bufs = 0, a_slots = 0, smem = 0;
   bool ok = false;
 };
-
-// Shared-memory plan of tc_dw_project_kernel.  expand: the expand layer is fused in (input patches as bf16 planes
-// of 64-byte rows, one fp32 patch per depthwise group, the block's expand weights beside its projection weights in
-// every ring stage, the expand bias beside the depthwise table).
-DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int stride, bool expand, int cin = 32) {
-  DwProjShape r;
-  if (out_mode != OUT_BF16X2 && out_mode != OUT_F32) return r;
-  if (res_mode == RES_SPLIT) return r;
-  if (stride != 1 && stride != 2) return r;
-  if (stride == 2 && !expand) return r;  // (patches loaded by TMA are built for stride 1 only)
-  const int step = 16;
-  const int n_tiles = (N + 255) / 256;
-  r.block_n = ((N + n_tiles - 1) / n_tiles + step - 1) / step * step;
-  if (r.block_n > 256 || r.block_n % 16 != 0) return r;
-  if (expand && r.block_n > 128) return r;  // (the expand accumulators take the TMEM columns past two 128-column ones)
+bool dw_project_formats(int out_mode, int res_mode) { return (out_mode == OUT_BF16X2 || out_mode == OUT_F32) && res_mode != RES_SPLIT; }
+// columns of a tile: N in as few tiles of at most `most` as it takes, all alike
+void dw_project_columns(DwProjShape& r, int N, int most) {
+  const int n_tiles = (N + most - 1) / most;
+  r.block_n = ((N + n_tiles - 1) / n_tiles + 15) / 16 * 16;
   r.tiles_n = (N + r.block_n - 1) / r.block_n;
   r.b_bytes = (r.block_n * 64 + 1023) / 1024 * 1024;
-  const int budget = kTcSmemBudget;
+}
+
+// Shared-memory plan of the pair.
+DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
+  DwProjShape r;
+  if (!dw_project_formats(out_mode, res_mode)) return r;
+  dw_project_columns(r, N, 256);
   const int c_pad = (C + kDwpChannels - 1) / kDwpChannels * kDwpChannels;
-  const int table = (c_pad * (expand ? 11 : 10) * 4 + 1023) / 1024 * 1024;  // depthwise filter and bias (+ expand bias)
-  const int stage = 2 * r.b_bytes + (expand ? 4096 : 0);
-  r.x_row_bytes = cin <= 16 ? 32 : 64;
-  r.x_plane_bytes = expand ? (dwp_patch_pixels(stride) * r.x_row_bytes + 1023) / 1024 * 1024 : 0;
-  // Deep patch ring first (a patch load outlasts one block's arithmetic), then three weight stages; the last
-  // resort is two of each.  With the expand layer: two input patch buffers if they
-  // fit, and never fewer than three stages (the expand MMAs run two blocks ahead of the projection's).
-  for (int min_stages : {4, 3, 2}) {
-    if (expand ? min_stages < 3 : min_stages > 3) continue;  // (without the expand layer three stages are plenty)
-    for (int x_bufs : {2, 1}) {
-      if (!expand && x_bufs != 2) continue;
-      // (an even ring only: the two depthwise groups take alternate blocks, so with an even depth a slot always
-      // belongs to the same group, which waits for its phases in order; with three slots a slot would alternate
-      // between the groups, a group would wait for every second phase of it, and a parity wait cannot tell a
-      // phase from the one two before it: a load delayed past a whole block's arithmetic let a group read a stale
-      // patch, about once in 10^5 loads with the L2 flushed)
-      for (int patches : {4, 2}) {
-        if (expand && patches != 2) continue;
-        const int fixed = (expand ? x_bufs * 2 * r.x_plane_bytes : 0) + patches * dwp_patch_bytes(stride, expand) +
-                          2 * 2 * dwp_a_plane_bytes(stride) + dwp_drain_warps(stride) * kDrainWarpBytes + table;
-        const int stages = std::min(kDwpMaxStages, (budget - fixed) / stage);
-        if (stages >= min_stages) {
-          r.stages = stages;
-          r.patches = patches;
-          r.x_bufs = expand ? x_bufs : 0;
-          r.smem = fixed + stages * stage + 1024;
-          r.ok = true;
-          return r;
-        }
+  const int table = (c_pad * 10 * 4 + 1023) / 1024 * 1024;  // depthwise filter and bias
+  const int stage = 2 * r.b_bytes;
+  // Deep patch ring first (a patch load outlasts one block's arithmetic), then three weight stages (plenty); the last
+  // resort is two of each.
+  for (int min_stages : {3, 2}) {
+    // (an even ring only: the two depthwise groups take alternate blocks, so with an even depth a slot always
+    // belongs to the same group, which waits for its phases in order; with three slots a slot would alternate
+    // between the groups, a group would wait for every second phase of it, and a parity wait cannot tell a
+    // phase from the one two before it: a load delayed past a whole block's arithmetic let a group read a stale
+    // patch, about once in 10^5 loads with the L2 flushed)
+    for (int patches : {4, 2}) {
+      const int fixed = patches * kDwpPatchBytes + 2 * 2 * kDwpAPlaneBytes + 8 * kDrainWarpBytes + table;
+      const int stages = std::min(kDwpMaxStages, (kTcSmemBudget - fixed) / stage);
+      if (stages >= min_stages) {
+        r.stages = stages;
+        r.patches = patches;
+        r.smem = fixed + stages * stage + 1024;
+        r.ok = true;
+        return r;
       }
     }
   }
+  return r;
+}
+
+// Shared and tensor memory plan of the whole block: all weights stay, so a block with too many of them for that is not taken.
+// Eight operand tiles before two input patches: four (one for each quarter of a set) leave the depthwise warps waiting for
+// the projection's MMAs, while a patch is needed by the expand MMAs only, which run ahead.
+DwProjShape block_shape(int N, int out_mode, int res_mode, int C, int stride, int cin) {
+  DwProjShape r;
+  if (!dw_project_formats(out_mode, res_mode) || (stride != 1 && stride != 2)) return r;
+  // two accumulators beside one buffer of each half's expanded pixels, or two where they fit
+  const int pixels = blk_in_cols(stride), most = (static_cast<int>(kTcTmemCols) - 2 * pixels) / 2 / 16 * 16;
+  dw_project_columns(r, N, std::min(128, most));
+  r.e_bufs = 2 * r.block_n + 4 * pixels <= static_cast<int>(kTcTmemCols) ? 2 : 1;
+  r.x_row_bytes = cin <= 16 ? 32 : 64;
+  r.x_plane_bytes = (dwp_patch_pixels(stride) * r.x_row_bytes + 1023) / 1024 * 1024;
+  const int c_blocks = (C + kDwpChannels - 1) / kDwpChannels, c_pad = c_blocks * kDwpChannels;
+  const int weights = 2 * c_pad * r.x_row_bytes + r.tiles_n * c_blocks * 2 * r.b_bytes;
+  const int table = (kBlkTableRows * c_pad * 4 + 1023) / 1024 * 1024;
+  const int fixed = weights + table + dwp_tile_h(stride) * kDwpTileW / 32 * kDrainWarpBytes;
+  for (int slots : {8, 4})
+    for (int x_bufs : {2, 1}) {
+      const int smem = fixed + x_bufs * 2 * r.x_plane_bytes + slots * 2 * blk_a_plane_bytes(stride);
+      if (smem > kTcSmemBudget) continue;
+      r.x_bufs = x_bufs;
+      r.a_slots = slots;
+      r.smem = smem + 1024;
+      r.ok = true;
+      return r;
+    }
   return r;
 }
 
@@ -1411,7 +1426,7 @@ bool tc_dw_project_applies(int C, int N, int H, int W, int out_mode, bool has_re
   if (!dw_project_fills(H, W, 1)) return false;
   const int res_mode = !has_res ? RES_NONE : (res_bf16 ? RES_BF16X2 : RES_F32);
   if (out_mode == OUT_F32 && N % 4 != 0) return false;
-  return dw_project_shape(N, out_mode, res_mode, C, 1, false).ok;
+  return dw_project_shape(N, out_mode, res_mode, C).ok;
 }
 
 bool tc_block_applies(int Cin, int C, int N, int OH, int OW, int stride, bool has_res) {
@@ -1423,7 +1438,7 @@ bool tc_block_applies(int Cin, int C, int N, int OH, int OW, int stride, bool ha
     for (int res_mode : {RES_NONE, RES_F32, RES_BF16X2}) {
       if (!has_res && res_mode != RES_NONE) continue;
       if (has_res && res_mode == RES_NONE) continue;
-      if (!dw_project_shape(N, out_mode, res_mode, C, stride, true, Cin).ok) return false;
+      if (!block_shape(N, out_mode, res_mode, C, stride, Cin).ok) return false;
     }
   return true;
 }
@@ -1437,7 +1452,8 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   if (!direct_rows(GEMM_BF16X3, e, c.out_channels, &p.wide)) return "the fused depthwise + projection kernel writes rows of 16-byte pieces";
   const bool expand = c.ex_w0 != nullptr;
   const int stride = c.stride;
-  const DwProjShape shape = dw_project_shape(c.out_channels, e.out_mode, res_mode, c.C, stride, expand, expand ? c.Cin : 32);
+  const DwProjShape shape = expand ? block_shape(c.out_channels, e.out_mode, res_mode, c.C, stride, c.Cin)
+                                   : (stride == 1 ? dw_project_shape(c.out_channels, e.out_mode, res_mode, c.C) : DwProjShape{});
   if (!shape.ok) return "the fused depthwise + projection kernel does not take this output format, width or stride";
   if (e.ldo != c.out_channels) return "the fused depthwise + projection kernel writes dense channel-last rows";
   const int x_channels = expand ? c.Cin : c.C;
@@ -1471,6 +1487,8 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   p.x_plane_bytes = shape.x_plane_bytes;
   p.x_row_bytes = shape.x_row_bytes;
   p.x_bufs = shape.x_bufs;
+  p.e_bufs = shape.e_bufs;
+  p.a_slots = shape.a_slots;
   p.ex_ksteps = expand ? (shape.x_row_bytes == 32 ? 1 : (c.Cin + 15) / 16) : 0;
   p.ex_bias = c.ex_bias;
   p.ex_act = c.ex_act;
@@ -1517,7 +1535,7 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
 }
 
 cudaError_t tc_launch_dw_project(const TcDwProjLaunch& L, cudaStream_t stream) {
-  KernelLaunchConfig lc(L.grid, kDwpThreads, L.smem_bytes, false, stream);
+  KernelLaunchConfig lc(L.grid, L.expand ? kBlkThreads : kDwpThreads, L.smem_bytes, false, stream);
   constexpr int max_smem = kTcSmemBudget + 1024;
   const cudaError_t e = with_form<GEMM_BF16X3, false>(L.p.out_mode, L.p.res_mode != RES_NONE, [&](auto form) {
     constexpr int EPI = decltype(form)::value;

@@ -273,6 +273,11 @@ __device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uin
 __device__ __forceinline__ void f32x2_fma(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ uint64_t f32x2_fma3(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
 __device__ __forceinline__ void f32x2_add(uint64_t& d, uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
 }
