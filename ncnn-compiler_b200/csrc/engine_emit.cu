@@ -600,9 +600,22 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         const dim3 grid(((node.OH + 7) / 8) * ((node.OW + 7) / 8), (ti.c / 4 + 7) / 8, static_cast<unsigned>(n));
         const int stride = node.sh;
         const float* wf = static_cast<const float*>(w);
-        s.kernel = "k_depthwise3x3_tile";
+        const int pairs = (node.OW + 1) / 2;
+        const long long threads = n * pairs * (ti.c / 4);
+        // A thread of the columns kernel walks OH rows one after the other (0.6 to 0.8 us each), so it needs enough of them.
+        // By events, tile / columns in us, around the line: 14x14x384 10 700 threads 12.7 / 14.3, 21 500 17.0 / 14.4;
+        // 28x28x192 10 700 16.4 / 18.6, 21 500 24.9 / 20.5; 112 -> 56x56x96 21 500 53 / 68, 43 000 96 / 86; 112x112x32
+        // 28 700 85 / 90, 57 300 160 / 107; 80 -> 40x40x144 23 000 47 / 52, 46 000 84 / 66.
+        const int clamp = node.act == ACT_RELU || node.act == ACT_CLIP ? 1 : 0;
+        const bool columns = in.fmt == FMT_F32 && (out.fmt == FMT_F32 || out.fmt == FMT_BF16X2) && (clamp || node.act == ACT_NONE) && !e.has_res &&
+                             threads >= (node.OH <= 32 ? 16384 : 40960) && n * pairs <= 0x7fffffffll && (threads + 255) / 256 <= 0x7fffffffll;
+        const float lo = node.act == ACT_CLIP ? e.act_a : 0.0f, hi = node.act == ACT_CLIP ? e.act_b : INFINITY;
+        const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
+        s.kernel = columns ? "k_depthwise3x3_columns" : "k_depthwise3x3_tile";
         s.run = [=](cudaStream_t st) {
-          if (stride == 1) launch_plain(k_depthwise3x3_tile<1>, grid, 256, 0, st, in, out, wf, g, e);
+          if (columns && stride == 1) launch_plain(k_depthwise3x3_columns<1>, blocks, 256, 0, st, in.p0, out, wf, e.bias, g, clamp, lo, hi, pairs, threads);
+          else if (columns) launch_plain(k_depthwise3x3_columns<2>, blocks, 256, 0, st, in.p0, out, wf, e.bias, g, clamp, lo, hi, pairs, threads);
+          else if (stride == 1) launch_plain(k_depthwise3x3_tile<1>, grid, 256, 0, st, in, out, wf, g, e);
           else launch_plain(k_depthwise3x3_tile<2>, grid, 256, 0, st, in, out, wf, g, e);
           return launch_ok();
         };

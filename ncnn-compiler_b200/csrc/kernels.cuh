@@ -702,6 +702,105 @@ static __global__ void __launch_bounds__(256) k_depthwise3x3_tile(ActRef in, Act
   }
 }
 
+// The same layer without shared memory, for many images: a thread owns four channels and two neighbouring columns of results
+// and walks down the image.  An input row (4 columns, 5 at stride 2) goes into the sums of every result row that it feeds,
+// while the next row's is on its way.  Activation none, or ReLU or clip (`clamp`) between `lo` and `hi`, and no residual; results
+// plain fp32 or bf16 pairs.
+// What bounds it: instructions.  The tile kernel spends 250 of them on four channels of a result (18 reads of shared memory,
+// every activation and format behind a branch); here it is packed FMAs and a clamp.  By events, tile kernel -> this one:
+// 7x7x960, 256 images (96 MB) 50.8 -> 28.6 us, 56x56x144 stride 1, 128 images 202 -> 119, 14x14x384, 64 images 25 -> 16.5.
+template <int STRIDE>
+static __global__ void __launch_bounds__(256, 2) k_depthwise3x3_columns(const float* __restrict__ in, ActRef out, const float* __restrict__ weights,
+                                                                        const float* __restrict__ bias_of, ConvGeom g, int clamp, float lo, float hi,
+                                                                        int pairs, long long threads) {
+  ptx::grid_begin();
+  constexpr int IC = STRIDE + 3;
+  const long long idx = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (idx >= threads) return;
+  const int cv = g.C / 4;
+  const int rest = static_cast<int>(idx / cv);  // (image and column pair: fewer than 2^31)
+  const int c = static_cast<int>(idx - static_cast<long long>(rest) * cv) * 4;
+  const int img = rest / pairs, ox = (rest - img * pairs) * 2;
+  const int ix0 = ox * STRIDE - g.pl;
+  ulonglong2 tap[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) tap[k] = *reinterpret_cast<const ulonglong2*>(weights + k * g.C + c);
+  const ulonglong2 bias = bias_of != nullptr ? *reinterpret_cast<const ulonglong2*>(bias_of + c) : make_ulonglong2(0ull, 0ull);
+  const float* column = in + (static_cast<long long>(img) * g.H * g.W + ix0) * g.C + c;  // row 0 of the image
+  const long long row_step = static_cast<long long>(g.W) * g.C;
+  bool inside[IC];
+#pragma unroll
+  for (int j = 0; j < IC; ++j) inside[j] = ix0 + j >= 0 && ix0 + j < g.W;
+  auto load = [&](int iy, ulonglong2 (&x)[IC]) {
+    const bool row = iy >= 0 && iy < g.H;
+    const float* const p = column + iy * row_step;
+#pragma unroll
+    for (int j = 0; j < IC; ++j) x[j] = row && inside[j] ? *reinterpret_cast<const ulonglong2*>(p + j * g.C) : make_ulonglong2(0ull, 0ull);
+  };
+  auto add = [&](ulonglong2 (&sum)[2], const ulonglong2 (&x)[IC], int kh) {
+#pragma unroll
+    for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const ulonglong2 v = x[q * STRIDE + kw], k = tap[kh * 3 + kw];
+        sum[q] = make_ulonglong2(f32x2_fma3(v.x, k.x, sum[q].x), f32x2_fma3(v.y, k.y, sum[q].y));
+      }
+  };
+  long long to = (static_cast<long long>(img) * g.OH * g.OW + ox) * g.C + c;
+  const long long to_step = static_cast<long long>(g.OW) * g.C;
+  auto put = [&](const ulonglong2 (&sum)[2]) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (q == 1 && ox + 1 >= g.OW) break;
+      const float2 a = f32x2_get(sum[q].x), b = f32x2_get(sum[q].y);
+      float4 y = make_float4(a.x, a.y, b.x, b.y);
+      if (clamp) y = make_float4(fminf(fmaxf(y.x, lo), hi), fminf(fmaxf(y.y, lo), hi), fminf(fmaxf(y.z, lo), hi), fminf(fmaxf(y.w, lo), hi));
+      const long long at = to + q * g.C;
+      if (out.fmt == FMT_BF16X2) {
+        uint2 h, m;
+        split_bf16x2(y.x, y.y, h.x, m.x);
+        split_bf16x2(y.z, y.w, h.y, m.y);
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out.p0) + at) = h;
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out.p1) + at) = m;
+      } else {
+        *reinterpret_cast<float4*>(out.p0 + at) = y;
+      }
+    }
+    to += to_step;
+  };
+  ulonglong2 x[IC], next[IC];
+  load(-g.pt, x);
+  if constexpr (STRIDE == 1) {
+    ulonglong2 a[2] = {bias, bias}, b[2] = {bias, bias};
+#pragma unroll 2
+    for (int t = 0; t < g.OH + 2; ++t) {  // input row t - pt
+      load(t + 1 < g.OH + 2 ? t + 1 - g.pt : -1, next);
+      ulonglong2 done[2] = {b[0], b[1]};
+      add(done, x, 2);
+      b[0] = a[0], b[1] = a[1];
+      add(b, x, 1);
+      a[0] = a[1] = bias;
+      add(a, x, 0);
+      if (t >= 2) put(done);
+#pragma unroll
+      for (int j = 0; j < IC; ++j) x[j] = next[j];
+    }
+  } else {
+    ulonglong2 b[2] = {bias, bias};
+#pragma unroll 1
+    for (int r = 0; r <= g.OH; ++r) {  // input row 2 r - pt, the third of result row r - 1 and the first of r, and 2 r + 1 - pt
+      load(r < g.OH ? 2 * r + 1 - g.pt : -1, next);
+      ulonglong2 done[2] = {b[0], b[1]};
+      add(done, x, 2);
+      b[0] = b[1] = bias;
+      add(b, x, 0);
+      load(r < g.OH ? 2 * r + 2 - g.pt : -1, x);
+      add(b, next, 1);
+      if (r > 0) put(done);
+    }
+  }
+}
+
 // 3x3 stride-2 max pooling through the same shared-memory tile as the depthwise kernel: the
 // 17x17 input patch of an 8x8 output tile is staged once for 32 channels (cp.async for plain
 // fp32 inputs), then every thread takes the maximum over the taps that lie inside the image

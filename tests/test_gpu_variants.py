@@ -378,6 +378,43 @@ def test_inner_product_sums_alike_whatever_the_rows_of_a_tile(pkg, tmp_path, k, 
             assert np.array_equal(model.run(x[:m])[0], want[:m]), m
 
 
+@pytest.mark.parametrize("h,w,c,stride,pad,act,n", [
+    (7, 7, 960, 1, 1, "clip", 18),     # bf16 pairs for the 1x1 layer behind it
+    (7, 7, 960, 1, 1, "", 18),
+    (5, 3, 512, 1, 0, "relu", 140),    # one column of results, no padding
+    (4, 9, 512, 1, 2, "clip", 36),     # two columns and rows of zeros on each side
+    (15, 14, 512, 2, 1, "clip", 33),   # stride 2, the last column is the last of its pair
+    (8, 9, 640, 2, 0, "", 60),
+    (9, 11, 512, 2, 2, "relu", 43),
+    (1, 1, 992, 1, 1, "clip", 70),
+    (6, 5, 36, 1, 1, "relu", 612),     # channels that no tensor-core layer takes as bf16 pairs: plain results only
+])
+def test_depthwise_by_columns(pkg, oracle, tmp_path, monkeypatch, h, w, c, stride, pad, act, n):
+    """Many images take the kernel that walks down columns; few take the tile kernel: the same bits, and the oracle's values."""
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    for tail in ((False, True) if c % 32 == 0 else (False,)):
+        net = pkg.zoo._Net(31 + h)
+        net.w.layer("Input", "input", [], ["data"], f"0={w} 1={h} 2={c}")
+        top = "d" if act or tail else "output"
+        net.depthwise("dw", "data", top, c, 3, stride, pad)
+        if act:
+            top, bottom = ("a" if tail else "output"), top
+            if act == "relu":
+                net.w.layer("ReLU", "act", [bottom], [top], "0=0.0")
+            else:
+                net.w.layer("Clip", "act", [bottom], [top], "0=-0.25 1=0.75")
+        if tail:
+            net.conv("project", top, "output", c, 32, 1, 1, 0, act=0, zero_bias=False)
+        param, bin_ = net.w.save(str(tmp_path / f"m{int(tail)}"))
+        x = np.random.default_rng(h * w + c).uniform(-2, 2, (n, c, h, w)).astype(np.float32)
+        model = pkg.Model(param, bin_)
+        kinds = lambda m: [r["kernel"] for r in model.profile(m, 1) if "depthwise" in r["kernel"]]
+        assert kinds(n) == ["k_depthwise3x3_columns"] and kinds(2) == ["k_depthwise3x3_tile"]
+        got = model.run(x)[0]
+        assert np.array_equal(got[-2:], model.run(x[-2:])[0])
+        assert rel_l2(got[0], oracle.Model(param, bin_).run([x[0]])[0]) <= (1e-4 if tail else 1e-6)
+
+
 @pytest.mark.parametrize("h,w,cin", [(1, 1, 64), (1, 7, 96), (3, 3, 32), (7, 9, 64), (8, 8, 40), (5, 13, 64), (11, 11, 64), (8, 16, 64)])
 def test_lone_tile_of_few_pixels(pkg, tmp_path, monkeypatch, h, w, cin):
     """A tile that is alone brings only the rows it has (1 to 128 of them): the bits of the same image in front of others."""
