@@ -1389,6 +1389,9 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
 DwProjShape block_shape(int N, int out_mode, int res_mode, int C, int stride, int cin) {
   DwProjShape r;
   if (!dw_project_formats(out_mode, res_mode) || (stride != 1 && stride != 2)) return r;
+  // A column tile is a whole tile of the kernel, its expand and depthwise work done once more.  64 images of 56x56x96 with 160
+  // outputs, two tiles: stride 1 227 us a call, 217 as expand layer and pair; stride 2 117, 102 as three layers.
+  if (N > 128) return r;
   // two accumulators beside one buffer of each half's expanded pixels, or two where they fit
   const int pixels = blk_in_cols(stride), most = (static_cast<int>(kTcTmemCols) - 2 * pixels) / 2 / 16 * 16;
   dw_project_columns(r, N, std::min(128, most));

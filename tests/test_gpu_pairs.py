@@ -529,3 +529,51 @@ def test_int8_k_blocks_per_stage_change_no_bit(pkg, oracle, tmp_path, monkeypatc
     m.close()
     want = np.stack([oracle.Model(param, bin_).run([xi])[0] for xi in x[:2]])
     assert np.array_equal(got[:2], want)
+
+
+# ------------------------------------------------------------------ whole blocks: which of them, and their bits
+def _block(pkg, prefix, h, w, cin, hidden, cout, stride=1, pads=(1, 1, 1, 1), expand_act=(0.0, 6.0), dw_act=(0.0, 6.0), residual=None, seed=70):
+    """One inverted-residual block with any activations (None, "relu" or the bounds of a clip) and pads (top, bottom, left, right)."""
+    net = pkg.zoo._Net(seed)
+    wr = net.w
+
+    def act(kind, name, bottom, top):
+        if kind == "relu":
+            wr.layer("ReLU", name, [bottom], [top], "0=0.0")
+        elif kind is not None:
+            wr.layer("Clip", name, [bottom], [top], f"0={kind[0]} 1={kind[1]}")
+
+    residual = stride == 1 and cin == cout if residual is None else residual
+    wr.layer("Input", "input", [], ["data"], f"0={w} 1={h} 2={cin}")
+    src = "data"
+    if residual:
+        wr.layer("Split", "split", ["data"], ["x", "id"])
+        src = "x"
+    net.conv("expand", src, "e" if expand_act is not None else "ea", cin, hidden, 1, 1, 0, zero_bias=False)
+    act(expand_act, "expand_act", "e", "ea")
+    filt = net._he((hidden, 1, 3, 3), 9)
+    wr.layer("ConvolutionDepthWise", "dw", ["ea"], ["d" if dw_act is not None else "da"],
+             f"0={hidden} 1=3 3={stride} 4={pads[2]} 15={pads[3]} 14={pads[0]} 16={pads[1]} 5=1 6={filt.size} 7={hidden}")
+    wr.f32(filt, tagged=True)
+    wr.f32((net.rng.standard_normal(hidden) * 0.1).astype(np.float32))
+    act(dw_act, "dw_act", "d", "da")
+    net.conv("project", "da", "p" if residual else "output", hidden, cout, 1, 1, 0, zero_bias=False)
+    if residual:
+        wr.layer("Eltwise", "add", ["p", "id"], ["output"], "0=1")
+    return wr.save(prefix)
+
+
+def _layers(kernels):
+    """The kernels between the conversions of the caller's arrays."""
+    return [k for k in kernels if not k.startswith(("k_chw_to_nhwc", "k_nhwc_to_chw"))]
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_blocks_of_more_than_128_outputs_are_not_whole(pkg, oracle, tmp_path, stride):
+    """A column tile repeats the expand layer and the depthwise filter: a projection past one tile stays with its pair or alone."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), 24, 16, 32, 96, 136, stride)
+    x = np.random.default_rng(stride).uniform(-2, 2, (3, 32, 24, 16)).astype(np.float32)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert not any("expand" in k for k in kernels), kernels
+    assert len(_layers(kernels)) == (2 if stride == 1 else 3) and (stride == 2 or "tc_dw_project_kernel<bf16x3>" in kernels), kernels
+    assert rel_l2(got, np.stack([oracle.Model(param, bin_).run([xi])[0] for xi in x])) <= 1e-4
