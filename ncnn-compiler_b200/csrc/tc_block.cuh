@@ -205,12 +205,12 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
   const uint32_t a_base = e_base + 2u * e_plane;
   const uint32_t b_bytes = static_cast<uint32_t>(p.b_bytes);
   const uint32_t b_base = a_base + slots * 2u * kAPlane;
-  const uint32_t drain = b_base + static_cast<uint32_t>(p.tiles_n * c_blocks) * 2u * b_bytes;
+  const uint32_t drain = b_base + static_cast<uint32_t>(c_blocks) * 2u * b_bytes;
   const uint32_t table = drain + static_cast<uint32_t>(TH * TW / 32) * kDrainWarpBytes;
-  // TMEM columns: the projection's two accumulators, then the halves' expanded pixels
+  // TMEM columns: the projection's accumulators, then the halves' expanded pixels
   const uint32_t acc_stride = static_cast<uint32_t>(p.block_n);
-  const uint32_t e_col0 = 2u * acc_stride;
-  const int total_tiles = p.images * p.tiles_y * p.tiles_x * p.tiles_n;
+  const uint32_t e_col0 = static_cast<uint32_t>(p.accs) * acc_stride;
+  const int total_tiles = p.images * p.tiles_y * p.tiles_x;
   volatile int* abort_ptr = &abort_flag;
 
   if (threadIdx.x == 0) {
@@ -260,16 +260,14 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
     if (elect_one() && static_cast<int>(blockIdx.x) < total_tiles) {
       const uint32_t wb = smem_u32(&w_full);
       const uint32_t e_tx = 2u * kDwpChannels * x_row, b_tx = 2u * static_cast<uint32_t>(p.block_n) * 64u;
-      mbar_arrive_expect_tx(wb, static_cast<uint32_t>(c_blocks) * (e_tx + static_cast<uint32_t>(p.tiles_n) * b_tx));
+      mbar_arrive_expect_tx(wb, static_cast<uint32_t>(c_blocks) * (e_tx + b_tx));
       for (int cb = 0; cb < c_blocks; ++cb) {
         const uint32_t e_at = e_base + static_cast<uint32_t>(cb * kDwpChannels) * x_row;
         tma_load_2d(e_at, &map_e0, wb, 0, cb * kDwpChannels);
         tma_load_2d(e_at + e_plane, &map_e1, wb, 0, cb * kDwpChannels);
-        for (int nb = 0; nb < p.tiles_n; ++nb) {
-          const uint32_t b_at = b_base + static_cast<uint32_t>(nb * c_blocks + cb) * 2u * b_bytes;
-          tma_load_2d(b_at, &map_b0, wb, cb * kDwpChannels, nb * p.block_n);
-          tma_load_2d(b_at + b_bytes, &map_b1, wb, cb * kDwpChannels, nb * p.block_n);
-        }
+        const uint32_t b_at = b_base + static_cast<uint32_t>(cb) * 2u * b_bytes;
+        tma_load_2d(b_at, &map_b0, wb, cb * kDwpChannels, 0);
+        tma_load_2d(b_at + b_bytes, &map_b1, wb, cb * kDwpChannels, 0);
       }
       grid_dependency_wait();
       const uint32_t x_tx = 2u * static_cast<uint32_t>(NPX) * x_row;
@@ -360,8 +358,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
         return true;
       };
       for (int i = 0; i < NB && ok; ++i) ok = issue_expand();
-      int acc = 0, n_blk = static_cast<int>(blockIdx.x) % p.tiles_n;
-      const int n_step = static_cast<int>(gridDim.x) % p.tiles_n;
+      int acc = 0;
       uint32_t acc_ph = 0, item = 0;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         if (!mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
@@ -385,7 +382,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
             }
             tc_fence_after_sync();
             const uint64_t a0 = a_first + static_cast<uint64_t>(slot * 2u * (kAPlane >> 4));
-            const uint64_t b0 = fixed_b + (((b_base + static_cast<uint32_t>(n_blk * c_blocks + cb) * 2u * b_bytes) & 0x3ffffu) >> 4);
+            const uint64_t b0 = fixed_b + (((b_base + static_cast<uint32_t>(cb) * 2u * b_bytes) & 0x3ffffu) >> 4);
             const uint64_t b1 = b0 + (b_bytes >> 4);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {  // two K steps of 16 channels: 2 KB of A, 32 bytes of a row of B
@@ -401,10 +398,8 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
         }
         if (!ok) break;
         tc_commit(smem_u32(&tfull_bar[acc]));
-        acc ^= 1;
+        if (p.accs == 2) acc ^= 1;
         if (acc == 0) acc_ph ^= 1u;
-        n_blk += n_step;
-        if (n_blk >= p.tiles_n) n_blk -= p.tiles_n;
       }
       if (!ok) {
         if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_MMA);

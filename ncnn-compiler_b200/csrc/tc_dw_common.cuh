@@ -35,6 +35,7 @@ struct TcDwProjParams {
                             // (16 channels) when the block's input has no more: two patch buffers then fit where one did
   int x_plane_bytes;        // one bf16 plane of an input patch buffer, rounded to 1 KB
   int x_bufs;               // input patch buffers: 2, or 1 when two do not fit
+  int accs;                 // accumulators of the projection: 2, or 1 when a second does not fit beside the expanded pixels
   int e_bufs;               // TMEM buffers of each half's expanded pixels: 2, or 1
   int a_slots;              // operand tiles: 8, or 4
   int ex_ksteps;            // K steps of 16 input channels the expand MMAs run: ceil(Cin / 16)
@@ -82,7 +83,8 @@ struct DwpWalk {
 };
 
 // Four epilogue warps (`quarter`: the TMEM lanes of this one) drain the projection's accumulators.  GROUPS = 2: two such groups
-// take alternate tiles, an accumulator each.  `drain`: kDrainWarpBytes for each warp of the group that has rows.
+// take alternate tiles, an accumulator each; GROUPS = 1: p.accs accumulators in turn.  `drain`: kDrainWarpBytes for each warp of
+// the group that has rows.
 template <int KIND, int STRIDE, int EPI, int GROUPS>
 __device__ __forceinline__ void dwp_epilogue(const TcDwProjParams& p, int group, int quarter, uint32_t drain, uint32_t tmem_base,
                                              uint32_t acc_stride, int total_tiles, uint64_t* tfull_bar, uint64_t* tempty_bar,
@@ -133,7 +135,7 @@ __device__ __forceinline__ void dwp_epilogue(const TcDwProjParams& p, int group,
     tc_fence_before_sync();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
-    if (GROUPS == 1) acc ^= 1;
+    if (GROUPS == 1 && lp.accs == 2) acc ^= 1;
     if (GROUPS == 2 || acc == 0) acc_ph ^= 1u;
   }
   if (!ok && lane == 0) {

@@ -1340,13 +1340,13 @@ cudaError_t tc_launch_conv_i8(const TcConvI8Launch& L, cudaStream_t stream) {
 namespace {
 
 struct DwProjShape {
-  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, e_bufs = 0, a_slots = 0, smem = 0;
+  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, accs = 2, e_bufs = 0, a_slots = 0, smem = 0;
   bool ok = false;
 };
 bool dw_project_formats(int out_mode, int res_mode) { return (out_mode == OUT_BF16X2 || out_mode == OUT_F32) && res_mode != RES_SPLIT; }
-// columns of a tile: N in as few tiles of at most `most` as it takes, all alike
-void dw_project_columns(DwProjShape& r, int N, int most) {
-  const int n_tiles = (N + most - 1) / most;
+// columns of a tile: N in as few tiles of at most 256 as it takes, all alike
+void dw_project_columns(DwProjShape& r, int N) {
+  const int n_tiles = (N + 255) / 256;
   r.block_n = ((N + n_tiles - 1) / n_tiles + 15) / 16 * 16;
   r.tiles_n = (N + r.block_n - 1) / r.block_n;
   r.b_bytes = (r.block_n * 64 + 1023) / 1024 * 1024;
@@ -1356,7 +1356,7 @@ void dw_project_columns(DwProjShape& r, int N, int most) {
 DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
   DwProjShape r;
   if (!dw_project_formats(out_mode, res_mode)) return r;
-  dw_project_columns(r, N, 256);
+  dw_project_columns(r, N);
   const int c_pad = (C + kDwpChannels - 1) / kDwpChannels * kDwpChannels;
   const int table = (c_pad * 10 * 4 + 1023) / 1024 * 1024;  // depthwise filter and bias
   const int stage = 2 * r.b_bytes;
@@ -1389,17 +1389,19 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
 DwProjShape block_shape(int N, int out_mode, int res_mode, int C, int stride, int cin) {
   DwProjShape r;
   if (!dw_project_formats(out_mode, res_mode) || (stride != 1 && stride != 2)) return r;
-  // A column tile is a whole tile of the kernel, its expand and depthwise work done once more.  64 images of 56x56x96 with 160
-  // outputs, two tiles: stride 1 227 us a call, 217 as expand layer and pair; stride 2 117, 102 as three layers.
+  // One column tile: a second is a whole tile of the kernel, its expand and depthwise work done once more.  64 images of
+  // 56x56x96 with 160 outputs in two: stride 1 227 us a call, 217 as expand layer and pair; stride 2 117, 102 as three layers.
   if (N > 128) return r;
-  // two accumulators beside one buffer of each half's expanded pixels, or two where they fit
-  const int pixels = blk_in_cols(stride), most = (static_cast<int>(kTcTmemCols) - 2 * pixels) / 2 / 16 * 16;
-  dw_project_columns(r, N, std::min(128, most));
-  r.e_bufs = 2 * r.block_n + 4 * pixels <= static_cast<int>(kTcTmemCols) ? 2 : 1;
+  dw_project_columns(r, N);
+  // Two accumulators beside one buffer of each half's expanded pixels, or two where they fit; past 96 columns at stride 2 one
+  // accumulator (56x56x144 -> 128, 64 images: a call takes 108 us, 131 with two accumulators and two column tiles).
+  const int pixels = blk_in_cols(stride), columns = static_cast<int>(kTcTmemCols);
+  r.accs = 2 * r.block_n + 2 * pixels <= columns ? 2 : 1;
+  r.e_bufs = 2 * r.block_n + 4 * pixels <= columns ? 2 : 1;
   r.x_row_bytes = cin <= 16 ? 32 : 64;
   r.x_plane_bytes = (dwp_patch_pixels(stride) * r.x_row_bytes + 1023) / 1024 * 1024;
   const int c_blocks = (C + kDwpChannels - 1) / kDwpChannels, c_pad = c_blocks * kDwpChannels;
-  const int weights = 2 * c_pad * r.x_row_bytes + r.tiles_n * c_blocks * 2 * r.b_bytes;
+  const int weights = 2 * c_pad * r.x_row_bytes + c_blocks * 2 * r.b_bytes;
   const int table = (kBlkTableRows * c_pad * 4 + 1023) / 1024 * 1024;
   const int fixed = weights + table + dwp_tile_h(stride) * kDwpTileW / 32 * kDrainWarpBytes;
   for (int slots : {8, 4})
@@ -1490,6 +1492,7 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   p.x_plane_bytes = shape.x_plane_bytes;
   p.x_row_bytes = shape.x_row_bytes;
   p.x_bufs = shape.x_bufs;
+  p.accs = shape.accs;
   p.e_bufs = shape.e_bufs;
   p.a_slots = shape.a_slots;
   p.ex_ksteps = expand ? (shape.x_row_bytes == 32 ? 1 : (c.Cin + 15) / 16) : 0;

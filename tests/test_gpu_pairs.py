@@ -577,3 +577,20 @@ def test_blocks_of_more_than_128_outputs_are_not_whole(pkg, oracle, tmp_path, st
     assert not any("expand" in k for k in kernels), kernels
     assert len(_layers(kernels)) == (2 if stride == 1 else 3) and (stride == 2 or "tc_dw_project_kernel<bf16x3>" in kernels), kernels
     assert rel_l2(got, np.stack([oracle.Model(param, bin_).run([xi])[0] for xi in x])) <= 1e-4
+
+
+@pytest.mark.parametrize("cin,hidden,cout,n", [
+    (24, 144, 128, 24),  # five blocks of 32 channels: sets of 4 and 1, three tiles to a CTA
+    (8, 32, 104, 40),    # a tile is one block: the accumulator changes hands with every item
+    (32, 96, 96, 24),    # the widest that still has two accumulators
+    (16, 96, 112, 3),
+])
+def test_whole_blocks_with_one_accumulator(pkg, tmp_path, monkeypatch, cin, hidden, cout, n):
+    """Past 96 outputs at stride 2 tensor memory has room for one accumulator: the bits of the three layers apart all the same."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), 61, 67, cin, hidden, cout, 2)
+    x = np.random.default_rng(cout).uniform(-2, 2, (n, cin, 61, 67)).astype(np.float32)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert _layers(kernels) == ["tc_dw_project_kernel:expand+stride2<bf16x3>"], kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, plain = _run(pkg, param, bin_, x)
+    assert len(_layers(plain)) == 3 and np.array_equal(got, base)
