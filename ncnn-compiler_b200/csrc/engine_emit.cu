@@ -602,13 +602,22 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         const float* wf = static_cast<const float*>(w);
         const int pairs = (node.OW + 1) / 2;
         const long long threads = n * pairs * (ti.c / 4);
-        // A thread of the columns kernel walks OH rows one after the other (0.6 to 0.8 us each), so it needs enough of them.
-        // By events, tile / columns in us, around the line: 14x14x384 10 700 threads 12.7 / 14.3, 21 500 17.0 / 14.4;
-        // 28x28x192 10 700 16.4 / 18.6, 21 500 24.9 / 20.5; 112 -> 56x56x96 21 500 53 / 68, 43 000 96 / 86; 112x112x32
-        // 28 700 85 / 90, 57 300 160 / 107; 80 -> 40x40x144 23 000 47 / 52, 46 000 84 / 66.
+        // A thread of the columns kernel walks OH rows one after the other, so it needs enough threads, and more the longer the
+        // walk.  At stride 2, whose rows come from memory twice as fast, it is only a little faster than the tile kernel when
+        // the last of its waves of 2 blocks an SM is full, and slower when that is not.  Whole calls of expand layer,
+        // depthwise layer and projection, tile / columns in us (the launch alone, its input in L2, flatters columns):
+        //   stride 1: 14x14x384  9 000 threads 24.6 / 30.7, 16 800 30.7 / 30.7, 24 200 34.8 / 32.8; 32x32x384 16 900 41.0 / 45.1,
+        //             24 600 49.2 / 47.1; 56x56x384 24 200 73.7 / 73.8, 37 600 108 / 98, 250 000 604 / 471
+        //   stride 2: 28 -> 14x14x384 16 800 43.0 / 45.1, 24 200 51.2 / 49.2; 56 -> 28x28x384 24 200 79.9 / 102, 75 300 (a wave)
+        //             212 / 194, 90 000 253 / 267; 64 -> 32x32x384 16 900 67.5 / 94.2, 75 300 229 / 219, 119 800 352 / 358;
+        //             112 -> 56x56x96 49 700 358 / 385, 75 300 531 / 527
+        const long long wave = 2ll * sm_count_ * 256, waves = (threads + wave - 1) / wave;
+        const bool enough = node.sh == 1       ? threads >= 16384 + 250 * std::max(0, node.OH - 8)
+                            : node.OH <= 16 ? threads >= 16384 + 1024 * std::max(0, node.OH - 8)
+                                            : threads * 100 >= waves * wave * (node.OH <= 28 ? 72 : 88);
         const int clamp = node.act == ACT_RELU || node.act == ACT_CLIP ? 1 : 0;
         const bool columns = in.fmt == FMT_F32 && (out.fmt == FMT_F32 || out.fmt == FMT_BF16X2) && (clamp || node.act == ACT_NONE) && !e.has_res &&
-                             threads >= (node.OH <= 32 ? 16384 : 40960) && n * pairs <= 0x7fffffffll && (threads + 255) / 256 <= 0x7fffffffll;
+                             enough && n * pairs <= 0x7fffffffll && (threads + 255) / 256 <= 0x7fffffffll;
         const float lo = node.act == ACT_CLIP ? e.act_a : 0.0f, hi = node.act == ACT_CLIP ? e.act_b : INFINITY;
         const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
         s.kernel = columns ? "k_depthwise3x3_columns" : "k_depthwise3x3_tile";

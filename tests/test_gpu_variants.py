@@ -675,3 +675,24 @@ def test_one_launch_under_the_callers_capture(pkg, tmp_path, int8):
         other = torch.zeros(2048, device="cuda")
         model.run_device(1, [source[i].data_ptr()], [other.data_ptr()], torch.cuda.current_stream().cuda_stream)
         assert np.array_equal(other.cpu().numpy(), want[i])
+
+
+@pytest.mark.parametrize("h,c,stride,n,kernel", [
+    (32, 96, 1, 44, "tile"),       # 16 896 threads of the columns kernel with 32 rows each
+    (32, 96, 1, 64, "columns"),    # 24 576
+    (56, 96, 2, 71, "tile"),       # a third of a wave at stride 2
+    (56, 96, 2, 223, "columns"),   # 0.99 of one
+    (56, 96, 2, 250, "tile"),      # one and a ninth
+    (28, 96, 2, 143, "columns"),   # short walks: as at stride 1
+])
+def test_depthwise_columns_where_they_are_faster(pkg, oracle, tmp_path, monkeypatch, h, c, stride, n, kernel):
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    net = pkg.zoo._Net(7)
+    net.w.layer("Input", "input", [], ["data"], f"0={h} 1={h} 2={c}")
+    net.depthwise("dw", "data", "output", c, 3, stride, 1)
+    param, bin_ = net.w.save(str(tmp_path / "m"))
+    x = np.random.default_rng(n).uniform(-2, 2, (n, c, h, h)).astype(np.float32)
+    model = pkg.Model(param, bin_)
+    assert [r["kernel"] for r in model.profile(n, 1) if "depthwise" in r["kernel"]] == ["k_depthwise3x3_" + kernel]
+    got = model.run(x)[0]
+    assert rel_l2(got[-1], oracle.Model(param, bin_).run([x[-1]])[0]) <= 1e-6
