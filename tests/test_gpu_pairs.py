@@ -594,3 +594,15 @@ def test_whole_blocks_with_one_accumulator(pkg, tmp_path, monkeypatch, cin, hidd
     monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
     base, plain = _run(pkg, param, bin_, x)
     assert len(_layers(plain)) == 3 and np.array_equal(got, base)
+
+
+@pytest.mark.parametrize("cin,cout,stride,n", [(32, 48, 2, 50), (8, 24, 2, 53), (16, 16, 1, 25), (8, 64, 1, 26)])
+def test_whole_blocks_of_one_channel_block(pkg, tmp_path, monkeypatch, cin, cout, stride, n):
+    """A tile is one item, its halves in quarters two apart; a CTA walks through more items than there are operand tiles."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), 59, 61, cin, 32, cout, stride)
+    x = np.random.default_rng(cout).uniform(-2, 2, (n, cin, 59, 61)).astype(np.float32)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert len(_layers(kernels)) == 1 and "expand" in _layers(kernels)[0], kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, plain = _run(pkg, param, bin_, x)
+    assert len(_layers(plain)) >= 3 and np.array_equal(got, base)
