@@ -410,7 +410,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
     }
   } else if (warp >= 4 && warp < 8) {
     // ------------------------------------------------------------ epilogue
-    dwp_epilogue<GEMM_BF16X3, STRIDE, EPI, 1>(p, 0, warp & 3, drain, tmem_base, acc_stride, total_tiles, tfull_bar, tempty_bar, abort_ptr);
+    dwp_epilogue<GEMM_BF16X3, STRIDE, EPI>(p, 1, 0, warp & 3, drain, tmem_base, acc_stride, total_tiles, tfull_bar, tempty_bar, abort_ptr);
   } else if (warp >= 8) {
     // ------------------------------------------------------------ depthwise
     const int q = warp & 3, h = (warp - 8) >> 2;

@@ -22,6 +22,7 @@ struct TcDwProjParams {
   int c_blocks;         // blocks of 32 channels (the last one may be partly past C: zero-filled)
   int pad_t, pad_l;
   int stages;           // weight ring depth
+  int drain_groups;     // groups of four epilogue warps in the pair: 2, or 1
   int patch_bufs;       // input patch ring depth, 2 or 4 (even: a slot then always serves the same depthwise group)
   int b_bytes;          // one plane of a weight stage, rounded to 1 KB
   int wide;             // rows of result and residual are multiples of 32 bytes, 32-byte aligned
@@ -82,11 +83,11 @@ struct DwpWalk {
   }
 };
 
-// Four epilogue warps (`quarter`: the TMEM lanes of this one) drain the projection's accumulators.  GROUPS = 2: two such groups
-// take alternate tiles, an accumulator each; GROUPS = 1: p.accs accumulators in turn.  `drain`: kDrainWarpBytes for each warp of
-// the group that has rows.
-template <int KIND, int STRIDE, int EPI, int GROUPS>
-__device__ __forceinline__ void dwp_epilogue(const TcDwProjParams& p, int group, int quarter, uint32_t drain, uint32_t tmem_base,
+// Four epilogue warps (`quarter`: the TMEM lanes of this one) drain the projection's accumulators.  Two such groups take
+// alternate tiles, an accumulator each; one takes p.accs accumulators in turn.  `drain`: kDrainWarpBytes for each warp of the
+// group that has rows.
+template <int KIND, int STRIDE, int EPI>
+__device__ __forceinline__ void dwp_epilogue(const TcDwProjParams& p, int groups, int group, int quarter, uint32_t drain, uint32_t tmem_base,
                                              uint32_t acc_stride, int total_tiles, uint64_t* tfull_bar, uint64_t* tempty_bar,
                                              volatile int* abort_ptr) {
   using namespace ptx;
@@ -102,11 +103,11 @@ __device__ __forceinline__ void dwp_epilogue(const TcDwProjParams& p, int group,
   d.wide = p.wide;
   const bool has_rows = quarter * 32 < TH * TW;  // (of a stride-2 tile only the first 64 rows are pixels)
   d.stage = drain + static_cast<uint32_t>(quarter) * kDrainWarpBytes;
-  int acc = GROUPS == 2 ? group : 0;
+  int acc = group;
   uint32_t acc_ph = 0;
   bool ok = true;
-  DwpWalk w(p, static_cast<int>(blockIdx.x + group * gridDim.x), static_cast<int>(GROUPS * gridDim.x));
-  for (int tile = blockIdx.x + group * gridDim.x; tile < total_tiles && ok; tile += GROUPS * gridDim.x, w.on(p)) {
+  DwpWalk w(p, static_cast<int>(blockIdx.x + group * gridDim.x), static_cast<int>(groups * gridDim.x));
+  for (int tile = blockIdx.x + group * gridDim.x; tile < total_tiles && ok; tile += groups * gridDim.x, w.on(p)) {
     const int oy0 = w.y * TH, ox0 = w.x * TW, n0 = w.n * p.block_n;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc) * acc_stride;
     const int oy = oy0 + (row >> 3), ox = ox0 + (row & 7);
@@ -135,8 +136,8 @@ __device__ __forceinline__ void dwp_epilogue(const TcDwProjParams& p, int group,
     tc_fence_before_sync();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
-    if (GROUPS == 1 && lp.accs == 2) acc ^= 1;
-    if (GROUPS == 2 || acc == 0) acc_ph ^= 1u;
+    if (groups == 1 && lp.accs == 2) acc ^= 1;
+    if (groups == 2 || acc == 0) acc_ph ^= 1u;
   }
   if (!ok && lane == 0) {
     if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_EPILOGUE);

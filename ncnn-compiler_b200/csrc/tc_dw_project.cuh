@@ -17,7 +17,7 @@
 // and the usual epilogue warps drain the accumulator (bias, residual, activation).
 // The operands, their order and the accumulation are those of the two separate kernels, so the results are the same bits.
 //
-// Warps (640 threads): 0 TMA producer, 1 MMA issuer, 4-11 epilogue (two groups on alternate tiles), 12-19 depthwise; registers
+// Warps (640 threads): 0 TMA producer, 1 MMA issuer, 4-11 epilogue (two groups on alternate tiles, or the first alone), 12-19 depthwise; registers
 // are split between the roles.  Every wait is bounded and ends in the status word.
 //
 // What bounds it: shared memory (~800 of a block's ~1 700 clocks are its own reads and writes, ~250 the MMAs') and the
@@ -70,7 +70,7 @@ __device__ __forceinline__ void dwp_pair_body(const TcDwProjParams& p, const CUt
   const int S = p.stages;
   // the depthwise filter and bias of every channel, [10][c_blocks * 32] fp32 (taps 0..8, then the bias; zero past C)
   const uint32_t drain = b_base + static_cast<uint32_t>(S) * b_stage_bytes;  // one block per epilogue warp
-  const uint32_t table = drain + 8u * kDrainWarpBytes;
+  const uint32_t table = drain + static_cast<uint32_t>(4 * p.drain_groups) * kDrainWarpBytes;
   const int c_pad = p.c_blocks * kDwpChannels;
   const uint32_t acc_stride = p.block_n > 128 ? 256u : 128u;  // TMEM columns of an accumulator
   const int tiles_per_image = p.tiles_y * p.tiles_x;
@@ -241,10 +241,11 @@ __device__ __forceinline__ void dwp_pair_body(const TcDwProjParams& p, const CUt
     }  // (warps 2 and 3 have no role: registers are split between whole warpgroups)
   } else if (warp < 12) {
     // ------------------------------------------------------------ epilogue (warps 4-11)
-    // two groups of four warps on alternate tiles, an accumulator each
+    // two groups of four warps on alternate tiles, an accumulator each; or one, where the second's shared memory is the rings'
     const int group = (warp - 4) >> 2;
-    dwp_epilogue<KIND, 1, EPI, 2>(p, group, warp & 3, drain + static_cast<uint32_t>(group) * 4u * kDrainWarpBytes, tmem_base, acc_stride, total_tiles,
-                                  tfull_bar, tempty_bar, abort_ptr);
+    if (group < p.drain_groups)
+      dwp_epilogue<KIND, 1, EPI>(p, p.drain_groups, group, warp & 3, drain + static_cast<uint32_t>(group) * 4u * kDrainWarpBytes, tmem_base,
+                                 acc_stride, total_tiles, tfull_bar, tempty_bar, abort_ptr);
   } else {
     // ------------------------------------------------------------ depthwise (warps 12-19, 256 threads)
     // Two groups of four warps take alternate channel blocks (group g: blocks g, g+2, ... of the CTA's sequence,

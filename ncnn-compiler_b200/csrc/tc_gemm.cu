@@ -1340,7 +1340,8 @@ cudaError_t tc_launch_conv_i8(const TcConvI8Launch& L, cudaStream_t stream) {
 namespace {
 
 struct DwProjShape {
-  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, accs = 2, e_bufs = 0, a_slots = 0, smem = 0;
+  int block_n = 0, tiles_n = 0, stages = 0, patches = 0, drain_groups = 0, b_bytes = 0, x_plane_bytes = 0, x_row_bytes = 64, x_bufs = 0, accs = 2, e_bufs = 0;
+  int a_slots = 0, smem = 0;
   bool ok = false;
 };
 bool dw_project_formats(int out_mode, int res_mode) { return (out_mode == OUT_BF16X2 || out_mode == OUT_F32) && res_mode != RES_SPLIT; }
@@ -1352,11 +1353,12 @@ void dw_project_columns(DwProjShape& r, int N) {
   r.b_bytes = (r.block_n * 64 + 1023) / 1024 * 1024;
 }
 
-// Shared-memory plan of the pair.
-DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
+// Shared-memory plan of the pair with one or two groups of epilogue warps.
+DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int drain_groups) {
   DwProjShape r;
   if (!dw_project_formats(out_mode, res_mode)) return r;
   dw_project_columns(r, N);
+  r.drain_groups = drain_groups;
   const int c_pad = (C + kDwpChannels - 1) / kDwpChannels * kDwpChannels;
   const int table = (c_pad * 10 * 4 + 1023) / 1024 * 1024;  // depthwise filter and bias
   const int stage = 2 * r.b_bytes;
@@ -1369,7 +1371,7 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
     // phase from the one two before it: a load delayed past a whole block's arithmetic let a group read a stale
     // patch, about once in 10^5 loads with the L2 flushed)
     for (int patches : {4, 2}) {
-      const int fixed = patches * kDwpPatchBytes + 2 * 2 * kDwpAPlaneBytes + 8 * kDrainWarpBytes + table;
+      const int fixed = patches * kDwpPatchBytes + 2 * 2 * kDwpAPlaneBytes + drain_groups * 4 * kDrainWarpBytes + table;
       const int stages = std::min(kDwpMaxStages, (kTcSmemBudget - fixed) / stage);
       if (stages >= min_stages) {
         r.stages = stages;
@@ -1381,6 +1383,16 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
     }
   }
   return r;
+}
+
+// The second group only where its 16 KB cost no patch and none of three weight stages.  Calls of 48x48x672 -> 112, 35 images:
+// four patches and one group 326 us, two and two 333; 16x16x1152 -> 96, 137 images 238, 244.  Where both leave the same rings the
+// second group wins on short chains: 84x84x96 -> 320, 9 images 141, 129.  What has no room for two groups even with two patches
+// and two stages is no pair: 1344 -> 256 takes 145 (14x14, 64 images), 489 (256) and 469 us (28x28, 64) as one, 135, 490 and 469
+// as two launches.
+DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
+  const DwProjShape one = dw_project_shape(N, out_mode, res_mode, C, 1), two = dw_project_shape(N, out_mode, res_mode, C, 2);
+  return !two.ok || (two.patches == one.patches && std::min(two.stages, 3) == std::min(one.stages, 3)) ? two : one;
 }
 
 // Shared and tensor memory plan of the whole block: all weights stay, so a block with too many of them for that is not taken.
@@ -1482,6 +1494,7 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   p.pad_l = c.pad_l;
   p.stages = shape.stages;
   p.patch_bufs = shape.patches;
+  p.drain_groups = shape.drain_groups;
   p.b_bytes = shape.b_bytes;
   p.dw_weights = c.dw_weights;
   p.dw_bias = c.dw_bias;

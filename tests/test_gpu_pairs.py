@@ -606,3 +606,26 @@ def test_whole_blocks_of_one_channel_block(pkg, tmp_path, monkeypatch, cin, cout
     monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
     base, plain = _run(pkg, param, bin_, x)
     assert len(_layers(plain)) >= 3 and np.array_equal(got, base)
+
+
+@pytest.mark.parametrize("h,c,cout,n", [
+    (16, 672, 112, 40),   # one epilogue group and four patches
+    (16, 768, 256, 40),   # one, three weight stages
+    (16, 96, 256, 160),   # two groups, several tiles to a CTA
+    (16, 1344, 128, 40),  # one, 42 blocks of channels
+])
+def test_pairs_with_one_and_two_epilogue_groups(pkg, tmp_path, monkeypatch, h, c, cout, n):
+    """A second group of epilogue warps only where its shared memory costs the rings nothing: the bits of the layers apart."""
+    net = pkg.zoo._Net(17)
+    net.w.layer("Input", "input", [], ["data"], f"0={h} 1={h} 2={c}")
+    net.depthwise("dw", "data", "d", c, 3, 1, 1)
+    net.w.layer("Clip", "relu6", ["d"], ["d6"], "0=0.0 1=6.0")
+    net.conv("project", "d6", "output", c, cout, 1, 1, 0, act=0, zero_bias=False)
+    param, bin_ = net.w.save(str(tmp_path / "p"))
+    x = np.random.default_rng(c).uniform(-3, 3, (n, c, h, h)).astype(np.float32)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert _layers(kernels) == ["tc_dw_project_kernel<bf16x3>"], kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, plain = _run(pkg, param, bin_, x)
+    assert len(_layers(plain)) == 2
+    assert np.array_equal(got, base)
