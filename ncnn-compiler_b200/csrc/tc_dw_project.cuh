@@ -32,7 +32,8 @@
 namespace nb {
 
 constexpr int kDwpThreads = 640;
-// registers a thread: at launch, of the issuing warpgroup, of the two epilogue groups and of the two depthwise groups
+// registers a thread: at launch (what the compiler gives 640 threads of one block; checked where a launch is planned), of the issuing
+// warpgroup, of the two epilogue groups and of the two depthwise groups
 constexpr int kDwpRegs = 96, kDwpIssueRegs = 56, kDwpDrainRegs = 96, kDwpFilterRegs = 112;
 static_assert(kDwpIssueRegs + 2 * kDwpDrainRegs + 2 * kDwpFilterRegs <= 5 * kDwpRegs, "what the launch gives the block");
 constexpr int kDwpMaxStages = 4;

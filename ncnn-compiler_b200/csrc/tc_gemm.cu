@@ -1436,6 +1436,24 @@ bool dw_project_fills(int H, int W, int stride) {
   return env_int("NCNN_B200_FUSE_DW", 1) >= 2 || static_cast<long long>(H) * W * 10 >= 6ll * tiles * th * kDwpTileW;
 }
 
+// The pair splits its registers between its roles (setmaxnreg): with fewer at launch than the split counts on, the depthwise warps
+// would wait for registers that nobody gives back, in an instruction that no time limit covers.
+std::string pair_registers(int out_mode, bool res) {
+  int regs = 0;
+  const cudaError_t e = with_form<GEMM_BF16X3, false>(out_mode, res, [&](auto form) {
+    cudaFuncAttributes a;
+    const cudaError_t q = cudaFuncGetAttributes(&a, tc_dw_project_kernel<GEMM_BF16X3, 1, false, decltype(form)::value>);
+    regs = q == cudaSuccess ? a.numRegs : 0;
+    return q;
+  });
+  if (e != cudaSuccess) return std::string("attributes of the fused depthwise + projection kernel: ") + cudaGetErrorString(e);
+  regs = env_int("NCNN_B200_TEST_PAIR_REGS", regs);  // (as if compiled for so many)
+  if (regs != kDwpRegs)
+    return "the fused depthwise + projection kernel was compiled for " + std::to_string(regs) + " registers a thread, its roles share " +
+           std::to_string(kDwpRegs);
+  return "";
+}
+
 }  // namespace
 
 bool tc_dw_project_applies(int C, int N, int H, int W, int out_mode, bool has_res, bool res_bf16) {
@@ -1473,6 +1491,8 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
                                    : (stride == 1 ? dw_project_shape(c.out_channels, e.out_mode, res_mode, c.C) : DwProjShape{});
   if (!shape.ok) return "the fused depthwise + projection kernel does not take this output format, width or stride";
   if (e.ldo != c.out_channels) return "the fused depthwise + projection kernel writes dense channel-last rows";
+  std::string err = expand ? std::string() : pair_registers(e.out_mode, res_mode != RES_NONE);
+  if (!err.empty()) return err;
   const int x_channels = expand ? c.Cin : c.C;
   if ((reinterpret_cast<uintptr_t>(c.x) & 15) != 0 || (static_cast<size_t>(x_channels) * (expand ? 2 : 4)) % 16 != 0 ||
       (expand && (c.x1 == nullptr || (reinterpret_cast<uintptr_t>(c.x1) & 15) != 0)))
@@ -1536,7 +1556,7 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   const uint32_t x_box = expand ? static_cast<uint32_t>(shape.x_row_bytes / 2) : kDwpChannels;
   const CUtensorMapSwizzle x_swizzle = !expand ? CU_TENSOR_MAP_SWIZZLE_NONE
                                                : (shape.x_row_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B);
-  std::string err = encode_tiled_4d(&L->map_x, expand, c.x, x_channels, c.Win, c.Hin, c.images, x_box, dwp_patch_w(stride),
+  err = encode_tiled_4d(&L->map_x, expand, c.x, x_channels, c.Win, c.Hin, c.images, x_box, dwp_patch_w(stride),
                                     dwp_patch_h(stride), x_swizzle);
   if (err.empty() && expand)
     err = encode_tiled_4d(&L->map_x1, true, c.x1, x_channels, c.Win, c.Hin, c.images, x_box, dwp_patch_w(stride),

@@ -629,3 +629,20 @@ def test_pairs_with_one_and_two_epilogue_groups(pkg, tmp_path, monkeypatch, h, c
     base, plain = _run(pkg, param, bin_, x)
     assert len(_layers(plain)) == 2
     assert np.array_equal(got, base)
+
+
+def test_pair_compiled_for_other_registers_is_an_error(pkg, tmp_path, monkeypatch):
+    """The pair's roles share the registers it is launched with.  A kernel compiled for fewer is refused before it is launched
+    (its warps would wait for registers without a limit); the environment variable stands for such a kernel."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), 16, 16, 64, 96, 24)
+    x = np.random.default_rng(1).uniform(-2, 2, (2, 64, 16, 16)).astype(np.float32)
+    good, kernels = _run(pkg, param, bin_, x)
+    assert "tc_dw_project_kernel<bf16x3>" in kernels, kernels
+    monkeypatch.setenv("NCNN_B200_TEST_PAIR_REGS", "88")
+    m = pkg.Model(param, bin_)
+    with pytest.raises(pkg.NcnnB200Error) as err:
+        m.run(x)
+    assert "88 registers" in str(err.value)
+    monkeypatch.delenv("NCNN_B200_TEST_PAIR_REGS")
+    assert np.array_equal(m.run(x)[0], good)
+    m.close()
