@@ -331,9 +331,7 @@ void EngineImpl::fuse_depthwise_projection() {
     // Measured on MobileNetV2 at batch 256, the block's three layers (stride 2) or expand layer and fused pair (stride 1)
     // against the whole block: 112x112x96 at stride 2 0.80 -> 0.30 ms, 56x56x144 0.38 -> 0.24 (stride 1) and 0.40 -> 0.16,
     // 28x28x192 0.134 -> 0.094 and 0.137 -> 0.053.  NCNN_B200_FUSE_EXPAND=1 keeps the stride-1 blocks apart.
-    // (Without an activation a NaN of the expand layer stays one in the layers apart; the whole block clamps to infinities.)
-    const int whole = env_int_or("NCNN_B200_FUSE_EXPAND", 3);
-    if (je >= 0 && dw.sh == 1 && (whole < 2 || (whole == 3 && nodes_[je].act == ACT_NONE))) je = -1;
+    if (je >= 0 && dw.sh == 1 && env_int_or("NCNN_B200_FUSE_EXPAND", 2) < 2) je = -1;
     if (je < 0 && dw.sh != 1) continue;
     if (dw.sh != 1 && dw.sh != 2) continue;
     if (uses[mid] != 1 || tin.rank != 3 || tin.fmt != FMT_F32 || tin.Cp != tin.c || tin.Wp != tin.w || tin.w_off != 0 ||

@@ -51,7 +51,7 @@ constexpr int kBlkTableRows = 11;
 // are carried from row to row by multiply-adds that write to another register than they read, and nothing is moved.
 template <int STRIDE, class F>
 __device__ __forceinline__ void blk_depthwise(uint32_t t_in, uint32_t table, int c_pad, int ch, int iy0, int h_in, uint32_t cols_in,
-                                              float ex_lo, float ex_hi, float lo, float hi, uint32_t a_at, uint32_t chunk0, F&& release) {
+                                              const DwpClamp& ex_act, const DwpClamp& act, uint32_t a_at, uint32_t chunk0, F&& release) {
   using namespace ptx;
   constexpr int PW = dwp_patch_w(STRIDE), ROWS = blk_half_rows(STRIDE), IN = blk_in_rows(STRIDE);
   constexpr uint32_t kPlane = blk_a_plane_bytes(STRIDE);
@@ -86,10 +86,10 @@ __device__ __forceinline__ void blk_depthwise(uint32_t t_in, uint32_t table, int
       uint64_t u;
       f32x2_add(u, f32x2_make(v[j], v[j + 1]), ex_bias2);
       const float2 f = f32x2_get(u);
-      v[j] = __float_as_uint(fminf(fmaxf(f.x, ex_lo), ex_hi));
-      v[j + 1] = __float_as_uint(fminf(fmaxf(f.y, ex_lo), ex_hi));
+      v[j] = __float_as_uint(ex_act(f.x));
+      v[j + 1] = __float_as_uint(ex_act(f.y));
     }
-    if (PW % 2 == 1) v[PW - 1] = __float_as_uint(fminf(fmaxf(__fadd_rn(__uint_as_float(v[PW - 1]), ex_bias), ex_lo), ex_hi));
+    if (PW % 2 == 1) v[PW - 1] = __float_as_uint(ex_act(__fadd_rn(__uint_as_float(v[PW - 1]), ex_bias)));
     if (cols_in != (1u << PW) - 1u) {
 #pragma unroll
       for (int j = 0; j < PW; ++j)
@@ -101,7 +101,7 @@ __device__ __forceinline__ void blk_depthwise(uint32_t t_in, uint32_t table, int
     uint32_t w_hi[4], w_mid[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c)
-      split_bf16x2(fminf(fmaxf(y[2 * c], lo), hi), fminf(fmaxf(y[2 * c + 1], lo), hi), w_hi[c], w_mid[c]);
+      split_bf16x2(act(y[2 * c]), act(y[2 * c + 1]), w_hi[c], w_mid[c]);
     // eight pixels of a row are one 16-byte chunk of the channel's 128 bytes, at chunk ^ (channel & 7)
     const uint32_t to = a_at + (chunk0 ^ to_chunk);
     to_chunk += 16u;
@@ -414,11 +414,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
   } else if (warp >= 8) {
     // ------------------------------------------------------------ depthwise
     const int q = warp & 3, h = (warp - 8) >> 2;
-    // none / ReLU / clip as one clamp: fminf(fmaxf(y, lo), hi) returns y itself between the bounds
-    const float act_lo = p.dw_act == ACT_RELU ? 0.0f : (p.dw_act == ACT_CLIP ? p.dw_act_a : -INFINITY);
-    const float act_hi = p.dw_act == ACT_CLIP ? p.dw_act_b : INFINITY;
-    const float ex_lo = p.ex_act == ACT_RELU ? 0.0f : (p.ex_act == ACT_CLIP ? p.ex_act_a : -INFINITY);
-    const float ex_hi = p.ex_act == ACT_CLIP ? p.ex_act_b : INFINITY;
+    const DwpClamp act(p.dw_act, p.dw_act_a, p.dw_act_b), ex_act(p.ex_act, p.ex_act_a, p.ex_act_b);
     // this thread's channel in an operand tile: eight channels to an atom; the half's 64 pixels (stride 2: its half of them)
     const uint32_t a_at = a_base + static_cast<uint32_t>(STRIDE == 1 ? h * 4096 : 0) + static_cast<uint32_t>((lane >> 3) * 1024 + (lane & 7) * 128);
     const uint32_t chunk0 = static_cast<uint32_t>(((lane & 7) ^ (STRIDE == 1 ? 0 : h * 4)) << 4);
@@ -454,7 +450,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
           ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&a_empty[slot]), ((mine >> slot_shift) & 1u) ^ 1u, abort_ptr, kTcWaitLimitNs) ? 1 : 0) != 0;
           if (!ok) break;
           const uint32_t t_in = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + e_col0 + static_cast<uint32_t>((h * NB + eb) * COLS);
-          blk_depthwise<STRIDE>(t_in, table, c_pad, (cb + q - q0) * kDwpChannels + lane, iy0, p.Hin, cols_in, ex_lo, ex_hi, act_lo, act_hi,
+          blk_depthwise<STRIDE>(t_in, table, c_pad, (cb + q - q0) * kDwpChannels + lane, iy0, p.Hin, cols_in, ex_act, act,
                                 a_at + slot * 2u * kAPlane, chunk0, release);
           fence_proxy_async_smem();  // the tensor core reads what these stores wrote
           __syncwarp();

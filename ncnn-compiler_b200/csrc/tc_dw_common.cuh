@@ -53,6 +53,18 @@ struct TcDwProjParams {
   int* status;
 };
 
+// None / ReLU / clip as one clamp, fminf(fmaxf(y, lo), hi).  Without an activation both bounds are NaN: the other operand comes
+// through whatever it is, a NaN too (which bounds of infinities would turn into one of them).
+struct DwpClamp {
+  float lo, hi;
+  __device__ __forceinline__ DwpClamp(int act, float a, float b) {
+    const float any = __int_as_float(0x7fffffff);
+    lo = act == ACT_NONE ? any : (act == ACT_CLIP ? a : 0.0f);
+    hi = act == ACT_NONE ? any : (act == ACT_CLIP ? b : INFINITY);
+  }
+  __device__ __forceinline__ float operator()(float y) const { return fminf(fmaxf(y, lo), hi); }
+};
+
 // The CTA's tiles: blockIdx.x + k * gridDim.x, column tiles of one pixel tile next to each other, so CTAs working side by
 // side share the patch in L2.  A walk takes every step-th of them by adding with carry: divisions in each role and tile
 // were a third of a one-block tile's instructions.

@@ -262,9 +262,7 @@ __device__ __forceinline__ void dwp_pair_body(const TcDwProjParams& p, const CUt
     const int col0 = ((t >> 4) % (TW / COLS)) * COLS;       // first of the thread's columns of the tile
     const int row0 = (((t & 127) >> 4) / (TW / COLS)) * R;  // first of the thread's rows
     bool ok = true;
-    // none / ReLU / clip as one clamp: fminf(fmaxf(y, lo), hi) returns y itself between the bounds
-    const float act_lo = p.dw_act == ACT_RELU ? 0.0f : (p.dw_act == ACT_CLIP ? p.dw_act_a : -INFINITY);
-    const float act_hi = p.dw_act == ACT_CLIP ? p.dw_act_b : INFINITY;
+    const DwpClamp act(p.dw_act, p.dw_act_a, p.dw_act_b);
     const uint32_t x_first = static_cast<uint32_t>(row0 * PW + col0) * kPitch + static_cast<uint32_t>(pair) * 8u;
     // Operand row = pixel (row, column) of the tile; 64-byte rows with the 64-byte swizzle: the 16-byte chunk j of row m
     // lives at m*64 + ((j ^ ((m >> 1) & 3)) * 16).  Rows of one parity share the lower or the upper half of the banks, so
@@ -325,7 +323,7 @@ __device__ __forceinline__ void dwp_pair_body(const TcDwProjParams& p, const CUt
 #pragma unroll
           for (int c = 0; c < COLS; ++c) {
             const float2 y = f32x2_get(acc[r][c]);
-            split_bf16x2(fminf(fmaxf(y.x, act_lo), act_hi), fminf(fmaxf(y.y, act_lo), act_hi), hi[c], mid[c]);
+            split_bf16x2(act(y.x), act(y.y), hi[c], mid[c]);
           }
 #pragma unroll
           for (int c = 0; c < COLS; ++c) {

@@ -646,3 +646,29 @@ def test_pair_compiled_for_other_registers_is_an_error(pkg, tmp_path, monkeypatc
     monkeypatch.delenv("NCNN_B200_TEST_PAIR_REGS")
     assert np.array_equal(m.run(x)[0], good)
     m.close()
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("expand_act,dw_act", [(None, (0.0, 6.0)), (None, None), ("relu", None), ((0.5, 2.0), "relu"), ((-0.25, 0.75), (0.5, 2.0))])
+def test_blocks_keep_what_is_no_number(pkg, tmp_path, monkeypatch, stride, expand_act, dw_act):
+    """NaN, infinities and sums past the largest number go through whole blocks, and through pairs, as through the layers apart."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), 24, 16, 16, 64, 24, stride, expand_act=expand_act, dw_act=dw_act)
+    x = np.random.default_rng(3).uniform(-2, 2, (4, 16, 24, 16)).astype(np.float32)
+    x[0, 3, 5, 7] = np.nan
+    x[0, 2, 20, 1] = -np.nan
+    x[1, 1, 0, 0] = np.inf
+    x[1, 9, 23, 15] = -np.inf
+    x[2, 4, 11, 3] = 3e38
+    x[2, 5, 11, 4] = -3e38
+    results = {}
+    for name, env in (("whole", {}), ("pair", {"NCNN_B200_FUSE_EXPAND": "0"}), ("apart", {"NCNN_B200_FUSE_DW": "0"})):
+        for k, v in env.items():
+            monkeypatch.setenv(k, v)
+        results[name], kernels = _run(pkg, param, bin_, x)
+        fused = [k for k in kernels if k.startswith("tc_dw_project_kernel")]
+        assert len(fused) == (0 if name == "apart" or (name == "pair" and stride == 2) else 1), kernels
+        assert name != "whole" or "expand" in fused[0], kernels
+        for k in env:
+            monkeypatch.delenv(k)
+    assert np.array_equal(results["whole"], results["apart"], equal_nan=True)
+    assert np.array_equal(results["pair"], results["apart"], equal_nan=True)
