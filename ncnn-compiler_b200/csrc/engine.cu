@@ -53,12 +53,13 @@ bool EngineImpl::build(const std::string& param, const std::string& bin, const E
   // workspace of the kernels that split sums between blocks: partial sums, and flags and counters (zero between launches);
   // all launches of a model run on one stream
   void* ws = nullptr;
-  constexpr size_t ws_bytes = kTcSplitWorkspaceBytes + kTcFlagWords * sizeof(int);
+  split_ws_bytes_ = split_workspace_bytes();
+  const size_t ws_bytes = split_ws_bytes_ + kTcFlagWords * sizeof(int);
   if (device_alloc(&ws, ws_bytes) != cudaSuccess) return fail(err, "out of device memory");
   cudaMemset(ws, 0, ws_bytes);
   device_allocs_.push_back(ws);
   d_split_ws_ = static_cast<uint32_t*>(ws);
-  d_split_flags_ = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + kTcSplitWorkspaceBytes);
+  d_split_flags_ = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + split_ws_bytes_);
   return true;
 }
 

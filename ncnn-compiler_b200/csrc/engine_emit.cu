@@ -124,6 +124,31 @@ static bool depthwise_apart(const Node& node, int64_t n) {
   return !node.ex_fused && blocks > 6 && blocks < kTcChunkFrom && n * node.OH * node.OW <= 256 && tc_row_bytes(GEMM_BF16X3, node.dw_c) != 0;
 }
 
+// And where a whole block is three launches again: blocks with too many weights to stay are long chains of channel blocks.  The
+// expanded tensor and the depthwise result then pass through the workspace.  Calls of stride-2 blocks in us, as three layers of
+// the network / whole:
+//   28x28x384 -> 64    images 1: 22.5 / 28.7    4: 28.6 / 28.7    8: 34.8 / 30.5   64: 73.7 / 47.1
+//   28x28x768 -> 128          1: 28.7 / 43.0    8: 36.9 / 43.0   16: 47.1 / 47.1   64: 133 / 75.8
+//   28x28x1024 -> 64          1: 30.7 / 51.2    8: 43.0 / 49.2   16: 55.3 / 51.2   64: 160 / 83.9
+//   56x56x384 -> 128          1: 28.6 / 28.7    4: 34.8 / 32.7    8: 47.1 / 34.8   64: 264 / 139
+// The crossover moves out with the channels, to ~2 400 result pixels.
+static int64_t block_apart_images(const Node& node) {
+  if (!node.ex_fused || env_int_or("NCNN_B200_FUSE_DW", 1) >= 2 || !tc_block_streams(node.ex_cin, node.dw_c, node.O, node.dw_stride) ||
+      tc_row_bytes(GEMM_BF16X3, node.dw_c) == 0 || tc_row_bytes(GEMM_BF16X3, node.ex_cin) == 0)
+    return 0;
+  return std::min(4 * (node.dw_c - 192), 2400) / (node.OH * node.OW);
+}
+// What they need for it: the depthwise result as two planes, then the expanded tensor.
+static size_t block_apart_bytes(const Node& node, int64_t n) {
+  return static_cast<size_t>(n) * (node.OH * node.OW + node.dw_hin * node.dw_win) * node.dw_c * 4 + 1024;
+}
+size_t EngineImpl::split_workspace_bytes() const {
+  size_t bytes = kTcSplitWorkspaceBytes;
+  for (const Node& node : nodes_)
+    if (const int64_t n = block_apart_images(node)) bytes = std::max(bytes, (block_apart_bytes(node, n) + 255) / 256 * 256);
+  return bytes;
+}
+
 // True when an InnerProduct / Gemm of this batch size runs on the kernel for a handful of rows (ip_rows.cuh): one pass
 // over the weights on the CUDA cores instead of mostly empty 128-row tiles.
 bool EngineImpl::takes_rows(const Node& node, int64_t n) const {
@@ -297,23 +322,65 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
       const char* kind_name = kind == GEMM_I8 ? "i8" : (kind == GEMM_TF32 ? "tf32" : (kind == GEMM_BF16X3 ? "bf16x3" : "tf32x3"));
       auto launch = std::make_shared<TcLaunch>();
       std::string perr;
-      if (node.dw_fused && depthwise_apart(node, n)) {
-        // the depthwise result as bf16 pairs in the workspace of split contractions, which this projection therefore goes
-        // without: its tiles stay whole, also where every other convolution is split (NCNN_B200_STREAMK=1)
+      if (node.dw_fused && (depthwise_apart(node, n) || (n <= block_apart_images(node) && block_apart_bytes(node, n) <= split_ws_bytes_))) {
+        // the depthwise result as bf16 pairs in the workspace of split contractions (a whole block's expanded tensor behind it),
+        // which these layers therefore go without: their tiles stay whole, also where every other convolution is split
+        // (NCNN_B200_STREAMK=1)
         te.sk_ws = nullptr;
         te.sk_flags = nullptr;
+        auto view = [&](const ActRef& x, int channels, int h, int w) {
+          TcIm2colView v;
+          v.plane0 = x.p0;
+          v.plane1 = x.p1;
+          v.C = channels;
+          v.W = v.OW = w;
+          v.H = v.OH = h;
+          v.N = n;
+          v.stride_w = static_cast<uint64_t>(channels) * 2;
+          v.stride_h = v.stride_w * w;
+          v.stride_n = v.stride_h * h;
+          return v;
+        };
         const size_t plane = (static_cast<size_t>(n) * node.OH * node.OW * node.dw_c * 2 + 255) / 256 * 256;
         ActRef mid;
         mid.fmt = FMT_BF16X2;
         mid.p0 = reinterpret_cast<float*>(d_split_ws_);
         mid.p1 = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(d_split_ws_) + plane);
+        ActRef wide = in;  // the depthwise layer's input
+        if (node.ex_fused) {
+          wide = ActRef{};
+          wide.fmt = FMT_F32;
+          wide.p0 = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(d_split_ws_) + 2 * plane);
+          TcEpilogue xe;
+          xe.bias = node.ex_bias;
+          xe.act = node.ex_act;
+          xe.act_a = node.ex_act_a;
+          xe.act_b = node.ex_act_b;
+          xe.out0 = wide.p0;
+          xe.ldo = node.dw_c;
+          xe.out_mode = OUT_F32;
+          xe.status = d_status_;
+          auto expand = std::make_shared<TcLaunch>();
+          perr = tc_plan_conv(expand.get(), GEMM_BF16X3, view(in, node.ex_cin, node.dw_hin, node.dw_win), node.ex_w0, node.ex_w1, node.dw_c, xe, sm_count_);
+          if (!perr.empty()) return fail(err, "layer " + node.ex_name + ": " + perr);
+          Step x = s;
+          x.name = node.ex_name;
+          x.kernel = "tc_gemm_kernel<bf16x3>";
+          x.flops = 2.0 * node.ex_cin * node.dw_c * node.dw_hin * node.dw_win * n;
+          x.run = [expand](cudaStream_t st) { return tc_launch(*expand, st); };
+          s.flops -= x.flops;
+          steps.push_back(std::move(x));
+        }
         ConvGeom g{};
         g.images = n;
-        g.H = g.OH = node.OH;
-        g.W = g.OW = node.OW;
+        g.H = node.dw_hin;
+        g.W = node.dw_win;
+        g.OH = node.OH;
+        g.OW = node.OW;
         g.C = g.O = node.dw_c;
         g.KH = g.KW = 3;
-        g.sh = g.sw = g.dh = g.dw = 1;
+        g.sh = g.sw = node.dw_stride;
+        g.dh = g.dw = 1;
         g.pt = node.dw_pt;
         g.pl = node.dw_pl;
         ConvEpilogue de{};
@@ -323,26 +390,16 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         de.act_b = node.dw_act_b;
         const dim3 grid(((node.OH + 7) / 8) * ((node.OW + 7) / 8), (node.dw_c / 4 + 7) / 8, static_cast<unsigned>(n));
         const float* dw = node.dw_w;
+        const int stride = node.dw_stride;
         Step d = s;
         d.name = node.dw_name;
         d.kernel = "k_depthwise3x3_tile";
         d.run = [=](cudaStream_t st) {
-          launch_plain(k_depthwise3x3_tile<1>, grid, 256, 0, st, in, mid, dw, g, de);
+          if (stride == 1) launch_plain(k_depthwise3x3_tile<1>, grid, 256, 0, st, wide, mid, dw, g, de);
+          else launch_plain(k_depthwise3x3_tile<2>, grid, 256, 0, st, wide, mid, dw, g, de);
           return launch_ok();
         };
-        TcIm2colView v;
-        v.plane0 = mid.p0;
-        v.plane1 = mid.p1;
-        v.C = node.dw_c;
-        v.W = node.OW;
-        v.H = node.OH;
-        v.N = n;
-        v.stride_w = static_cast<uint64_t>(node.dw_c) * 2;
-        v.stride_h = v.stride_w * node.OW;
-        v.stride_n = v.stride_h * node.OH;
-        v.OH = node.OH;
-        v.OW = node.OW;
-        perr = tc_plan_conv(launch.get(), GEMM_BF16X3, v, node.d_w0, node.d_w1, node.O, te, sm_count_);
+        perr = tc_plan_conv(launch.get(), GEMM_BF16X3, view(mid, node.dw_c, node.OH, node.OW), node.d_w0, node.d_w1, node.O, te, sm_count_);
         if (!perr.empty()) return fail(err, "layer " + node.name + ": " + perr);
         d.flops = 18.0 * node.dw_c * node.OH * node.OW * n;
         s.flops -= d.flops;

@@ -276,6 +276,7 @@ class EngineImpl {
   void fold_channel_concats();
   void fuse_quantize_steps();
   void fuse_depthwise_projection();
+  size_t split_workspace_bytes() const;
   void fuse_stem_pooling();
   int profile(int64_t n, int repeat, std::vector<LayerTiming>* out);
   Plan* plan_for(int64_t n);
@@ -297,6 +298,7 @@ class EngineImpl {
   uint64_t use_counter_ = 0;
   int* d_status_ = nullptr;
   uint32_t* d_split_ws_ = nullptr;
+  size_t split_ws_bytes_ = 0;  // kTcSplitWorkspaceBytes, or more where a block that runs as three layers passes tensors through it
   int* d_split_flags_ = nullptr;
   int sm_count_ = 148;
   cudaStream_t stream_ = nullptr;

@@ -18,7 +18,10 @@
 // that nobody reads).
 //
 // Warps (512 threads): 0 TMA producer (input patches; all weights once), 1 MMA issuer, 4-7 epilogue, 8-15 depthwise.  Every
-// wait is bounded and ends in the status word.
+// wait is bounded and ends in the status word.  Where a stride-2 block has too many weights to stay in shared memory (`stages` > 0),
+// warp 2 brings a set's expand weights at a time, each block's where its quarter expects it, and warp 3 the projection's through a
+// ring of blocks: two more producers, because the expand MMAs run a set ahead of the projection's and with one of them for both,
+// or for the patches too, each could wait for what the other has yet to free.
 //
 // What bounds it: the depthwise warps' instructions (~1 500 for half an item, two warps to a scheduler, about every second
 // slot), and for stride 2, whose pixels fill tensor memory once, the wait for the next set's expand MMAs.  With the expanded
@@ -36,6 +39,7 @@ namespace nb {
 
 constexpr int kBlkThreads = 512;
 constexpr int kBlkMaxSlots = 8;
+constexpr int kBlkMaxStages = 8;
 
 // a half of a tile: result rows, input rows, and TMEM columns of its input pixels
 __host__ __device__ constexpr int blk_half_rows(int stride) { return dwp_tile_h(stride) / 2; }
@@ -182,7 +186,8 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
   grid_dependency_trigger();  // the next kernel of the stream may begin its preamble
 
   extern __shared__ uint8_t dwp_smem_raw[];
-  __shared__ __align__(8) uint64_t x_full[2], x_empty[2], w_full;
+  __shared__ __align__(8) uint64_t x_full[2], x_empty[2], w_full;  // (w_full, w_empty: all weights, or a set's expand weights)
+  __shared__ __align__(8) uint64_t w_empty, b_full[kBlkMaxStages], b_empty[kBlkMaxStages];
   __shared__ __align__(8) uint64_t e_full[4], e_empty[4];  // [half][buffer]
   __shared__ __align__(8) uint64_t a_full[kBlkMaxSlots], a_empty[kBlkMaxSlots];
   __shared__ __align__(8) uint64_t tfull_bar[2], tempty_bar[2];
@@ -199,13 +204,14 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
   const uint32_t slot_shift = slots == 8u ? 3u : 2u;
   // input patches (hi, mid planes), expand weights, operand tiles, projection weights, the epilogue's, tables.  (An expand
   // MMA may read up to 96 weight rows ahead of a plane or behind it: the patches lie before, the operand tiles behind.)
+  const bool streamed = STRIDE == 2 && p.stages > 0;
   const uint32_t x_base = smem_base;
-  const uint32_t e_plane = static_cast<uint32_t>(c_pad) * x_row;
+  const uint32_t e_plane = static_cast<uint32_t>(streamed ? 4 * kDwpChannels : c_pad) * x_row;
   const uint32_t e_base = x_base + static_cast<uint32_t>(XB) * 2u * x_plane;
   const uint32_t a_base = e_base + 2u * e_plane;
   const uint32_t b_bytes = static_cast<uint32_t>(p.b_bytes);
   const uint32_t b_base = a_base + slots * 2u * kAPlane;
-  const uint32_t drain = b_base + static_cast<uint32_t>(c_blocks) * 2u * b_bytes;
+  const uint32_t drain = b_base + static_cast<uint32_t>(streamed ? p.stages : c_blocks) * 2u * b_bytes;
   const uint32_t table = drain + static_cast<uint32_t>(TH * TW / 32) * kDrainWarpBytes;
   // TMEM columns: the projection's accumulators, then the halves' expanded pixels
   const uint32_t acc_stride = static_cast<uint32_t>(p.block_n);
@@ -214,6 +220,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
   // With one block of channels a tile is one item, and a single buffer lets no second one run beside it: its halves then go to
   // quarters two apart, so that their two warps have a scheduler each (28x28x32 -> 48 at stride 2, 3 281 images: 698 -> 651 us).
   const int apart = c_blocks == 1 ? 2 : 0;
+  const uint32_t e_tx = 2u * kDwpChannels * x_row, b_tx = 2u * static_cast<uint32_t>(p.block_n) * 64u;  // a block's weights
   volatile int* abort_ptr = &abort_flag;
 
   if (threadIdx.x == 0) {
@@ -225,6 +232,11 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
       mbar_init(smem_u32(&tempty_bar[i]), 4);
     }
     mbar_init(smem_u32(&w_full), 1);
+    mbar_init(smem_u32(&w_empty), 1);
+    for (int i = 0; i < kBlkMaxStages; ++i) {
+      mbar_init(smem_u32(&b_full[i]), 1);
+      mbar_init(smem_u32(&b_empty[i]), 1);
+    }
     for (int i = 0; i < 4; ++i) {
       mbar_init(smem_u32(&e_full[i]), 1);
       mbar_init(smem_u32(&e_empty[i]), 4);  // the half's four warps, those without an item in the set too
@@ -262,9 +274,8 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
     // ------------------------------------------------------------ producer (one elected thread: tc_gemm.cuh says why)
     if (elect_one() && static_cast<int>(blockIdx.x) < total_tiles) {
       const uint32_t wb = smem_u32(&w_full);
-      const uint32_t e_tx = 2u * kDwpChannels * x_row, b_tx = 2u * static_cast<uint32_t>(p.block_n) * 64u;
-      mbar_arrive_expect_tx(wb, static_cast<uint32_t>(c_blocks) * (e_tx + b_tx));
-      for (int cb = 0; cb < c_blocks; ++cb) {
+      if (!streamed) mbar_arrive_expect_tx(wb, static_cast<uint32_t>(c_blocks) * (e_tx + b_tx));
+      for (int cb = 0; cb < c_blocks && !streamed; ++cb) {
         const uint32_t e_at = e_base + static_cast<uint32_t>(cb * kDwpChannels) * x_row;
         tma_load_2d(e_at, &map_e0, wb, 0, cb * kDwpChannels);
         tma_load_2d(e_at + e_plane, &map_e1, wb, 0, cb * kDwpChannels);
@@ -301,7 +312,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
       if (*abort_ptr != 0) {
         // copies issued by this thread may still be landing: wait (bounded) for the last ones
         int zero = 0;
-        mbar_wait_bounded(wb, 0u, &zero, 200000000ull);
+        if (!streamed) mbar_wait_bounded(wb, 0u, &zero, 200000000ull);
         for (long long i = issued > XB ? issued - XB : 0; i < issued; ++i)
           mbar_wait_bounded(smem_u32(&x_full[i % XB]), static_cast<uint32_t>((i / XB) & 1), &zero, 200000000ull);
       }
@@ -315,19 +326,20 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
       // (a stride-2 tile has 64 rows: its second 64 are the first once more, into accumulator rows that nobody reads)
       const uint64_t a_first = smem_desc_mnmajor(a_base, STRIDE == 1 ? 4096u : 0u, 1024u);
       const int my_tiles = (total_tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1;
-      bool ok = mbar_wait_bounded(smem_u32(&w_full), 0u, abort_ptr, kTcWaitLimitNs);
+      bool ok = streamed || mbar_wait_bounded(smem_u32(&w_full), 0u, abort_ptr, kTcWaitLimitNs);
       // expand: the next set in order
       int e_tiles = 0, e_cb = 0, xb = 0, eb = 0;
-      uint32_t e_item = 0, x_ph = 0, e_ph = 0;
+      uint32_t e_item = 0, x_ph = 0, e_ph = 0, w_ph = 0;
       auto issue_expand = [&]() -> bool {
         if (e_tiles == my_tiles) return true;  // (the last sets have no successors)
         if (e_cb == 0 && !mbar_wait_bounded(smem_u32(&x_full[xb]), x_ph, abort_ptr, kTcWaitLimitNs)) return false;
         const int q0 = static_cast<int>(e_item & 3u);
         const int count = min(4 - q0, c_blocks - e_cb);
+        if (streamed && !mbar_wait_bounded(smem_u32(&w_full), w_ph, abort_ptr, kTcWaitLimitNs)) return false;
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           // the rows of block e_cb in its quarter: the operand starts so many blocks ahead of it
-          const uint32_t wa = e_base + static_cast<uint32_t>((e_cb - ((q0 + h * apart) & 3)) * kDwpChannels) * x_row;
+          const uint32_t wa = streamed ? e_base : e_base + static_cast<uint32_t>((e_cb - ((q0 + h * apart) & 3)) * kDwpChannels) * x_row;
           const uint64_t w0 = fixed_x + ((wa & 0x3ffffu) >> 4), w1 = w0 + (e_plane >> 4);
           if (!mbar_wait_bounded(smem_u32(&e_empty[h * 2 + eb]), e_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) return false;
           tc_fence_after_sync();
@@ -342,6 +354,10 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
             mma_f16(d, w0 + 2u * k, x0 + 2u * k, idesc_e, 1u);           // hi * hi
           }
           tc_commit(smem_u32(&e_full[h * 2 + eb]));
+        }
+        if (streamed) {
+          tc_commit(smem_u32(&w_empty));
+          w_ph ^= 1u;
         }
         if (++eb == NB) {
           eb = 0;
@@ -361,8 +377,8 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
         return true;
       };
       for (int i = 0; i < NB && ok; ++i) ok = issue_expand();
-      int acc = 0;
-      uint32_t acc_ph = 0, item = 0;
+      int acc = 0, bs = 0;
+      uint32_t acc_ph = 0, item = 0, b_ph = 0;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         if (!mbar_wait_bounded(smem_u32(&tempty_bar[acc]), acc_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) {
           ok = false;
@@ -379,13 +395,14 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
           if (expand_first) ok = issue_expand();
           for (int i = 0; i < count && ok; ++i, ++item, ++cb) {
             const uint32_t slot = item & (slots - 1u);
-            if (!mbar_wait_bounded(smem_u32(&a_full[slot]), (item >> slot_shift) & 1u, abort_ptr, kTcWaitLimitNs)) {
+            if (!mbar_wait_bounded(smem_u32(&a_full[slot]), (item >> slot_shift) & 1u, abort_ptr, kTcWaitLimitNs) ||
+                (streamed && !mbar_wait_bounded(smem_u32(&b_full[bs]), b_ph, abort_ptr, kTcWaitLimitNs))) {
               ok = false;
               break;
             }
             tc_fence_after_sync();
             const uint64_t a0 = a_first + static_cast<uint64_t>(slot * 2u * (kAPlane >> 4));
-            const uint64_t b0 = fixed_b + (((b_base + static_cast<uint32_t>(cb) * 2u * b_bytes) & 0x3ffffu) >> 4);
+            const uint64_t b0 = fixed_b + (((b_base + static_cast<uint32_t>(streamed ? bs : cb) * 2u * b_bytes) & 0x3ffffu) >> 4);
             const uint64_t b1 = b0 + (b_bytes >> 4);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {  // two K steps of 16 channels: 2 KB of A, 32 bytes of a row of B
@@ -396,6 +413,13 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
               accumulate = 1u;
             }
             tc_commit(smem_u32(&a_empty[slot]));
+            if (streamed) {
+              tc_commit(smem_u32(&b_empty[bs]));
+              if (++bs == p.stages) {
+                bs = 0;
+                b_ph ^= 1u;
+              }
+            }
           }
           if (!expand_first && ok) ok = issue_expand();
         }
@@ -408,10 +432,67 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
         if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_MMA);
       }
     }
-  } else if (warp >= 4 && warp < 8) {
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ producer of a set's expand weights
+    if (STRIDE == 2 && streamed && elect_one()) {
+      const uint32_t full = smem_u32(&w_full);
+      uint32_t item = 0, ph = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x)
+        for (int cb = 0; cb < c_blocks;) {
+          const int q0 = static_cast<int>(item & 3u);
+          const int count = min(4 - q0, c_blocks - cb);
+          ok = mbar_wait_bounded(smem_u32(&w_empty), ph ^ 1u, abort_ptr, kTcWaitLimitNs);
+          if (!ok) break;
+          mbar_arrive_expect_tx(full, static_cast<uint32_t>(count) * e_tx);
+          for (int i = 0; i < count; ++i) {
+            const uint32_t at = e_base + static_cast<uint32_t>((q0 + i) * kDwpChannels) * x_row;
+            tma_load_2d(at, &map_e0, full, 0, (cb + i) * kDwpChannels);
+            tma_load_2d(at + e_plane, &map_e1, full, 0, (cb + i) * kDwpChannels);
+          }
+          ph ^= 1u;
+          item += static_cast<uint32_t>(count);
+          cb += count;
+        }
+      if (!ok) {
+        if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
+      }
+      int zero = 0;
+      if (*abort_ptr != 0 && item > 0) mbar_wait_bounded(full, ph ^ 1u, &zero, 200000000ull);  // the last set's copies may still be landing
+    }
+  } else if (warp == 3) {
+    // ------------------------------------------------------------ producer of the projection's weights, a block to a stage
+    if (STRIDE == 2 && streamed && elect_one()) {
+      const int S = p.stages;
+      int s = 0;
+      uint32_t ph = 0;
+      long long issued = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x)
+        for (int cb = 0; cb < c_blocks; ++cb) {
+          ok = mbar_wait_bounded(smem_u32(&b_empty[s]), ph ^ 1u, abort_ptr, kTcWaitLimitNs);
+          if (!ok) break;
+          const uint32_t full = smem_u32(&b_full[s]), at = b_base + static_cast<uint32_t>(s) * 2u * b_bytes;
+          mbar_arrive_expect_tx(full, b_tx);
+          tma_load_2d(at, &map_b0, full, cb * kDwpChannels, 0);
+          tma_load_2d(at + b_bytes, &map_b1, full, cb * kDwpChannels, 0);
+          ++issued;
+          if (++s == S) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+      if (!ok) {
+        if (atomicCAS(const_cast<int*>(abort_ptr), 0, 1) == 0) atomicCAS(p.status, 0, TC_TIMEOUT_PRODUCER);
+      }
+      int zero = 0;
+      for (long long i = *abort_ptr != 0 && issued > S ? issued - S : 0; *abort_ptr != 0 && i < issued; ++i)
+        mbar_wait_bounded(smem_u32(&b_full[i % S]), static_cast<uint32_t>((i / S) & 1), &zero, 200000000ull);
+    }
+  } else if (warp < 8) {
     // ------------------------------------------------------------ epilogue
     dwp_epilogue<GEMM_BF16X3, STRIDE, EPI>(p, 1, 0, warp & 3, drain, tmem_base, acc_stride, total_tiles, tfull_bar, tempty_bar, abort_ptr);
-  } else if (warp >= 8) {
+  } else {
     // ------------------------------------------------------------ depthwise
     const int q = warp & 3, h = (warp - 8) >> 2;
     const DwpClamp act(p.dw_act, p.dw_act_a, p.dw_act_b), ex_act(p.ex_act, p.ex_act_a, p.ex_act_b);

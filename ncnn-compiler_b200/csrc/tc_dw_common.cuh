@@ -21,7 +21,7 @@ struct TcDwProjParams {
   int tiles_y, tiles_x, tiles_n, block_n;
   int c_blocks;         // blocks of 32 channels (the last one may be partly past C: zero-filled)
   int pad_t, pad_l;
-  int stages;           // weight ring depth
+  int stages;           // weight ring depth; whole blocks: 0 where all weights stay
   int drain_groups;     // groups of four epilogue warps in the pair: 2, or 1
   int patch_bufs;       // input patch ring depth, 2 or 4 (even: a slot then always serves the same depthwise group)
   int b_bytes;          // one plane of a weight stage, rounded to 1 KB

@@ -1395,7 +1395,8 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
   return !two.ok || (two.patches == one.patches && std::min(two.stages, 3) == std::min(one.stages, 3)) ? two : one;
 }
 
-// Shared and tensor memory plan of the whole block: all weights stay, so a block with too many of them for that is not taken.
+// Shared and tensor memory plan of the whole block.  Where its weights do not stay, stride-2 blocks stream them (64 images of
+// 28x28x384 -> 64: 47 us a call, 74 as three layers; 56x56x384 -> 128 139, 264).
 // Eight operand tiles before two input patches: four (one for each quarter of a set) leave the depthwise warps waiting for
 // the projection's MMAs, while a patch is needed by the expand MMAs only, which run ahead.
 DwProjShape block_shape(int N, int out_mode, int res_mode, int C, int stride, int cin) {
@@ -1413,19 +1414,28 @@ DwProjShape block_shape(int N, int out_mode, int res_mode, int C, int stride, in
   r.x_row_bytes = cin <= 16 ? 32 : 64;
   r.x_plane_bytes = (dwp_patch_pixels(stride) * r.x_row_bytes + 1023) / 1024 * 1024;
   const int c_blocks = (C + kDwpChannels - 1) / kDwpChannels, c_pad = c_blocks * kDwpChannels;
-  const int weights = 2 * c_pad * r.x_row_bytes + c_blocks * 2 * r.b_bytes;
   const int table = (kBlkTableRows * c_pad * 4 + 1023) / 1024 * 1024;
-  const int fixed = weights + table + dwp_tile_h(stride) * kDwpTileW / 32 * kDrainWarpBytes;
-  for (int slots : {8, 4})
-    for (int x_bufs : {2, 1}) {
-      const int smem = fixed + x_bufs * 2 * r.x_plane_bytes + slots * 2 * blk_a_plane_bytes(stride);
-      if (smem > kTcSmemBudget) continue;
-      r.x_bufs = x_bufs;
-      r.a_slots = slots;
-      r.smem = smem + 1024;
-      r.ok = true;
-      return r;
-    }
+  const int fixed = table + dwp_tile_h(stride) * kDwpTileW / 32 * kDrainWarpBytes;
+  const int stage = 2 * r.b_bytes;
+  for (bool streamed : {false, true}) {
+    if (streamed && stride == 1) break;
+    const int weights = streamed ? 2 * 4 * kDwpChannels * r.x_row_bytes : 2 * c_pad * r.x_row_bytes + c_blocks * stage;
+    for (int slots : {8, 4})
+      for (int x_bufs : {2, 1}) {
+        int smem = fixed + weights + x_bufs * 2 * r.x_plane_bytes + slots * 2 * blk_a_plane_bytes(stride);
+        if (streamed) {
+          r.stages = std::min(kBlkMaxStages, (kTcSmemBudget - smem) / stage);
+          if (r.stages < (slots == 8 || x_bufs == 2 ? 4 : 2)) continue;
+          smem += r.stages * stage;
+        }
+        if (smem > kTcSmemBudget) continue;
+        r.x_bufs = x_bufs;
+        r.a_slots = slots;
+        r.smem = smem + 1024;
+        r.ok = true;
+        return r;
+      }
+  }
   return r;
 }
 
@@ -1467,6 +1477,7 @@ bool tc_dw_project_applies(int C, int N, int H, int W, int out_mode, bool has_re
 bool tc_block_applies(int Cin, int C, int N, int OH, int OW, int stride, bool has_res) {
   if (Cin < 8 || Cin > 32 || Cin % 8 != 0 || C % 8 != 0 || C < 32 || N % 8 != 0 || OH < 1 || OW < 1) return false;
   if (has_res && stride != 1) return false;
+  if (C > (kTcChunkFrom - 1) * kDwpChannels) return false;  // (a projection that deep may be summed in chunks, the block sums it whole)
   if (!dw_project_fills(OH, OW, stride)) return false;
   // whatever formats the planner gives the output and the residual later
   for (int out_mode : {OUT_F32, OUT_BF16X2})
@@ -1477,6 +1488,8 @@ bool tc_block_applies(int Cin, int C, int N, int OH, int OW, int stride, bool ha
     }
   return true;
 }
+
+bool tc_block_streams(int Cin, int C, int N, int stride) { return block_shape(N, OUT_F32, RES_NONE, C, stride, Cin).stages > 0; }
 
 std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const TcEpilogue& e, int sm_count) {
   load_driver_entry_points();

@@ -252,6 +252,8 @@ bool tc_dw_project_applies(int C, int N, int H, int W, int out_mode, bool has_re
 // stride 1 or 2 with output OH x OW, 1x1 projection C -> N) fits the fused kernel, whatever formats its output and
 // residual get.
 bool tc_block_applies(int Cin, int C, int N, int OH, int OW, int stride, bool has_res);
+// True when such a block has more weights than shared memory keeps and brings them in for every tile.
+bool tc_block_streams(int Cin, int C, int N, int stride);
 std::string tc_plan_dw_project(TcDwProjLaunch* launch, const TcDwProjConv& conv, const TcEpilogue& epilogue, int sm_count);
 cudaError_t tc_launch_dw_project(const TcDwProjLaunch& launch, cudaStream_t stream);
 

@@ -672,3 +672,37 @@ def test_blocks_keep_what_is_no_number(pkg, tmp_path, monkeypatch, stride, expan
             monkeypatch.delenv(k)
     assert np.array_equal(results["whole"], results["apart"], equal_nan=True)
     assert np.array_equal(results["pair"], results["apart"], equal_nan=True)
+
+
+@pytest.mark.parametrize("h,w,cin,hidden,cout,n,fuse", [
+    (28, 28, 32, 384, 64, 150, "1"),   # twelve blocks, four tiles to a CTA
+    (27, 21, 16, 424, 128, 60, "1"),   # the last set and the last block are not full; 32-byte rows, one accumulator
+    (29, 30, 24, 832, 88, 45, "1"),    # 26 blocks: sets of 4 and 2
+    (15, 16, 32, 1000, 128, 40, "2"),  # one patch, four operand tiles
+    (33, 17, 32, 352, 112, 1, "2"),    # fewer tiles than CTAs
+])
+def test_whole_blocks_whose_weights_are_streamed(pkg, tmp_path, monkeypatch, h, w, cin, hidden, cout, n, fuse):
+    """Stride-2 blocks with more weights than shared memory holds: a set's expand weights and a ring of the projection's."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), h, w, cin, hidden, cout, 2)
+    x = np.random.default_rng(hidden).uniform(-2, 2, (n, cin, h, w)).astype(np.float32)
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", fuse)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert _layers(kernels) == ["tc_dw_project_kernel:expand+stride2<bf16x3>"], kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, plain = _run(pkg, param, bin_, x)
+    assert len(_layers(plain)) == 3 and np.array_equal(got, base)
+
+
+@pytest.mark.parametrize("h,w,cin,hidden,cout,n", [(28, 28, 32, 384, 64, 1), (27, 31, 16, 424, 120, 3), (14, 16, 24, 1000, 64, 12)])
+def test_streamed_blocks_of_few_pixels_are_three_launches(pkg, oracle, tmp_path, monkeypatch, h, w, cin, hidden, cout, n):
+    """The batch decides between one kernel and three launches through the workspace, so both give the same bits."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), h, w, cin, hidden, cout, 2)
+    x = np.random.default_rng(hidden).uniform(-2, 2, (64, cin, h, w)).astype(np.float32)
+    m = pkg.Model(param, bin_)
+    assert [k.split(":")[0] for k in _layers(_kernels(m, n))] == ["tc_gemm_kernel<bf16x3>", "k_depthwise3x3_tile", "tc_gemm_kernel<bf16x3>"]
+    assert _layers(_kernels(m, 64)) == ["tc_dw_project_kernel:expand+stride2<bf16x3>"]
+    few = m.run(x[:n])[0].copy()
+    many = m.run(x)[0]
+    assert np.array_equal(few, many[:n])
+    assert rel_l2(few[0], oracle.Model(param, bin_).run([x[0]])[0]) <= 1e-4
+    m.close()
