@@ -706,3 +706,79 @@ def test_streamed_blocks_of_few_pixels_are_three_launches(pkg, oracle, tmp_path,
     assert np.array_equal(few, many[:n])
     assert rel_l2(few[0], oracle.Model(param, bin_).run([x[0]])[0]) <= 1e-4
     m.close()
+
+
+@pytest.mark.parametrize("h,w,cin,hidden,cout,stride,n", [
+    (56, 56, 24, 144, 24, 1, 12),  # two buffers of expanded pixels, five channel blocks that rotate through the quarters
+    (40, 40, 16, 96, 48, 1, 30),   # one buffer at stride 1
+    (28, 28, 32, 192, 64, 1, 40),  # one buffer and four operand tiles
+    (30, 24, 8, 40, 32, 1, 60),    # a block of eight channels behind a full one, 32-byte rows
+    (57, 57, 32, 160, 24, 2, 25),  # five blocks at stride 2
+    (57, 57, 24, 224, 40, 2, 25),  # seven
+    (33, 47, 16, 72, 96, 2, 40),   # three, the widest projection with two accumulators
+])
+def test_whole_blocks_equal_the_layers_apart(pkg, oracle, tmp_path, monkeypatch, h, w, cin, hidden, cout, stride, n):
+    """More than two tiles to a CTA, so that every ring, buffer and quarter comes round again: the bits of the layers apart."""
+    param, bin_ = _block(pkg, str(tmp_path / "b"), h, w, cin, hidden, cout, stride)
+    x = np.random.default_rng(h + hidden).uniform(-2, 2, (n, cin, h, w)).astype(np.float32)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert _layers(kernels) == ["tc_dw_project_kernel:expand" + ("+stride2" if stride == 2 else "") + "<bf16x3>"], kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, plain = _run(pkg, param, bin_, x)
+    assert not any(k.startswith("tc_dw_project_kernel") for k in plain) and np.array_equal(got, base)
+    assert rel_l2(got[-1], oracle.Model(param, bin_).run([x[-1]])[0]) <= 1e-4
+
+
+@pytest.mark.parametrize("stride,pads,expand_act,dw_act", [
+    (1, (1, 1, 1, 1), None, "relu"),
+    (1, (0, 2, 0, 2), (0.5, 2.0), None),         # outside the image the filter sees zeros, not the clip's lower bound
+    (1, (2, 0, 2, 0), "relu", (-0.25, 0.75)),
+    (1, (2, 0, 0, 2), (-0.25, 0.75), (0.5, 2.0)),
+    (2, (1, 1, 1, 1), None, None),
+    (2, (0, 0, 0, 0), "relu", (0.5, 2.0)),
+    (2, (2, 2, 2, 2), (0.5, 2.0), "relu"),
+    (2, (1, 0, 0, 1), (-0.25, 0.75), None),
+    (2, (0, 1, 1, 0), (0.5, 2.0), (-0.25, 0.75)),
+])
+def test_whole_blocks_with_any_clamp_and_pads(pkg, oracle, tmp_path, monkeypatch, stride, pads, expand_act, dw_act):
+    param, bin_ = _block(pkg, str(tmp_path / "b"), 24, 25, 16, 72, 16, stride, pads=pads, expand_act=expand_act, dw_act=dw_act)
+    x = np.random.default_rng(sum(pads)).uniform(-2, 2, (3, 16, 24, 25)).astype(np.float32)
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "2")  # also where the image fills its tiles badly
+    got, kernels = _run(pkg, param, bin_, x)
+    assert len(_layers(kernels)) == 1 and "expand" in _layers(kernels)[0], kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, _ = _run(pkg, param, bin_, x)
+    assert np.array_equal(got, base)
+    assert rel_l2(got, np.stack([oracle.Model(param, bin_).run([xi])[0] for xi in x])) <= 1e-4
+
+
+@pytest.mark.parametrize("expand_act", [None, "relu", (0.0, 6.0)])
+def test_which_blocks_run_whole(pkg, tmp_path, monkeypatch, expand_act):
+    """By default all whose input has at most 32 channels; NCNN_B200_FUSE_EXPAND=1 keeps stride 1 apart, 0 both."""
+    found = {}
+    for stride in (1, 2):
+        param, bin_ = _block(pkg, str(tmp_path / f"b{stride}"), 32, 32, 24, 96, 24, stride, expand_act=expand_act)
+        wide, wide_bin = _block(pkg, str(tmp_path / f"w{stride}"), 32, 32, 40, 96, 24, stride, expand_act=expand_act)
+        for level in (None, "2", "1", "0"):
+            if level is not None:
+                monkeypatch.setenv("NCNN_B200_FUSE_EXPAND", level)
+            m = pkg.Model(param, bin_)
+            found[stride, level] = len(_layers(_kernels(m, 4)))
+            m.close()
+        monkeypatch.delenv("NCNN_B200_FUSE_EXPAND")
+        m = pkg.Model(wide, wide_bin)
+        found[stride, "wide"] = len(_layers(_kernels(m, 4)))
+        m.close()
+    # (a pair takes the residual with it; at stride 2 there is none)
+    assert [found[1, k] for k in (None, "2", "1", "0", "wide")] == [1, 1, 2, 2, 2], found
+    assert [found[2, k] for k in (None, "2", "1", "0", "wide")] == [1, 1, 1, 3, 3], found
+
+
+def test_mobilenet_v2_has_the_bits_of_its_layers_apart(pkg, tmp_path, monkeypatch):
+    param, bin_ = pkg.zoo.mobilenet_v2(str(tmp_path / "mbv2"))
+    x = np.random.default_rng(9).uniform(-1, 1, (5, 3, 224, 224)).astype(np.float32)
+    got, kernels = _run(pkg, param, bin_, x)
+    assert sum("expand" in k for k in kernels) == 6, kernels
+    monkeypatch.setenv("NCNN_B200_FUSE_DW", "0")
+    base, plain = _run(pkg, param, bin_, x)
+    assert not any(k.startswith("tc_dw_project_kernel") for k in plain) and np.array_equal(got, base)
