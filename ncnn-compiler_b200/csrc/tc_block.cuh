@@ -174,7 +174,8 @@ __device__ __forceinline__ void blk_depthwise(uint32_t t_in, uint32_t table, int
   }
 }
 
-template <int STRIDE, int EPI>
+// (STREAMED: weights that do not stay; in the same code the branches cost the issuing thread 2 to 3 % of every stride-2 block)
+template <int STRIDE, int EPI, bool STREAMED>
 __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUtensorMap& map_x, const CUtensorMap& map_x1,
                                               const CUtensorMap& map_e0, const CUtensorMap& map_e1, const CUtensorMap& map_b0,
                                               const CUtensorMap& map_b1) {
@@ -204,14 +205,13 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
   const uint32_t slot_shift = slots == 8u ? 3u : 2u;
   // input patches (hi, mid planes), expand weights, operand tiles, projection weights, the epilogue's, tables.  (An expand
   // MMA may read up to 96 weight rows ahead of a plane or behind it: the patches lie before, the operand tiles behind.)
-  const bool streamed = STRIDE == 2 && p.stages > 0;
   const uint32_t x_base = smem_base;
-  const uint32_t e_plane = static_cast<uint32_t>(streamed ? 4 * kDwpChannels : c_pad) * x_row;
+  const uint32_t e_plane = static_cast<uint32_t>(STREAMED ? 4 * kDwpChannels : c_pad) * x_row;
   const uint32_t e_base = x_base + static_cast<uint32_t>(XB) * 2u * x_plane;
   const uint32_t a_base = e_base + 2u * e_plane;
   const uint32_t b_bytes = static_cast<uint32_t>(p.b_bytes);
   const uint32_t b_base = a_base + slots * 2u * kAPlane;
-  const uint32_t drain = b_base + static_cast<uint32_t>(streamed ? p.stages : c_blocks) * 2u * b_bytes;
+  const uint32_t drain = b_base + static_cast<uint32_t>(STREAMED ? p.stages : c_blocks) * 2u * b_bytes;
   const uint32_t table = drain + static_cast<uint32_t>(TH * TW / 32) * kDrainWarpBytes;
   // TMEM columns: the projection's accumulators, then the halves' expanded pixels
   const uint32_t acc_stride = static_cast<uint32_t>(p.block_n);
@@ -232,10 +232,12 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
       mbar_init(smem_u32(&tempty_bar[i]), 4);
     }
     mbar_init(smem_u32(&w_full), 1);
-    mbar_init(smem_u32(&w_empty), 1);
-    for (int i = 0; i < kBlkMaxStages; ++i) {
-      mbar_init(smem_u32(&b_full[i]), 1);
-      mbar_init(smem_u32(&b_empty[i]), 1);
+    if constexpr (STREAMED) {
+      mbar_init(smem_u32(&w_empty), 1);
+      for (int i = 0; i < kBlkMaxStages; ++i) {
+        mbar_init(smem_u32(&b_full[i]), 1);
+        mbar_init(smem_u32(&b_empty[i]), 1);
+      }
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(smem_u32(&e_full[i]), 1);
@@ -274,8 +276,8 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
     // ------------------------------------------------------------ producer (one elected thread: tc_gemm.cuh says why)
     if (elect_one() && static_cast<int>(blockIdx.x) < total_tiles) {
       const uint32_t wb = smem_u32(&w_full);
-      if (!streamed) mbar_arrive_expect_tx(wb, static_cast<uint32_t>(c_blocks) * (e_tx + b_tx));
-      for (int cb = 0; cb < c_blocks && !streamed; ++cb) {
+      if (!STREAMED) mbar_arrive_expect_tx(wb, static_cast<uint32_t>(c_blocks) * (e_tx + b_tx));
+      for (int cb = 0; cb < c_blocks && !STREAMED; ++cb) {
         const uint32_t e_at = e_base + static_cast<uint32_t>(cb * kDwpChannels) * x_row;
         tma_load_2d(e_at, &map_e0, wb, 0, cb * kDwpChannels);
         tma_load_2d(e_at + e_plane, &map_e1, wb, 0, cb * kDwpChannels);
@@ -312,7 +314,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
       if (*abort_ptr != 0) {
         // copies issued by this thread may still be landing: wait (bounded) for the last ones
         int zero = 0;
-        if (!streamed) mbar_wait_bounded(wb, 0u, &zero, 200000000ull);
+        if (!STREAMED) mbar_wait_bounded(wb, 0u, &zero, 200000000ull);
         for (long long i = issued > XB ? issued - XB : 0; i < issued; ++i)
           mbar_wait_bounded(smem_u32(&x_full[i % XB]), static_cast<uint32_t>((i / XB) & 1), &zero, 200000000ull);
       }
@@ -326,7 +328,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
       // (a stride-2 tile has 64 rows: its second 64 are the first once more, into accumulator rows that nobody reads)
       const uint64_t a_first = smem_desc_mnmajor(a_base, STRIDE == 1 ? 4096u : 0u, 1024u);
       const int my_tiles = (total_tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1;
-      bool ok = streamed || mbar_wait_bounded(smem_u32(&w_full), 0u, abort_ptr, kTcWaitLimitNs);
+      bool ok = STREAMED || mbar_wait_bounded(smem_u32(&w_full), 0u, abort_ptr, kTcWaitLimitNs);
       // expand: the next set in order
       int e_tiles = 0, e_cb = 0, xb = 0, eb = 0;
       uint32_t e_item = 0, x_ph = 0, e_ph = 0, w_ph = 0;
@@ -335,11 +337,11 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
         if (e_cb == 0 && !mbar_wait_bounded(smem_u32(&x_full[xb]), x_ph, abort_ptr, kTcWaitLimitNs)) return false;
         const int q0 = static_cast<int>(e_item & 3u);
         const int count = min(4 - q0, c_blocks - e_cb);
-        if (streamed && !mbar_wait_bounded(smem_u32(&w_full), w_ph, abort_ptr, kTcWaitLimitNs)) return false;
+        if (STREAMED && !mbar_wait_bounded(smem_u32(&w_full), w_ph, abort_ptr, kTcWaitLimitNs)) return false;
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
           // the rows of block e_cb in its quarter: the operand starts so many blocks ahead of it
-          const uint32_t wa = streamed ? e_base : e_base + static_cast<uint32_t>((e_cb - ((q0 + h * apart) & 3)) * kDwpChannels) * x_row;
+          const uint32_t wa = STREAMED ? e_base : e_base + static_cast<uint32_t>((e_cb - ((q0 + h * apart) & 3)) * kDwpChannels) * x_row;
           const uint64_t w0 = fixed_x + ((wa & 0x3ffffu) >> 4), w1 = w0 + (e_plane >> 4);
           if (!mbar_wait_bounded(smem_u32(&e_empty[h * 2 + eb]), e_ph ^ 1u, abort_ptr, kTcWaitLimitNs)) return false;
           tc_fence_after_sync();
@@ -355,7 +357,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
           }
           tc_commit(smem_u32(&e_full[h * 2 + eb]));
         }
-        if (streamed) {
+        if (STREAMED) {
           tc_commit(smem_u32(&w_empty));
           w_ph ^= 1u;
         }
@@ -396,13 +398,13 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
           for (int i = 0; i < count && ok; ++i, ++item, ++cb) {
             const uint32_t slot = item & (slots - 1u);
             if (!mbar_wait_bounded(smem_u32(&a_full[slot]), (item >> slot_shift) & 1u, abort_ptr, kTcWaitLimitNs) ||
-                (streamed && !mbar_wait_bounded(smem_u32(&b_full[bs]), b_ph, abort_ptr, kTcWaitLimitNs))) {
+                (STREAMED && !mbar_wait_bounded(smem_u32(&b_full[bs]), b_ph, abort_ptr, kTcWaitLimitNs))) {
               ok = false;
               break;
             }
             tc_fence_after_sync();
             const uint64_t a0 = a_first + static_cast<uint64_t>(slot * 2u * (kAPlane >> 4));
-            const uint64_t b0 = fixed_b + (((b_base + static_cast<uint32_t>(streamed ? bs : cb) * 2u * b_bytes) & 0x3ffffu) >> 4);
+            const uint64_t b0 = fixed_b + (((b_base + static_cast<uint32_t>(STREAMED ? bs : cb) * 2u * b_bytes) & 0x3ffffu) >> 4);
             const uint64_t b1 = b0 + (b_bytes >> 4);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {  // two K steps of 16 channels: 2 KB of A, 32 bytes of a row of B
@@ -413,7 +415,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
               accumulate = 1u;
             }
             tc_commit(smem_u32(&a_empty[slot]));
-            if (streamed) {
+            if (STREAMED) {
               tc_commit(smem_u32(&b_empty[bs]));
               if (++bs == p.stages) {
                 bs = 0;
@@ -434,7 +436,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------ producer of a set's expand weights
-    if (STRIDE == 2 && streamed && elect_one()) {
+    if (STREAMED && elect_one()) {
       const uint32_t full = smem_u32(&w_full);
       uint32_t item = 0, ph = 0;
       bool ok = true;
@@ -462,7 +464,7 @@ __device__ __forceinline__ void tc_block_body(const TcDwProjParams& p, const CUt
     }
   } else if (warp == 3) {
     // ------------------------------------------------------------ producer of the projection's weights, a block to a stage
-    if (STRIDE == 2 && streamed && elect_one()) {
+    if (STREAMED && elect_one()) {
       const int S = p.stages;
       int s = 0;
       uint32_t ph = 0;

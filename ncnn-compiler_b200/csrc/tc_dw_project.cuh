@@ -349,14 +349,14 @@ __device__ __forceinline__ void dwp_pair_body(const TcDwProjParams& p, const CUt
   if (warp == 1) tmem_dealloc(tmem_base, kTcTmemCols);
 }
 
-// (KIND: the projection's arithmetic; bf16 pairs are the only form built.  EXPAND: the whole block.)
-template <int KIND, int STRIDE, bool EXPAND, int EPI>
+// (KIND: the projection's arithmetic; bf16 pairs are the only form built.  EXPAND: the whole block; STREAMED: its weights do not stay.)
+template <int KIND, int STRIDE, bool EXPAND, int EPI, bool STREAMED = false>
 __global__ void __launch_bounds__(EXPAND ? kBlkThreads : kDwpThreads, 1)
 tc_dw_project_kernel(const __grid_constant__ TcDwProjParams p, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ CUtensorMap map_x1, const __grid_constant__ CUtensorMap map_e0,
                      const __grid_constant__ CUtensorMap map_e1,
                      const __grid_constant__ CUtensorMap map_b0, const __grid_constant__ CUtensorMap map_b1) {
-  if constexpr (EXPAND) tc_block_body<STRIDE, EPI>(p, map_x, map_x1, map_e0, map_e1, map_b0, map_b1);
+  if constexpr (EXPAND) tc_block_body<STRIDE, EPI, STREAMED>(p, map_x, map_x1, map_e0, map_e1, map_b0, map_b1);
   else dwp_pair_body<KIND, EPI>(p, map_x, map_b0, map_b1);
 }
 

@@ -1593,6 +1593,7 @@ cudaError_t tc_launch_dw_project(const TcDwProjLaunch& L, cudaStream_t stream) {
     constexpr int EPI = decltype(form)::value;
     if (!L.expand) return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 1, false, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
     if (L.stride == 1) return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 1, true, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
+    if (L.p.stages > 0) return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 2, true, EPI, true>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
     return launch_opted(tc_dw_project_kernel<GEMM_BF16X3, 2, true, EPI>, max_smem, lc, L.p, L.map_x, L.map_x1, L.map_e0, L.map_e1, L.map_b0, L.map_b1);
   });
   return e != cudaSuccess ? e : cudaGetLastError();
