@@ -1385,14 +1385,17 @@ DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C, int drain
   return r;
 }
 
-// The second group only where its 16 KB cost no patch and none of three weight stages.  Calls of 48x48x672 -> 112, 35 images:
-// four patches and one group 326 us, two and two 333; 16x16x1152 -> 96, 137 images 238, 244.  Where both leave the same rings the
-// second group wins on short chains: 84x84x96 -> 320, 9 images 141, 129.  What has no room for two groups even with two patches
-// and two stages is no pair: 1344 -> 256 takes 145 (14x14, 64 images), 489 (256) and 469 us (28x28, 64) as one, 135, 490 and 469
-// as two launches.
+// A second group hides the drain of a tile behind the next one, which counts on short chains of channel blocks; on long ones its
+// 16 KB may be two of four patches or one of three weight stages, which count more.  Calls in us, one group / two where the
+// rings differ: 48x48x32 -> 384, 30 images 137 / 117; 48x48x128 -> 208, 59 images 220 / 204; 24x24x192 -> 352, 106 images 181 / 173;
+// 24x24x256 -> 320, 160 images 269 / 273; 48x48x288 -> 320, 38 images 258 / 262; 14x14x384 -> 288, 356 images 279 / 285; 48x48x672 -> 112,
+// 35 images 326 / 333; 16x16x1152 -> 96, 137 images 238 / 244.  Where both leave the same rings two never lose.
+// What has no room for two groups even with two patches and two stages is no pair: 1344 -> 256 takes 145 (14x14, 64 images), 489
+// (256) and 469 us (28x28, 64) as one, 135, 490 and 469 as two launches.
 DwProjShape dw_project_shape(int N, int out_mode, int res_mode, int C) {
   const DwProjShape one = dw_project_shape(N, out_mode, res_mode, C, 1), two = dw_project_shape(N, out_mode, res_mode, C, 2);
-  return !two.ok || (two.patches == one.patches && std::min(two.stages, 3) == std::min(one.stages, 3)) ? two : one;
+  const bool same_rings = two.patches == one.patches && std::min(two.stages, 3) == std::min(one.stages, 3);
+  return !two.ok || C <= 8 * kDwpChannels || same_rings ? two : one;
 }
 
 // Shared and tensor memory plan of the whole block.  Where its weights do not stay, stride-2 blocks stream them (64 images of
