@@ -663,15 +663,16 @@ bool EngineImpl::emit_node(std::vector<Step>& steps, const Node& node, int64_t n
         // walk.  At stride 2, whose rows come from memory twice as fast, it is only a little faster than the tile kernel when
         // the last of its waves of 2 blocks an SM is full, and slower when that is not.  Whole calls of expand layer,
         // depthwise layer and projection, tile / columns in us (the launch alone, its input in L2, flatters columns):
-        //   stride 1: 14x14x384  9 000 threads 24.6 / 30.7, 16 800 30.7 / 30.7, 24 200 34.8 / 32.8; 32x32x384 16 900 41.0 / 45.1,
-        //             24 600 49.2 / 47.1; 56x56x384 24 200 73.7 / 73.8, 37 600 108 / 98, 250 000 604 / 471
-        //   stride 2: 28 -> 14x14x384 16 800 43.0 / 45.1, 24 200 51.2 / 49.2; 56 -> 28x28x384 24 200 79.9 / 102, 75 300 (a wave)
-        //             212 / 194, 90 000 253 / 267; 64 -> 32x32x384 16 900 67.5 / 94.2, 75 300 229 / 219, 119 800 352 / 358;
-        //             112 -> 56x56x96 49 700 358 / 385, 75 300 531 / 527
+        //   stride 1: 14x14x384 8 700 threads 24.6 / 30.7, 16 800 30.7 / 30.7, 24 200 36.8 / 32.8; 32x32x384 16 900 41.0 / 45.1,
+        //             24 600 49.2 / 47.1; 56x56x384 24 200 73.7 / 73.8, 37 600 109 / 98, 250 000 604 / 471
+        //   stride 2: 28 -> 14x14x384 16 800 43.0 / 45.1, 24 200 51.2 / 49.2; 34 -> 17x17x384 51 000 102 / 90; 40 -> 20x20x384
+        //             38 400 90.1 / 96.3, 49 900 117 / 115; 56 -> 28x28x384 24 200 79.9 / 102, 75 300 (a wave)
+        //             215 / 197, 90 000 252 / 266; 64 -> 32x32x384 16 900 65.6 / 94.2, 75 300 232 / 221, 119 800 352 / 358;
+        //             112 -> 56x56x96 49 700 361 / 389, 75 300 533 / 528
         const long long wave = 2ll * sm_count_ * 256, waves = (threads + wave - 1) / wave;
-        const bool enough = node.sh == 1       ? threads >= 16384 + 250 * std::max(0, node.OH - 8)
+        const bool enough = node.sh == 1       ? threads >= 16384 + 250 * std::max(0, node.OH - 14)
                             : node.OH <= 16 ? threads >= 16384 + 1024 * std::max(0, node.OH - 8)
-                                            : threads * 100 >= waves * wave * (node.OH <= 28 ? 72 : 88);
+                                            : threads * 100 >= waves * wave * (node.OH <= 20 ? 62 : node.OH <= 28 ? 72 : 88);
         const int clamp = node.act == ACT_RELU || node.act == ACT_CLIP ? 1 : 0;
         const bool columns = in.fmt == FMT_F32 && (out.fmt == FMT_F32 || out.fmt == FMT_BF16X2) && (clamp || node.act == ACT_NONE) && !e.has_res &&
                              enough && n * pairs <= 0x7fffffffll && (threads + 255) / 256 <= 0x7fffffffll;
