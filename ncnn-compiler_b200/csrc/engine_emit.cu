@@ -136,7 +136,7 @@ static int64_t block_apart_images(const Node& node) {
   if (!node.ex_fused || env_int_or("NCNN_B200_FUSE_DW", 1) >= 2 || !tc_block_streams(node.ex_cin, node.dw_c, node.O, node.dw_stride) ||
       tc_row_bytes(GEMM_BF16X3, node.dw_c) == 0 || tc_row_bytes(GEMM_BF16X3, node.ex_cin) == 0)
     return 0;
-  return std::min(4 * (node.dw_c - 192), 2400) / (node.OH * node.OW);
+  return std::max(0, std::min(4 * (node.dw_c - 192), 2400)) / (node.OH * node.OW);
 }
 // What they need for it: the depthwise result as two planes, then the expanded tensor.
 static size_t block_apart_bytes(const Node& node, int64_t n) {

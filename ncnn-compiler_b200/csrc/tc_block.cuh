@@ -17,8 +17,9 @@
 // pixels (the A descriptor starts so many rows ahead that every block lands in its quarter; the other lanes hold products
 // that nobody reads).
 //
-// Warps (512 threads): 0 TMA producer (input patches; all weights once), 1 MMA issuer, 4-7 epilogue, 8-15 depthwise.  Every
-// wait is bounded and ends in the status word.  Where a stride-2 block has too many weights to stay in shared memory (`stages` > 0),
+// Warps (512 threads): 0 TMA producer (input patches; all weights once), 1 MMA issuer, 4-7 epilogue, 8-15 depthwise.  Every wait is
+// bounded and ends in the status word.  Tensor memory holds the projection's accumulators, two, or one of more than 96 columns at
+// stride 2, and one or two buffers of each half's expanded pixels.  Where a stride-2 block has too many weights to stay in shared memory (`stages` > 0),
 // warp 2 brings a set's expand weights at a time, each block's where its quarter expects it, and warp 3 the projection's through a
 // ring of blocks: two more producers, because the expand MMAs run a set ahead of the projection's and with one of them for both,
 // or for the patches too, each could wait for what the other has yet to free.
@@ -27,7 +28,8 @@
 // slot), and for stride 2, whose pixels fill tensor memory once, the wait for the next set's expand MMAs.  With the expanded
 // pixels in a shared-memory patch instead (two channels and a square of results to a thread) the kernel was bound by that
 // memory, 80 % of its cycles with the MMAs' reads.  256 images, the patch form -> this one: 56x56x144 stride 1 289 -> 240 us,
-// stride 2 184 -> 162, 28x28x192 stride 1 105 -> 94, stride 2 66 -> 53, 112x112x96 stride 2 290 -> 299.
+// stride 2 184 -> 162, 28x28x192 stride 1 105 -> 94, stride 2 66 -> 53, 112x112x96 stride 2 290 -> 299: three blocks that rotate
+// through the quarters are 1.5 sets a tile where one would do, and with a single buffer of expanded pixels sets wait for one another.
 // Measured without gain: sixteen depthwise warps (279 us where eight take 260: what they share is the clamps' pipe), rows
 // loaded one step ahead (a load takes 65 clocks), packed multiply-adds of two columns (275: the odd pairs cost moves),
 // every step unrolled (474: the warps wait for instructions).

@@ -30,8 +30,7 @@ struct TcDwProjParams {
   const float* dw_bias;     // [C] or null
   int dw_act;
   float dw_act_a, dw_act_b;
-  // expand layer inside (tc_block.cuh): x is [image][Hin][Win][Cin] as bf16 hi / mid planes, weights packed [C][32] bf16 hi / mid
-  int Cin;
+  // expand layer inside (tc_block.cuh): x is [image][Hin][Win][input channels] as bf16 hi / mid planes, weights packed [C][32] bf16 hi / mid
   int x_row_bytes;          // operand rows of the input patch and of the expand weights: 64 bytes (32 channels), or 32
                             // (16 channels) when the block's input has no more: two patch buffers then fit where one did
   int x_plane_bytes;        // one bf16 plane of an input patch buffer, rounded to 1 KB
@@ -39,7 +38,7 @@ struct TcDwProjParams {
   int accs;                 // accumulators of the projection: 2, or 1 when a second does not fit beside the expanded pixels
   int e_bufs;               // TMEM buffers of each half's expanded pixels: 2, or 1
   int a_slots;              // operand tiles: 8, or 4
-  int ex_ksteps;            // K steps of 16 input channels the expand MMAs run: ceil(Cin / 16)
+  int ex_ksteps;            // K steps of 16 input channels the expand MMAs run
   const float* ex_bias;     // [C] or null
   int ex_act;
   float ex_act_a, ex_act_b;

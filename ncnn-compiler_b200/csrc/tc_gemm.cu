@@ -1537,7 +1537,6 @@ std::string tc_plan_dw_project(TcDwProjLaunch* L, const TcDwProjConv& c, const T
   p.dw_act = c.dw_act;
   p.dw_act_a = c.dw_act_a;
   p.dw_act_b = c.dw_act_b;
-  p.Cin = expand ? c.Cin : 0;
   p.x_plane_bytes = shape.x_plane_bytes;
   p.x_row_bytes = shape.x_row_bytes;
   p.x_bufs = shape.x_bufs;
